@@ -23,6 +23,12 @@ __device__ __forceinline__ void cp_async_elem(float2 *dst, const float2 *src) {
 // every cp.async this thread issued has landed
 __device__ __forceinline__ void async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
+// groups of copies: everything this thread issued since the last commit is
+// one group; wait until at most N groups are still in flight
+__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void async_wait_group() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
 // the staged tile is complete and visible to the whole CTA
 __device__ __forceinline__ void staged_sync() {
     async_wait_all();

@@ -111,6 +111,9 @@ extern "C" int gm_engine_create(int device, const gm_config *cfg, gm_engine **ou
     GM_CUDA(cudaEventCreate(&e->ev_s0));
     GM_CUDA(cudaEventCreate(&e->ev_s1));
     GM_CUDA(cudaEventCreate(&e->ev_sm));
+    GM_CUDA(cudaStreamCreateWithFlags(&e->st2, cudaStreamNonBlocking));
+    GM_CUDA(cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming));
+    GM_CUDA(cudaEventCreateWithFlags(&e->ev_join, cudaEventDisableTiming));
     if ((rc = gm::noalloc_prepare(device))) return rc;
 
     const gm::Symbolic &s = e->sym;
@@ -153,13 +156,37 @@ extern "C" int gm_engine_create(int device, const gm_config *cfg, gm_engine **ou
         L.ent_count = (int64_t)ent_dst.size() - L.ent_first;
     }
     ent_lvl_off[s.nnodes] = (int64_t)ent_dst.size();
+    // levels with more than 32 pivots: rows of the pivot workspace, and each
+    // front's part of the triangle-inversion scratch (one level at a time)
+    std::vector<int64_t> y_off(s.nnodes, -1), tri_off(s.nnodes, 0);
+    int64_t y_total = 0;
+    for (const gm::LevelInfo &L : e->levels) {
+        if (L.max_piv <= 32) continue;
+        int64_t tri = 0;
+        for (int t = L.first; t < L.first + L.count; ++t) {
+            const int v = s.lvl_nodes[t];
+            y_off[v] = y_total;
+            y_total += s.npiv[v];
+            tri_off[v] = tri;
+            tri += (int64_t)s.npiv[v] * s.npiv[v];
+        }
+        e->tri_total = std::max(e->tri_total, tri);
+    }
+    std::vector<gm::NodeDesc> desc(s.nnodes);
+    for (int t = 0; t < s.nnodes; ++t) {
+        const int v = s.lvl_nodes[t];
+        desc[t] = gm::NodeDesc{s.front_off[v], s.var_off[v], s.inv_off[v], s.rhs_off[v], y_off[v],
+                               v, s.nfront[v], s.npiv[v], s.child0[v], s.child1[v], 0};
+    }
     int rc2;
+    if ((rc2 = upload(e->d_desc, desc, e->st))) return rc2;
     if ((rc2 = upload(e->d_npiv, s.npiv, e->st)) || (rc2 = upload(e->d_nfront, s.nfront, e->st)) ||
         (rc2 = upload(e->d_child0, s.child0, e->st)) || (rc2 = upload(e->d_child1, s.child1, e->st)) ||
         (rc2 = upload(e->d_vars, s.vars, e->st)) || (rc2 = upload(e->d_inv, s.inv, e->st)) ||
         (rc2 = upload(e->d_lvl_nodes, s.lvl_nodes, e->st)) || (rc2 = upload(e->d_front_off, s.front_off, e->st)) ||
         (rc2 = upload(e->d_var_off, s.var_off, e->st)) || (rc2 = upload(e->d_inv_off, s.inv_off, e->st)) ||
         (rc2 = upload(e->d_rhs_off, s.rhs_off, e->st)) || (rc2 = upload(e->d_ent_dst, ent_dst, e->st)) ||
+        (rc2 = upload(e->d_y_off, y_off, e->st)) || (rc2 = upload(e->d_tri_off, tri_off, e->st)) ||
         (rc2 = upload(e->d_ent_src, ent_src, e->st)) || (rc2 = upload(e->d_ent_lvl_off, ent_lvl_off, e->st)))
         return rc2;
     GM_CUDA(cudaStreamSynchronize(e->st));
@@ -171,6 +198,8 @@ extern "C" int gm_engine_create(int device, const gm_config *cfg, gm_engine **ou
     d.front_off = e->d_front_off.as<int64_t>(); d.var_off = e->d_var_off.as<int64_t>();
     d.inv_off = e->d_inv_off.as<int64_t>(); d.rhs_off = e->d_rhs_off.as<int64_t>();
     d.front_total = s.front_total; d.rhs_total = s.rhs_total;
+    d.desc = e->d_desc.as<gm::NodeDesc>();
+    d.y_off = e->d_y_off.as<int64_t>(); d.y_total = y_total;
 
     gm_stats &st = e->stats;
     st.n = s.n;
@@ -383,6 +412,7 @@ static int factor_batch(gm_engine *e, double pivscale) {
     static const bool no_graph = std::getenv("GM_NO_GRAPH") != nullptr;
     const int nl = (int)e->levels.size();
     auto launch_levels = [&](cudaEvent_t *evs) {
+        bool forked = false;
         for (int h = 0; h < nl; ++h) {
             if (small_factor_level<R>(e->levels[h])) {
                 launch_factor_small<R>(a, e->levels[h], e->st);
@@ -397,7 +427,17 @@ static int factor_batch(gm_engine *e, double pivscale) {
                 else
                     launch_gemm_sub_cc<R>(probs + pl.prob_off, tiles + pl.tile_off, pl.ntiles, e->st);
             }
+            if (e->levels[h].max_piv > 32) {   // beside the levels above (the last level's: nothing is)
+                cudaEventRecord(e->ev_fork, e->st);
+                cudaStreamWaitEvent(e->st2, e->ev_fork, 0);
+                launch_tri_inverse<R>(a, e->levels[h], e->d_tri.p, e->tri_total, e->d_tri_off.as<int64_t>(), e->st2);
+                forked = true;
+            }
             if (evs) cudaEventRecord(evs[1 + h], e->st);
+        }
+        if (forked) {
+            cudaEventRecord(e->ev_join, e->st2);
+            cudaStreamWaitEvent(e->st, e->ev_join, 0);
         }
     };
     if (!trace && !no_graph && !e->fgraph_broken) {
@@ -407,7 +447,7 @@ static int factor_batch(gm_engine *e, double pivscale) {
         // attributes outside any capture), the second captures the graph.
         gm_engine::FactorGraphKey key;
         key.front = e->d_front.p; key.A = e->d_A.p; key.amax = e->d_amax.p; key.npert = e->d_npert.p;
-        key.pivsrc = e->d_pivsrc.p;
+        key.pivsrc = e->d_pivsrc.p; key.tri = e->d_tri.p;
         key.tcerr = e->d_tcerr.p; key.probs = probs; key.tiles = tiles; key.nf = e->nf; key.fp64 = sizeof(R) == 8;
         if (!(e->fgraph && key == e->fgraph_key) && key == e->fgraph_seen) {
             if (e->fgraph) cudaGraphExecDestroy(e->fgraph);
@@ -496,6 +536,7 @@ static int factor_assembled(gm_engine *e) {
     GM_ALLOC(e->d_front, fbytes);
     GM_ALLOC(e->d_npert, 2 * sizeof(unsigned long long));   // perturbed pivots, row exchanges
     GM_ALLOC(e->d_amax, sizeof(unsigned long long));
+    GM_ALLOC(e->d_tri, (size_t)e->nf * e->tri_total * e->csize());
     if (e->cfg.pivot_tol > 0) {
         GM_ALLOC(e->d_pivsrc, (size_t)e->nf * e->n);
         const int rc = init_pivsrc(e);
@@ -614,9 +655,10 @@ extern "C" int gm_get_triplets(gm_engine *e, int ifreq, double *Ar, double *Ai, 
 namespace gm {
 
 // One substitution over the right-hand sides in xT; fmap (device, nfz
-// entries) restricts it to those matrices of the batch (NULL: all).
+// entries) restricts it to those matrices of the batch (NULL: all); y is the
+// pivot workspace.
 template <class R>
-static void substitute(gm_engine *e, void *xT, int nrhs, int trans, const unsigned char *mask = nullptr,
+static void substitute(gm_engine *e, void *xT, void *y, int nrhs, int trans, const unsigned char *mask = nullptr,
                        const int *fmap = nullptr, int nfz = 0, const int *xmap = nullptr,
                        const SpikeRhs *spikes = nullptr) {
     cudaEventRecord(e->ev_s0, e->st);
@@ -626,6 +668,7 @@ static void substitute(gm_engine *e, void *xT, int nrhs, int trans, const unsign
     a.pivsrc = e->cfg.pivot_tol > 0 ? e->d_pivsrc.as<unsigned char>() : nullptr;
     a.x = xT;
     a.w = e->d_w.p;
+    a.y = y;
     a.nf = e->nf;
     a.fmap = fmap;
     a.nfz = nfz;
@@ -738,6 +781,14 @@ static const unsigned char *build_mask(gm_engine *e, int nrhs, const RhsPattern 
                                    e->st) == cudaSuccess;
     cudaStreamSynchronize(e->st);   // m and work are released on return
     return e->d_mask.as<unsigned char>();
+}
+
+// Pivot workspace of the substitutions over d_t (the refinement sweeps, the
+// complex64 path) and over GMRES's vectors.  The first FP64 substitution
+// works in x and takes d_t, which is free then.
+static int ensure_y(gm_engine *e, int nrhs) {
+    GM_ALLOC(e->d_y, (size_t)e->nf * e->dsym.y_total * nrhs * e->csize());
+    return GM_OK;
 }
 
 // serialises the GMRES workspace sizing of engines on different host threads
@@ -895,7 +946,7 @@ static int gmres_refine(gm_engine *e, int sys, int nrhs, double2 *d_x, const Res
             GM_CUDA(cudaMemcpy(d_scal, hs.data(), hs.size() * sizeof(double), cudaMemcpyHostToDevice));
             launch_scale_down<R>(V + jj * vstride, Z + jj * vstride, d_scal, d_zm, ni, n, nrhs, e->st);
             // Z_jj <- M~^-1 Z_jj (working-precision substitution in place)
-            substitute<R>(e, Z + jj * vstride, nrhs, sys, nullptr, d_fm, ni, d_zm);
+            substitute<R>(e, Z + jj * vstride, e->d_y.p, nrhs, sys, nullptr, d_fm, ni, d_zm);
             // V_jj+1 = M' Z_jj (FP64)
             ResidArgs pa = ra;
             pa.fmap = d_fm; pa.nfz = ni; pa.xmap = d_zm; pa.omap = d_zm;
@@ -1048,11 +1099,12 @@ int engine_solve_device(gm_engine *e, int sys, int nrhs, double2 *d_x, const dou
     if (implicit && !lazy_b) launch_spikes(d_x, e->n, e->nf, nrhs, spikes->k, spikes->amp, e->st);   // x = b
     if (fp64) {
         if (!implicit) GM_CUDA(cudaMemcpyAsync(d_x, d_b, cnt * sizeof(double2), cudaMemcpyDeviceToDevice, e->st));
-        substitute<double>(e, d_x, nrhs, sys, mask, nullptr, 0, nullptr, lazy_b ? spikes : nullptr);
+        substitute<double>(e, d_x, e->d_t.p, nrhs, sys, mask, nullptr, 0, nullptr, lazy_b ? spikes : nullptr);
     } else {
+        if (const int rc = ensure_y(e, nrhs)) return rc;
         launch_convert_down<float>(implicit ? d_x : d_b, e->d_t.p, cnt, e->st);
         GM_CUDA(cudaMemsetAsync(d_x, 0, cnt * sizeof(double2), e->st));
-        substitute<float>(e, e->d_t.p, nrhs, sys, mask);
+        substitute<float>(e, e->d_t.p, e->d_y.p, nrhs, sys, mask);
         launch_add_up<float>(d_x, e->d_t.p, cnt, e->st);
     }
     GM_CUDA(cudaGetLastError());
@@ -1132,6 +1184,7 @@ int engine_solve_device(gm_engine *e, int sys, int nrhs, double2 *d_x, const dou
             std::fprintf(stderr, "\n");
         }
         if (next.empty() || it >= e->cfg.ir_max_iter) break;
+        if (const int rc = ensure_y(e, nrhs)) return rc;
         // Matrices that go on with GMRES-IR: all of them in GMRES mode; in
         // auto mode those whose plain sweeps cannot reach the target within
         // the sweeps left at the contraction of the last one (or did not
@@ -1181,10 +1234,10 @@ int engine_solve_device(gm_engine *e, int sys, int nrhs, double2 *d_x, const dou
         if (!rhs) launch_residual_t<double>(ra, e->d_t.p, e->d_part.as<double>(), nblk_max, e->st);
         const size_t per_f = (size_t)e->n * nrhs;
         if (fp64) {
-            substitute<double>(e, e->d_t.p, nrhs, sys, nullptr, d_act, nn);
+            substitute<double>(e, e->d_t.p, e->d_y.p, nrhs, sys, nullptr, d_act, nn);
             launch_add_up_f<double>(d_x, e->d_t.p, per_f, d_act, nn, e->st);
         } else {
-            substitute<float>(e, e->d_t.p, nrhs, sys, nullptr, d_act, nn);
+            substitute<float>(e, e->d_t.p, e->d_y.p, nrhs, sys, nullptr, d_act, nn);
             launch_add_up_f<float>(d_x, e->d_t.p, per_f, d_act, nn, e->st);
         }
         for (int f : act) {
@@ -1217,6 +1270,7 @@ static void time_levels(gm_engine *e, void *xT, int nrhs, std::vector<float> &fw
     a.pivsrc = e->cfg.pivot_tol > 0 ? e->d_pivsrc.as<unsigned char>() : nullptr;
     a.x = xT;
     a.w = e->d_w.p;
+    a.y = e->d_y.p;
     a.nf = e->nf;
     a.nrhs = nrhs;
     a.ldr = nrhs;
@@ -1255,6 +1309,7 @@ extern "C" int gm_autotune(gm_engine *e, int nrhs, int reps) {
     const size_t cnt = (size_t)e->nf * e->n * nrhs;
     GM_ALLOC(e->d_t, cnt * e->csize());
     GM_ALLOC(e->d_w, (size_t)e->nf * e->sym.rhs_total * nrhs * e->csize());
+    if (const int rc = gm::ensure_y(e, nrhs)) return rc;
     GM_CUDA(cudaMemsetAsync(e->d_t.p, 0, cnt * e->csize(), e->st));   // the pass's cost does not depend on the values
     const int nl = (int)e->levels.size();
     // per level, each pass direction: the fastest of the candidate tiles

@@ -53,7 +53,8 @@ struct gm_engine {
 
     // device copy of the symbolic structure
     gm::DevBuf d_npiv, d_nfront, d_child0, d_child1, d_vars, d_inv, d_lvl_nodes;
-    gm::DevBuf d_front_off, d_var_off, d_inv_off, d_rhs_off;
+    gm::DevBuf d_front_off, d_var_off, d_inv_off, d_rhs_off, d_y_off, d_tri_off, d_desc;
+    int64_t tri_total = 0;   // entries of the triangle-inversion scratch per matrix
     gm::DevBuf d_ent_dst, d_ent_src, d_ent_lvl_off;
     std::vector<gm::LevelInfo> levels;
     gm::DevSym dsym{};
@@ -67,7 +68,7 @@ struct gm_engine {
     int nf = 0;
     std::vector<float> freqs;
     std::vector<int> models;    // material model of each matrix of the batch
-    gm::DevBuf d_A, d_mass, d_pml, d_fq, d_front, d_npert, d_amax;
+    gm::DevBuf d_A, d_mass, d_pml, d_fq, d_front, d_npert, d_amax, d_tri;
     // threshold pivoting record [nf][n] (FactorArgs::pivsrc): every slot up
     // to pivsrc_ready_nf of the buffer at pivsrc_ready holds the identity
     // outside the pivoted levels
@@ -88,20 +89,25 @@ struct gm_engine {
     // the buffers and the batch it was captured for stay the same
     struct FactorGraphKey {
         const void *front = nullptr, *A = nullptr, *amax = nullptr, *npert = nullptr, *tcerr = nullptr;
-        const void *probs = nullptr, *tiles = nullptr, *pivsrc = nullptr;
+        const void *probs = nullptr, *tiles = nullptr, *pivsrc = nullptr, *tri = nullptr;
         int nf = 0, fp64 = 0;
         bool operator==(const FactorGraphKey &o) const {
             return front == o.front && A == o.A && amax == o.amax && npert == o.npert && tcerr == o.tcerr &&
-                   probs == o.probs && tiles == o.tiles && pivsrc == o.pivsrc && nf == o.nf && fp64 == o.fp64;
+                   probs == o.probs && tiles == o.tiles && pivsrc == o.pivsrc && tri == o.tri && nf == o.nf &&
+                   fp64 == o.fp64;
         }
     };
     FactorGraphKey fgraph_key, fgraph_seen;
     cudaGraphExec_t fgraph = nullptr;
     long long fgraph_kernels = 0;
     bool fgraph_broken = false;   // capture failed once: launch directly
+    // the pivot-triangle inversions run beside the levels above theirs
+    cudaStream_t st2 = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
 
     // solve workspaces
     gm::DevBuf d_x, d_b, d_r, d_t, d_w, d_part, d_norm;
+    gm::DevBuf d_y;   // pivot workspace (SolveArgs::y) of the substitutions that work in d_t
     gm::DevBuf d_fmap;                          // matrices still refined (device list)
     // GMRES-IR: Krylov vectors [m+1][ng][n][nrhs] c128, preconditioned
     // vectors [m][ng][n][nrhs] (working precision), reductions, coefficients
@@ -148,7 +154,10 @@ struct gm_engine {
         if (ev_s0) cudaEventDestroy(ev_s0);
         if (ev_s1) cudaEventDestroy(ev_s1);
         if (ev_sm) cudaEventDestroy(ev_sm);
+        if (ev_fork) cudaEventDestroy(ev_fork);
+        if (ev_join) cudaEventDestroy(ev_join);
         if (fgraph) cudaGraphExecDestroy(fgraph);
+        if (st2) cudaStreamDestroy(st2);
         if (st) cudaStreamDestroy(st);
     }
 

@@ -203,11 +203,12 @@ int residuals(gm_engine *e, int ns, int ntr, const float *pobs, int stf_inv, int
 namespace {
 
 // Device bytes per shot of one block solve over the batch: the FP64
-// solutions, the working-precision copy, the front update vectors and the
-// residual partial sums.
+// solutions, the working-precision copy, the front update vectors, the
+// complex64 path's pivot workspace and the residual partial sums.
 size_t bytes_per_shot(const gm_engine *e) {
     const size_t n = (size_t)e->n, nf = (size_t)e->nf;
-    return nf * (n * sizeof(double2) + n * e->csize() + (size_t)e->sym.rhs_total * e->csize() +
+    const size_t y = e->cfg.precision == GM_PREC_FP64 ? 0 : (size_t)e->dsym.y_total;
+    return nf * (n * sizeof(double2) + n * e->csize() + ((size_t)e->sym.rhs_total + y) * e->csize() +
                  (size_t)gm::residual_blocks(e->cfg.nx, e->cfg.ny) * 2 * sizeof(double) + 2 * sizeof(double));
 }
 
@@ -216,7 +217,8 @@ size_t bytes_per_shot(const gm_engine *e) {
 // workspaces already hold, less a reserve of 5 % of the device and 1 GB),
 // or the caller's cap (gm_set_shot_block).
 int shot_block(const gm_engine *e, int nshots) {
-    const size_t held = e->d_xf.bytes + e->d_t.bytes + e->d_w.bytes + e->d_part.bytes + e->d_norm.bytes;
+    const size_t held = e->d_xf.bytes + e->d_t.bytes + e->d_w.bytes + e->d_part.bytes + e->d_norm.bytes +
+                        (e->cfg.precision == GM_PREC_FP64 ? 0 : e->d_y.bytes);
     const size_t per = std::max<size_t>(1, bytes_per_shot(e));
     if (e->shot_block <= 0 && per * (size_t)nshots <= held) return nshots;   // workspaces in place already
     size_t fr = 0, tot = 0;
@@ -239,8 +241,8 @@ extern "C" int gm_set_shot_block(gm_engine *e, int max_shots) {
 extern "C" int gm_memory_estimate(gm_engine *e, int nmat, size_t *factor_bytes, size_t *shot_bytes) {
     if (!e || nmat <= 0) return fail(GM_ERROR_INVALID, "gm_memory_estimate: bad argument");
     const size_t n = (size_t)e->n, m = (size_t)nmat;
-    if (factor_bytes)   // fronts, assembled stencils, mass / stiffness, PML profiles
-        *factor_bytes = m * ((size_t)e->sym.front_total * e->csize() + 9 * n * sizeof(double2) + n * sizeof(float2) +
+    if (factor_bytes)   // fronts, triangle-inversion scratch, assembled stencils, mass / stiffness, PML profiles
+        *factor_bytes = m * (((size_t)e->sym.front_total + (size_t)e->tri_total) * e->csize() + 9 * n * sizeof(double2) + n * sizeof(float2) +
                              n * sizeof(float) + (4 * ((size_t)e->cfg.nx + 2) + 4 * ((size_t)e->cfg.ny + 2)) * 4);
     if (shot_bytes) {
         const int nf = e->nf;

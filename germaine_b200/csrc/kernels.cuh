@@ -40,11 +40,23 @@ void launch_assemble(const AsmArgs &a, const float *m0, const float *m1, const A
                      cudaStream_t st);
 
 // ---------------- symbolic structure on the device ----------------
+// what a kernel needs of one front, in level order (one 64-byte load instead
+// of a chain of table look-ups)
+struct alignas(16) NodeDesc {
+    int64_t front_off, var_off, inv_off, rhs_off, y_off;
+    int node, nfront, npiv, child0, child1, pad;
+};
+
 struct DevSym {
     int n, nnodes;
+    const NodeDesc *desc;   // [level position], parallel to lvl_nodes
     const int *npiv, *nfront, *child0, *child1, *vars, *inv, *lvl_nodes;
     const int64_t *front_off, *var_off, *inv_off, *rhs_off;
     int64_t front_total, rhs_total;
+    // pivot workspace of the substitution: first row of each node of the
+    // levels with more than 32 pivots (-1 elsewhere), rows in all
+    const int64_t *y_off;
+    int64_t y_total;
 };
 
 // ---------------- K2-K4 numeric factorisation ----------------
@@ -118,6 +130,13 @@ template <class R>
 bool level_pivots(const LevelInfo &L);
 template <class R>
 void launch_factor_mid(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_t st);
+// The level's 32 x 32 diagonal-block inverses extended to the inverses of the
+// fronts' whole pivot triangles (levels with more than 32 pivots; what the
+// substitution multiplies by there).  scratch: [nf][scratch_total] cplx<R>,
+// npiv^2 entries per node of the level at scratch_off[node].
+template <class R>
+void launch_tri_inverse(const FactorArgs<R> &a, const LevelInfo &L, void *scratch, int64_t scratch_total,
+                        const int64_t *scratch_off, cudaStream_t st);
 
 
 // one dense product C -= A * B (column-major, complex<R>)
@@ -140,6 +159,7 @@ struct SolveArgs {
     const void *front;        // cplx<R> factors [nf][front_total]
     void *x;                  // cplx<R> [nf][n][ldr], rhs in, solution out
     void *w;                  // cplx<R> [nf][rhs_total][ldr] update vectors (ring rows)
+    void *y;                  // cplx<R> [nf][y_total][ldr] pivot rows of the levels with more than 32 pivots
     int nf, nrhs, ldr;
     int rch;                  // right-hand sides per CTA (<= 32)
     int trans;                // 0: M x = b, 1: M^T x = b
@@ -170,10 +190,10 @@ struct SolveArgs {
     const int *spike_k;
     const double2 *spike_amp;
     // row exchanges of the factorisation's threshold pivoting (FactorArgs::
-    // pivsrc; NULL: none): within each 32-pivot block of the fronts solved
-    // by the ring / pivot kernels, the forward pass of M x = b gathers the
-    // block's right-hand-side rows through it, the backward pass of
-    // M^T x = b scatters the block's solution rows through it
+    // pivsrc; NULL: none): within each 32-pivot block of the pivoted fronts,
+    // the forward pass of M x = b gathers the block's right-hand-side rows
+    // through it, the backward pass of M^T x = b scatters the block's
+    // solution rows through it
     const unsigned char *pivsrc;
 };
 

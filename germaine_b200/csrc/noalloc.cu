@@ -73,13 +73,14 @@ bool device_reachable(const void *p) {
 }
 
 template <class R>
-void substitute_into(gm_engine *e, void *xT, void *w, int nrhs, int trans) {
+void substitute_into(gm_engine *e, void *xT, void *w, void *y, int nrhs, int trans) {
     gm::SolveArgs<R> a{};
     a.s = e->dsym;
     a.front = e->d_front.p;
     a.pivsrc = e->cfg.pivot_tol > 0 ? e->d_pivsrc.as<unsigned char>() : nullptr;
     a.x = xT;
     a.w = w;
+    a.y = y;   // [nf][y_total][nrhs], y_total <= n
     a.nf = e->nf;
     a.nrhs = nrhs;
     a.ldr = nrhs;
@@ -157,13 +158,14 @@ extern "C" int gm_solve_noalloc(gm_engine *e, int sys, int nrhs, const double *d
     const double2 *b = reinterpret_cast<const double2 *>(d_b);
     double2 *x = reinterpret_cast<double2 *>(d_x);
 
-    // initial solve in working precision, x = 0 + t
+    // initial solve in working precision, x = 0 + t (the residual's buffer is
+    // free while a substitution runs: it holds the pivot workspace)
     NA_CUDA(cudaEventRecord(e->ev0, e->st));
     if (fp64) gm::launch_convert_down<double>(b, t, cnt, e->st);
     else gm::launch_convert_down<float>(b, t, cnt, e->st);
     NA_CUDA(cudaMemsetAsync(x, 0, cnt * sizeof(double2), e->st));
-    if (fp64) substitute_into<double>(e, t, w, nrhs, sys);
-    else substitute_into<float>(e, t, w, nrhs, sys);
+    if (fp64) substitute_into<double>(e, t, w, r, nrhs, sys);
+    else substitute_into<float>(e, t, w, r, nrhs, sys);
     if (fp64) gm::launch_add_up<double>(x, t, cnt, e->st);
     else gm::launch_add_up<float>(x, t, cnt, e->st);
     NA_CUDA(cudaGetLastError());
@@ -207,8 +209,8 @@ extern "C" int gm_solve_noalloc(gm_engine *e, int sys, int nrhs, const double *d
         if (worst <= e->cfg.ir_tol || it >= e->cfg.ir_max_iter) break;
         if (fp64) gm::launch_convert_down<double>(r, t, cnt, e->st);
         else gm::launch_convert_down<float>(r, t, cnt, e->st);
-        if (fp64) substitute_into<double>(e, t, w, nrhs, sys);
-        else substitute_into<float>(e, t, w, nrhs, sys);
+        if (fp64) substitute_into<double>(e, t, w, r, nrhs, sys);
+        else substitute_into<float>(e, t, w, r, nrhs, sys);
         if (fp64) gm::launch_add_up<double>(x, t, cnt, e->st);
         else gm::launch_add_up<float>(x, t, cnt, e->st);
         e->stats.n_subst += 1;

@@ -5,286 +5,33 @@
 //
 // Right-hand sides / solutions are [nf][n][ldr] complex, right-hand side
 // fastest.  Work units are (front, frequency, slice of 32 or 40 right-hand
-// sides).  The factorisation stores, in every 32 x 32 diagonal block, the
-// inverses of the block's triangles, so every step below is a small GEMM on
-// CUDA cores: 128 threads, each owning a (RT/16) x B complex register tile
-// of an RT-row x 8B-right-hand-side output tile, operands staged in shared
-// memory.
+// sides).  The factorisation stores the inverse of every pivot triangle (of
+// the 32 x 32 diagonal block of the fronts with at most 32 pivots, of the
+// whole triangle above that, tri.cu), so every step below is a small GEMM:
+// 128 threads fill an RT-row x 8B-right-hand-side output tile, operands
+// staged in shared memory (solve_tile.cuh).
 //
-// Pivot rows are solved in place in x (their rows of x hold the right-hand
-// side, then y, then the solution); the workspace w holds only each front's
-// update vector for its parent (its ring rows).  Per elimination-tree level:
+// x holds the right-hand side, then the solution; the workspace w holds each
+// front's update vector for its parent (its ring rows).  Per
+// elimination-tree level, fronts of at most 32 pivots take one fused kernel
+// per pass (k_fwd_small, k_bwd_small), the others
 //   forward  (leaves -> root)
-//     k_fwd_piv   add the children's update vectors (by the extend-add
-//                 inverse maps) into x at the pivots, then per 32-pivot block:
-//                 y_b = L_bb^-1 x_b, x_rest -= L_rb y_b over the remaining
-//                 pivot rows;
+//     k_fwd_rhs   the children's update vectors added into x at the pivots;
+//     k_fwd_tri   y = L^-1 x_piv into the pivot workspace, 32-row tiles;
 //     k_fwd_ring  w_ring = (children's update vectors at the ring rows)
-//                 - L_ring,piv * y over 64-row tiles of the ring (many CTAs
-//                 per front: the wide part of the level);
+//                 - L_ring,piv * y over RT-row tiles of the ring;
 //   backward (root -> leaves)
-//     k_bwd_ring  x_piv -= U_piv,ring * x_ring (x_ring = final values of the
-//                 ancestors' variables), 64-row tiles of the pivot rows;
-//     k_bwd_piv   per block from the last: x_b = U_bb^-1 x_b,
-//                 x_above -= U_ab x_b.
+//     k_bwd_ring  t = y - U_piv,ring * x_ring (x_ring = final values of the
+//                 ancestors' variables) in the pivot workspace;
+//     k_bwd_tri   x_piv = U^-1 t, 32-row tiles.
 // trans = 1 solves M^T x = b with the same factors: M^T = U^T L^T, the
 // forward pass runs with U^T and the backward pass with L^T; only the
 // factor indexing and which stored inverse is used change.
 #include <cstdlib>
 
-#include "kernels.cuh"
-#include "cplx.cuh"
-#include "async_copy.cuh"
+#include "solve_tile.cuh"
 
 namespace gm {
-
-constexpr int SNB = 32;   // pivot block (= factorisation block)
-constexpr int NT = 128;   // threads per CTA
-// Template parameters of the kernels:
-//   RT (output rows per tile, 64 or 32): 64-row tiles reuse each staged
-//      right-hand-side row over more factor rows; 32-row tiles halve the
-//      accumulators and the factor tile, so more CTAs fit on an SM -- the
-//      better trade on the small fronts of the lower tree levels;
-//   B (right-hand sides per CTA = 8 B): every slice re-stages the front's
-//      factor tiles, so wider slices read the factors fewer times.
-
-// Tile rows are padded by SPAD elements: the complex128 tile product reads
-// 8 x 4 fragments (4 pivots x 8 rows), which a stride of RT + 2 spreads over
-// distinct shared-memory banks.
-constexpr int SPAD = 2;
-
-template <class C, int RT, int B>
-struct SolveSmem {
-    C L[SNB][RT + SPAD];       // factor tile, [pivot q][row]
-    C Y[SNB][8 * B + SPAD];    // right operand, [pivot q][rhs]
-};
-
-// factor element M'(i, c) of the forward (L') or backward (U') factor:
-// F[i + c f] for M x = b, F[c + i f] for M^T x = b
-template <class C, bool TRANS>
-__device__ __forceinline__ C elem(const C *F, int f, int i, int c) {
-    return TRANS ? F[c + (size_t)i * f] : F[i + (size_t)c * f];
-}
-
-// The staging helpers below issue asynchronous copies (every load of the
-// tile in flight at once, no register round trip); the tile is complete
-// after staged_sync().
-//
-// sm.L[q][row] = M'(i0 + row, c0 + q) for row < rows, q < qb.  Entries
-// outside are left as they are: tile_mma reads only q < qb, and rows >= rows
-// (or right-hand sides >= rn) only feed accumulators that are never stored,
-// so partial tiles stage only what they use.
-// (the _p forms take the tile by pointer and the participating threads as
-// lt = 0 .. nt - 1; the SolveSmem forms are the CTA-wide ones)
-template <class C, bool TRANS, int RT>
-__device__ __forceinline__ void stage_factor_p(C (*L)[RT + SPAD], const C *F, int f, int i0, int rows, int c0, int qb,
-                                               int lt, int nt) {
-    if (!TRANS) {
-        for (int t = lt; t < RT * qb; t += nt) {
-            const int row = t % RT, q = t / RT;
-            if (row < rows) cp_async_elem(&L[q][row], F + (i0 + row) + (size_t)(c0 + q) * f);
-        }
-    } else {
-        for (int t = lt; t < SNB * rows; t += nt) {
-            const int q = t % SNB, row = t / SNB;
-            if (q < qb) cp_async_elem(&L[q][row], F + (c0 + q) + (size_t)(i0 + row) * f);
-        }
-    }
-}
-template <class C, bool TRANS, int RT, int B>
-__device__ __forceinline__ void stage_factor(SolveSmem<C, RT, B> &sm, const C *F, int f, int i0, int rows, int c0, int qb) {
-    stage_factor_p<C, TRANS, RT>(sm.L, F, f, i0, rows, c0, qb, threadIdx.x, NT);
-}
-
-// sm.L[q][p] = the inverse diagonal-block operator of pivot block k0:
-//   FWD && !TRANS: L^-1        FWD && TRANS: (U^-1)^T
-//   !FWD && !TRANS: U^-1       !FWD && TRANS: (L^-1)^T
-// The stored block holds L^-1 strictly below the diagonal (unit diagonal
-// implied) and U^-1 on and above it.
-template <class C, bool FWD, bool TRANS, int RT>
-__device__ __forceinline__ void stage_dinv_p(C (*L)[RT + SPAD], const C *F, int f, int k0, int kb, int lt, int nt) {
-    for (int t = lt; t < SNB * kb; t += nt) {
-        const int p = t % SNB, q = t / SNB;   // operator entry (p, q) -> L[q][p], q < kb
-        if (p >= kb) continue;
-        const bool lower_src = FWD != TRANS;         // L^-1 (or its transpose) wanted
-        const int r = TRANS ? q : p, c = TRANS ? p : q;  // position in the stored block
-        const bool stored = lower_src ? r > c : r <= c;
-        if (stored) {
-            cp_async_elem(&L[q][p], F + (k0 + r) + (size_t)(k0 + c) * f);
-        } else {
-            using RR = decltype(L[0][0].x);
-            L[q][p] = (lower_src && r == c) ? mk(RR(1), RR(0)) : czero<C>();
-        }
-    }
-}
-template <class C, bool FWD, bool TRANS, int RT, int B>
-__device__ __forceinline__ void stage_dinv(SolveSmem<C, RT, B> &sm, const C *F, int f, int k0, int kb) {
-    stage_dinv_p<C, FWD, TRANS, RT>(sm.L, F, f, k0, kb, threadIdx.x, NT);
-}
-
-// Per-thread accumulators of an RT x 8B complex output tile (128 threads,
-// lt = 0 .. 127), in the layout of the tile product that fills them.
-template <class C, int RT, int B>
-struct TileAcc;
-
-// complex64: CUDA-core FMAs; thread (tr, tc) = (lt / 8, lt % 8) owns rows
-// tr + 16 i and columns tc + 8 j
-template <int RT, int B>
-struct TileAcc<float2, RT, B> {
-    static constexpr int NR = RT / 16, NC = B;
-    float2 v[NR][NC];
-    __device__ __forceinline__ static int row(int i, int lt) { return lt / 8 + 16 * i; }
-    __device__ __forceinline__ static int col(int j, int lt) { return lt % 8 + 8 * j; }
-};
-
-// complex128: FP64 matrix instructions (mma.sync m8n8k4 f64) on 8 x 8
-// blocks; warp w owns row blocks w + 4 i, lane l row 8 (w + 4 i) + l / 4 of
-// them and columns 8 c + 2 (l % 4) + {0, 1} of every column block c
-template <int RT, int B>
-struct TileAcc<double2, RT, B> {
-    static constexpr int NR = RT / 32, NC = 2 * B;
-    double2 v[NR][NC];
-    __device__ __forceinline__ static int row(int i, int lt) { return 8 * ((lt >> 5) + 4 * i) + ((lt & 31) >> 2); }
-    __device__ __forceinline__ static int col(int j, int lt) { return 8 * (j >> 1) + 2 * (lt & 3) + (j & 1); }
-};
-
-template <class C, int RT, int B>
-__device__ __forceinline__ void zero_acc(TileAcc<C, RT, B> &acc) {
-#pragma unroll
-    for (int i = 0; i < TileAcc<C, RT, B>::NR; ++i)
-#pragma unroll
-        for (int j = 0; j < TileAcc<C, RT, B>::NC; ++j) acc.v[i][j] = czero<C>();
-}
-
-// f(row, col, value) for the thread's accumulators with row < rows, col < rn
-template <class C, int RT, int B, class F>
-__device__ __forceinline__ void for_acc(const TileAcc<C, RT, B> &acc, int rows, int rn, int lt, F f) {
-    using A = TileAcc<C, RT, B>;
-#pragma unroll
-    for (int i = 0; i < A::NR; ++i) {
-        const int row = A::row(i, lt);
-        if (row >= rows) continue;
-#pragma unroll
-        for (int j = 0; j < A::NC; ++j) {
-            const int col = A::col(j, lt);
-            if (col < rn) f(row, col, acc.v[i][j]);
-        }
-    }
-}
-
-// acc += L'[rows x qb] Y[qb x rn]: L[q][row] holds operator entry (row, q),
-// Y[q][col] the right operand.  Rows >= `rows` and columns >= rn of the
-// tile only feed accumulators that are never stored; row and column groups
-// that lie entirely outside are skipped warp-uniformly, so small fronts and
-// short slices do not pay for the full tile.  TRI: 0 a full operator;
-// TRI_LOWER / TRI_UPPER a triangular one (the diagonal-block inverses),
-// whose column q has no entries above / below row q: row groups that column
-// q does not reach are skipped for that q.
-constexpr int TRI_LOWER = 1, TRI_UPPER = 2;
-
-// complex64: each thread accumulates its 16-row-strided rows x 8-column-
-// strided columns with CUDA-core FMAs, one pivot q at a time
-template <int TRI, int RT, int B>
-__device__ __forceinline__ void tile_mma_p(const float2 (*L)[RT + SPAD], const float2 (*Y)[8 * B + SPAD], int qb,
-                                           TileAcc<float2, RT, B> &acc, int rows, int rn, int lt) {
-    constexpr int A = RT / 16;
-    const int tr = lt / 8, tc = lt % 8;
-    const int wrow = (lt >> 5) * 4;   // a warp owns rows 4w .. 4w + 3 of each 16-row group
-    const int na = rows <= wrow ? 0 : min(A, (rows - wrow + 15) / 16);
-    const int nb = min(B, (rn + 7) / 8);
-    if (na == 0) return;   // warp-uniform: this warp owns no row of the tile
-#pragma unroll 2
-    for (int q = 0; q < qb; ++q) {
-        const int alo = TRI == TRI_LOWER ? q / 16 : 0;       // rows >= q only
-        const int ahi = TRI == TRI_UPPER ? q / 16 : A - 1;   // rows <= q only
-        float2 l[A], y[B];
-#pragma unroll
-        for (int a = 0; a < A; ++a) l[a] = a < na && a >= alo && a <= ahi ? L[q][tr + 16 * a] : czero<float2>();
-#pragma unroll
-        for (int b = 0; b < B; ++b) y[b] = b < nb ? Y[q][tc + 8 * b] : czero<float2>();
-#pragma unroll
-        for (int a = 0; a < A; ++a) {
-            if (a >= na) break;
-            if (a < alo || a > ahi) continue;
-#pragma unroll
-            for (int b = 0; b < B; ++b)
-                if (b < nb) cfma(acc.v[a][b], l[a], y[b]);
-        }
-    }
-}
-
-// d = a b + d on one 8 x 8 x 4 FP64 block (warp-wide; a: this lane's entry
-// of the 8 x 4 row-major left block, b: of the 4 x 8 column-major right
-// block, d: this lane's two entries of the 8 x 8 result)
-__device__ __forceinline__ void dmma_884(double a, double b, double &d0, double &d1) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
-}
-
-// complex128: per 4 pivots and per 8 x 8 block, four FP64 matrix
-// instructions (Re += Ar Br - Ai Bi, Im += Ar Bi + Ai Br); a lane loads one
-// complex entry of each left and right fragment.  Pivots q >= qb enter as
-// zeros.
-template <int TRI, int RT, int B>
-__device__ __forceinline__ void tile_mma_p(const double2 (*L)[RT + SPAD], const double2 (*Y)[8 * B + SPAD], int qb,
-                                           TileAcc<double2, RT, B> &acc, int rows, int rn, int lt) {
-    constexpr int NRB = RT / 32;
-    const int w = lt >> 5, lane = lt & 31;
-    const int nb = min(B, (rn + 7) / 8);
-    for (int k0 = 0; k0 < qb; k0 += 4) {
-        const int kk = k0 + (lane & 3);
-        const bool kin = kk < qb;
-        double2 bf[B];
-#pragma unroll
-        for (int b = 0; b < B; ++b) bf[b] = kin && b < nb ? Y[kk][8 * b + (lane >> 2)] : czero<double2>();
-#pragma unroll
-        for (int i = 0; i < NRB; ++i) {
-            const int rb = w + 4 * i;   // row block: rows 8 rb .. 8 rb + 7
-            if (8 * rb >= rows) break;   // warp-uniform
-            if (TRI == TRI_UPPER && 8 * rb > k0 + 3) continue;   // rows <= q only
-            if (TRI == TRI_LOWER && 8 * rb + 7 < k0) continue;   // rows >= q only
-            const double2 af = kin ? L[kk][8 * rb + (lane >> 2)] : czero<double2>();
-#pragma unroll
-            for (int b = 0; b < B; ++b) {
-                if (b >= nb) break;
-                double2 &d0 = acc.v[i][2 * b], &d1 = acc.v[i][2 * b + 1];
-                dmma_884(af.x, bf[b].x, d0.x, d1.x);
-                dmma_884(-af.y, bf[b].y, d0.x, d1.x);
-                dmma_884(af.x, bf[b].y, d0.y, d1.y);
-                dmma_884(af.y, bf[b].x, d0.y, d1.y);
-            }
-        }
-    }
-}
-
-template <int TRI = 0, class C, int RT, int B>
-__device__ __forceinline__ void tile_mma(const SolveSmem<C, RT, B> &sm, int qb, TileAcc<C, RT, B> &acc, int rows,
-                                         int rn) {
-    tile_mma_p<TRI, RT, B>(sm.L, sm.Y, qb, acc, rows, rn, threadIdx.x);
-}
-
-// row_ptr(row)[col] -= acc for the thread's rows (< rows) and columns (< rn)
-template <class C, int RT, int B, class RowPtr>
-__device__ __forceinline__ void sub_acc(RowPtr row_ptr, int rows, int rn, const TileAcc<C, RT, B> &acc) {
-    for_acc(acc, rows, rn, threadIdx.x, [&](int row, int col, const C &v) {
-        C *x = row_ptr(row);
-        x[col] = csub(x[col], v);
-    });
-}
-
-// Y[q][r] = row_ptr(q)[r] for q < qb, r < rn (entries outside: as above)
-template <class C, int TC, class RowPtr>
-__device__ __forceinline__ void stage_rows_p(C (*Y)[TC + SPAD], RowPtr row_ptr, int qb, int rn, int lt, int nt) {
-    for (int t = lt; t < qb * TC; t += nt) {
-        const int q = t / TC, r = t % TC;
-        if (r < rn) cp_async_elem(&Y[q][r], row_ptr(q) + r);
-    }
-}
-template <class C, int RT, int B, class RowPtr>
-__device__ __forceinline__ void stage_rows(SolveSmem<C, RT, B> &sm, RowPtr row_ptr, int qb, int rn) {
-    stage_rows_p<C, 8 * B>(sm.Y, row_ptr, qb, rn, threadIdx.x, NT);
-}
 
 // false when right-hand sides r0 .. r0 + rn - 1 are zero throughout node v's
 // subtree (forward-pass pruning mask; no mask: always true)
@@ -328,16 +75,17 @@ template <class R, int TC>
 __device__ __forceinline__ Ctx<R> make_ctx(const SolveArgs<R> &a, int lvl_first, int chunk, int pos = -1) {
     using C = cplx<R>;
     Ctx<R> c;
-    c.node = a.s.lvl_nodes[lvl_first + (pos < 0 ? (int)blockIdx.y : pos)];
-    c.f = a.s.nfront[c.node];
-    c.s = a.s.npiv[c.node];
+    const NodeDesc d = a.s.desc[lvl_first + (pos < 0 ? (int)blockIdx.y : pos)];
+    c.node = d.node;
+    c.f = d.nfront;
+    c.s = d.npiv;
     const int r0 = chunk * TC;
     c.rn = min(TC, a.nrhs - r0);
     const size_t fz = solve_matrix(a), xz = solve_slot(a);
-    c.F = reinterpret_cast<const C *>(a.front) + fz * a.s.front_total + a.s.front_off[c.node];
-    c.vars = a.s.vars + a.s.var_off[c.node];
+    c.F = reinterpret_cast<const C *>(a.front) + fz * a.s.front_total + d.front_off;
+    c.vars = a.s.vars + d.var_off;
     c.X = reinterpret_cast<C *>(a.x) + xz * (size_t)a.s.n * a.ldr + r0;
-    c.W = reinterpret_cast<C *>(a.w) + xz * (size_t)a.s.rhs_total * a.ldr + r0 + (size_t)a.s.rhs_off[c.node] * a.ldr;
+    c.W = reinterpret_cast<C *>(a.w) + xz * (size_t)a.s.rhs_total * a.ldr + r0 + (size_t)d.rhs_off * a.ldr;
     return c;
 }
 
@@ -368,77 +116,154 @@ __device__ __forceinline__ void pivot_rhs(const SolveArgs<R> &a, const Ctx<R> &c
     __syncthreads();
 }
 
-// Forward pass, pivot part: add the children's update vectors (gathered by
-// the extend-add inverse maps) into x at this front's pivots, then solve the
-// pivot rows in place in x, 32-pivot block by block.
-template <class R, bool TRANS, int RT, int B>
-__global__ void __launch_bounds__(NT) k_fwd_piv(SolveArgs<R> a, int lvl_first, int fused) {
+// ---- fronts of the levels with more than 32 pivots ----
+// The factorisation leaves the full inverses of both pivot triangles there
+// (tri.cu), so the pivot rows are products too, over as many CTAs as they
+// have 32-row tiles, and no CTA walks a chain of 32-pivot blocks: in one
+// CTA per front and slice that chain was the longest part of every upper
+// level (1030 pivots, one matrix, 100 right-hand sides: 2.8 ms for the
+// forward and 2.6 ms for the backward pivot rows of two such fronts).
+// y goes to the separate pivot workspace a.y, since every tile reads all the
+// rows above (below) it.
+
+// Product of rows i0 .. i0 + rows of a factor with the right operand rows
+// row_ptr(k), k = k0 .. k1 - 1, accumulated in chunks of PKC pivots staged PST
+// deep: the next chunks' copies are in flight while one is multiplied.  TRI:
+// i0 is a multiple of 32 and the chunks inside i0 .. i0 + 31 belong to the
+// diagonal block's stored inverse (of the forward or the backward operator).
+// Two 16-pivot chunks take the shared memory of one 32-pivot tile, so six
+// CTAs still fit an SM; measured at 841 x 227 (10 x 100), backward levels
+// 7-10 (52-113 pivots): 1.11 ms unpiped in 32-pivot tiles, 1.27 ms with two
+// 32-pivot chunks (three CTAs per SM), 1.03 ms so; three or four chunks in
+// flight 1.16 and 1.28 ms.
+constexpr int PKC = 16, PST = 2;
+
+template <class C, int RT, int B>
+struct PipeStage {
+    C L[PKC][RT + SPAD];       // factor tile, [pivot q][row]
+    C Y[PKC][8 * B + SPAD];    // right operand, [pivot q][rhs]
+};
+
+template <class R, bool TRANS, bool FWD, bool TRI, int RT, int B, class RowPtr>
+__device__ __forceinline__ void pipe_product(PipeStage<cplx<R>, RT, B> *st, const cplx<R> *F, int f, int i0, int rows,
+                                             int k0, int k1, RowPtr row_ptr, int rn, TileAcc<cplx<R>, RT, B> &acc) {
     using C = cplx<R>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    SolveSmem<C, RT, B> &sm = *reinterpret_cast<SolveSmem<C, RT, B> *>(smem_raw);
-    constexpr int TC = 8 * B;
-    const Ctx<R> c = make_ctx<R, TC>(a, lvl_first, blockIdx.x);
-    if (c.rn <= 0) return;
-    const int r0 = blockIdx.x * TC;
+    const int nc = (k1 - k0 + PKC - 1) / PKC;
+    auto stage = [&](int j) {
+        if (j < nc) {
+            PipeStage<C, RT, B> &sm = st[j % PST];
+            const int q0 = k0 + j * PKC, qb = min(PKC, k1 - q0);
+            if (TRI && q0 >= i0 && q0 < i0 + SNB)
+                stage_dinv_p<C, FWD, TRANS, RT, PKC>(sm.L, F, f, i0, rows, q0 - i0, qb, threadIdx.x, NT);
+            else
+                stage_factor_p<C, TRANS, RT, PKC>(sm.L, F, f, i0, rows, q0, qb, threadIdx.x, NT);
+            stage_rows_p<C, 8 * B>(sm.Y, [&](int q) { return row_ptr(q0 + q); }, qb, rn, threadIdx.x, NT);
+        }
+        async_commit();
+    };
+#pragma unroll
+    for (int j = 0; j < PST - 1; ++j) stage(j);
+    for (int j = 0; j < nc; ++j) {
+        async_wait_group<PST - 2>();   // chunk j has landed
+        __syncthreads();               // and every warp is past chunk j - 1
+        stage(j + PST - 1);
+        const PipeStage<C, RT, B> &sm = st[j % PST];
+        tile_mma_p<0, RT, B>(sm.L, sm.Y, min(PKC, k1 - k0 - j * PKC), acc, rows, rn, threadIdx.x);
+    }
+}
+
+// rows of this front in the pivot workspace, this slice's columns
+template <class R, int TC>
+__device__ __forceinline__ cplx<R> *pivot_work(const SolveArgs<R> &a, int node, int chunk) {
+    return reinterpret_cast<cplx<R> *>(a.y) + (solve_slot(a) * (size_t)a.s.y_total + (size_t)a.s.y_off[node]) * a.ldr +
+           chunk * TC;
+}
+
+// Forward pass, right-hand sides: the children's update vectors (gathered by
+// the extend-add inverse maps) are added into x at this front's pivots, one
+// 32-pivot block x slice per CTA; for M x = b with row exchanges the block's
+// rows are left in pivot order (prow[q]: the block row at pivot position q).
+// blockIdx.x = chunk + nchunk * block
+template <class R, bool TRANS, int B>
+__global__ void __launch_bounds__(NT) k_fwd_rhs(SolveArgs<R> a, int lvl_first, int nchunk) {
+    using C = cplx<R>;
+    constexpr int TC = 8 * B, NE = SNB * TC / NT;
+    const int chunk = blockIdx.x % nchunk, k0 = blockIdx.x / nchunk * SNB;
+    const Ctx<R> c = make_ctx<R, TC>(a, lvl_first, chunk);
+    if (c.rn <= 0 || k0 >= c.s) return;
+    const int r0 = chunk * TC;
     if (!live(a, c.node, r0, c.rn)) return;   // y and the update vector are zero
-    (void)fused;
     const int *inv = a.s.inv + a.s.inv_off[c.node];
-    const size_t xz = solve_slot(a);
-    const C *Wall = reinterpret_cast<const C *>(a.w) + xz * (size_t)a.s.rhs_total * a.ldr + r0;
+    const C *Wall = reinterpret_cast<const C *>(a.w) + solve_slot(a) * (size_t)a.s.rhs_total * a.ldr + r0;
     const int c0 = a.s.child0[c.node], c1 = a.s.child1[c.node];
     const C *W0 = c0 >= 0 && live(a, c0, r0, c.rn) ? Wall + (size_t)a.s.rhs_off[c0] * a.ldr : nullptr;
     const C *W1 = c1 >= 0 && live(a, c1, r0, c.rn) ? Wall + (size_t)a.s.rhs_off[c1] * a.ldr : nullptr;
     const size_t ldr = a.ldr;
-
-    pivot_rhs(a, c, inv, W0, W1, r0, ldr);   // (the ring part is k_fwd_ring's)
-
-    auto xrow = [&](int k) { return c.X + (size_t)c.vars[k] * ldr; };
-    // M x = b with row exchanges: block k0's right-hand-side rows are taken
-    // in pivot order (prow[q]: the block row at pivot position q), y is
-    // written in pivot order (rows of L' below the block stay in equation
-    // order until their own block)
-    __shared__ unsigned char prow[SNB];
+    const bool implicit = a.spike_k != nullptr;
     const bool pv = !TRANS && a.pivsrc;
+    if (!(W0 || W1 || implicit || pv)) return;   // CTA-uniform: x holds the block's right-hand sides already
     const unsigned char *psrc = pv ? a.pivsrc + solve_matrix(a) * (size_t)a.s.n : nullptr;
-    TileAcc<C, RT, B> acc;
-    for (int k0 = 0; k0 < c.s; k0 += SNB) {
-        const int kb = min(SNB, c.s - k0);
-        if (pv) {   // the previous block's reads of prow ended before its staged_sync
-            if (threadIdx.x < kb) prow[threadIdx.x] = psrc[c.vars[k0 + threadIdx.x]];
-            __syncthreads();
+    const C amp = implicit ? cconv<C>(a.spike_amp[solve_matrix(a)]) : czero<C>();
+    const int kb = min(SNB, c.s - k0);
+    C v[NE];   // all of the block's rows are read before any is written
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+        const int t = threadIdx.x + NT * e, q = t / TC, r = t % TC;
+        v[e] = czero<C>();
+        if (q < kb && r < c.rn) {
+            const int p = k0 + (pv ? psrc[c.vars[k0 + q]] : q);
+            const int row = c.vars[p];
+            const int q0 = W0 ? inv[p] : -1, q1 = W1 ? inv[c.f + p] : -1;
+            if (implicit) {
+                if (a.spike_k[r0 + r] == row) v[e] = amp;
+            } else {
+                v[e] = c.X[(size_t)row * ldr + r];
+            }
+            C g = czero<C>();
+            if (q0 >= 0) g = cadd(g, W0[(size_t)q0 * ldr + r]);
+            if (q1 >= 0) g = cadd(g, W1[(size_t)q1 * ldr + r]);
+            v[e] = cadd(v[e], g);
         }
-        stage_dinv<C, true, TRANS, RT, B>(sm, c.F, c.f, k0, kb);
-        stage_rows(sm, [&](int q) { return xrow(k0 + (pv ? prow[q] : q)); }, kb, c.rn);
-        staged_sync();
-        zero_acc(acc);
-        tile_mma<TRI_LOWER>(sm, kb, acc, kb, c.rn);   // y_b = Dinv w_b
-        __syncthreads();
-        for_acc(acc, kb, c.rn, threadIdx.x, [&](int row, int col, const C &v) { sm.Y[row][col] = v; });
-        __syncthreads();
-        for (int t = threadIdx.x; t < kb * TC; t += NT) {
-            const int q = t / TC, r = t % TC;
-            if (r < c.rn) xrow(k0 + q)[r] = sm.Y[q][r];
-        }
-        for (int i0 = k0 + kb; i0 < c.s; i0 += RT) {
-            const int rows = min(RT, c.s - i0);
-            stage_factor<C, TRANS, RT, B>(sm, c.F, c.f, i0, rows, k0, kb);
-            staged_sync();
-            zero_acc(acc);
-            tile_mma(sm, kb, acc, rows, c.rn);
-            sub_acc([&](int row) { return xrow(i0 + row); }, rows, c.rn, acc);
-            __syncthreads();
-        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+        const int t = threadIdx.x + NT * e, q = t / TC, r = t % TC;
+        if (q < kb && r < c.rn) c.X[(size_t)c.vars[k0 + q] * ldr + r] = v[e];
     }
 }
 
+// Forward pass, pivot part: y = (inverse of the forward triangle) x[pivots],
+// one 32-row tile x slice per CTA; zero where the pruned pass skips the
+// front.  blockIdx.x = chunk + nchunk * tile
+template <class R, bool TRANS, int B>
+__global__ void __launch_bounds__(NT) k_fwd_tri(SolveArgs<R> a, int lvl_first, int nchunk) {
+    using C = cplx<R>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    auto *st = reinterpret_cast<PipeStage<C, SNB, B> *>(smem_raw);
+    constexpr int TC = 8 * B;
+    const int chunk = blockIdx.x % nchunk, i0 = blockIdx.x / nchunk * SNB;
+    const Ctx<R> c = make_ctx<R, TC>(a, lvl_first, chunk);
+    if (c.rn <= 0 || i0 >= c.s) return;
+    const int rows = min(SNB, c.s - i0);
+    const size_t ldr = a.ldr;
+    C *Y = pivot_work<R, TC>(a, c.node, chunk);
+    TileAcc<C, SNB, B> acc;
+    zero_acc(acc);
+    if (live(a, c.node, chunk * TC, c.rn))
+        pipe_product<R, TRANS, true, true, SNB, B>(st, c.F, c.f, i0, rows, 0, i0 + rows,
+                                                   [&](int k) { return c.X + (size_t)c.vars[k] * ldr; }, c.rn, acc);
+    for_acc(acc, rows, c.rn, threadIdx.x, [&](int row, int r, const C &v) { Y[(size_t)(i0 + row) * ldr + r] = v; });
+}
+
 // Forward pass, ring part: update vector = children's update vectors at the
-// ring rows - L'(ring, pivots) y, 64-row tiles of the ring over many CTAs;
+// ring rows - L'(ring, pivots) y, RT-row tiles of the ring over many CTAs;
 // blockIdx.x = chunk + nchunk * tile
 template <class R, bool TRANS, int RT, int B>
 __global__ void __launch_bounds__(NT) k_fwd_ring(SolveArgs<R> a, int lvl_first, int nchunk) {
     using C = cplx<R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    SolveSmem<C, RT, B> &sm = *reinterpret_cast<SolveSmem<C, RT, B> *>(smem_raw);
+    auto *st = reinterpret_cast<PipeStage<C, RT, B> *>(smem_raw);
     constexpr int TC = 8 * B;
     const int chunk = blockIdx.x % nchunk, tile = blockIdx.x / nchunk;
     const Ctx<R> c = make_ctx<R, TC>(a, lvl_first, chunk);
@@ -447,39 +272,37 @@ __global__ void __launch_bounds__(NT) k_fwd_ring(SolveArgs<R> a, int lvl_first, 
     if (!live(a, c.node, chunk * TC, c.rn)) return;   // the update vector is zero (never read)
     const int rows = min(RT, c.f - i0);
     const size_t ldr = a.ldr;
-    TileAcc<C, RT, B> acc;
-    zero_acc(acc);
-    for (int q0 = 0; q0 < c.s; q0 += SNB) {
-        const int qb = min(SNB, c.s - q0);
-        stage_factor<C, TRANS, RT, B>(sm, c.F, c.f, i0, rows, q0, qb);
-        stage_rows(sm, [&](int q) { return c.X + (size_t)c.vars[q0 + q] * ldr; }, qb, c.rn);
-        staged_sync();
-        tile_mma(sm, qb, acc, rows, c.rn);
-        __syncthreads();
-    }
-    // w = (children's update vectors at the ring rows) - L'(ring, piv) y
+    const C *Y = pivot_work<R, TC>(a, c.node, chunk);
+    // the accumulators start from minus the children's update vectors, whose
+    // loads then overlap the first chunk's copies
     const int *inv = a.s.inv + a.s.inv_off[c.node];
     const C *Wall = reinterpret_cast<const C *>(a.w) + solve_slot(a) * a.s.rhs_total * a.ldr + chunk * TC;
     const int c0 = a.s.child0[c.node], c1 = a.s.child1[c.node];
     const C *W0 = c0 >= 0 && live(a, c0, chunk * TC, c.rn) ? Wall + (size_t)a.s.rhs_off[c0] * a.ldr : nullptr;
     const C *W1 = c1 >= 0 && live(a, c1, chunk * TC, c.rn) ? Wall + (size_t)a.s.rhs_off[c1] * a.ldr : nullptr;
-    for_acc(acc, rows, c.rn, threadIdx.x, [&](int row, int r, const C &v) {
+    TileAcc<C, RT, B> acc;
+    zero_acc(acc);
+    for_acc(acc, rows, c.rn, threadIdx.x, [&](int row, int r, C &v) {
         const int i = i0 + row;
         const int q0 = W0 ? inv[i] : -1, q1 = W1 ? inv[c.f + i] : -1;
-        C g = czero<C>();
-        if (q0 >= 0) g = cadd(g, W0[(size_t)q0 * ldr + r]);
-        if (q1 >= 0) g = cadd(g, W1[(size_t)q1 * ldr + r]);
-        c.W[(size_t)(i - c.s) * ldr + r] = csub(g, v);
+        if (q0 >= 0) v = csub(v, W0[(size_t)q0 * ldr + r]);
+        if (q1 >= 0) v = csub(v, W1[(size_t)q1 * ldr + r]);
+    });
+    pipe_product<R, TRANS, true, false, RT, B>(st, c.F, c.f, i0, rows, 0, c.s,
+                                               [&](int k) { return Y + (size_t)k * ldr; }, c.rn, acc);
+    for_acc(acc, rows, c.rn, threadIdx.x, [&](int row, int r, const C &v) {
+        c.W[(size_t)(i0 + row - c.s) * ldr + r] = csub(czero<C>(), v);
     });
 }
 
-// Backward pass, ring part: x[pivots] -= U'(pivots, ring) x[ring]
-// (final values of the ancestors' variables); blockIdx.x = chunk + nchunk * tile
+// Backward pass, ring part: t = y - U'(pivots, ring) x[ring] (final values
+// of the ancestors' variables) in the pivot workspace; blockIdx.x = chunk +
+// nchunk * tile
 template <class R, bool TRANS, int RT, int B>
 __global__ void __launch_bounds__(NT) k_bwd_ring(SolveArgs<R> a, int lvl_first, int nchunk) {
     using C = cplx<R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    SolveSmem<C, RT, B> &sm = *reinterpret_cast<SolveSmem<C, RT, B> *>(smem_raw);
+    auto *st = reinterpret_cast<PipeStage<C, RT, B> *>(smem_raw);
     constexpr int TC = 8 * B;
     const int chunk = blockIdx.x % nchunk, tile = blockIdx.x / nchunk;
     const Ctx<R> c = make_ctx<R, TC>(a, lvl_first, chunk);
@@ -487,96 +310,60 @@ __global__ void __launch_bounds__(NT) k_bwd_ring(SolveArgs<R> a, int lvl_first, 
     if (c.rn <= 0 || i0 >= c.s || c.f == c.s) return;
     const int rows = min(RT, c.s - i0);
     const size_t ldr = a.ldr;
-    TileAcc<C, RT, B> acc;
+    C *Y = pivot_work<R, TC>(a, c.node, chunk);
+    TileAcc<C, RT, B> acc;   // starts from -y: its loads overlap the first chunk's copies
     zero_acc(acc);
-    for (int j0 = c.s; j0 < c.f; j0 += SNB) {
-        const int jb = min(SNB, c.f - j0);
-        stage_factor<C, TRANS, RT, B>(sm, c.F, c.f, i0, rows, j0, jb);
-        stage_rows(sm, [&](int q) { return c.X + (size_t)c.vars[j0 + q] * ldr; }, jb, c.rn);
-        staged_sync();
-        tile_mma(sm, jb, acc, rows, c.rn);
-        __syncthreads();
-    }
-    // y = 0 at the pivot rows in the right-hand sides the pruned forward
-    // pass skipped for this front (x is not cleared there when the
-    // right-hand sides are implicit spikes)
-    for_acc(acc, rows, c.rn, threadIdx.x, [&](int row, int col, const C &v) {
-        C &x = c.X[(size_t)c.vars[i0 + row] * ldr + col];
-        x = csub(a.spike_k && !col_live(a, c.node, chunk * TC + col) ? czero<C>() : x, v);
+    for_acc(acc, rows, c.rn, threadIdx.x,
+            [&](int row, int r, C &v) { v = csub(v, Y[(size_t)(i0 + row) * ldr + r]); });
+    pipe_product<R, TRANS, false, false, RT, B>(st, c.F, c.f, i0, rows, c.s, c.f,
+                                                [&](int k) { return c.X + (size_t)c.vars[k] * ldr; }, c.rn, acc);
+    for_acc(acc, rows, c.rn, threadIdx.x,
+            [&](int row, int r, const C &v) { Y[(size_t)(i0 + row) * ldr + r] = csub(czero<C>(), v); });
+}
+
+// Backward pass, pivot part: x[pivots] = (inverse of the backward triangle)
+// t, one 32-row tile x slice per CTA; for M^T x = b with row exchanges the
+// result comes out in pivot order and is scattered to equation order within
+// its block (prow[q]: the block row at pivot position q).
+template <class R, bool TRANS, int B>
+__global__ void __launch_bounds__(NT) k_bwd_tri(SolveArgs<R> a, int lvl_first, int nchunk) {
+    using C = cplx<R>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    auto *st = reinterpret_cast<PipeStage<C, SNB, B> *>(smem_raw);
+    constexpr int TC = 8 * B;
+    const int chunk = blockIdx.x % nchunk, i0 = blockIdx.x / nchunk * SNB;
+    const Ctx<R> c = make_ctx<R, TC>(a, lvl_first, chunk);
+    if (c.rn <= 0 || i0 >= c.s) return;
+    const int rows = min(SNB, c.s - i0);
+    const size_t ldr = a.ldr;
+    const C *Y = pivot_work<R, TC>(a, c.node, chunk);
+    const bool pv = TRANS && a.pivsrc;
+    const unsigned char *psrc = pv ? a.pivsrc + solve_matrix(a) * (size_t)a.s.n : nullptr;
+    TileAcc<C, SNB, B> acc;
+    zero_acc(acc);
+    pipe_product<R, TRANS, false, true, SNB, B>(st, c.F, c.f, i0, rows, i0, c.s,
+                                                [&](int k) { return Y + (size_t)k * ldr; }, c.rn, acc);
+    for_acc(acc, rows, c.rn, threadIdx.x, [&](int row, int r, const C &v) {
+        const int p = i0 + (pv ? psrc[c.vars[i0 + row]] : row);
+        c.X[(size_t)c.vars[p] * ldr + r] = v;
     });
 }
 
-// Backward pass, pivot part: block by block from the last, x_b = Dinv t_b in
-// place in x, then t_above -= U'(above, b) x_b.
-template <class R, bool TRANS, int RT, int B>
-__global__ void __launch_bounds__(NT) k_bwd_piv(SolveArgs<R> a, int lvl_first, int fused) {
-    using C = cplx<R>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    SolveSmem<C, RT, B> &sm = *reinterpret_cast<SolveSmem<C, RT, B> *>(smem_raw);
-    constexpr int TC = 8 * B;
-    const Ctx<R> c = make_ctx<R, TC>(a, lvl_first, blockIdx.x);
-    if (c.rn <= 0) return;
-    (void)fused;
-    const size_t ldr = a.ldr;
-    auto xrow = [&](int k) { return c.X + (size_t)c.vars[k] * ldr; };
-    if (c.f == c.s && a.spike_k) {
-        // no ring (k_bwd_ring did not set y): y = 0 at the pivot rows in the
-        // right-hand sides the pruned forward pass skipped for this front
-        for (int t = threadIdx.x; t < c.s * TC; t += NT) {
-            const int q = t / TC, r = t % TC;
-            if (r < c.rn && !col_live(a, c.node, blockIdx.x * TC + r)) xrow(q)[r] = czero<C>();
-        }
-        __syncthreads();
-    }
-    // M^T x = b with row exchanges: the block's result comes out in pivot
-    // order and is scattered to equation order (prow[q]: the block row at
-    // pivot position q), where the updates of the blocks above read it
-    __shared__ unsigned char prow[SNB];
-    const bool pv = TRANS && a.pivsrc;
-    const unsigned char *psrc = pv ? a.pivsrc + solve_matrix(a) * (size_t)a.s.n : nullptr;
-    TileAcc<C, RT, B> acc;
-    const int nblk = (c.s + SNB - 1) / SNB;
-    for (int b = nblk - 1; b >= 0; --b) {
-        const int k0 = b * SNB, kb = min(SNB, c.s - k0);
-        if (pv && threadIdx.x < kb) prow[threadIdx.x] = psrc[c.vars[k0 + threadIdx.x]];   // read after staged_sync
-        stage_dinv<C, false, TRANS, RT, B>(sm, c.F, c.f, k0, kb);
-        stage_rows(sm, [&](int q) { return xrow(k0 + q); }, kb, c.rn);
-        staged_sync();
-        zero_acc(acc);
-        tile_mma<TRI_UPPER>(sm, kb, acc, kb, c.rn);   // x_b = Dinv t_b
-        __syncthreads();
-        for_acc(acc, kb, c.rn, threadIdx.x, [&](int row, int col, const C &v) { sm.Y[pv ? prow[row] : row][col] = v; });
-        __syncthreads();
-        for (int t = threadIdx.x; t < kb * TC; t += NT) {
-            const int q = t / TC, r = t % TC;
-            if (r < c.rn) xrow(k0 + q)[r] = sm.Y[q][r];
-        }
-        for (int i0 = 0; i0 < k0; i0 += RT) {
-            const int rows = min(RT, k0 - i0);
-            stage_factor<C, TRANS, RT, B>(sm, c.F, c.f, i0, rows, k0, kb);
-            staged_sync();
-            zero_acc(acc);
-            tile_mma(sm, kb, acc, rows, c.rn);
-            sub_acc([&](int row) { return xrow(i0 + row); }, rows, c.rn, acc);
-            __syncthreads();
-        }
-    }
-}
-
-// (The complex128 small-front kernels are held to 80 registers, six CTAs per
-// SM: measured on the leaf levels they stall on global loads first, so more
-// resident warps pay; the complex64 ones need fewer registers anyway.)
+// (The small-front kernels are held to 80 registers, six CTAs per SM: they
+// stall on global loads first, so more resident warps pay.  Measured at
+// 841 x 227, 10 matrices x 100 right-hand sides, complex64 forward levels 0-6:
+// 18.0 -> 14.4 ms over three passes against the unbounded 118 registers.)
 //
 // Forward pass of a whole front whose pivots fit one 32-pivot block (the
 // small fronts of the lower levels): the children's update vectors are added
 // into x at the pivots, y = Dinv x_piv is formed in shared memory and written
 // back to x, and the update vector w = (children's update vectors at the
 // ring rows) - L'(ring, pivots) y follows tile by tile with y kept in shared
-// memory -- k_fwd_piv and k_fwd_ring in one CTA, y read once.
+// memory -- k_fwd_tri and k_fwd_ring in one CTA, y read once.
 // wofs >= 0: the CTA's (front position, slice) is work[wofs + blockIdx.x],
 // the live pairs of a pruned pass; wofs < 0: (blockIdx.y, blockIdx.x).
 template <class R, bool TRANS, int B>
-__global__ void __launch_bounds__(NT, sizeof(R) == 8 ? 6 : 1) k_fwd_small(SolveArgs<R> a, int lvl_first, int wofs) {
+__global__ void __launch_bounds__(NT, 6) k_fwd_small(SolveArgs<R> a, int lvl_first, int wofs) {
     using C = cplx<R>;
     constexpr int RT = 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -642,10 +429,10 @@ __global__ void __launch_bounds__(NT, sizeof(R) == 8 ? 6 : 1) k_fwd_small(SolveA
 // Backward pass of a whole front whose pivots fit one 32-pivot block (the
 // small fronts of the lower levels): t = y - U'(pivots, ring) x[ring] with
 // the product accumulated in registers over 32-column ring blocks, t placed
-// in shared memory, then x_piv = Dinv t -- k_bwd_ring and k_bwd_piv in one
+// in shared memory, then x_piv = Dinv t -- k_bwd_ring and k_bwd_tri in one
 // CTA, without writing t to x in between.
 template <class R, bool TRANS, int B>
-__global__ void __launch_bounds__(NT, sizeof(R) == 8 ? 6 : 1) k_bwd_small(SolveArgs<R> a, int lvl_first) {
+__global__ void __launch_bounds__(NT, 6) k_bwd_small(SolveArgs<R> a, int lvl_first) {
     using C = cplx<R>;
     constexpr int RT = 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -698,23 +485,33 @@ template <class R, int RT, int B>
 static size_t solve_smem() { return sizeof(SolveSmem<cplx<R>, RT, B>); }
 
 template <class R, int RT, int B>
+static size_t pipe_smem() { return PST * sizeof(PipeStage<cplx<R>, RT, B>); }
+
+template <class K>
+static void set_smem(K kernel, size_t bytes) {
+    cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
+template <class R, int RT, int B>
 static void set_attrs() {
     static bool done = false;
     if (done) return;
-    const int sm = (int)solve_smem<R, RT, B>();
-    cudaFuncSetAttribute((const void *)k_fwd_piv<R, false, RT, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute((const void *)k_fwd_piv<R, true, RT, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute((const void *)k_fwd_ring<R, false, RT, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute((const void *)k_fwd_ring<R, true, RT, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute((const void *)k_bwd_ring<R, false, RT, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute((const void *)k_bwd_ring<R, true, RT, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute((const void *)k_bwd_piv<R, false, RT, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute((const void *)k_bwd_piv<R, true, RT, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    const size_t sm = pipe_smem<R, RT, B>(), sms = solve_smem<R, RT, B>();
+    set_smem(k_fwd_ring<R, false, RT, B>, sm);
+    set_smem(k_fwd_ring<R, true, RT, B>, sm);
+    set_smem(k_bwd_ring<R, false, RT, B>, sm);
+    set_smem(k_bwd_ring<R, true, RT, B>, sm);
     if (RT == 32) {
-        cudaFuncSetAttribute((const void *)k_bwd_small<R, false, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        cudaFuncSetAttribute((const void *)k_bwd_small<R, true, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        cudaFuncSetAttribute((const void *)k_fwd_small<R, false, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        cudaFuncSetAttribute((const void *)k_fwd_small<R, true, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        set_smem(k_fwd_tri<R, false, B>, sm);
+        set_smem(k_fwd_tri<R, true, B>, sm);
+        set_smem(k_bwd_tri<R, false, B>, sm);
+        set_smem(k_bwd_tri<R, true, B>, sm);
+        set_smem(k_fwd_rhs<R, false, B>, 0);
+        set_smem(k_fwd_rhs<R, true, B>, 0);
+        set_smem(k_fwd_small<R, false, B>, sms);
+        set_smem(k_fwd_small<R, true, B>, sms);
+        set_smem(k_bwd_small<R, false, B>, sms);
+        set_smem(k_bwd_small<R, true, B>, sms);
     }
     done = true;
 }
@@ -750,13 +547,16 @@ static int slice_b(int nrhs) {
 template <class R>
 static int solve_nfz(const SolveArgs<R> &a) { return a.fmap ? a.nfz : a.nf; }
 
+// Levels with at most 32 pivots per front take the fused small-front kernels
+// whatever the tile height; the others the four kernels above, RT being the
+// tile height of their ring parts.
 template <class R, int RT, int B>
 static void forward_level(const SolveArgs<R> &a, const LevelInfo &L, cudaStream_t st) {
+    set_attrs<R, 32, B>();
     set_attrs<R, RT, B>();
-    const size_t smem = solve_smem<R, RT, B>();
+    const size_t smem = solve_smem<R, 32, B>();
     const int nchunk = (a.nrhs + 8 * B - 1) / (8 * B);
-    static const bool no_small = env_int("GM_NO_FWD_SMALL") != 0;
-    if (RT == 32 && L.max_piv <= SNB && !no_small) {   // one pivot block per front: fused pivot + ring kernel
+    if (L.max_piv <= SNB) {   // one pivot block per front: fused pivot + ring kernel
         if (a.work && a.work_w[L.index] == 8 * B) {   // pruned pass: only the live (front, slice) pairs
             const int wofs = a.work_off[L.index];
             const int nlive = a.work_off[L.index + 1] - wofs;
@@ -773,47 +573,49 @@ static void forward_level(const SolveArgs<R> &a, const LevelInfo &L, cudaStream_
         });
         return;
     }
-    const int fused = 0;   // separate ring kernel: more parallelism per level
+    const int nblk = (L.max_piv + SNB - 1) / SNB;
     for_level_pieces(L, [&](int first, int count) {
-        dim3 g1(nchunk, count, solve_nfz(a));
-        if (a.trans) (k_fwd_piv<R, true, RT, B><<<g1, NT, smem, st>>>(a, first, fused), note_launch());
-        else (k_fwd_piv<R, false, RT, B><<<g1, NT, smem, st>>>(a, first, fused), note_launch());
-    });
-    if (L.max_ring > 0) {
-        for_level_pieces(L, [&](int first, int count) {
+        dim3 g(nchunk * nblk, count, solve_nfz(a));
+        if (a.trans) {
+            (k_fwd_rhs<R, true, B><<<g, NT, 0, st>>>(a, first, nchunk), note_launch());
+            (k_fwd_tri<R, true, B><<<g, NT, pipe_smem<R, 32, B>(), st>>>(a, first, nchunk), note_launch());
+        } else {
+            (k_fwd_rhs<R, false, B><<<g, NT, 0, st>>>(a, first, nchunk), note_launch());
+            (k_fwd_tri<R, false, B><<<g, NT, pipe_smem<R, 32, B>(), st>>>(a, first, nchunk), note_launch());
+        }
+        if (L.max_ring > 0) {
+            const size_t smr = pipe_smem<R, RT, B>();
             dim3 g2(nchunk * ((L.max_ring + RT - 1) / RT), count, solve_nfz(a));
-            if (a.trans) (k_fwd_ring<R, true, RT, B><<<g2, NT, smem, st>>>(a, first, nchunk), note_launch());
-            else (k_fwd_ring<R, false, RT, B><<<g2, NT, smem, st>>>(a, first, nchunk), note_launch());
-        });
-    }
+            if (a.trans) (k_fwd_ring<R, true, RT, B><<<g2, NT, smr, st>>>(a, first, nchunk), note_launch());
+            else (k_fwd_ring<R, false, RT, B><<<g2, NT, smr, st>>>(a, first, nchunk), note_launch());
+        }
+    });
 }
 
 template <class R, int RT, int B>
 static void backward_level(const SolveArgs<R> &a, const LevelInfo &L, cudaStream_t st) {
+    set_attrs<R, 32, B>();
     set_attrs<R, RT, B>();
-    const size_t smem = solve_smem<R, RT, B>();
     const int nchunk = (a.nrhs + 8 * B - 1) / (8 * B);
-    static const bool no_small = env_int("GM_NO_BWD_SMALL") != 0;
-    if (RT == 32 && L.max_piv <= SNB && !no_small) {   // one pivot block per front: fused ring + pivot kernel
+    if (L.max_piv <= SNB) {   // one pivot block per front: fused ring + pivot kernel
         for_level_pieces(L, [&](int first, int count) {
             dim3 g(nchunk, count, solve_nfz(a));
-            if (a.trans) (k_bwd_small<R, true, B><<<g, NT, smem, st>>>(a, first), note_launch());
-            else (k_bwd_small<R, false, B><<<g, NT, smem, st>>>(a, first), note_launch());
+            if (a.trans) (k_bwd_small<R, true, B><<<g, NT, solve_smem<R, 32, B>(), st>>>(a, first), note_launch());
+            else (k_bwd_small<R, false, B><<<g, NT, solve_smem<R, 32, B>(), st>>>(a, first), note_launch());
         });
         return;
     }
-    const int fused = 0;
-    if (L.max_ring > 0) {
-        for_level_pieces(L, [&](int first, int count) {
-            dim3 g1(nchunk * ((L.max_piv + RT - 1) / RT), count, solve_nfz(a));
-            if (a.trans) (k_bwd_ring<R, true, RT, B><<<g1, NT, smem, st>>>(a, first, nchunk), note_launch());
-            else (k_bwd_ring<R, false, RT, B><<<g1, NT, smem, st>>>(a, first, nchunk), note_launch());
-        });
-    }
+    const int nblk = (L.max_piv + SNB - 1) / SNB;
     for_level_pieces(L, [&](int first, int count) {
-        dim3 g2(nchunk, count, solve_nfz(a));
-        if (a.trans) (k_bwd_piv<R, true, RT, B><<<g2, NT, smem, st>>>(a, first, fused), note_launch());
-        else (k_bwd_piv<R, false, RT, B><<<g2, NT, smem, st>>>(a, first, fused), note_launch());
+        if (L.max_ring > 0) {
+            const size_t smr = pipe_smem<R, RT, B>();
+            dim3 g1(nchunk * ((L.max_piv + RT - 1) / RT), count, solve_nfz(a));
+            if (a.trans) (k_bwd_ring<R, true, RT, B><<<g1, NT, smr, st>>>(a, first, nchunk), note_launch());
+            else (k_bwd_ring<R, false, RT, B><<<g1, NT, smr, st>>>(a, first, nchunk), note_launch());
+        }
+        dim3 g2(nchunk * nblk, count, solve_nfz(a));
+        if (a.trans) (k_bwd_tri<R, true, B><<<g2, NT, pipe_smem<R, 32, B>(), st>>>(a, first, nchunk), note_launch());
+        else (k_bwd_tri<R, false, B><<<g2, NT, pipe_smem<R, 32, B>(), st>>>(a, first, nchunk), note_launch());
     });
 }
 

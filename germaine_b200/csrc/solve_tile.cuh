@@ -1,0 +1,254 @@
+// Tile machinery shared by the substitution kernels (solve.cu) and the
+// triangle inversion (tri.cu): small GEMMs of 32- or 64-row factor tiles
+// with 32- or 40-column right operands, both staged in shared memory by
+// asynchronous copies, 128 threads per CTA.
+#pragma once
+#include "kernels.cuh"
+#include "cplx.cuh"
+#include "async_copy.cuh"
+
+namespace gm {
+
+constexpr int SNB = 32;   // pivot block (= factorisation block)
+constexpr int NT = 128;   // threads per CTA
+// Template parameters of the kernels:
+//   RT (output rows per tile, 64 or 32): 64-row tiles reuse each staged
+//      right-hand-side row over more factor rows; 32-row tiles halve the
+//      accumulators and the factor tile, so more CTAs fit on an SM -- the
+//      better trade on the small fronts of the lower tree levels;
+//   B (right-hand sides per CTA = 8 B): every slice re-stages the front's
+//      factor tiles, so wider slices read the factors fewer times.
+
+// Tile rows are padded by SPAD elements: the complex128 tile product reads
+// 8 x 4 fragments (4 pivots x 8 rows), which a stride of RT + 2 spreads over
+// distinct shared-memory banks.
+constexpr int SPAD = 2;
+
+template <class C, int RT, int B>
+struct SolveSmem {
+    C L[SNB][RT + SPAD];       // factor tile, [pivot q][row]
+    C Y[SNB][8 * B + SPAD];    // right operand, [pivot q][rhs]
+};
+
+// factor element M'(i, c) of the forward (L') or backward (U') factor:
+// F[i + c f] for M x = b, F[c + i f] for M^T x = b
+template <class C, bool TRANS>
+__device__ __forceinline__ C elem(const C *F, int f, int i, int c) {
+    return TRANS ? F[c + (size_t)i * f] : F[i + (size_t)c * f];
+}
+
+// The staging helpers below issue asynchronous copies (every load of the
+// tile in flight at once, no register round trip); the tile is complete
+// after staged_sync().
+//
+// sm.L[q][row] = M'(i0 + row, c0 + q) for row < rows, q < qb.  Entries
+// outside are left as they are: tile_mma reads only q < qb, and rows >= rows
+// (or right-hand sides >= rn) only feed accumulators that are never stored,
+// so partial tiles stage only what they use.
+// (the _p forms take the tile by pointer and the participating threads as
+// lt = 0 .. nt - 1; the SolveSmem forms are the CTA-wide ones)
+template <class C, bool TRANS, int RT, int KQ = SNB>
+__device__ __forceinline__ void stage_factor_p(C (*L)[RT + SPAD], const C *F, int f, int i0, int rows, int c0, int qb,
+                                               int lt, int nt) {
+    if (!TRANS) {
+        for (int t = lt; t < RT * qb; t += nt) {
+            const int row = t % RT, q = t / RT;
+            if (row < rows) cp_async_elem(&L[q][row], F + (i0 + row) + (size_t)(c0 + q) * f);
+        }
+    } else {
+        for (int t = lt; t < KQ * rows; t += nt) {
+            const int q = t % KQ, row = t / KQ;
+            if (q < qb) cp_async_elem(&L[q][row], F + (c0 + q) + (size_t)(i0 + row) * f);
+        }
+    }
+}
+template <class C, bool TRANS, int RT, int B>
+__device__ __forceinline__ void stage_factor(SolveSmem<C, RT, B> &sm, const C *F, int f, int i0, int rows, int c0, int qb) {
+    stage_factor_p<C, TRANS, RT>(sm.L, F, f, i0, rows, c0, qb, threadIdx.x, NT);
+}
+
+// L[q][p] = entry (p, q0 + q) of the inverse diagonal-block operator of
+// pivot block k0, p < rows, q < qb:
+//   FWD && !TRANS: L^-1        FWD && TRANS: (U^-1)^T
+//   !FWD && !TRANS: U^-1       !FWD && TRANS: (L^-1)^T
+// The stored block holds L^-1 strictly below the diagonal (unit diagonal
+// implied) and U^-1 on and above it.
+template <class C, bool FWD, bool TRANS, int RT, int KQ = SNB>
+__device__ __forceinline__ void stage_dinv_p(C (*L)[RT + SPAD], const C *F, int f, int k0, int rows, int q0, int qb,
+                                             int lt, int nt) {
+    constexpr int IN = TRANS ? KQ : SNB;   // the index along the stored columns runs fastest
+    for (int t = lt; t < IN * (TRANS ? rows : qb); t += nt) {
+        const int p = TRANS ? t / IN : t % IN, q = TRANS ? t % IN : t / IN;
+        if (TRANS ? q >= qb : p >= rows) continue;
+        const bool lower_src = FWD != TRANS;         // L^-1 (or its transpose) wanted
+        const int r = TRANS ? q0 + q : p, c = TRANS ? p : q0 + q;  // position in the stored block
+        const bool stored = lower_src ? r > c : r <= c;
+        if (stored) {
+            cp_async_elem(&L[q][p], F + (k0 + r) + (size_t)(k0 + c) * f);
+        } else {
+            using RR = decltype(L[0][0].x);
+            L[q][p] = (lower_src && r == c) ? mk(RR(1), RR(0)) : czero<C>();
+        }
+    }
+}
+template <class C, bool FWD, bool TRANS, int RT, int B>
+__device__ __forceinline__ void stage_dinv(SolveSmem<C, RT, B> &sm, const C *F, int f, int k0, int kb) {
+    stage_dinv_p<C, FWD, TRANS, RT>(sm.L, F, f, k0, kb, 0, kb, threadIdx.x, NT);
+}
+
+// Per-thread accumulators of an RT x 8B complex output tile (128 threads,
+// lt = 0 .. 127), in the layout of the tile product that fills them.
+template <class C, int RT, int B>
+struct TileAcc;
+
+// complex64: CUDA-core FMAs; thread (tr, tc) = (lt / 8, lt % 8) owns rows
+// tr + 16 i and columns tc + 8 j
+template <int RT, int B>
+struct TileAcc<float2, RT, B> {
+    static constexpr int NR = RT / 16, NC = B;
+    float2 v[NR][NC];
+    __device__ __forceinline__ static int row(int i, int lt) { return lt / 8 + 16 * i; }
+    __device__ __forceinline__ static int col(int j, int lt) { return lt % 8 + 8 * j; }
+};
+
+// complex128: FP64 matrix instructions (mma.sync m8n8k4 f64) on 8 x 8
+// blocks; warp w owns row blocks w + 4 i, lane l row 8 (w + 4 i) + l / 4 of
+// them and columns 8 c + 2 (l % 4) + {0, 1} of every column block c
+template <int RT, int B>
+struct TileAcc<double2, RT, B> {
+    static constexpr int NR = RT / 32, NC = 2 * B;
+    double2 v[NR][NC];
+    __device__ __forceinline__ static int row(int i, int lt) { return 8 * ((lt >> 5) + 4 * i) + ((lt & 31) >> 2); }
+    __device__ __forceinline__ static int col(int j, int lt) { return 8 * (j >> 1) + 2 * (lt & 3) + (j & 1); }
+};
+
+template <class C, int RT, int B>
+__device__ __forceinline__ void zero_acc(TileAcc<C, RT, B> &acc) {
+#pragma unroll
+    for (int i = 0; i < TileAcc<C, RT, B>::NR; ++i)
+#pragma unroll
+        for (int j = 0; j < TileAcc<C, RT, B>::NC; ++j) acc.v[i][j] = czero<C>();
+}
+
+// f(row, col, value) for the thread's accumulators with row < rows, col < rn
+template <class C, int RT, int B, class F>
+__device__ __forceinline__ void for_acc(TileAcc<C, RT, B> &acc, int rows, int rn, int lt, F f) {
+    using A = TileAcc<C, RT, B>;
+#pragma unroll
+    for (int i = 0; i < A::NR; ++i) {
+        const int row = A::row(i, lt);
+        if (row >= rows) continue;
+#pragma unroll
+        for (int j = 0; j < A::NC; ++j) {
+            const int col = A::col(j, lt);
+            if (col < rn) f(row, col, acc.v[i][j]);
+        }
+    }
+}
+
+// acc += L'[rows x qb] Y[qb x rn]: L[q][row] holds operator entry (row, q),
+// Y[q][col] the right operand.  Rows >= `rows` and columns >= rn of the
+// tile only feed accumulators that are never stored; row and column groups
+// that lie entirely outside are skipped warp-uniformly, so small fronts and
+// short slices do not pay for the full tile.  TRI: 0 a full operator;
+// TRI_LOWER / TRI_UPPER a triangular one (the diagonal-block inverses),
+// whose column q has no entries above / below row q: row groups that column
+// q does not reach are skipped for that q.
+constexpr int TRI_LOWER = 1, TRI_UPPER = 2;
+
+// complex64: each thread accumulates its 16-row-strided rows x 8-column-
+// strided columns with CUDA-core FMAs, one pivot q at a time
+template <int TRI, int RT, int B>
+__device__ __forceinline__ void tile_mma_p(const float2 (*L)[RT + SPAD], const float2 (*Y)[8 * B + SPAD], int qb,
+                                           TileAcc<float2, RT, B> &acc, int rows, int rn, int lt, int q0 = 0) {
+    constexpr int A = RT / 16;
+    const int tr = lt / 8, tc = lt % 8;
+    const int wrow = (lt >> 5) * 4;   // a warp owns rows 4w .. 4w + 3 of each 16-row group
+    const int na = rows <= wrow ? 0 : min(A, (rows - wrow + 15) / 16);
+    const int nb = min(B, (rn + 7) / 8);
+    if (na == 0) return;   // warp-uniform: this warp owns no row of the tile
+#pragma unroll 2
+    for (int q = 0; q < qb; ++q) {
+        const int alo = TRI == TRI_LOWER ? (q0 + q) / 16 : 0;       // rows >= q only
+        const int ahi = TRI == TRI_UPPER ? (q0 + q) / 16 : A - 1;   // rows <= q only
+        float2 l[A], y[B];
+#pragma unroll
+        for (int a = 0; a < A; ++a) l[a] = a < na && a >= alo && a <= ahi ? L[q][tr + 16 * a] : czero<float2>();
+#pragma unroll
+        for (int b = 0; b < B; ++b) y[b] = b < nb ? Y[q][tc + 8 * b] : czero<float2>();
+#pragma unroll
+        for (int a = 0; a < A; ++a) {
+            if (a >= na) break;
+            if (a < alo || a > ahi) continue;
+#pragma unroll
+            for (int b = 0; b < B; ++b)
+                if (b < nb) cfma(acc.v[a][b], l[a], y[b]);
+        }
+    }
+}
+
+// d = a b + d on one 8 x 8 x 4 FP64 block (warp-wide; a: this lane's entry
+// of the 8 x 4 row-major left block, b: of the 4 x 8 column-major right
+// block, d: this lane's two entries of the 8 x 8 result)
+__device__ __forceinline__ void dmma_884(double a, double b, double &d0, double &d1) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                 : "+d"(d0), "+d"(d1)
+                 : "d"(a), "d"(b));
+}
+
+// complex128: per 4 pivots and per 8 x 8 block, four FP64 matrix
+// instructions (Re += Ar Br - Ai Bi, Im += Ar Bi + Ai Br); a lane loads one
+// complex entry of each left and right fragment.  Pivots q >= qb enter as
+// zeros.
+template <int TRI, int RT, int B>
+__device__ __forceinline__ void tile_mma_p(const double2 (*L)[RT + SPAD], const double2 (*Y)[8 * B + SPAD], int qb,
+                                           TileAcc<double2, RT, B> &acc, int rows, int rn, int lt, int q0 = 0) {
+    constexpr int NRB = RT / 32;
+    const int w = lt >> 5, lane = lt & 31;
+    const int nb = min(B, (rn + 7) / 8);
+    for (int k0 = 0; k0 < qb; k0 += 4) {
+        const int kk = k0 + (lane & 3);
+        const bool kin = kk < qb;
+        double2 bf[B];
+#pragma unroll
+        for (int b = 0; b < B; ++b) bf[b] = kin && b < nb ? Y[kk][8 * b + (lane >> 2)] : czero<double2>();
+#pragma unroll
+        for (int i = 0; i < NRB; ++i) {
+            const int rb = w + 4 * i;   // row block: rows 8 rb .. 8 rb + 7
+            if (8 * rb >= rows) break;   // warp-uniform
+            if (TRI == TRI_UPPER && 8 * rb > q0 + k0 + 3) continue;   // rows <= q only
+            if (TRI == TRI_LOWER && 8 * rb + 7 < q0 + k0) continue;   // rows >= q only
+            const double2 af = kin ? L[kk][8 * rb + (lane >> 2)] : czero<double2>();
+#pragma unroll
+            for (int b = 0; b < B; ++b) {
+                if (b >= nb) break;
+                double2 &d0 = acc.v[i][2 * b], &d1 = acc.v[i][2 * b + 1];
+                dmma_884(af.x, bf[b].x, d0.x, d1.x);
+                dmma_884(-af.y, bf[b].y, d0.x, d1.x);
+                dmma_884(af.x, bf[b].y, d0.y, d1.y);
+                dmma_884(af.y, bf[b].x, d0.y, d1.y);
+            }
+        }
+    }
+}
+
+template <int TRI = 0, class C, int RT, int B>
+__device__ __forceinline__ void tile_mma(const SolveSmem<C, RT, B> &sm, int qb, TileAcc<C, RT, B> &acc, int rows,
+                                         int rn) {
+    tile_mma_p<TRI, RT, B>(sm.L, sm.Y, qb, acc, rows, rn, threadIdx.x);
+}
+
+// Y[q][r] = row_ptr(q)[r] for q < qb, r < rn (entries outside: as above)
+template <class C, int TC, class RowPtr>
+__device__ __forceinline__ void stage_rows_p(C (*Y)[TC + SPAD], RowPtr row_ptr, int qb, int rn, int lt, int nt) {
+    for (int t = lt; t < qb * TC; t += nt) {
+        const int q = t / TC, r = t % TC;
+        if (r < rn) cp_async_elem(&Y[q][r], row_ptr(q) + r);
+    }
+}
+template <class C, int RT, int B, class RowPtr>
+__device__ __forceinline__ void stage_rows(SolveSmem<C, RT, B> &sm, RowPtr row_ptr, int qb, int rn) {
+    stage_rows_p<C, 8 * B>(sm.Y, row_ptr, qb, rn, threadIdx.x, NT);
+}
+
+}  // namespace gm
