@@ -175,8 +175,10 @@ extern "C" int gm_engine_create(int device, const gm_config *cfg, gm_engine **ou
     std::vector<gm::NodeDesc> desc(s.nnodes);
     for (int t = 0; t < s.nnodes; ++t) {
         const int v = s.lvl_nodes[t];
-        desc[t] = gm::NodeDesc{s.front_off[v], s.var_off[v], s.inv_off[v], s.rhs_off[v], y_off[v],
-                               v, s.nfront[v], s.npiv[v], s.child0[v], s.child1[v], 0};
+        const auto cb = [&](int c) { return c < 0 ? 0 : s.front_off[c] + s.npiv[c] + (int64_t)s.npiv[c] * s.nfront[c]; };
+        const int c0 = s.child0[v], c1 = s.child1[v];
+        desc[t] = gm::NodeDesc{s.front_off[v], s.var_off[v], s.inv_off[v], s.rhs_off[v], y_off[v], cb(c0), cb(c1),
+                               v, s.nfront[v], s.npiv[v], c0, c1, c0 < 0 ? 0 : s.nfront[c0], c1 < 0 ? 0 : s.nfront[c1], 0};
     }
     int rc2;
     if ((rc2 = upload(e->d_desc, desc, e->st))) return rc2;
@@ -347,9 +349,16 @@ static int build_cb_plan(gm_engine *e) {
             max_cb = std::max(max_cb, s.nfront[v] - s.npiv[v]);
         }
         const int backend = (c64 && max_cb >= kTcMinBlock) ? 1 : 0;
-        const int tr = backend ? cgemm_tile_rows() : kGemmTileCC, tc = backend ? cgemm_tile_cols() : kGemmTileCC;
+        int64_t n64 = 0;   // 64 x 64 tiles of the level
+        for (int t = L.first; t < L.first + L.count; ++t) {
+            const int64_t nt = (s.nfront[s.lvl_nodes[t]] - s.npiv[s.lvl_nodes[t]] + kGemmTileCC - 1) / kGemmTileCC;
+            n64 += e->nf * nt * nt;
+        }
+        const int tile = n64 < kGemmTileFill ? 32 : kGemmTileCC;
+        const int tr = backend ? cgemm_tile_rows() : tile, tc = backend ? cgemm_tile_cols() : tile;
         auto &pl = e->cb_plan[h];
         pl.backend = backend;
+        pl.tile = tile;
         pl.prob_off = (int64_t)probs.size();
         pl.tile_off = (int64_t)tiles.size();
         if (small_factor_level<R>(L) || use_mid_factor<R>(L)) {   // fused kernels form the Schur complement themselves
@@ -425,7 +434,7 @@ static int factor_batch(gm_engine *e, double pivscale) {
                     launch_cgemm_sub(1, reinterpret_cast<const CgemmProb *>(probs + pl.prob_off), tiles + pl.tile_off,
                                      pl.ntiles, e->d_tcerr.as<int>(), e->st);
                 else
-                    launch_gemm_sub_cc<R>(probs + pl.prob_off, tiles + pl.tile_off, pl.ntiles, e->st);
+                    launch_gemm_sub_cc<R>(probs + pl.prob_off, tiles + pl.tile_off, pl.ntiles, pl.tile, e->st);
             }
             if (e->levels[h].max_piv > 32) {   // beside the levels above (the last level's: nothing is)
                 cudaEventRecord(e->ev_fork, e->st);

@@ -80,7 +80,7 @@ struct gm_engine {
 
     // contribution-block GEMM plan per level (rebuilt when the front
     // storage moves or the batch size changes)
-    struct CbPlan { int backend; int64_t prob_off, tile_off; int ntiles; };
+    struct CbPlan { int backend; int64_t prob_off, tile_off; int ntiles, tile; };
     std::vector<CbPlan> cb_plan;
     gm::DevBuf d_cb_probs, d_cb_tiles, d_tcerr;
     const void *cb_plan_base = nullptr;

@@ -6,8 +6,8 @@
 // (one block per node per frequency).  A level is processed by
 //   K2 gather   -- each front pulls its children's contribution blocks
 //                  (extend-add by inverse maps: deterministic, no atomics),
-//   K2 scatter  -- adds the operator entries owned by the front,
-//   K3 diag     -- per NB-wide pivot block: LU of the diagonal block with
+//   K3 diag     -- adds the operator entries owned by the front (first block),
+//                  then per NB-wide pivot block: LU of the diagonal block with
 //                  threshold partial pivoting inside the block (static
 //                  pivots as the last resort) and the inverses of its two
 //                  triangles, factored once per front (the first block by
@@ -16,7 +16,7 @@
 //   K3 panels   -- L21 = A21 U11^-1 and U12 = L11^-1 P A12 as products with
 //                  those inverses (FP64 matrix instructions in complex128),
 //   K4 update   -- rank-NB Schur update of the pivot rows and columns still
-//                  to come, 64x64 tiles.
+//                  to come, 64x64 or 32x32 tiles.
 // K3/K4 alternate ceil(max_piv/NB) times per level.  After the last step a
 // front holds L (unit lower) and U in its first npiv rows/columns -- except
 // that each NB x NB diagonal block holds the INVERSES of its two triangles
@@ -34,7 +34,9 @@
 //                   and applies the Schur update to the contribution block
 //                   once, in place of K3 / K4 and the contribution GEMM.
 // The remaining (upper) levels take the blocked K2-K4 sequence.
+#include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 #include "kernels.cuh"
 #include "cplx.cuh"
 #include "async_copy.cuh"
@@ -42,44 +44,46 @@
 namespace gm {
 
 constexpr int NB = 32;       // pivot block width
-constexpr int TILE = 64;     // Schur-update tile
+constexpr int TILE = 64;     // panel and Schur-update tile
+constexpr int kTileFill = kGemmTileFill;
 
 constexpr int GATHER_COLS = 4;   // front columns per CTA of the extend-add gather
 constexpr int TSTR = TILE + 2;   // padded row stride of staged 64-wide tiles (conflict-free 8 x 4 fragments)
 
-// 64 x 64 complex output tile of a 256-thread CTA, in the layout of the
-// product that fills it: complex64 with CUDA-core FMAs, thread t owning
+// TL x TL complex output tile (TL 64 or 32) of a 256-thread CTA, in the layout
+// of the product that fills it: complex64 with CUDA-core FMAs, thread t owning
 // rows t % 16 + 16 i and columns t / 16 + 16 j (v[i][j]); complex128 on FP64
-// matrix instructions (mma.sync m8n8k4 f64) on 8 x 8 blocks, warp w owning
-// row blocks w % 4 and w % 4 + 4 of column blocks 4 (w / 4) .. 4 (w / 4) + 3
-// (so a tile with few rows still keeps six of the eight warps busy), lane l
-// row 8 rb + l / 4 and columns 8 cb + 2 (l % 4) + j of each owned block;
-// v[4 rbi + cbi][j] for row block w % 4 + 4 rbi, column block 4 (w / 4) + cbi.
-template <class C, bool MMA>
-struct Tile64;
-template <class C>
-struct Tile64<C, false> {   // CUDA-core FMAs (complex64, or complex128 where short K suits them better)
-    static constexpr int NI = 4, NJ = 4;
+// matrix instructions (mma.sync m8n8k4 f64) on 8 x 8 blocks, lane l holding
+// row 8 rb + l / 4 and columns 8 cb + 2 (l % 4) + j of each block its warp w
+// owns: for TL = 64 row blocks w % 4 and w % 4 + 4 of column blocks 4 (w / 4)
+// .. 4 (w / 4) + 3 (v[4 rbi + cbi], so a tile with few rows still keeps six of
+// the eight warps busy), for TL = 32 row block w % 4 of column blocks
+// 2 (w / 4) and 2 (w / 4) + 1 (v[cbi]).
+template <class C, bool MMA, int TL>
+struct TileCC;
+template <class C, int TL>
+struct TileCC<C, false, TL> {   // CUDA-core FMAs (complex64, or complex128 where short K suits them better)
+    static constexpr int NI = TL / 16, NJ = TL / 16;
     C v[NI][NJ];
     __device__ __forceinline__ static int row(int i, int, int t) { return t % 16 + 16 * i; }
     __device__ __forceinline__ static int col(int, int j, int t) { return t / 16 + 16 * j; }
 };
-template <>
-struct Tile64<double2, true> {   // FP64 matrix instructions
-    static constexpr int NI = 8, NJ = 2;
+template <int TL>
+struct TileCC<double2, true, TL> {   // FP64 matrix instructions
+    static constexpr int NRB = TL / 32, NCB = TL / 16, NI = NRB * NCB, NJ = 2;
     double2 v[NI][NJ];
     __device__ __forceinline__ static int row(int i, int, int t) {
-        return 8 * ((t >> 5) % 4 + 4 * (i / 4)) + ((t & 31) >> 2);
+        return 8 * ((t >> 5) % 4 + 4 * (i / NCB)) + ((t & 31) >> 2);
     }
     __device__ __forceinline__ static int col(int i, int j, int t) {
-        return 8 * (4 * ((t >> 5) / 4) + i % 4) + 2 * (t & 3) + j;
+        return 8 * (NCB * ((t >> 5) / 4) + i % NCB) + 2 * (t & 3) + j;
     }
 };
 
 // f(row, col, value) over the thread's entries of the tile
-template <class C, bool MMA, class F>
-__device__ __forceinline__ void for_tile64(Tile64<C, MMA> &acc, int t, F f) {
-    using T = Tile64<C, MMA>;
+template <class C, bool MMA, int TL, class F>
+__device__ __forceinline__ void for_tile(TileCC<C, MMA, TL> &acc, int t, F f) {
+    using T = TileCC<C, MMA, TL>;
 #pragma unroll
     for (int i = 0; i < T::NI; ++i)
 #pragma unroll
@@ -89,22 +93,23 @@ __device__ __forceinline__ void for_tile64(Tile64<C, MMA> &acc, int t, F f) {
 // acc += A B (NEG: acc -= A B) over k < kb, A(r, k) = As[k * ak + r * ar]
 // for rows r < mrows, B(k, c) = Bs[k * bk + c * bc] for columns c < ncols
 // (entries outside read as zero)
-template <bool NEG, class C>
-__device__ __forceinline__ void mma64(const C *As, int ak, int ar, const C *Bs, int bk, int bc, int kb, int mrows,
-                                      int ncols, Tile64<C, false> &acc, int t) {
+template <bool NEG, class C, int TL>
+__device__ __forceinline__ void mma_tile(const C *As, int ak, int ar, const C *Bs, int bk, int bc, int kb, int mrows,
+                                         int ncols, TileCC<C, false, TL> &acc, int t) {
+    constexpr int NT = TL / 16;
     const int tx = t % 16, ty = t / 16;
     for (int k = 0; k < kb; ++k) {
-        C lv[4], uv[4];
+        C lv[NT], uv[NT];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < NT; ++i)
             lv[i] = tx + 16 * i < mrows ? As[(size_t)k * ak + (size_t)(tx + 16 * i) * ar] : czero<C>();
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < NT; ++j)
             uv[j] = ty + 16 * j < ncols ? Bs[(size_t)k * bk + (size_t)(ty + 16 * j) * bc] : czero<C>();
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < NT; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < NT; ++j) {
                 if (NEG) cfms(acc.v[i][j], lv[i], uv[j]);
                 else cfma(acc.v[i][j], lv[i], uv[j]);
             }
@@ -117,36 +122,41 @@ __device__ __forceinline__ void dmma_884(double a, double b, double &d0, double 
                  : "d"(a), "d"(b));
 }
 
-template <bool NEG>
-__device__ __forceinline__ void mma64(const double2 *As, int ak, int ar, const double2 *Bs, int bk, int bc, int kb,
-                                      int mrows, int ncols, Tile64<double2, true> &acc, int t) {
+// one complex 8 x 8 x 4 block
+__device__ __forceinline__ void cmma_884(const double2 &a, const double2 &b, double2 &d0, double2 &d1) {
+    dmma_884(a.x, b.x, d0.x, d1.x);    // Re += Ar Br
+    dmma_884(-a.y, b.y, d0.x, d1.x);   //     - Ai Bi
+    dmma_884(a.x, b.y, d0.y, d1.y);    // Im += Ar Bi
+    dmma_884(a.y, b.x, d0.y, d1.y);    //     + Ai Br
+}
+
+template <bool NEG, int TL>
+__device__ __forceinline__ void mma_tile(const double2 *As, int ak, int ar, const double2 *Bs, int bk, int bc, int kb,
+                                         int mrows, int ncols, TileCC<double2, true, TL> &acc, int t) {
+    using T = TileCC<double2, true, TL>;
     const int w = t >> 5, lane = t & 31, g = lane >> 2;
-    const int rb0 = w % 4, cb0 = 4 * (w / 4);
+    const int rb0 = w % 4, cb0 = T::NCB * (w / 4);
     if (8 * rb0 >= mrows || 8 * cb0 >= ncols) return;   // warp-uniform: none of this warp's blocks is used
     for (int k0 = 0; k0 < kb; k0 += 4) {
         const int kk = k0 + (lane & 3);
         const bool kin = kk < kb;
-        double2 bf[4];
+        double2 bf[T::NCB];
 #pragma unroll
-        for (int ci = 0; ci < 4; ++ci) {
+        for (int ci = 0; ci < T::NCB; ++ci) {
             const int c = 8 * (cb0 + ci) + g;
             bf[ci] = kin && c < ncols ? Bs[(size_t)kk * bk + (size_t)c * bc] : czero<double2>();
         }
 #pragma unroll
-        for (int ri = 0; ri < 2; ++ri) {
+        for (int ri = 0; ri < T::NRB; ++ri) {
             const int rb = rb0 + 4 * ri;
             if (8 * rb >= mrows) break;   // warp-uniform
             const int r = 8 * rb + g;
             double2 af = kin && r < mrows ? As[(size_t)kk * ak + (size_t)r * ar] : czero<double2>();
             if (NEG) af = make_double2(-af.x, -af.y);
 #pragma unroll
-            for (int ci = 0; ci < 4; ++ci) {
+            for (int ci = 0; ci < T::NCB; ++ci) {
                 if (8 * (cb0 + ci) >= ncols) break;   // warp-uniform
-                double2 &d0 = acc.v[4 * ri + ci][0], &d1 = acc.v[4 * ri + ci][1];
-                dmma_884(af.x, bf[ci].x, d0.x, d1.x);    // Re += Ar Br
-                dmma_884(-af.y, bf[ci].y, d0.x, d1.x);   //     - Ai Bi
-                dmma_884(af.x, bf[ci].y, d0.y, d1.y);    // Im += Ar Bi
-                dmma_884(af.y, bf[ci].x, d0.y, d1.y);    //     + Ai Br
+                cmma_884(af, bf[ci], acc.v[T::NCB * ri + ci][0], acc.v[T::NCB * ri + ci][1]);
             }
         }
     }
@@ -155,26 +165,17 @@ __device__ __forceinline__ void mma64(const double2 *As, int ak, int ar, const d
 template <class R>
 __global__ void k_front_gather(FactorArgs<R> a, int lvl_first) {
     using C = cplx<R>;
-    const int node = a.s.lvl_nodes[lvl_first + blockIdx.y];
-    const int f = a.s.nfront[node];
+    const NodeDesc d = a.s.desc[lvl_first + blockIdx.y];
+    const int f = d.nfront;
     const int j = blockIdx.x * GATHER_COLS + (threadIdx.x >> 5);   // one warp per front column
     if (j >= f) return;   // warp-uniform (no barrier below)
     C *base = reinterpret_cast<C *>(a.front) + (size_t)blockIdx.z * a.s.front_total;
-    C *F = base + a.s.front_off[node];
-    const int *inv = a.s.inv + a.s.inv_off[node];
-    const int c0 = a.s.child0[node], c1 = a.s.child1[node];
-    const int b0 = c0 >= 0 ? inv[j] : -1;
-    const int b1 = c1 >= 0 ? inv[f + j] : -1;
-    const C *cb0 = nullptr, *cb1 = nullptr;
-    int f0 = 0, f1 = 0;
-    if (b0 >= 0) {
-        const int s0 = a.s.npiv[c0]; f0 = a.s.nfront[c0];
-        cb0 = base + a.s.front_off[c0] + s0 + (size_t)(s0 + b0) * f0;
-    }
-    if (b1 >= 0) {
-        const int s1 = a.s.npiv[c1]; f1 = a.s.nfront[c1];
-        cb1 = base + a.s.front_off[c1] + s1 + (size_t)(s1 + b1) * f1;
-    }
+    C *F = base + d.front_off;
+    const int *inv = a.s.inv + d.inv_off;
+    const int b0 = d.child0 >= 0 ? inv[j] : -1;
+    const int b1 = d.child1 >= 0 ? inv[f + j] : -1;
+    const C *cb0 = b0 >= 0 ? base + d.cb0 + (size_t)b0 * d.ld0 : nullptr;
+    const C *cb1 = b1 >= 0 ? base + d.cb1 + (size_t)b1 * d.ld1 : nullptr;
     for (int i = threadIdx.x & 31; i < f; i += 32) {
         C v = czero<C>();
         if (cb0) { const int r = inv[i]; if (r >= 0) v = cadd(v, cb0[r]); }
@@ -183,15 +184,18 @@ __global__ void k_front_gather(FactorArgs<R> a, int lvl_first) {
     }
 }
 
+// the operator entries owned by the front at level position pos, added into
+// it by one CTA (positions are distinct)
 template <class R>
-__global__ void k_entry_scatter(FactorArgs<R> a, int64_t e0, int64_t cnt) {
+__device__ __forceinline__ void add_entries(const FactorArgs<R> &a, int pos, int z) {
     using C = cplx<R>;
-    const int64_t e = e0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= e0 + cnt) return;
-    C *F = reinterpret_cast<C *>(a.front) + (size_t)blockIdx.y * a.s.front_total;
-    const double2 v = a.A[(size_t)blockIdx.y * 9 * a.s.n + a.ent_src[e]];
-    C &d = F[a.ent_dst[e]];
-    d = cadd(d, cconv<C>(v));
+    C *F = reinterpret_cast<C *>(a.front) + (size_t)z * a.s.front_total;
+    const double2 *A = a.A + (size_t)z * 9 * a.s.n;
+    const int64_t e1 = a.ent_lvl_off[pos + 1];
+    for (int64_t e = a.ent_lvl_off[pos] + threadIdx.x; e < e1; e += blockDim.x) {
+        C &d = F[a.ent_dst[e]];
+        d = cadd(d, cconv<C>(A[a.ent_src[e]]));
+    }
 }
 
 // Static pivoting: a pivot of magnitude below pivtol (or NaN) is replaced by
@@ -216,170 +220,263 @@ __device__ __forceinline__ cplx<R> static_pivot(cplx<R> piv, R pivtol, int &nper
 
 // LU of the kb x kb diagonal block at (k0, k0) of the front F (leading
 // dimension f), with threshold row exchanges inside the block or without
-// (below), a pivot that stays tiny replaced as static_pivot does; the
-// inverses of its two triangles are written back in its place (all that
-// the panel products and the substitution use): L^-1 in the strict lower
-// part (unit diagonal implied), U^-1 in the upper part with the diagonal.
+// (PIV), a pivot that stays tiny replaced as static_pivot does; the inverses
+// of its two triangles are written back in its place (all that the panel
+// products and the substitution use): L^-1 in the strict lower part (unit
+// diagonal implied), U^-1 in the upper part with the diagonal.
 //
-// The inverses are built during the elimination, one rank-1 step per pivot
-// p over every entry outside the leading (p+1) x (p+1) block, with l = the
-// scaled column p of L and u = row p of U over the pivot:
-//   trailing   D(r, c) -= l_r D(p, c)             r, c > p
-//   L^-1       X(r, c) -= l_r X(p, c)             r > p >= c   (X = I initially)
-//   unit U^-1  Z(r, c) -= Z(r, p) D(p, c) / piv   r <= p < c   (Z = I initially)
-// (X = L_p^-1 ... L_0^-1 and Z = M_0^-1 ... M_p^-1 for the elementary
-// factors L = L_0 L_1 ... and unit U = ... M_1 M_0), and U^-1 = Z diag(1/piv).
-// All three are T(r, c) -= (a_r / piv) b_c with a = column p and b = row p
-// of D where they lie beyond p, of X / Z otherwise; X and Z share one array
-// (strict lower / upper part).  The regions are disjoint and read only row
-// and column p, so one barrier per pivot suffices.  Each thread owns the
-// entries (t % NB, t / NB + 8 k), k < 4 (256 threads), updated without
-// branches.  (With three barriers per pivot and the inverses as column
-// recurrences afterwards the block took about twice as long; the chain is
-// the serial part of every pivot step of the upper levels.)
+// Both inverses are built during the elimination, in place, by 8-pivot
+// panels q.  With the panel's own triangles L_q, U_q, the block rows / columns
+// it meets change as
+//   row q     X_qc := L_q^-1 X_qc (c < q),   U_qc = L_q^-1 D_qc,  Z_qc := -U_q^-1 U_qc (c > q)
+//   column q  Z_rq := Z_rq U_q^-1 (r < q),   L_rq = D_rq U_q^-1,  X_rq := -L_rq L_q^-1 (r > q)
+//   others    T_rc -= a_r b_c with a = Z_rq or L_rq, b = X_qc or U_qc, except r < q and c < q
+// (X the finished part of L^-1 below, Z that of U^-1 above the diagonal; one
+// array holds D, X and Z).  Per panel:
+//   1. warp 0 factors it with a row per lane and its 8 columns in registers:
+//      the pivot row goes round by shuffles, so a pivot costs no block
+//      barrier, and its reciprocal is formed while the search (one warp
+//      reduction) is still out;
+//   2. warp 0 solves with L_q for the 24 other columns and the identity (b),
+//      warp 1 with U_q for the 24 other rows and the identity (a), a column /
+//      row per lane;
+//   3. all warps form the 16 products a_r b_c on 8 x 8 blocks.
+// Row exchanges: position p goes to the row of largest |D(r, p)| among those
+// left (by the leading 32 bits of |D|^2) when the row there has |D(p, p)|^2 <
+// pivtau2 |D(r, p)|^2; whole rows of the array trade places (a few per front).
+// The block's permutation goes to pivsrc[vars[k0 + q]] (q: pivot position,
+// value: block row in equation order); columns right of the block are
+// exchanged when the U panel is staged, columns left of it (earlier blocks'
+// multipliers) stay in equation order -- the forward substitution gathers the
+// block's rows at the same point of the elimination.
 //
-// Without row exchanges (PIV false) thread 0 forms the next pivot from row
-// and column p before the step and publishes its reciprocal.  With them,
-// warp 0 picks pivot p after step p - 1 (a second barrier): the row r >= p
-// of largest |D(r, p)| is exchanged with row p when |D(p, p)|^2 <
-// pivtau2 |D(r, p)|^2 -- the whole row of D (its multipliers included) and
-// the finished part of X (columns < p: X' = P X P for the exchange P);
-// Z only holds finished rows < p.  The block's permutation goes to
-// pivsrc[vars[k0 + q]] (q: pivot position, value: block row in equation
-// order); columns right of the block are exchanged when the U panel is
-// staged, columns left of it (earlier blocks' multipliers) stay in equation
-// order -- the forward substitution gathers the block's rows at the same
-// point of the elimination.  The CTA has DIAG_THREADS threads; sm is shared
-// scratch of DIAG_SCRATCH complex values.
-constexpr int DIAG_SCRATCH = 2 * NB * (NB + 1) + NB;
+// The block is the serial part of every pivot step of the upper levels.
+// Pivot by pivot over all 256 threads (two barriers and ~155 dependent
+// instructions each) k_diag took 31 us for 32 complex128 pivots alone on an
+// SM; so it takes 21 us (24.5k cycles after the loads: four panels of 4250,
+// the triangle solves 520 each, the products 1400 each), and an update launch
+// of a top level, which ends in one, 22.5 us instead of 48.  The CTA has DIAG_THREADS threads; sm is shared scratch of
+// DIAG_SCRATCH complex values.
+constexpr int PW8 = 8;       // panel width
+constexpr int DSTR = NB + 1;
+constexpr int ASTR = PW8 + 4, BSTR = NB + 2;   // strides of conflict-free 8 x 4 / 4 x 8 fragments
+constexpr int DIAG_SCRATCH = NB * DSTR + NB * ASTR + PW8 * BSTR + NB;
 constexpr int DIAG_THREADS = 256;
+
+// leading bits of a non-negative value: ordered as the value is
+__device__ __forceinline__ int lead_bits(double v) { return __double2hiint(v); }
+__device__ __forceinline__ int lead_bits(float v) { return __float_as_int(v); }
+__device__ __forceinline__ double from_lead(int b, double) { return __hiloint2double(b, 0); }
+__device__ __forceinline__ float from_lead(int b, float) { return __int_as_float(b); }
+
+// acc (this lane's two entries of an 8 x 8 block: row l / 4, columns
+// 2 (l % 4) + {0, 1}) -= A B, A(r, j) = Ab[r * sa + j], B(j, c) = Bb[j * sb + c], j < 8
+__device__ __forceinline__ void block8_sub(const double2 *Ab, int sa, const double2 *Bb, int sb, double2 *acc, int lane) {
+    const int g = lane >> 2, kq = lane & 3;
+#pragma unroll
+    for (int j = 0; j < PW8; j += 4) {
+        const double2 v = Ab[g * sa + j + kq];
+        cmma_884(make_double2(-v.x, -v.y), Bb[(j + kq) * sb + g], acc[0], acc[1]);
+    }
+}
+__device__ __forceinline__ void block8_sub(const float2 *Ab, int sa, const float2 *Bb, int sb, float2 *acc, int lane) {
+    const int g = lane >> 2, kq = lane & 3;
+#pragma unroll
+    for (int j = 0; j < PW8; ++j) {
+        const float2 v = Ab[g * sa + j];
+        cfms(acc[0], v, Bb[j * sb + 2 * kq]);
+        cfms(acc[1], v, Bb[j * sb + 2 * kq + 1]);
+    }
+}
 
 template <class R, bool PIV>
 __device__ void factor_diag_block(const FactorArgs<R> &a, cplx<R> *F, int f, int k0, int kb, cplx<R> *sm,
                                   unsigned char *src, const int *vars) {
     using C = cplx<R>;
-    constexpr int NE = NB * NB / DIAG_THREADS;   // entries per thread
-    auto D = reinterpret_cast<C (*)[NB + 1]>(sm);
-    auto W = reinterpret_cast<C (*)[NB + 1]>(sm + NB * (NB + 1));   // X (strict lower) and Z (upper)
-    C *rdiag = sm + 2 * NB * (NB + 1);
-    __shared__ int rowof[NB];   // PIV: block row (equation order) at pivot position q
+    constexpr unsigned ALL = 0xffffffffu;
+    C *T = sm;                                // [NB][DSTR]
+    C *Ab = T + NB * DSTR;                    // [NB][ASTR]
+    C *Bb = Ab + NB * ASTR;                   // [PW8][BSTR]
+    C *rd = Bb + PW8 * BSTR;                  // [NB] reciprocal pivots
+    __shared__ int rowat[NB];                 // block row (equation order) at pivot position q
     const R pivtol = (R)(a.pivscale * __longlong_as_double((long long)*a.amax));
-    int np = 0, nsw = 0;   // pivots this thread perturbed / exchanged
-    const int r = threadIdx.x % NB, cb = threadIdx.x / NB;
-    if (PIV && threadIdx.x < NB) rowof[threadIdx.x] = threadIdx.x;
-#pragma unroll
-    for (int e = 0; e < NE; ++e) {
-        const int c = cb + (DIAG_THREADS / NB) * e;
-        if (r < kb && c < kb) {
-            C v = F[(k0 + r) + (size_t)(k0 + c) * f];
-            if (!PIV && r == 0 && c == 0) {
-                v = static_pivot<R>(v, pivtol, np);
-                rdiag[0] = crcp(v);
-            }
-            D[r][c] = v;
-            W[r][c] = r == c ? mk(R(1), R(0)) : czero<C>();
-        }
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid < NB) {
+        rowat[tid] = tid;
+        rd[tid] = czero<C>();
+    }
+    for (int t = tid; t < NB * NB; t += DIAG_THREADS) {   // rows and columns beyond kb: zero throughout
+        const int r = t % NB, c = t / NB;
+        T[r * DSTR + c] = r < kb && c < kb ? F[(k0 + r) + (size_t)(k0 + c) * f] : czero<C>();
     }
     __syncthreads();
-    for (int p = 0; p < kb; ++p) {
-        if (PIV) {
-            if (threadIdx.x < 32) {   // warp 0: pivot p
-                const int lane = threadIdx.x;
-                R m2 = lane >= p && lane < kb ? cabs2(D[lane][p]) : R(-1);
-                int arg = lane;
+    int np = 0, nsw = 0;      // pivots perturbed / exchanged (warp 0: the same in every lane)
+#pragma unroll 1
+    for (int q = 0; q * PW8 < kb; ++q) {
+        const int p0 = q * PW8, pw = min(PW8, kb - p0);
+        C *Tq = T + p0 * DSTR + p0;   // the panel's own 8 x 8 block
+        if (warp == 0) {   // 1. the panel: x[i] = this row's entry in column p + i
+            C x[PW8];
+            C *own = T + lane * DSTR;
 #pragma unroll
-                for (int o = 16; o; o >>= 1) {
-                    const R om = __shfl_xor_sync(0xffffffffu, m2, o);
-                    const int oa = __shfl_xor_sync(0xffffffffu, arg, o);
-                    if (om > m2 || (om == m2 && oa < arg)) {
-                        m2 = om;
-                        arg = oa;
-                    }
-                }
-                m2 = __shfl_sync(0xffffffffu, m2, 0);   // lane 0's result for all (NaN entries
-                arg = __shfl_sync(0xffffffffu, arg, 0);  // could leave the lanes disagreeing)
-                const bool swap = arg != p && cabs2(D[p][p]) < (R)a.pivtau2 * m2;   // warp-uniform
-                if (swap) {
-                    if (lane < kb) {
-                        const C t = D[p][lane];
-                        D[p][lane] = D[arg][lane];
-                        D[arg][lane] = t;
-                        if (lane < p) {
-                            const C u = W[p][lane];
-                            W[p][lane] = W[arg][lane];
-                            W[arg][lane] = u;
+            for (int i = 0; i < PW8; ++i) x[i] = own[p0 + i];
+            // pivots j0 .. j1 - 1 of the panel, W of its columns still live (no
+            // divergent branch: each costs the chain)
+            auto pivots = [&](auto width, int j0, int j1) {
+                constexpr int W = decltype(width)::value;
+#pragma unroll 1
+                for (int j = j0; j < j1; ++j) {
+                    const int p = p0 + j;
+                    C pr[W];   // the pivot row
+#pragma unroll
+                    for (int i = 0; i < W; ++i) pr[i] = mk(__shfl_sync(ALL, x[i].x, p), __shfl_sync(ALL, x[i].y, p));
+                    C rp = crcp(pr[0]);
+                    if (PIV) {
+                        const R m2 = cabs2(x[0]);
+                        const int key = lane >= p && lane < kb ? lead_bits(m2) : -1;
+                        const int top = __reduce_max_sync(ALL, key);
+                        if (cabs2(pr[0]) < (R)a.pivtau2 * from_lead(top, R(0))) {   // warp-uniform
+                            const int arg = __ffs(__ballot_sync(ALL, key == top)) - 1;
+                            if (arg > p) {   // rows p and arg trade places
+                                const int from = lane == p ? arg : lane == arg ? p : lane;
+#pragma unroll
+                                for (int i = 0; i < W; ++i) {
+                                    pr[i] = mk(__shfl_sync(ALL, x[i].x, arg), __shfl_sync(ALL, x[i].y, arg));
+                                    x[i] = mk(__shfl_sync(ALL, x[i].x, from), __shfl_sync(ALL, x[i].y, from));
+                                }
+                                const C u = T[p * DSTR + lane], v = T[arg * DSTR + lane];
+                                T[p * DSTR + lane] = v;
+                                T[arg * DSTR + lane] = u;
+                                if (lane == 0) {
+                                    const int t = rowat[p];
+                                    rowat[p] = rowat[arg];
+                                    rowat[arg] = t;
+                                }
+                                __syncwarp();
+                                rp = crcp(pr[0]);
+                                ++nsw;
+                            }
                         }
                     }
-                    if (lane == 0) {
-                        const int t = rowof[p];
-                        rowof[p] = rowof[arg];
-                        rowof[arg] = t;
-                        ++nsw;
+                    C piv = pr[0];
+                    if (!(cabs2(piv) >= pivtol * pivtol) || !(pivtol > R(0))) {   // rare, off the chain: rp is formed already
+                        piv = static_pivot<R>(piv, pivtol, np);
+                        rp = crcp(piv);
                     }
-                    __syncwarp();
-                }
-                if (lane == 0) rdiag[p] = crcp(static_pivot<R>(D[p][p], pivtol, np));
-            }
-            __syncthreads();
-            if (p + 1 == kb) break;
-        } else if (p + 1 == kb) {
-            break;
-        }
-        const C rp = rdiag[p];
-        if (!PIV && threadIdx.x == 0) {
-            C v = D[p + 1][p + 1];
-            cfms(v, cmul(D[p + 1][p], rp), D[p][p + 1]);
-            v = static_pivot<R>(v, pivtol, np);
-            rdiag[p + 1] = crcp(v);
-        }
+                    const C l = lane > p ? cmul(x[0], rp) : czero<C>();   // rows p and above are final
+                    own[p] = lane > p ? l : lane == p ? piv : x[0];
+                    if (lane == p) rd[p] = rp;
 #pragma unroll
-        for (int e = 0; e < NE; ++e) {
-            const int c = cb + (DIAG_THREADS / NB) * e;
-            if (r < kb && c < kb && (r > p || c > p) && (PIV || !(r == p + 1 && c == p + 1))) {
-                const C av = r > p ? D[r][p] : W[r][p];
-                const C bv = c > p ? D[p][c] : W[p][c];
-                C &T = (r > p && c > p) ? D[r][c] : W[r][c];
-                C v = T;
-                cfms(v, cmul(av, rp), bv);
-                T = v;
+                    for (int i = 1; i < W; ++i) {
+                        C v = x[i];
+                        cfms(v, l, pr[i]);
+                        x[i - 1] = v;
+                    }
+                    x[W - 1] = czero<C>();
+                }
+            };
+            pivots(std::integral_constant<int, PW8>(), 0, min(pw, PW8 / 2));
+            pivots(std::integral_constant<int, PW8 / 2>(), PW8 / 2, pw);
+        }
+        __syncthreads();
+        // 2. the panel's triangles applied to its rows and columns (rows and
+        // columns beyond kb hold zeros: no cases for a short last panel)
+        const int ql = lane - p0;   // 0 .. 7: this lane takes a column / row of the identity
+        const bool mid = ql >= 0 && ql < PW8;
+        if (warp == 0) {   // b: columns `lane` of the panel's rows
+            C v[PW8];
+#pragma unroll
+            for (int j = 0; j < PW8; ++j)
+                v[j] = mid ? mk(R(j == ql && j < pw), R(0)) : T[(p0 + j) * DSTR + lane];
+#pragma unroll
+            for (int i = 0; i + 1 < PW8; ++i)
+#pragma unroll
+                for (int j = i + 1; j < PW8; ++j) cfms(v[j], Tq[j * DSTR + i], v[i]);
+#pragma unroll
+            for (int j = 0; j < PW8; ++j) Bb[j * BSTR + lane] = v[j];
+        } else if (warp == 1) {   // a: rows `lane` of the panel's columns
+            C v[PW8];
+#pragma unroll
+            for (int j = 0; j < PW8; ++j)
+                v[j] = mid ? mk(R(j == ql && j < pw), R(0)) : T[lane * DSTR + p0 + j];
+            if (ql < PW8) {   // (rows below hold their multipliers already)
+#pragma unroll
+                for (int i = 0; i < PW8; ++i) {
+                    v[i] = cmul(v[i], rd[p0 + i]);
+#pragma unroll
+                    for (int j = i + 1; j < PW8; ++j) cfms(v[j], v[i], Tq[i * DSTR + j]);
+                }
             }
+#pragma unroll
+            for (int j = 0; j < PW8; ++j) Ab[lane * ASTR + j] = v[j];
+        }
+        __syncthreads();
+        // 3. 8 x 8 blocks (bi, bj) of the array, two per warp
+        const int g = lane >> 2, kq = lane & 3;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int bi = warp & 3, bj = (warp >> 2) + 2 * e;
+            if (bi < q && bj < q) continue;
+            C *d = T + (8 * bi + g) * DSTR + 8 * bj + 2 * kq;
+            const C *ar = Ab + (8 * bi + g) * ASTR + 2 * kq, *bc = Bb + g * BSTR + 8 * bj + 2 * kq;
+            C v[2];
+            if (bi == q && bj == q) {   // L_q^-1 below, U_q^-1 on and above the diagonal
+                v[0] = g > 2 * kq ? bc[0] : ar[0];
+                v[1] = g > 2 * kq + 1 ? bc[1] : ar[1];
+            } else if (bi == q && bj < q) {
+                v[0] = bc[0];
+                v[1] = bc[1];
+            } else if (bi < q && bj == q) {
+                v[0] = ar[0];
+                v[1] = ar[1];
+            } else {   // T - a b, the panel's own rows and columns starting from zero
+                v[0] = v[1] = czero<C>();
+                if (bi != q && bj != q) {
+                    v[0] = d[0];
+                    v[1] = d[1];
+                }
+                block8_sub(Ab + 8 * bi * ASTR, ASTR, Bb + 8 * bj, BSTR, v, lane);
+            }
+            d[0] = v[0];
+            d[1] = v[1];
         }
         __syncthreads();
     }
-#pragma unroll
-    for (int e = 0; e < NE; ++e) {
-        const int c = cb + (DIAG_THREADS / NB) * e;
-        if (r < kb && c < kb) F[(k0 + r) + (size_t)(k0 + c) * f] = r > c ? W[r][c] : cmul(W[r][c], rdiag[c]);
+    for (int t = tid; t < NB * NB; t += DIAG_THREADS) {
+        const int r = t % NB, c = t / NB;
+        if (r < kb && c < kb) F[(k0 + r) + (size_t)(k0 + c) * f] = T[r * DSTR + c];
     }
-    if (PIV && threadIdx.x < kb) src[vars[k0 + threadIdx.x]] = (unsigned char)rowof[threadIdx.x];
-    if (np) atomicAdd(a.npert, (unsigned long long)np);
-    if (PIV && nsw) atomicAdd(a.nswap, (unsigned long long)nsw);
+    if (PIV && tid < kb) src[vars[k0 + tid]] = (unsigned char)rowat[tid];
+    if (tid == 0) {
+        if (np) atomicAdd(a.npert, (unsigned long long)np);
+        if (PIV && nsw) atomicAdd(a.nswap, (unsigned long long)nsw);
+    }
 }
 
-// the diagonal block (k0, kb) of front `node` in matrix z, with row
-// exchanges when piv (the level's fronts have more than NB pivots)
+// the diagonal block (k0, kb) of the front in matrix z, with row exchanges
+// when piv (the level's fronts have more than NB pivots)
 template <class R>
-__device__ __forceinline__ void diag_block(const FactorArgs<R> &a, cplx<R> *F, int node, int z, int k0, int kb,
+__device__ __forceinline__ void diag_block(const FactorArgs<R> &a, cplx<R> *F, const NodeDesc &d, int z, int k0, int kb,
                                            cplx<R> *sm, bool piv) {
-    const int f = a.s.nfront[node];
     if (piv) {
-        factor_diag_block<R, true>(a, F, f, k0, kb, sm, a.pivsrc + (size_t)z * a.s.n, a.s.vars + a.s.var_off[node]);
+        factor_diag_block<R, true>(a, F, d.nfront, k0, kb, sm, a.pivsrc + (size_t)z * a.s.n, a.s.vars + d.var_off);
     } else {
-        factor_diag_block<R, false>(a, F, f, k0, kb, sm, nullptr, nullptr);
+        factor_diag_block<R, false>(a, F, d.nfront, k0, kb, sm, nullptr, nullptr);
     }
 }
 
-// K3a: the first diagonal block of every front of the level (the later
-// ones are factored by the first CTA of the preceding trailing update)
+// K2 + K3a: the front's operator entries, then its first diagonal block (the
+// later ones are factored by the first CTA of the preceding trailing update)
 template <class R>
 __global__ void __launch_bounds__(DIAG_THREADS) k_diag(FactorArgs<R> a, int lvl_first, int piv) {
     using C = cplx<R>;
-    const int node = a.s.lvl_nodes[lvl_first + blockIdx.x];
-    const int s = a.s.npiv[node];
-    if (s <= 0) return;
-    C *F = reinterpret_cast<C *>(a.front) + (size_t)blockIdx.y * a.s.front_total + a.s.front_off[node];
-    extern __shared__ unsigned char smem_raw[];
-    diag_block<R>(a, F, node, blockIdx.y, 0, min(NB, s), reinterpret_cast<C *>(smem_raw), piv != 0);
+    const NodeDesc d = a.s.desc[lvl_first + blockIdx.x];
+    if (d.npiv <= 0) return;
+    C *F = reinterpret_cast<C *>(a.front) + (size_t)blockIdx.y * a.s.front_total + d.front_off;
+    add_entries(a, lvl_first + blockIdx.x, blockIdx.y);
+    __syncthreads();   // the entries are visible to the CTA
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    diag_block<R>(a, F, d, blockIdx.y, 0, min(NB, d.npiv), reinterpret_cast<C *>(smem_raw), piv != 0);
 }
 
 // K3b: the L and U panels of pivot block k0 as products with the inverted
@@ -392,19 +489,19 @@ __global__ void __launch_bounds__(DIAG_THREADS) k_diag(FactorArgs<R> a, int lvl_
 template <class R>
 __global__ void __launch_bounds__(256) k_panel_mm(FactorArgs<R> a, int lvl_first, int k0, int ntmax, int piv) {
     using C = cplx<R>;
-    const int node = a.s.lvl_nodes[lvl_first + blockIdx.y];
-    const int s = a.s.npiv[node];
+    const NodeDesc d = a.s.desc[lvl_first + blockIdx.y];
+    const int s = d.npiv;
     if (k0 >= s) return;
-    const int f = a.s.nfront[node];
+    const int f = d.nfront;
     const int kb = min(NB, s - k0);
     const int i0 = k0 + kb;
     const bool upper = blockIdx.x >= (unsigned)ntmax;
     const int x0 = i0 + (upper ? blockIdx.x - ntmax : blockIdx.x) * TILE;   // first row (L) / column (U)
     if (x0 >= f) return;
     const int nx = min(TILE, f - x0);
-    C *F = reinterpret_cast<C *>(a.front) + (size_t)blockIdx.z * a.s.front_total + a.s.front_off[node];
+    C *F = reinterpret_cast<C *>(a.front) + (size_t)blockIdx.z * a.s.front_total + d.front_off;
 
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     C *Is = reinterpret_cast<C *>(smem_raw);   // [NB][TSTR]: Is[k * TSTR + r] = triangle-inverse factor (r, k)
     C *Ps = Is + NB * TSTR;                    // [NB][TSTR]: Ps[k * TSTR + x] = panel entry (k, x)
     const C *Dg = F + k0 + (size_t)k0 * f;    // the inverted diagonal block
@@ -424,7 +521,7 @@ __global__ void __launch_bounds__(256) k_panel_mm(FactorArgs<R> a, int lvl_first
     if (upper) {
         if (threadIdx.x < NB)
             rsrc[threadIdx.x] = piv && threadIdx.x < kb
-                                    ? a.pivsrc[(size_t)blockIdx.z * a.s.n + a.s.vars[a.s.var_off[node] + k0 + threadIdx.x]]
+                                    ? a.pivsrc[(size_t)blockIdx.z * a.s.n + a.s.vars[d.var_off + k0 + threadIdx.x]]
                                     : (unsigned char)threadIdx.x;
         __syncthreads();
     }
@@ -438,10 +535,10 @@ __global__ void __launch_bounds__(256) k_panel_mm(FactorArgs<R> a, int lvl_first
         }
     }
     staged_sync();
-    Tile64<C, sizeof(R) == 8> acc;
-    for_tile64(acc, threadIdx.x, [](int, int, C &v) { v = czero<C>(); });
-    mma64<false>(Is, TSTR, 1, Ps, TSTR, 1, kb, kb, nx, acc, threadIdx.x);
-    for_tile64(acc, threadIdx.x, [&](int k, int x, C &v) {
+    TileCC<C, sizeof(R) == 8, TILE> acc;
+    for_tile(acc, threadIdx.x, [](int, int, C &v) { v = czero<C>(); });
+    mma_tile<false>(Is, TSTR, 1, Ps, TSTR, 1, kb, kb, nx, acc, threadIdx.x);
+    for_tile(acc, threadIdx.x, [&](int k, int x, C &v) {
         if (k < kb && x < nx) {
             if (upper) F[(k0 + k) + (size_t)(x0 + x) * f] = v;
             else F[(x0 + x) + (size_t)(k0 + k) * f] = v;
@@ -449,115 +546,129 @@ __global__ void __launch_bounds__(256) k_panel_mm(FactorArgs<R> a, int lvl_first
     });
 }
 
-// Trailing update C -= Lp * Up on one TILE x TILE tile; 256 threads, each
-// owns a 4 x 4 complex sub-tile with rows tx + 16a and columns ty + 16b.
-// Only the part of the trailing matrix that still belongs to pivot rows or
-// pivot columns is updated here; the contribution block (rows and columns
-// >= npiv) receives all pivot steps at once in one K = npiv GEMM at the end
-// of the level (launch_cb_gemm).
+// Trailing update C -= Lp * Up on TL x TL tiles, 256 threads.  Only the part
+// of the trailing matrix that still belongs to pivot rows or pivot columns is
+// updated here; the contribution block (rows and columns >= npiv) receives
+// all pivot steps at once in one K = npiv GEMM at the end of the level
+// (launch_gemm_sub_cc).  The first CTA takes the next diagonal block alone,
+// updates and factors it (it starts first, so this overlaps the tiles); the
+// others take tile blockIdx.x - 1 without that block.
+//
+// Tile size: a 64 x 64 x 32 complex128 product keeps one SM's FP64 pipe busy
+// for 4.3 us, a 32 x 32 one for 1.1 us, so where the level's 64-row tiles do
+// not fill the chip twice (kTileFill CTAs) the smaller ones shorten the step:
+// one 241 x 141 matrix, contribution GEMMs of the top levels 22-39 -> 11-15 us,
+// updates without a diagonal block behind them 19 -> 11 us.
 static_assert(DIAG_THREADS == 256, "k_update's first CTA factors the next diagonal block");
-template <class R>
+template <class R, int TL>
 __global__ void __launch_bounds__(256) k_update(FactorArgs<R> a, int lvl_first, int k0, int ntmax, int piv) {
     using C = cplx<R>;
-    const int node = a.s.lvl_nodes[lvl_first + blockIdx.y];
-    const int s = a.s.npiv[node];
+    constexpr int SS = TL + 2;   // padded row stride of the staged operands
+    const NodeDesc d = a.s.desc[lvl_first + blockIdx.y];
+    const int s = d.npiv;
     if (k0 >= s) return;
-    const int f = a.s.nfront[node];
+    const int f = d.nfront;
     const int kb = min(NB, s - k0);
     const int i0 = k0 + kb, m = f - i0;
-    const int nt = (m + TILE - 1) / TILE;
-    C *F = reinterpret_cast<C *>(a.front) + (size_t)blockIdx.z * a.s.front_total + a.s.front_off[node];
-    const int ti = blockIdx.x / ntmax, tj = blockIdx.x % ntmax;
+    const int nt = (m + TL - 1) / TL;
+    C *F = reinterpret_cast<C *>(a.front) + (size_t)blockIdx.z * a.s.front_total + d.front_off;
+    const bool next = blockIdx.x == 0;   // the next diagonal block
+    const int ti = next ? 0 : (blockIdx.x - 1) / ntmax, tj = next ? 0 : (blockIdx.x - 1) % ntmax;
     if (ti >= nt || tj >= nt) return;
-    if (i0 + ti * TILE >= s && i0 + tj * TILE >= s) return;   // tile inside the contribution block
+    if (i0 + ti * TL >= s && i0 + tj * TL >= s) return;   // tile inside the contribution block
+    const int nd = min(NB, s - i0);                        // size of the next diagonal block
+    const bool first = !next && ti == 0 && tj == 0;        // the tile that holds it
+    if (first && TL <= NB && nd == NB) return;
+    if (next && nd <= 0) return;
 
-    extern __shared__ unsigned char smem_raw[];
-    C *Ls = reinterpret_cast<C *>(smem_raw);   // [NB][TSTR]: Ls[c * TSTR + r]
-    C *Us = Ls + NB * TSTR;                    // [NB][TSTR]: Us[c * TSTR + col]
-    const int r0 = i0 + ti * TILE, c0 = i0 + tj * TILE;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C *Ls = reinterpret_cast<C *>(smem_raw);   // [NB][SS]: Ls[c * SS + r]
+    C *Us = Ls + NB * SS;                      // [NB][SS]: Us[c * SS + col]
+    const int r0 = i0 + ti * TL, c0 = i0 + tj * TL;
     // a tile whose columns all lie in the contribution block needs only its
     // pivot rows (and the other way round): the product is cut to them
-    const int mrows = c0 >= s ? min(TILE, s - r0) : min(TILE, f - r0);
-    const int ncols = r0 >= s ? min(TILE, s - c0) : min(TILE, f - c0);
+    const int mrows = next ? nd : c0 >= s ? min(TL, s - r0) : min(TL, f - r0);
+    const int ncols = next ? nd : r0 >= s ? min(TL, s - c0) : min(TL, f - c0);
     // asynchronous copies, all in flight at once; entries outside those rows
     // and columns or beyond kb are not staged (the product reads k < kb only
     // and treats rows / columns outside them as zero)
-    for (int t = threadIdx.x; t < NB * TILE; t += blockDim.x) {
-        const int r = t % TILE, c = t / TILE;
-        if (c < kb && r < mrows) cp_async_elem(Ls + c * TSTR + r, F + (r0 + r) + (size_t)(k0 + c) * f);
+    for (int t = threadIdx.x; t < NB * TL; t += blockDim.x) {
+        const int r = t % TL, c = t / TL;
+        if (c < kb && r < mrows) cp_async_elem(Ls + c * SS + r, F + (r0 + r) + (size_t)(k0 + c) * f);
         const int col = t / NB, cc = t % NB;   // U: contiguous along the pivot index
-        if (cc < kb && col < ncols) cp_async_elem(Us + cc * TSTR + col, F + (k0 + cc) + (size_t)(c0 + col) * f);
+        if (cc < kb && col < ncols) cp_async_elem(Us + cc * SS + col, F + (k0 + cc) + (size_t)(c0 + col) * f);
     }
     // the tile's current values go into the accumulators while the staged
     // operands land (read after the products, their latency was exposed)
-    Tile64<C, sizeof(R) == 8> acc;
-    auto mine = [&](int rr, int cc) { return rr < mrows && cc < ncols && (r0 + rr < s || c0 + cc < s); };
-    for_tile64(acc, threadIdx.x, [&](int rr, int cc, C &v) {
+    TileCC<C, sizeof(R) == 8, TL> acc;
+    auto mine = [&](int rr, int cc) {
+        return rr < mrows && cc < ncols && (r0 + rr < s || c0 + cc < s) && !(first && rr < nd && cc < nd);
+    };
+    for_tile(acc, threadIdx.x, [&](int rr, int cc, C &v) {
         v = mine(rr, cc) ? F[(r0 + rr) + (size_t)(c0 + cc) * f] : czero<C>();
     });
     staged_sync();
-    mma64<true>(Ls, TSTR, 1, Us, TSTR, 1, kb, mrows, ncols, acc, threadIdx.x);
-    for_tile64(acc, threadIdx.x, [&](int rr, int cc, C &v) {
+    mma_tile<true>(Ls, SS, 1, Us, SS, 1, kb, mrows, ncols, acc, threadIdx.x);
+    for_tile(acc, threadIdx.x, [&](int rr, int cc, C &v) {
         if (mine(rr, cc)) F[(r0 + rr) + (size_t)(c0 + cc) * f] = v;
     });
-    if (blockIdx.x == 0) {
-        // the first tile holds the next diagonal block, now final: factor it
-        // here (the first CTA starts first, so this overlaps the other tiles)
-        __syncthreads();   // the tile's global writes are visible; Ls / Us are free
-        diag_block<R>(a, F, node, blockIdx.z, i0, min(NB, s - i0), Ls, piv != 0);
+    if (next) {
+        __syncthreads();   // the block's global writes are visible; Ls / Us are free
+        diag_block<R>(a, F, d, blockIdx.z, i0, nd, Ls, piv != 0);
     }
 }
 
-// Batched C -= A * B on CUDA cores (64 x 64 output tiles, 4 x 4 complex
-// register tile per thread): the contribution-block update of every front
-// of a level in one launch.  K runs in chunks of GKC staged through shared
-// memory by asynchronous copies, two buffers: the next chunk's loads are in
-// flight while the current one is multiplied.  Tile entries outside A's
-// rows or B's columns are not staged (they only feed accumulators that are
-// never stored); the chunk loop reads only the k < kb part.
+// Batched C -= A * B (TL x TL output tiles, 256 threads): the
+// contribution-block update of every front of a level in one launch.  K runs
+// in chunks of GKC staged through shared memory by asynchronous copies, two
+// buffers: the next chunk's loads are in flight while the current one is
+// multiplied.  Tile entries outside A's rows or B's columns are not staged
+// (they only feed accumulators that are never stored); the chunk loop reads
+// only the k < kb part.
 constexpr int GKC = 16;
 
-template <class R>
+template <class R, int TL>
 __global__ void __launch_bounds__(256) k_gemm_sub_cc(const GemmProb<R> *__restrict__ probs,
                                                      const int4 *__restrict__ tiles) {
     using C = cplx<R>;
+    constexpr int SS = TL + 2;
     const int4 tl = tiles[blockIdx.x];
     const GemmProb<R> p = probs[tl.x];
-    const int r0 = tl.y * TILE, c0 = tl.z * TILE;
-    extern __shared__ unsigned char smem_raw[];
-    C *As = reinterpret_cast<C *>(smem_raw);   // [2][GKC][TSTR]: As[c * TSTR + r]
-    C *Bs = As + 2 * GKC * TSTR;               // [2][GKC][TSTR]: Bs[c * TSTR + col]
+    const int r0 = tl.y * TL, c0 = tl.z * TL;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C *As = reinterpret_cast<C *>(smem_raw);   // [2][GKC][SS]: As[c * SS + r]
+    C *Bs = As + 2 * GKC * SS;                 // [2][GKC][SS]: Bs[c * SS + col]
     auto stage = [&](int buf, int k0) {
         const int kb = min(GKC, p.k - k0);
-        C *Ab = As + buf * GKC * TSTR, *Bb = Bs + buf * GKC * TSTR;
-        for (int t = threadIdx.x; t < GKC * TILE; t += blockDim.x) {
-            const int r = t % TILE, c = t / TILE;
-            if (c < kb && r0 + r < p.m) cp_async_elem(Ab + c * TSTR + r, p.A + (size_t)(r0 + r) + (size_t)(k0 + c) * p.lda);
+        C *Ab = As + buf * GKC * SS, *Bb = Bs + buf * GKC * SS;
+        for (int t = threadIdx.x; t < GKC * TL; t += blockDim.x) {
+            const int r = t % TL, c = t / TL;
+            if (c < kb && r0 + r < p.m) cp_async_elem(Ab + c * SS + r, p.A + (size_t)(r0 + r) + (size_t)(k0 + c) * p.lda);
             const int col = t / GKC, cc = t % GKC;   // B: contiguous along k
             if (cc < kb && c0 + col < p.n)
-                cp_async_elem(Bb + cc * TSTR + col, p.B + (size_t)(k0 + cc) + (size_t)(c0 + col) * p.ldb);
+                cp_async_elem(Bb + cc * SS + col, p.B + (size_t)(k0 + cc) + (size_t)(c0 + col) * p.ldb);
         }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        async_commit();
     };
-    Tile64<C, sizeof(R) == 8> acc;
-    for_tile64(acc, threadIdx.x, [](int, int, C &v) { v = czero<C>(); });
-    const int mrows = min(TILE, p.m - r0), ncols = min(TILE, p.n - c0);
+    TileCC<C, sizeof(R) == 8, TL> acc;
+    for_tile(acc, threadIdx.x, [](int, int, C &v) { v = czero<C>(); });
+    const int mrows = min(TL, p.m - r0), ncols = min(TL, p.n - c0);
     const int nk = (p.k + GKC - 1) / GKC;
     if (nk > 0) stage(0, 0);
     for (int kc = 0; kc < nk; ++kc) {
         if (kc + 1 < nk) {
             stage((kc + 1) & 1, (kc + 1) * GKC);
-            asm volatile("cp.async.wait_group 1;\n" ::: "memory");   // chunk kc has landed
+            async_wait_group<1>();   // chunk kc has landed
         } else {
-            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            async_wait_group<0>();
         }
         __syncthreads();
         const int kb = min(GKC, p.k - kc * GKC);
-        mma64<false>(As + (kc & 1) * GKC * TSTR, TSTR, 1, Bs + (kc & 1) * GKC * TSTR, TSTR, 1, kb, mrows, ncols, acc,
-                     threadIdx.x);
+        mma_tile<false>(As + (kc & 1) * GKC * SS, SS, 1, Bs + (kc & 1) * GKC * SS, SS, 1, kb, mrows, ncols, acc,
+                        threadIdx.x);
         __syncthreads();   // this buffer is staged again for chunk kc + 2
     }
-    for_tile64(acc, threadIdx.x, [&](int rr, int cc, C &v) {
+    for_tile(acc, threadIdx.x, [&](int rr, int cc, C &v) {
         const int row = r0 + rr, col = c0 + cc;
         if (row < p.m && col < p.n) {
             C &d = p.C[(size_t)row + (size_t)col * p.ldc];
@@ -566,20 +677,39 @@ __global__ void __launch_bounds__(256) k_gemm_sub_cc(const GemmProb<R> *__restri
     });
 }
 
-template <class R>
-void launch_gemm_sub_cc(const GemmProb<R> *d_probs, const int4 *d_tiles, int ntiles, cudaStream_t st) {
-    if (ntiles <= 0) return;
-    const size_t smem = 4 * GKC * TSTR * sizeof(cplx<R>);
+template <class R, int TL>
+static void launch_gemm_tl(const GemmProb<R> *d_probs, const int4 *d_tiles, int ntiles, cudaStream_t st) {
+    const size_t smem = 4 * GKC * (TL + 2) * sizeof(cplx<R>);
     static bool attr = false;
     if (!attr) {
-        cudaFuncSetAttribute(k_gemm_sub_cc<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_gemm_sub_cc<R, TL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         attr = true;
     }
-    (k_gemm_sub_cc<R><<<ntiles, 256, smem, st>>>(d_probs, d_tiles), note_launch());
+    (k_gemm_sub_cc<R, TL><<<ntiles, 256, smem, st>>>(d_probs, d_tiles), note_launch());
 }
 
-template void launch_gemm_sub_cc<double>(const GemmProb<double> *, const int4 *, int, cudaStream_t);
-template void launch_gemm_sub_cc<float>(const GemmProb<float> *, const int4 *, int, cudaStream_t);
+template <class R>
+void launch_gemm_sub_cc(const GemmProb<R> *d_probs, const int4 *d_tiles, int ntiles, int tile, cudaStream_t st) {
+    if (ntiles <= 0) return;
+    if (tile == 32) launch_gemm_tl<R, 32>(d_probs, d_tiles, ntiles, st);
+    else launch_gemm_tl<R, 64>(d_probs, d_tiles, ntiles, st);
+}
+
+template void launch_gemm_sub_cc<double>(const GemmProb<double> *, const int4 *, int, int, cudaStream_t);
+template void launch_gemm_sub_cc<float>(const GemmProb<float> *, const int4 *, int, int, cudaStream_t);
+
+// trailing update of pivot block k0 over TL x TL tiles
+template <class R, int TL>
+static void launch_update(const FactorArgs<R> &a, int first, int count, int mmax, int k0, int piv, cudaStream_t st) {
+    const size_t smem = std::max<size_t>(2 * NB * (TL + 2), DIAG_SCRATCH) * sizeof(cplx<R>);
+    static bool attr = false;
+    if (!attr) {
+        cudaFuncSetAttribute(k_update<R, TL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        attr = true;
+    }
+    const int nt = (mmax + TL - 1) / TL;
+    (k_update<R, TL><<<dim3(nt * nt + 1, count, a.nf), 256, smem, st>>>(a, first, k0, nt, piv), note_launch());
+}
 
 template <class R>
 void launch_factor_level(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_t st) {
@@ -590,15 +720,9 @@ void launch_factor_level(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_
                              st>>>(a, first),
          note_launch());
     });
-    if (L.ent_count > 0) {
-        const int tpb = 256;
-        (k_entry_scatter<R><<<dim3((unsigned)((L.ent_count + tpb - 1) / tpb), a.nf), tpb, 0, st>>>(a, L.ent_first,
-                                                                                                  L.ent_count), note_launch());
-    }
     const size_t smem = 2 * NB * TSTR * sizeof(C);
     static bool attr_set = false;
     if (!attr_set) {
-        cudaFuncSetAttribute(k_update<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaFuncSetAttribute(k_panel_mm<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         attr_set = true;
     }
@@ -618,8 +742,8 @@ void launch_factor_level(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_
         // pivot block there is nothing left for them
         if (ntmax > 0 && L.max_piv > k0 + NB)
             for_level_pieces(L, [&](int first, int count) {
-                (k_update<R><<<dim3(ntmax * ntmax, count, a.nf), 256, smem, st>>>(a, first, k0, ntmax, piv),
-                 note_launch());
+                if ((int64_t)ntmax * ntmax * L.count * a.nf < kTileFill) launch_update<R, 32>(a, first, count, mmax, k0, piv, st);
+                else launch_update<R, 64>(a, first, count, mmax, k0, piv, st);
             });
     }
 }
@@ -1025,14 +1149,16 @@ __global__ void __launch_bounds__(MID_FT) k_factor_mid(FactorArgs<R> a, int lvl_
     __shared__ C rd[NPR];        // reciprocal pivots
     __shared__ int perm[NB];     // front row at pivot position q (row exchanges)
     __shared__ int npert;
-    const int node = a.s.lvl_nodes[lvl_first + blockIdx.x];
-    const int f = a.s.nfront[node], s = a.s.npiv[node], m = f - s;
+    const NodeDesc d = a.s.desc[lvl_first + blockIdx.x];
+    const int f = d.nfront, s = d.npiv, m = f - s;
     if (s == 0) return;   // the gathered front is already the contribution block
+    add_entries(a, lvl_first + blockIdx.x, blockIdx.y);
+    __syncthreads();   // the entries are visible to the CTA
     const int ldp = f + 1, ldu = s | 1;
     C *P = reinterpret_cast<C *>(smem_raw);
     C *U = P + (size_t)ldp * s;
     const int tid = threadIdx.x;
-    C *F = reinterpret_cast<C *>(a.front) + (size_t)blockIdx.y * a.s.front_total + a.s.front_off[node];
+    C *F = reinterpret_cast<C *>(a.front) + (size_t)blockIdx.y * a.s.front_total + d.front_off;
     const R pivtol = (R)(a.pivscale * __longlong_as_double((long long)*a.amax));
     if (tid == 0) npert = 0;
 
@@ -1097,7 +1223,7 @@ __global__ void __launch_bounds__(MID_FT) k_factor_mid(FactorArgs<R> a, int lvl_
     if (np) atomicAdd(&npert, np);
     if (tid == 0 && nsw) atomicAdd(a.nswap, (unsigned long long)nsw);
     staged_sync();
-    if (piv && tid < s) a.pivsrc[(size_t)blockIdx.y * a.s.n + a.s.vars[a.s.var_off[node] + tid]] = (unsigned char)perm[tid];
+    if (piv && tid < s) a.pivsrc[(size_t)blockIdx.y * a.s.n + a.s.vars[d.var_off + tid]] = (unsigned char)perm[tid];
 
     // 2. U12 = L11^-1 A12, one column per thread of warps 2 .. 7, while
     // warps 0 and 1 invert the pivot block's triangles (3.)
@@ -1154,14 +1280,14 @@ __global__ void __launch_bounds__(MID_FT) k_factor_mid(FactorArgs<R> a, int lvl_
     // values loaded into the accumulators first
     for (int i0 = 0; i0 < m; i0 += 64)
         for (int j0 = 0; j0 < m; j0 += 64) {
-            Tile64<C, (sizeof(R) == 8 && NPR > 16)> acc;   // short K (<= 16 pivots): CUDA-core FMAs
-            for_tile64(acc, tid, [&](int rr, int cc, C &v) {
+            TileCC<C, (sizeof(R) == 8 && NPR > 16), 64> acc;   // short K (<= 16 pivots): CUDA-core FMAs
+            for_tile(acc, tid, [&](int rr, int cc, C &v) {
                 const int i = i0 + rr, j = j0 + cc;
                 v = (i < m && j < m) ? F[s + i + (size_t)(s + j) * f] : czero<C>();
             });
-            mma64<true>(P + s + i0, ldp, 1, U + (size_t)j0 * ldu, 1, ldu, s, min(64, m - i0), min(64, m - j0), acc,
+            mma_tile<true>(P + s + i0, ldp, 1, U + (size_t)j0 * ldu, 1, ldu, s, min(64, m - i0), min(64, m - j0), acc,
                         tid);
-            for_tile64(acc, tid, [&](int rr, int cc, C &v) {
+            for_tile(acc, tid, [&](int rr, int cc, C &v) {
                 const int i = i0 + rr, j = j0 + cc;
                 if (i < m && j < m) F[s + i + (size_t)(s + j) * f] = v;
             });
@@ -1203,12 +1329,6 @@ void launch_factor_mid(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_t 
                              st>>>(a, first),
          note_launch());
     });
-    if (L.ent_count > 0) {
-        const int tpb = 256;
-        (k_entry_scatter<R><<<dim3((unsigned)((L.ent_count + tpb - 1) / tpb), a.nf), tpb, 0, st>>>(a, L.ent_first,
-                                                                                                  L.ent_count),
-         note_launch());
-    }
     if (L.max_piv <= 16)
         launch_mid<R, 16>(a, L, st);
     else

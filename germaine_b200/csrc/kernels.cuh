@@ -44,7 +44,8 @@ void launch_assemble(const AsmArgs &a, const float *m0, const float *m1, const A
 // of a chain of table look-ups)
 struct alignas(16) NodeDesc {
     int64_t front_off, var_off, inv_off, rhs_off, y_off;
-    int node, nfront, npiv, child0, child1, pad;
+    int64_t cb0, cb1;   // the children's contribution blocks (offsets as front_off), leading dimensions ld0, ld1
+    int node, nfront, npiv, child0, child1, ld0, ld1, pad;
 };
 
 struct DevSym {
@@ -147,10 +148,12 @@ struct GemmProb {
     cplx_any<R> *C;
     int lda, ldb, ldc, m, n, k;
 };
-// CUDA-core batched GEMM over 64 x 64 tiles: tiles[t] = (problem, tile row, tile col)
+// batched GEMM over tile x tile output tiles (64 or 32): tiles[t] = (problem, tile row, tile col)
 template <class R>
-void launch_gemm_sub_cc(const GemmProb<R> *d_probs, const int4 *d_tiles, int ntiles, cudaStream_t st);
+void launch_gemm_sub_cc(const GemmProb<R> *d_probs, const int4 *d_tiles, int ntiles, int tile, cudaStream_t st);
 constexpr int kGemmTileCC = 64;
+// fewer 64 x 64 tiles than this in a launch: 32 x 32 ones instead (two per SM)
+constexpr int kGemmTileFill = 2 * 148;
 
 // ---------------- K5 multi-RHS substitution ----------------
 template <class R>
