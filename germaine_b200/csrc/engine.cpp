@@ -133,10 +133,12 @@ extern "C" int gm_engine_create(int device, const gm_config *cfg, gm_engine **ou
         L.max_piv = s.lvl_max_piv[h];
         L.max_ring = 0;
         L.mid_words = 0;
+        L.front_words = 0;
         for (int t = L.first; t < L.first + L.count; ++t) {
             const int v = s.lvl_nodes[t], fv = s.nfront[v], sv = s.npiv[v];
             L.max_ring = std::max(L.max_ring, fv - sv);
             L.mid_words = std::max(L.mid_words, (int64_t)(fv + 1) * sv + (int64_t)(sv | 1) * (fv - sv));
+            L.front_words = std::max(L.front_words, gm::front_words_of(fv, sv));
         }
         L.ent_first = (int64_t)ent_dst.size();
         for (int t = L.first; t < L.first + L.count; ++t) {
@@ -178,10 +180,18 @@ extern "C" int gm_engine_create(int device, const gm_config *cfg, gm_engine **ou
         const auto cb = [&](int c) { return c < 0 ? 0 : s.front_off[c] + s.npiv[c] + (int64_t)s.npiv[c] * s.nfront[c]; };
         const int c0 = s.child0[v], c1 = s.child1[v];
         desc[t] = gm::NodeDesc{s.front_off[v], s.var_off[v], s.inv_off[v], s.rhs_off[v], y_off[v], cb(c0), cb(c1),
-                               v, s.nfront[v], s.npiv[v], c0, c1, c0 < 0 ? 0 : s.nfront[c0], c1 < 0 ? 0 : s.nfront[c1], 0};
+                               v, s.nfront[v], s.npiv[v], c0, c1, c0 < 0 ? 0 : s.nfront[c0], c1 < 0 ? 0 : s.nfront[c1],
+                               c0 < 0 ? 0 : s.nfront[c0] - s.npiv[c0], c1 < 0 ? 0 : s.nfront[c1] - s.npiv[c1],
+                               (int)(ent_lvl_off[t + 1] - ent_lvl_off[t]), ent_lvl_off[t]};
+    }
+    std::vector<gm::NodeDesc> fdesc = desc;
+    for (gm::LevelInfo &L : e->levels) {
+        std::stable_sort(fdesc.begin() + L.first, fdesc.begin() + L.first + L.count,
+                         [](const gm::NodeDesc &x, const gm::NodeDesc &y) { return x.nfront > y.nfront; });
+        L.classes = gm::front_classes(fdesc.data() + L.first, L.count, e->csize());
     }
     int rc2;
-    if ((rc2 = upload(e->d_desc, desc, e->st))) return rc2;
+    if ((rc2 = upload(e->d_desc, desc, e->st)) || (rc2 = upload(e->d_fdesc, fdesc, e->st))) return rc2;
     if ((rc2 = upload(e->d_npiv, s.npiv, e->st)) || (rc2 = upload(e->d_nfront, s.nfront, e->st)) ||
         (rc2 = upload(e->d_child0, s.child0, e->st)) || (rc2 = upload(e->d_child1, s.child1, e->st)) ||
         (rc2 = upload(e->d_vars, s.vars, e->st)) || (rc2 = upload(e->d_inv, s.inv, e->st)) ||
@@ -189,7 +199,7 @@ extern "C" int gm_engine_create(int device, const gm_config *cfg, gm_engine **ou
         (rc2 = upload(e->d_var_off, s.var_off, e->st)) || (rc2 = upload(e->d_inv_off, s.inv_off, e->st)) ||
         (rc2 = upload(e->d_rhs_off, s.rhs_off, e->st)) || (rc2 = upload(e->d_ent_dst, ent_dst, e->st)) ||
         (rc2 = upload(e->d_y_off, y_off, e->st)) || (rc2 = upload(e->d_tri_off, tri_off, e->st)) ||
-        (rc2 = upload(e->d_ent_src, ent_src, e->st)) || (rc2 = upload(e->d_ent_lvl_off, ent_lvl_off, e->st)))
+        (rc2 = upload(e->d_ent_src, ent_src, e->st)))
         return rc2;
     GM_CUDA(cudaStreamSynchronize(e->st));
     gm::DevSym &d = e->dsym;
@@ -201,6 +211,7 @@ extern "C" int gm_engine_create(int device, const gm_config *cfg, gm_engine **ou
     d.inv_off = e->d_inv_off.as<int64_t>(); d.rhs_off = e->d_rhs_off.as<int64_t>();
     d.front_total = s.front_total; d.rhs_total = s.rhs_total;
     d.desc = e->d_desc.as<gm::NodeDesc>();
+    d.fdesc = e->d_fdesc.as<gm::NodeDesc>();
     d.y_off = e->d_y_off.as<int64_t>(); d.y_total = y_total;
 
     gm_stats &st = e->stats;
@@ -303,8 +314,8 @@ static int assemble_batch(gm_engine *e) {
 // their output tiles: tcgen05 tiles (128 x 64) for the complex64 path on
 // levels whose blocks are large enough to fill them, CUDA-core tiles
 // (64 x 64) otherwise.
-// Levels of fronts with at most 16 pivots that are too large for the small
-// kernel go to the fused mid-level kernel; GM_NO_FACTOR_MID=1 keeps them on
+// Levels of fronts with at most 16 pivots that are too large for the
+// whole-front kernel go to the fused mid-level kernel; GM_NO_FACTOR_MID=1 keeps them on
 // the blocked diagonal / panel / contribution-GEMM sequence.  With 17-32
 // pivots the fused kernel holds 32-entry pivot rows in registers and fits
 // one CTA per SM; measured at 841 x 227 (10 frequencies) the blocked
@@ -361,7 +372,7 @@ static int build_cb_plan(gm_engine *e) {
         pl.tile = tile;
         pl.prob_off = (int64_t)probs.size();
         pl.tile_off = (int64_t)tiles.size();
-        if (small_factor_level<R>(L) || use_mid_factor<R>(L)) {   // fused kernels form the Schur complement themselves
+        if (front_factor_level<R>(L) || use_mid_factor<R>(L)) {   // fused kernels form the Schur complement themselves
             pl.ntiles = 0;
             continue;
         }
@@ -401,7 +412,6 @@ static int factor_batch(gm_engine *e, double pivscale) {
     a.A = e->d_A.as<double2>();
     a.ent_dst = e->d_ent_dst.as<int64_t>();
     a.ent_src = e->d_ent_src.as<int>();
-    a.ent_lvl_off = e->d_ent_lvl_off.as<int64_t>();
     a.nf = e->nf;
     a.amax = e->d_amax.as<unsigned long long>();
     a.pivscale = pivscale;
@@ -423,8 +433,10 @@ static int factor_batch(gm_engine *e, double pivscale) {
     auto launch_levels = [&](cudaEvent_t *evs) {
         bool forked = false;
         for (int h = 0; h < nl; ++h) {
-            if (small_factor_level<R>(e->levels[h])) {
-                launch_factor_small<R>(a, e->levels[h], e->st);
+            bool inverted = false;   // the whole-front kernel leaves whole triangle inverses
+            if (front_factor_level<R>(e->levels[h])) {
+                launch_factor_front<R>(a, e->levels[h], e->st);
+                inverted = true;
             } else if (use_mid_factor<R>(e->levels[h])) {
                 launch_factor_mid<R>(a, e->levels[h], e->st);
             } else {
@@ -436,7 +448,7 @@ static int factor_batch(gm_engine *e, double pivscale) {
                 else
                     launch_gemm_sub_cc<R>(probs + pl.prob_off, tiles + pl.tile_off, pl.ntiles, pl.tile, e->st);
             }
-            if (e->levels[h].max_piv > 32) {   // beside the levels above (the last level's: nothing is)
+            if (e->levels[h].max_piv > 32 && !inverted) {   // beside the levels above (the last level's: nothing is)
                 cudaEventRecord(e->ev_fork, e->st);
                 cudaStreamWaitEvent(e->st2, e->ev_fork, 0);
                 launch_tri_inverse<R>(a, e->levels[h], e->d_tri.p, e->tri_total, e->d_tri_off.as<int64_t>(), e->st2);
@@ -502,7 +514,7 @@ static int factor_batch(gm_engine *e, double pivscale) {
             const LevelInfo &L = e->levels[h];
             std::fprintf(stderr, "factor %s level %2d: fronts %5d max_front %4d max_piv %4d %s %.3f ms\n",
                          sizeof(R) == 8 ? "c128" : "c64", h, L.count, L.max_front, L.max_piv,
-                         small_factor_level<R>(L) ? "small" : use_mid_factor<R>(L) ? "mid" : "tiled", ms);
+                         front_factor_level<R>(L) ? (level_pivots<R>(L) ? "front" : "small") : use_mid_factor<R>(L) ? "mid" : "tiled", ms);
         }
         for (auto &x : ev) cudaEventDestroy(x);
     }

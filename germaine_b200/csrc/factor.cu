@@ -27,7 +27,7 @@
 // permutation is in FactorArgs::pivsrc.
 //
 // Two fused kernels leave the same layout on the levels where they pay:
-//   k_factor_small  fronts that fit shared memory whole (the lower levels):
+//   k_factor_front  fronts that fit shared memory whole (the lower levels):
 //                   extend-add, entries, LU and Schur complement in one CTA;
 //   k_factor_mid    fronts with at most NB pivots and at most 256 rows above
 //                   those: after K2, one CTA factorises the pivot columns
@@ -184,15 +184,15 @@ __global__ void k_front_gather(FactorArgs<R> a, int lvl_first) {
     }
 }
 
-// the operator entries owned by the front at level position pos, added into
-// it by one CTA (positions are distinct)
+// the operator entries owned by the front, added into it by one CTA
+// (positions are distinct)
 template <class R>
-__device__ __forceinline__ void add_entries(const FactorArgs<R> &a, int pos, int z) {
+__device__ __forceinline__ void add_entries(const FactorArgs<R> &a, const NodeDesc &nd, int z) {
     using C = cplx<R>;
     C *F = reinterpret_cast<C *>(a.front) + (size_t)z * a.s.front_total;
     const double2 *A = a.A + (size_t)z * 9 * a.s.n;
-    const int64_t e1 = a.ent_lvl_off[pos + 1];
-    for (int64_t e = a.ent_lvl_off[pos] + threadIdx.x; e < e1; e += blockDim.x) {
+    const int64_t e1 = nd.ent_first + nd.ent_count;
+    for (int64_t e = nd.ent_first + threadIdx.x; e < e1; e += blockDim.x) {
         C &d = F[a.ent_dst[e]];
         d = cadd(d, cconv<C>(A[a.ent_src[e]]));
     }
@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(DIAG_THREADS) k_diag(FactorArgs<R> a, int lvl_
     const NodeDesc d = a.s.desc[lvl_first + blockIdx.x];
     if (d.npiv <= 0) return;
     C *F = reinterpret_cast<C *>(a.front) + (size_t)blockIdx.y * a.s.front_total + d.front_off;
-    add_entries(a, lvl_first + blockIdx.x, blockIdx.y);
+    add_entries(a, d, blockIdx.y);
     __syncthreads();   // the entries are visible to the CTA
     extern __shared__ __align__(16) unsigned char smem_raw[];
     diag_block<R>(a, F, d, blockIdx.y, 0, min(NB, d.npiv), reinterpret_cast<C *>(smem_raw), piv != 0);
@@ -752,301 +752,488 @@ template void launch_factor_level<double>(const FactorArgs<double> &, const Leve
 template void launch_factor_level<float>(const FactorArgs<float> &, const LevelInfo &, cudaStream_t);
 
 // ---------------------------------------------------------------------
-// Small fronts (the lower levels of the tree): one CTA assembles and
-// factorises a whole front in shared memory -- extend-add of the children's
-// contribution blocks, the operator entries, right-looking LU of the npiv
-// pivot columns with the same static pivoting as factor_diag_block, the Schur
-// complement of the contribution block, and the inverses of the NB x NB
-// diagonal blocks -- and writes the front back once.  The result has the
-// layout the blocked path leaves (L below, U above, diagonal-block inverses,
-// contribution block), in one launch per level instead of the
-// gather / scatter / ceil(npiv/NB) x (panel + update) / contribution GEMM
-// sequence.  S[i + j * ld] holds front entry (i, j).
+// Fronts that fit shared memory whole (the lower levels of the tree): one CTA
+// assembles and factorises a front -- extend-add of the children's
+// contribution blocks, the operator entries, LU of the npiv pivot columns,
+// the inverses of both pivot triangles and the Schur complement of the
+// contribution block -- and writes it back once, in one launch per level and
+// size class instead of the gather / diagonal / panel / update / contribution
+// GEMM sequence.  The result has the layout the blocked path leaves.
+//
+// The front is held in 8 x 8 blocks, the pivots padded to a multiple of 8 by
+// decoupled unit pivots: S[i + j ld], pivot k at position k, ring variable i
+// at i - npiv + sp.  Per 8-pivot panel q the three steps of
+// factor_diag_block, over the whole front:
+//   1. one warp factors the panel's pivot rows (a row per lane, up to 32 below
+//      the panel's first; row exchanges inside them when PIV);
+//   2. a thread per column solves with L_q (b), a thread per row with U_q (a);
+//      the ring parts are final (U12 and L21) and stay in S, the pivot parts
+//      and the panel's triangle inverses go to Bb and Ab;
+//   3. the warps form T - a b on 8 x 8 blocks (FP64 matrix instructions in
+//      complex128): the trailing front, the finished rows and columns of the
+//      inverses, the panel's own inverse rows and columns.  The panels' warp
+//      takes the next one's pivot blocks and goes on with its step 1 beside
+//      the others.
+// So a front costs three barriers per 8 pivots and the inverses no pass of
+// their own.  (Before: one barrier per pivot or two per 4 pivots, then one
+// thread per inverse column chaining up to 435 multiply-adds, and from 80 rows
+// on the gathered front passed through global memory twice more.  841 x 227,
+// 10 matrices, complex128, levels 0-4: 3.87, 0.73, 1.03, 1.47, 1.04 ms then;
+// 2.58, 0.57, 0.59, 0.83, 0.92 ms now.  complex64: 2.90, 0.63, 0.67, 0.69,
+// 0.93 -> 1.85, 0.38, 0.36, 0.56, 0.73 ms.)
+//
+// What bounds it: the pivots' latency chain (about 420 cycles each, 3 to 8
+// fronts per SM side by side), then the shared-memory traffic of the 8 x 8
+// blocks (16-byte elements, 128 B a cycle).  Fronts are launched largest
+// first in classes of like size, so a class's shared memory, and with it the
+// fronts per SM, follows its own largest front.  (The substitution keeps the
+// dissection's order: neighbouring fronts share rows of x in L2.)
 // ---------------------------------------------------------------------
-constexpr int SMALL_FT = 256;   // threads per CTA
+constexpr size_t FRONT_SMEM = 226 << 10;   // largest dynamic shared memory of a CTA (1 KB left for static)
 
-// (register bounds: three CTAs per SM for the blocked form, whose panel
-// registers would otherwise cost one; four for the per-pivot form, which the
-// smaller fronts of levels 1-2 fit in shared memory -- without a bound the
-// compiler takes 88 registers and two CTAs, and those levels run 2x slower)
-template <class R, int SROWS, bool BLOCKED>
-__global__ void __launch_bounds__(SMALL_FT, BLOCKED ? 3 : 4) k_factor_small(FactorArgs<R> a, int lvl_first, int ld) {
+__host__ __device__ constexpr int front_sp(int s) { return (s + PW8 - 1) / PW8 * PW8; }
+__host__ __device__ constexpr int front_fp(int f, int s) { return f - s + front_sp(s); }
+// column stride: whole blocks of rows (zero below the front), odd (conflict-free blocks)
+__host__ __device__ constexpr int front_ld(int fp) { return (fp + PW8 - 1) / PW8 * PW8 + 1; }
+// elements: S, Ab [8][sp + 2], Bb [sp][12], rd [sp]
+static size_t front_words(int fp, int sp) { return (size_t)front_ld(fp) * fp + 8 * (sp + 2) + 12 * (size_t)sp + sp; }
+
+// Right operand of a column of 8 x 8 blocks, held by the warp: B(k, c) =
+// pb[k + c bc] for k < 8, c < nc; sub() subtracts A B from this lane's two
+// entries of a block (row l / 4, columns 2 (l % 4) + {0, 1}); pa points at the
+// lane's part of A (left()), A's pivots being ak apart.
+template <class C>
+struct BlockCol;
+template <>
+struct BlockCol<double2> {
+    double by[2], nx[2], ny[2];   // b and -b: the matrix instructions take no negated operands
+    __device__ __forceinline__ static int left(int ak, int lane) { return (lane >> 2) + (lane & 3) * ak; }
+    __device__ __forceinline__ void load(const double2 *pb, int bc, int nc, int lane) {
+        const int g = lane >> 2, kq = lane & 3;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const double2 w = g < nc ? pb[4 * h + kq + g * bc] : czero<double2>();
+            by[h] = w.y; nx[h] = -w.x; ny[h] = -w.y;
+        }
+    }
+    __device__ __forceinline__ void sub(const double2 *pa, int ak, double2 &a0, double2 &a1) const {
+        const double2 v0 = pa[0], v1 = pa[4 * ak];
+        dmma_884(v0.x, nx[0], a0.x, a1.x);   // Re -= Ar Br - Ai Bi
+        dmma_884(v0.x, ny[0], a0.y, a1.y);   // Im -= Ar Bi + Ai Br
+        dmma_884(v0.y, by[0], a0.x, a1.x);
+        dmma_884(v0.y, nx[0], a0.y, a1.y);
+        dmma_884(v1.x, nx[1], a0.x, a1.x);
+        dmma_884(v1.x, ny[1], a0.y, a1.y);
+        dmma_884(v1.y, by[1], a0.x, a1.x);
+        dmma_884(v1.y, nx[1], a0.y, a1.y);
+    }
+};
+template <>
+struct BlockCol<float2> {
+    float2 b[2][PW8];
+    __device__ __forceinline__ static int left(int, int lane) { return lane >> 2; }
+    __device__ __forceinline__ void load(const float2 *pb, int bc, int nc, int lane) {
+        const int c = 2 * (lane & 3);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int k = 0; k < PW8; ++k) b[h][k] = c + h < nc ? pb[k + (c + h) * bc] : czero<float2>();
+    }
+    __device__ __forceinline__ void sub(const float2 *pa, int ak, float2 &a0, float2 &a1) const {
+#pragma unroll
+        for (int k = 0; k < PW8; ++k) {
+            const float2 v = pa[k * ak];
+            cfms(a0, v, b[0][k]);
+            cfms(a1, v, b[1][k]);
+        }
+    }
+};
+
+template <class R, int NTH, bool PIV>
+__global__ void __launch_bounds__(NTH, NTH == 128 ? (sizeof(R) == 8 ? 5 : 8) : NTH == 256 ? (sizeof(R) == 8 ? 2 : 3) : 1) k_factor_front(FactorArgs<R> a, int lvl_first) {
     using C = cplx<R>;
+    constexpr unsigned ALL = 0xffffffffu;
+    constexpr int NW = NTH / 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int rowat[PIV ? NB : 1];      // PIV: front row at pivot position k (npiv <= NB)
+    __shared__ int pm[NTH == 128 ? 64 : NTH == 256 ? 96 : 128];   // a child's ring positions here
+    __shared__ int swaps[PW8 + 1];           // the panel's row exchanges: count, then p | arg << 16
+    const NodeDesc d = a.s.fdesc[lvl_first + blockIdx.x];
+    const int f = d.nfront, s = d.npiv, sp = front_sp(s), fp = front_fp(f, s), ld = front_ld(fp);
+    const int nb = (fp + PW8 - 1) / PW8, npb = sp / PW8;
     C *S = reinterpret_cast<C *>(smem_raw);
-    __shared__ C Dinv[NB][NB + 1];
-    __shared__ int npert;
-    const int pos = lvl_first + blockIdx.x;
-    const int node = a.s.lvl_nodes[pos];
-    const int f = a.s.nfront[node], s = a.s.npiv[node];
-    C *rd = S + (size_t)ld * f;   // reciprocal pivots
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = SMALL_FT / 32;
+    C *Ab = S + (size_t)ld * fp;             // [PW8][sp + 2]: Ab[k * (sp + 2) + r], pivot rows r
+    C *Bb = Ab + PW8 * (sp + 2);             // [sp][12]: Bb[c * 12 + k], pivot columns c
+    C *rd = Bb + 12 * sp;                    // reciprocal pivots
+    const int sa = sp + 2;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // wi 0 factors the panels: another of the CTA's first four warps in every
+    // CTA, so that the panels of the fronts on an SM meet all its schedulers
+    // (all on the first one they took twice as long)
+    const int wi = (warp + NW - ((blockIdx.x + blockIdx.y) & 3)) % NW;
     const size_t fz = blockIdx.y;
     C *base = reinterpret_cast<C *>(a.front) + fz * a.s.front_total;
-    C *F = base + a.s.front_off[node];
+    C *F = base + d.front_off;
 
-    // extend-add of the children's contribution blocks (zero for leaves)
-    const int *inv = a.s.inv + a.s.inv_off[node];
-    const int c0 = a.s.child0[node], c1 = a.s.child1[node];
-    const C *cb0 = nullptr, *cb1 = nullptr;
-    int f0 = 0, f1 = 0;
-    if (c0 >= 0) { const int s0 = a.s.npiv[c0]; f0 = a.s.nfront[c0]; cb0 = base + a.s.front_off[c0] + s0 + (size_t)s0 * f0; }
-    if (c1 >= 0) { const int s1 = a.s.npiv[c1]; f1 = a.s.nfront[c1]; cb1 = base + a.s.front_off[c1] + s1 + (size_t)s1 * f1; }
-    for (int j = warp; j < f; j += nw) {
-        const int j0 = cb0 ? inv[j] : -1, j1 = cb1 ? inv[f + j] : -1;
-        for (int i = lane; i < f; i += 32) {
-            C v = czero<C>();
-            if (j0 >= 0) { const int r = inv[i]; if (r >= 0) v = cadd(v, cb0[r + (size_t)j0 * f0]); }
-            if (j1 >= 0) { const int r = inv[f + i]; if (r >= 0) v = cadd(v, cb1[r + (size_t)j1 * f1]); }
-            S[i + j * ld] = v;
-        }
+    // the operator entries owned by the front (positions are distinct): the
+    // first NE per thread are requested before anything else
+    constexpr int NE = NTH == 128 ? 2 : 1;
+    const double2 *A = a.A + fz * 9 * (size_t)a.s.n;
+    double2 ev[NE];
+    int ep[NE];
+#pragma unroll
+    for (int x = 0; x < NE; ++x) {
+        const int e = tid + x * NTH;
+        ep[x] = e < d.ent_count ? (int)(a.ent_dst[d.ent_first + e] - d.front_off) : -1;
+        ev[x] = ep[x] >= 0 ? A[a.ent_src[d.ent_first + e]] : make_double2(0.0, 0.0);
     }
-    if (tid == 0) npert = 0;
-    __syncthreads();
-    // operator entries owned by the front (positions are distinct)
-    {
-        const int64_t e0 = a.ent_lvl_off[pos], e1 = a.ent_lvl_off[pos + 1];
-        const int64_t fo = a.s.front_off[node];
-        const double2 *A = a.A + fz * 9 * (size_t)a.s.n;
-        for (int64_t e = e0 + tid; e < e1; e += SMALL_FT) {
-            const int p = (int)(a.ent_dst[e] - fo);
-            const int i = p % f, j = p / f;
-            C &d = S[i + j * ld];
-            d = cadd(d, cconv<C>(A[a.ent_src[e]]));
-        }
-    }
-    __syncthreads();
-
-    // right-looking LU of the pivot columns; the trailing update covers the
-    // contribution block too (its Schur complement).  Warp 0 updates column
-    // k + 1 first in step k, so it can take the next pivot (static pivoting
-    // as in factor_diag_block) and scale the next L column while the other warps are
-    // still updating: one barrier per pivot.
-    const R pivtol = (R)(a.pivscale * __longlong_as_double((long long)*a.amax));
-    auto take_pivot = [&](int k) {   // warp 0 only: pivot k, reciprocal, L column k scaled
-        if (lane == 0) {
-            const C piv = static_pivot<R>(S[k + k * ld], pivtol, npert);
-            S[k + k * ld] = piv;
-            rd[k] = crcp(piv);
-        }
-        __syncwarp();
-        const C rk = rd[k];
-        for (int i = k + 1 + lane; i < f; i += 32) S[i + k * ld] = cmul(S[i + k * ld], rk);
-        __syncwarp();
+    auto add_entry = [&](int q, const double2 &v) {
+        int i = q % f, j = q / f;
+        if (i >= s) i += sp - s;
+        if (j >= s) j += sp - s;
+        C &t = S[i + j * ld];
+        t = cadd(t, cconv<C>(v));
     };
-    if constexpr (BLOCKED) {
-        // complex128, fronts with many pivots: blocked by 4-pivot panels.  Warp 0 factors a panel's
-        // columns (static pivoting, L columns scaled) and applies each pivot
-        // to the panel rows right of the panel (the U rows); then every warp
-        // applies the rank-4 update to the trailing block on FP64 matrix
-        // instructions, one 8 x 8 block per warp at a time.  Two barriers per
-        // panel instead of one per pivot.
-        constexpr int PW = 4;
-        const int g = lane >> 2, kq = lane & 3;
-        for (int kb0 = 0; kb0 < s; kb0 += PW) {
-            const int kend = min(s, kb0 + PW);
-            if (warp == 0) {
-                // the panel in registers: lane l holds rows l and l + 32
-                // (fronts of at most 64 rows) of the panel's columns; the
-                // pivot row's entries come from their owner by shuffles, so
-                // each pivot costs shuffles and FMAs, no shared-memory round
-                // trip or warp barrier
-                C pv[2][PW];
+    // extend-add: zeros, then each child's contribution block read once down
+    // its columns (GB of them in flight per warp) and added at its rows'
+    // positions here (pm: the inverse of the extend-add map)
+    constexpr int NR = NTH == 128 ? 2 : NTH == 256 ? 3 : 4;   // rows per lane (launch condition)
+    constexpr int GB = NTH == 128 ? 4 : 2;
+    {
+        const int pad = sp - s;
+        for (int t = tid; t < ld * fp; t += NTH) S[t] = czero<C>();
+#pragma unroll 1
+        for (int ch = 0; ch < 2; ++ch) {
+            if ((ch ? d.child1 : d.child0) < 0) continue;   // CTA-uniform
+            const int *inv = a.s.inv + d.inv_off + (ch ? f : 0);
+            const int ldc = ch ? d.ld1 : d.ld0;
+            const C *cb = base + (ch ? d.cb1 : d.cb0);
+            for (int i = tid; i < f; i += NTH) {
+                const int r = inv[i];
+                if (r >= 0) pm[r] = i < s ? i : i + pad;
+            }
+            const int m = ch ? d.ring1 : d.ring0;   // the child's ring, which lies in this front whole
+            __syncthreads();
+#pragma unroll 1
+            for (int j = warp; j < m; j += GB * NW) {
+                C v[GB][NR];
 #pragma unroll
-                for (int q = 0; q < 2; ++q)
+                for (int w = 0; w < GB; ++w)
 #pragma unroll
-                    for (int j = 0; j < PW; ++j) {
-                        const int i = lane + 32 * q;
-                        pv[q][j] = i < f && kb0 + j < kend ? S[i + (kb0 + j) * ld] : czero<C>();
+                    for (int u = 0; u < NR; ++u) {
+                        const int jw = j + w * NW, i = lane + 32 * u;
+                        v[w][u] = jw < m && i < m ? cb[i + (size_t)jw * ldc] : czero<C>();
                     }
 #pragma unroll
-                for (int jk = 0; jk < PW; ++jk) {
-                    const int k = kb0 + jk;
-                    if (k >= kend) break;   // warp-uniform
-                    const int owner = k & 31;
-                    C prow[PW];   // row k of the panel
+                for (int w = 0; w < GB; ++w)
 #pragma unroll
-                    for (int j = 0; j < PW; ++j) {
-                        const C v = k >= 32 ? pv[1][j] : pv[0][j];
-                        prow[j] = make_double2(__shfl_sync(0xffffffffu, v.x, owner), __shfl_sync(0xffffffffu, v.y, owner));
-                    }
-                    int np = 0;
-                    const C piv = static_pivot<R>(prow[jk], pivtol, np);   // every lane: the same pivot
-                    const C rk = crcp(piv);
-                    if (lane == 0) {
-                        rd[k] = rk;
-                        npert += np;
-                    }
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        const int i = lane + 32 * q;
-                        if (i == k) pv[q][jk] = piv;   // the (perturbed) pivot
-                        if (i > k && i < f) {
-                            const C l = cmul(pv[q][jk], rk);
-                            pv[q][jk] = l;
-#pragma unroll
-                            for (int j = jk + 1; j < PW; ++j) cfms(pv[q][j], l, prow[j]);
+                    for (int u = 0; u < NR; ++u) {
+                        const int jw = j + w * NW, i = lane + 32 * u;
+                        if (jw < m && i < m) {
+                            C &t = S[pm[i] + pm[jw] * ld];
+                            t = cadd(t, v[w][u]);
                         }
                     }
-                }
-#pragma unroll
-                for (int q = 0; q < 2; ++q)
-#pragma unroll
-                    for (int j = 0; j < PW; ++j) {
-                        const int i = lane + 32 * q;
-                        if (i < f && kb0 + j < kend) S[i + (kb0 + j) * ld] = pv[q][j];
-                    }
-                __syncwarp();
-                // the panel's U rows right of the panel: unit lower solve with
-                // the panel's diagonal block, one column per lane
-                const int pw = kend - kb0;
-                for (int j = kend + lane; j < f; j += 32) {
-                    C u[PW];
-#pragma unroll
-                    for (int r = 0; r < PW; ++r) {
-                        if (r >= pw) break;
-                        C v = S[kb0 + r + j * ld];
-#pragma unroll
-                        for (int t = 0; t < r; ++t) cfms(v, S[kb0 + r + (kb0 + t) * ld], u[t]);
-                        u[r] = v;
-                        S[kb0 + r + j * ld] = v;
-                    }
-                }
-            }
-            __syncthreads();
-            const int mt = f - kend, nbt = (mt + 7) / 8;
-            for (int bi = warp; bi < nbt * nbt; bi += nw) {   // trailing block -= L(:, panel) U(panel, :)
-                const int r = kend + 8 * (bi % nbt) + g, c0 = kend + 8 * (bi / nbt);
-                const int cl = c0 + 2 * kq;
-                double2 d0 = r < f && cl < f ? S[r + cl * ld] : czero<C>();
-                double2 d1 = r < f && cl + 1 < f ? S[r + (cl + 1) * ld] : czero<C>();
-                const int kk = kb0 + kq;
-                const bool kin = kk < kend;
-                double2 af = kin && r < f ? S[r + kk * ld] : czero<C>();
-                af = make_double2(-af.x, -af.y);
-                const int cb = c0 + g;
-                const double2 bf = kin && cb < f ? S[kk + cb * ld] : czero<C>();
-                dmma_884(af.x, bf.x, d0.x, d1.x);
-                dmma_884(-af.y, bf.y, d0.x, d1.x);
-                dmma_884(af.x, bf.y, d0.y, d1.y);
-                dmma_884(af.y, bf.x, d0.y, d1.y);
-                if (r < f && cl < f) S[r + cl * ld] = d0;
-                if (r < f && cl + 1 < f) S[r + (cl + 1) * ld] = d1;
             }
             __syncthreads();
         }
-    } else {
-        if (warp == 0 && s > 0) take_pivot(0);
+        if (PIV && tid < NB) rowat[tid] = tid;
+        for (int k = tid; k < sp; k += NTH) rd[k] = mk(R(1), R(0));
         __syncthreads();
-        // Each lane holds its rows of the scaled L column k in registers for the
-        // whole step (SROWS x 32 >= the level's largest front), so an entry's
-        // update reads shared memory once, not twice.
-        for (int k = 0; k < s; ++k) {
-            const int m = f - k - 1;
-            C lk[SROWS];
+        if (tid < pad) S[(s + tid) * (ld + 1)] = mk(R(1), R(0));   // decoupled unit pivots
 #pragma unroll
-            for (int q = 0; q < SROWS; ++q) {
-                const int ii = lane + 32 * q;
-                lk[q] = ii < m ? S[k + 1 + ii + k * ld] : czero<C>();
-            }
-            for (int jj = warp; jj < m; jj += nw) {
-                C *col = S + (k + 1 + jj) * ld;
-                const C u = col[k];
-#pragma unroll
-                for (int q = 0; q < SROWS; ++q) {
-                    const int ii = lane + 32 * q;
-                    if (ii < m) cfms(col[k + 1 + ii], lk[q], u);
-                }
-                if (jj == 0 && k + 1 < s) {   // warp 0 just finished column k + 1
-                    __syncwarp();
-                    take_pivot(k + 1);
-                }
-            }
-            __syncthreads();
-        }
-    }
-
-    // inverses of the NB x NB diagonal blocks: L^-1 strictly below the
-    // diagonal (unit diagonal implied), U^-1 on and above it
-    for (int k0 = 0; k0 < s; k0 += NB) {
-        const int kb = min(NB, s - k0);
-        auto D = [&](int r, int q) { return S[(k0 + r) + (k0 + q) * ld]; };
-        if (tid < kb) {
-            const int c = tid;
-            for (int r = c + 1; r < kb; ++r) {
-                C acc = D(r, c);
-                for (int q = c + 1; q < r; ++q) cfma(acc, D(r, q), Dinv[q][c]);
-                Dinv[r][c] = mk(-acc.x, -acc.y);
-            }
-        } else if (tid >= 32 && tid < 32 + kb) {
-            const int c = tid - 32;
-            Dinv[c][c] = rd[k0 + c];
-            for (int r = c - 1; r >= 0; --r) {
-                C acc = czero<C>();
-                for (int q = r + 1; q <= c; ++q) cfma(acc, D(r, q), Dinv[q][c]);
-                Dinv[r][c] = cmul(mk(-acc.x, -acc.y), rd[k0 + r]);
-            }
-        }
-        __syncthreads();
-        for (int t = tid; t < kb * kb; t += SMALL_FT) {
-            const int r = t % kb, c = t / kb;
-            S[(k0 + r) + (k0 + c) * ld] = Dinv[r][c];
-        }
+        for (int x = 0; x < NE; ++x)
+            if (ep[x] >= 0) add_entry(ep[x], ev[x]);
+        for (int e = tid + NE * NTH; e < d.ent_count; e += NTH)
+            add_entry((int)(a.ent_dst[d.ent_first + e] - d.front_off), A[a.ent_src[d.ent_first + e]]);
         __syncthreads();
     }
 
-    for (int j = warp; j < f; j += nw)
-        for (int i = lane; i < f; i += 32) F[i + (size_t)j * f] = S[i + j * ld];
-    if (tid == 0 && npert) atomicAdd(a.npert, (unsigned long long)npert);
+    const R pivtol = (R)(a.pivscale * __longlong_as_double((long long)*a.amax));
+    int np = 0, nsw = 0;   // the panels' warp: the same in every lane
+    // 1. the panel at p0 (one warp): lane l holds pivot row p0 + l in registers,
+    // x[i] its entry in column p + i
+    auto panel = [&](int p0) {
+        C *own = S + p0 + lane;
+        const bool in = p0 + lane < sp;
+        C x[PW8];
+#pragma unroll
+        for (int i = 0; i < PW8; ++i) x[i] = in ? own[(p0 + i) * ld] : czero<C>();
+        int nx = 0;
+        const int pw = min(PW8, s - p0);
+#pragma unroll 1
+        for (int j = 0; j < pw; ++j) {
+            const int p = p0 + j;
+            C piv = mk(__shfl_sync(ALL, x[0].x, j), __shfl_sync(ALL, x[0].y, j));
+            C rp = crcp(piv);
+            if (PIV) {
+                const int key = lane >= j && p0 + lane < s ? lead_bits(cabs2(x[0])) : -1;
+                const int top = __reduce_max_sync(ALL, key);
+                if (cabs2(piv) < (R)a.pivtau2 * from_lead(top, R(0))) {   // warp-uniform
+                    const int arg = __ffs(__ballot_sync(ALL, key == top)) - 1;
+                    if (arg > j) {   // rows p and p0 + arg trade places: the panel's columns here, the others in step 2
+                        const int from = lane == j ? arg : lane == arg ? j : lane;
+#pragma unroll
+                        for (int i = 0; i < PW8; ++i)
+                            x[i] = mk(__shfl_sync(ALL, x[i].x, from), __shfl_sync(ALL, x[i].y, from));
+                        piv = mk(__shfl_sync(ALL, x[0].x, j), __shfl_sync(ALL, x[0].y, j));
+                        if (lane < j) {   // the multipliers stored so far
+                            C *c = S + (p0 + lane) * ld;
+                            const C t = c[p];
+                            c[p] = c[p0 + arg];
+                            c[p0 + arg] = t;
+                        }
+                        if (lane == 0) {
+                            const int t = rowat[p];
+                            rowat[p] = rowat[p0 + arg];
+                            rowat[p0 + arg] = t;
+                            swaps[1 + nx] = p | (p0 + arg) << 16;
+                        }
+                        __syncwarp();
+                        ++nx;
+                        rp = crcp(piv);
+                    }
+                }
+            }
+            if (!(cabs2(piv) >= pivtol * pivtol) || !(pivtol > R(0))) {   // rare, off the chain: rp is formed already
+                piv = static_pivot<R>(piv, pivtol, np);
+                rp = crcp(piv);
+            }
+            const C l = lane > j ? cmul(x[0], rp) : czero<C>();   // rows p and above are final
+            if (in) own[p * ld] = lane > j ? l : lane == j ? piv : x[0];
+            if (lane == j) rd[p] = rp;
+#pragma unroll
+            for (int i = 1; i < PW8; ++i) {   // less the pivot row's entry, from its lane
+                const C v = mk(__shfl_sync(ALL, x[i].x, j), __shfl_sync(ALL, x[i].y, j));
+                cfms(x[i], l, v);
+                x[i - 1] = x[i];
+            }
+            x[PW8 - 1] = czero<C>();
+        }
+        if (PIV && lane == 0) swaps[0] = nx;
+        nsw += nx;
+    };
+    // 3. blocks bi0 .. bi1 - 1 of block column bj in step q: T - a b, or its
+    // special forms on the panel's row and column and the finished parts of
+    // the inverses
+    const int g = lane >> 2, kq = lane & 3;
+    auto column = [&](int q, int bj, int bi0, int bi1) {
+        const bool rj = bj >= npb;   // ring columns
+        if (rj) bi0 = max(bi0, q + 1);                  // (U12 above is final)
+        else if (bj < q) bi0 = max(bi0, q), bi1 = min(bi1, npb);
+        else if (bj == q) bi1 = min(bi1, npb);          // (L21 is final)
+        if (bi0 >= bi1) return;
+        const int c = 8 * bj + 2 * kq, nc = fp - 8 * bj;
+        const bool in0 = c < fp, in1 = c + 1 < fp;
+        BlockCol<C> b;
+        b.load(rj ? S + q * PW8 + 8 * bj * ld : Bb + 8 * bj * 12, rj ? ld : 12, nc, lane);
+        const C *paA = Ab + BlockCol<C>::left(sa, lane), *paS = S + q * PW8 * ld + BlockCol<C>::left(ld, lane);
+        C *t = S + 8 * bi0 + g + c * ld;
+#pragma unroll 1
+        for (int bi = bi0; bi < bi1; ++bi, t += PW8) {
+            C a0 = czero<C>(), a1 = czero<C>();
+            if (bi <= q && bj <= q) {   // X's row q, L_q^-1; Z's column q, U_q^-1 (bi == q or bj == q)
+                const bool x0 = bi == q && (bj < q || g > 2 * kq), x1 = bi == q && (bj < q || g > 2 * kq + 1);
+                a0 = x0 ? Bb[c * 12 + g] : Ab[2 * kq * sa + 8 * bi + g];
+                a1 = x1 ? Bb[(c + 1) * 12 + g] : Ab[(2 * kq + 1) * sa + 8 * bi + g];
+            } else {
+                if (bi != q && bj != q) {
+                    if (in0) a0 = t[0];
+                    if (in1) a1 = t[ld];
+                }
+                const bool ri = bi >= npb;
+                b.sub((ri ? paS : paA) + 8 * bi, ri ? ld : sa, a0, a1);
+            }
+            if (in0) t[0] = a0;
+            if (in1) t[ld] = a1;
+        }
+    };
+
+    // q = -1: the first panel alone
+    const int nseg = 1 + (nb - npb + 3) / 4;   // pieces of a block column: its pivot rows, four blocks of ring rows each
+#pragma unroll 1
+    for (int q = npb > 0 ? -1 : 0; q < npb; ++q) {
+        const int p0 = q * PW8, p1 = p0 + PW8;
+        if (q >= 0) {
+            __syncthreads();
+            // 2. a and b (the panel's own rows and columns take the identity)
+            const C *Tq = S + p0 + p0 * ld;
+            constexpr int HALF = NTH / 2;
+            if (tid < HALF) {
+                for (int r = tid; r < fp; r += HALF) {
+                    C v[PW8];
+                    const int ql = r - p0;
+#pragma unroll
+                    for (int j = 0; j < PW8; ++j)
+                        v[j] = ql >= 0 && ql < PW8 ? mk(R(j == ql), R(0)) : S[r + (p0 + j) * ld];
+                    if (!(r >= p1 && r < min(sp, p0 + 32))) {   // (the panel's lanes hold their multipliers already)
+#pragma unroll
+                        for (int i = 0; i < PW8; ++i) {
+                            v[i] = cmul(v[i], rd[p0 + i]);
+#pragma unroll
+                            for (int j = i + 1; j < PW8; ++j) cfms(v[j], v[i], Tq[i + j * ld]);
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < PW8; ++j) {
+                        if (r < sp) Ab[j * sa + r] = v[j];
+                        else S[r + (p0 + j) * ld] = v[j];
+                    }
+                }
+            } else {
+                const int nx = PIV ? swaps[0] : 0;
+                for (int c = tid - HALF; c < fp; c += HALF) {
+                    C v[PW8];
+                    const int ql = c - p0;
+                    const bool mid = ql >= 0 && ql < PW8;
+                    C *col = S + c * ld;
+                    if (PIV && !mid)
+                        for (int x = 0; x < nx; ++x) {
+                            const int w = swaps[1 + x], u = w & 0xffff, z = w >> 16;
+                            const C t = col[u];
+                            col[u] = col[z];
+                            col[z] = t;
+                        }
+#pragma unroll
+                    for (int j = 0; j < PW8; ++j) v[j] = mid ? mk(R(j == ql), R(0)) : col[p0 + j];
+#pragma unroll
+                    for (int i = 0; i + 1 < PW8; ++i)
+#pragma unroll
+                        for (int j = i + 1; j < PW8; ++j) cfms(v[j], Tq[j + i * ld], v[i]);
+#pragma unroll
+                    for (int j = 0; j < PW8; ++j) {
+                        if (c < sp) Bb[c * 12 + j] = v[j];
+                        else col[p0 + j] = v[j];
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        const bool more = q + 1 < npb, ahead = more && wi == 0;   // one warp goes on with the next panel
+        if (q >= 0) {
+            const int e1 = ahead ? 0 : nb * nseg, step = ahead ? 1 : more ? NW - 1 : NW;
+#pragma unroll 1
+            for (int e = ahead ? -1 : more ? wi - 1 : wi; e < e1; e += step) {
+                int bj = q + 1, b0 = q + 1, b1 = npb;   // ahead: the next panel's pivot blocks
+                if (!ahead) {
+                    const int seg = e % nseg;
+                    bj = nb - 1 - e / nseg;
+                    b0 = seg ? npb + 4 * (seg - 1) : 0;
+                    b1 = seg ? min(nb, b0 + 4) : more && bj == q + 1 ? q + 1 : npb;
+                }
+                column(q, bj, b0, b1);
+            }
+        }
+        if (ahead) {
+            __syncwarp();
+            panel(p1);
+        }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int j = warp; j < f; j += GB * NW) {
+        C v[GB][NR];
+#pragma unroll
+        for (int w = 0; w < GB; ++w)
+#pragma unroll
+            for (int u = 0; u < NR; ++u) {
+                const int jw = j + w * NW, i = lane + 32 * u;
+                if (jw < f && i < f) v[w][u] = S[(i < s ? i : i + sp - s) + (jw < s ? jw : jw + sp - s) * ld];
+            }
+#pragma unroll
+        for (int w = 0; w < GB; ++w)
+#pragma unroll
+            for (int u = 0; u < NR; ++u) {
+                const int jw = j + w * NW, i = lane + 32 * u;
+                if (jw < f && i < f) F[i + (size_t)jw * f] = v[w][u];
+            }
+    }
+    if (PIV && tid < s) a.pivsrc[fz * (size_t)a.s.n + a.s.vars[d.var_off + tid]] = (unsigned char)rowat[tid];
+    if (wi == 0 && lane == 0) {
+        if (np) atomicAdd(a.npert, (unsigned long long)np);
+        if (PIV && nsw) atomicAdd(a.nswap, (unsigned long long)nsw);
+    }
 }
 
-constexpr size_t SMALL_FACTOR_SMEM = 100 << 10;
-
+// Levels whose fronts take static pivots: those of at most 100 KB.  (The
+// larger fronts' levels exchange rows; the line is the one the exchanges were
+// measured with: with them on the levels above it the direct solves' worst
+// residual on the 841 x 227 operators fell from 3.1e-11 to 1.5e-11, on the
+// lower levels a replay finds nothing more to gain.)
 template <class R>
-static size_t small_factor_smem(int fmax) {
-    const int ld = fmax + 1;
-    return ((size_t)ld * fmax + fmax) * sizeof(cplx<R>);
+static bool static_pivot_level(const LevelInfo &L) {
+    const int f = L.max_front;
+    return L.count > 0 && f <= 128 && ((size_t)(f + 1) * f + f) * sizeof(cplx<R>) <= (size_t)100 << 10;
 }
 
+// Row exchanges happen on every other level
 template <class R>
-bool small_factor_level(const LevelInfo &L) {   // (the shared-memory bound keeps fronts below 4 x 32 rows)
-    return L.count > 0 && L.max_front <= 128 && small_factor_smem<R>(L.max_front) <= SMALL_FACTOR_SMEM;
+bool level_pivots(const LevelInfo &L) {
+    return L.count > 0 && !static_pivot_level<R>(L);
 }
+template bool level_pivots<double>(const LevelInfo &);
+template bool level_pivots<float>(const LevelInfo &);
 
 template <class R>
-void launch_factor_small(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_t st) {
+bool front_factor_level(const LevelInfo &L) {
+    return L.count > 0 && (size_t)L.front_words * sizeof(cplx<R>) <= FRONT_SMEM &&
+           L.max_front + PW8 - 1 <= 128 && (L.max_piv <= NB || static_pivot_level<R>(L));
+}
+
+// Size classes of a level whose nodes are ordered by front size, largest
+// first: a class is closed where the next front's shared memory lets more
+// fronts share an SM, once it holds kMinClass fronts.
+constexpr int kMinClass = 1024;
+std::vector<FrontClass> front_classes(const NodeDesc *desc, int count, size_t csize) {
+    std::vector<FrontClass> out;
+    auto fit = [](size_t bytes) { return (int)std::min<size_t>(16, (FRONT_SMEM + 1024) / (bytes + 1024)); };
+    for (int t = 0; t < count; ++t) {
+        const int f = desc[t].nfront, s = desc[t].npiv;
+        const size_t bytes = front_words(front_fp(f, s), front_sp(s)) * csize;
+        if (out.empty() || (out.back().count >= kMinClass && fit(bytes) > fit(out.back().smem)))
+            out.push_back(FrontClass{t, 0, 0, 0});
+        FrontClass &c = out.back();
+        ++c.count;
+        c.max_rows = std::max(c.max_rows, front_ld(front_fp(f, s)) - 1);
+        c.smem = std::max(c.smem, bytes);
+    }
+    return out;
+}
+
+template <class R, int NTH, bool PIV>
+static void launch_front_class(const FactorArgs<R> &a, const LevelInfo &L, const FrontClass &c, cudaStream_t st) {
     static bool attr_set = false;
     if (!attr_set) {
-        cudaFuncSetAttribute(k_factor_small<R, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMALL_FACTOR_SMEM);
-        cudaFuncSetAttribute(k_factor_small<R, 3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMALL_FACTOR_SMEM);
-        cudaFuncSetAttribute(k_factor_small<R, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMALL_FACTOR_SMEM);
-        if (sizeof(R) == 8)
-            cudaFuncSetAttribute(k_factor_small<R, 2, sizeof(R) == 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)SMALL_FACTOR_SMEM);
+        cudaFuncSetAttribute(k_factor_front<R, NTH, PIV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FRONT_SMEM);
         attr_set = true;
     }
-    const size_t smem = small_factor_smem<R>(L.max_front);
-    const dim3 grid(L.count, a.nf);
-    const int ld = L.max_front + 1;
-    // the blocked complex128 LU pays on fronts with many pivots (the leaf
-    // level: 5.4 -> 4.6 ms); with 7-13 pivots its one-warp panels are slower
-    // GM_BLOCKED_LU_MIN_PIV=<n> moves the threshold (a large n: the
-    // per-pivot kernel everywhere)
-    static const int min_piv = [] {
-        const char *v = std::getenv("GM_BLOCKED_LU_MIN_PIV");
-        return v ? std::atoi(v) : 16;
-    }();
-    if (sizeof(R) == 8 && L.max_piv >= min_piv && L.max_front <= 64)   // (the blocked panel holds 64 rows)
-        (k_factor_small<R, 2, sizeof(R) == 8><<<grid, SMALL_FT, smem, st>>>(a, L.first, ld), note_launch());
-    else if (L.max_front <= 64) (k_factor_small<R, 2, false><<<grid, SMALL_FT, smem, st>>>(a, L.first, ld), note_launch());
-    else if (L.max_front <= 96) (k_factor_small<R, 3, false><<<grid, SMALL_FT, smem, st>>>(a, L.first, ld), note_launch());
-    else (k_factor_small<R, 4, false><<<grid, SMALL_FT, smem, st>>>(a, L.first, ld), note_launch());
+    (k_factor_front<R, NTH, PIV><<<dim3(c.count, a.nf), NTH, c.smem, st>>>(a, L.first + c.first), note_launch());
 }
 
-template bool small_factor_level<double>(const LevelInfo &);
-template bool small_factor_level<float>(const LevelInfo &);
-template void launch_factor_small<double>(const FactorArgs<double> &, const LevelInfo &, cudaStream_t);
-template void launch_factor_small<float>(const FactorArgs<float> &, const LevelInfo &, cudaStream_t);
+// Threads per front: 128 up to 64 rows (several fronts per SM hide each
+// other's chains), 256 up to 96 and 512 up to 128, where one or two fronts
+// fill the SM.
+template <class R>
+void launch_factor_front(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_t st) {
+    const bool piv = level_pivots<R>(L) && a.pivsrc && a.pivtau2 > 0;
+    for (const FrontClass &c : L.classes) {
+        if (piv) {
+            if (c.max_rows <= 64) launch_front_class<R, 128, true>(a, L, c, st);
+            else if (c.max_rows <= 96) launch_front_class<R, 256, true>(a, L, c, st);
+            else launch_front_class<R, 512, true>(a, L, c, st);
+        } else {
+            if (c.max_rows <= 64) launch_front_class<R, 128, false>(a, L, c, st);
+            else if (c.max_rows <= 96) launch_front_class<R, 256, false>(a, L, c, st);
+            else launch_front_class<R, 512, false>(a, L, c, st);
+        }
+    }
+}
+
+template bool front_factor_level<double>(const LevelInfo &);
+template bool front_factor_level<float>(const LevelInfo &);
+template void launch_factor_front<double>(const FactorArgs<double> &, const LevelInfo &, cudaStream_t);
+template void launch_factor_front<float>(const FactorArgs<float> &, const LevelInfo &, cudaStream_t);
+int64_t front_words_of(int f, int s) { return (int64_t)front_words(front_fp(f, s), front_sp(s)); }
 
 // Grid-stride max of |A| with one atomicMax per warp.  Non-negative doubles
 // order like their bit patterns read as unsigned integers.
@@ -1086,7 +1273,7 @@ namespace gm {
 
 // ---------------------------------------------------------------------
 // Mid-level fronts: at most NB pivots and at most MID_FT rows, but too
-// large for the small kernel's whole-front tile.  After the extend-add
+// large for the whole-front kernel.  After the extend-add
 // gather and the operator entries (K2), one CTA per front and frequency
 //   1. factorises the pivot columns (f x s) right-looking with each thread
 //      holding one front row in registers: per pivot, warp 0 picks the
@@ -1152,7 +1339,7 @@ __global__ void __launch_bounds__(MID_FT) k_factor_mid(FactorArgs<R> a, int lvl_
     const NodeDesc d = a.s.desc[lvl_first + blockIdx.x];
     const int f = d.nfront, s = d.npiv, m = f - s;
     if (s == 0) return;   // the gathered front is already the contribution block
-    add_entries(a, lvl_first + blockIdx.x, blockIdx.y);
+    add_entries(a, d, blockIdx.y);
     __syncthreads();   // the entries are visible to the CTA
     const int ldp = f + 1, ldu = s | 1;
     C *P = reinterpret_cast<C *>(smem_raw);
@@ -1298,18 +1485,9 @@ constexpr size_t MID_FACTOR_SMEM = 200 << 10;
 
 template <class R>
 bool mid_factor_level(const LevelInfo &L) {
-    return L.count > 0 && L.max_piv <= NB && L.max_front <= MID_FT && !small_factor_level<R>(L) &&
+    return L.count > 0 && L.max_piv <= NB && L.max_front <= MID_FT &&
            (size_t)L.mid_words * sizeof(cplx<R>) <= MID_FACTOR_SMEM;
 }
-
-// Row exchanges happen on every level but those of the small-front kernel
-// (whose fronts fit shared memory whole: the lower levels)
-template <class R>
-bool level_pivots(const LevelInfo &L) {
-    return L.count > 0 && !small_factor_level<R>(L);
-}
-template bool level_pivots<double>(const LevelInfo &);
-template bool level_pivots<float>(const LevelInfo &);
 
 template <class R, int NPR>
 static void launch_mid(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_t st) {

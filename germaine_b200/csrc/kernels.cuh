@@ -1,6 +1,7 @@
 // Device-side argument blocks and launch wrappers shared by the engine.
 #pragma once
 #include <cstdint>
+#include <vector>
 #include <cuda_runtime.h>
 
 #include "../../include/germaine_gpu.h"
@@ -40,17 +41,20 @@ void launch_assemble(const AsmArgs &a, const float *m0, const float *m1, const A
                      cudaStream_t st);
 
 // ---------------- symbolic structure on the device ----------------
-// what a kernel needs of one front, in level order (one 64-byte load instead
-// of a chain of table look-ups)
+// what a kernel needs of one front, in level order (one record instead of a
+// chain of table look-ups)
 struct alignas(16) NodeDesc {
     int64_t front_off, var_off, inv_off, rhs_off, y_off;
     int64_t cb0, cb1;   // the children's contribution blocks (offsets as front_off), leading dimensions ld0, ld1
-    int node, nfront, npiv, child0, child1, ld0, ld1, pad;
+    int node, nfront, npiv, child0, child1, ld0, ld1, ring0, ring1;   // ring: rows of a child's block
+    int ent_count;      // operator entries owned by the front: ent_dst / ent_src[ent_first ..]
+    int64_t ent_first;
 };
 
 struct DevSym {
     int n, nnodes;
     const NodeDesc *desc;   // [level position], parallel to lvl_nodes
+    const NodeDesc *fdesc;  // the same with every level ordered by front size, largest first
     const int *npiv, *nfront, *child0, *child1, *vars, *inv, *lvl_nodes;
     const int64_t *front_off, *var_off, *inv_off, *rhs_off;
     int64_t front_total, rhs_total;
@@ -61,6 +65,10 @@ struct DevSym {
 };
 
 // ---------------- K2-K4 numeric factorisation ----------------
+struct FrontClass {   // fronts first .. first + count - 1 of a level ordered by front size
+    int first, count, max_rows;
+    size_t smem;      // dynamic shared memory of the class's largest front
+};
 struct LevelInfo {
     int first;      // offset into lvl_nodes
     int count;      // nodes in the level
@@ -68,6 +76,8 @@ struct LevelInfo {
     int64_t ent_first, ent_count;  // level's entry range in ent_dst/ent_src
     int64_t mid_words;  // largest (f + 1) s + (s | 1)(f - s) of the level's fronts: k_factor_mid's tile
     int index;          // the level's height
+    int64_t front_words;               // largest shared-memory need of the whole-front kernel (elements)
+    std::vector<FrontClass> classes;   // its launches, over DevSym::fdesc
 };
 
 // Launches that put a level's fronts on grid.y are split into pieces of at
@@ -100,8 +110,6 @@ struct FactorArgs {
     double pivtau2;
     unsigned char *pivsrc;
     unsigned long long *nswap;
-    const int64_t *ent_lvl_off; // entries of level position t (index into lvl_nodes):
-                                // ent_dst/ent_src[ent_lvl_off[t] .. ent_lvl_off[t + 1])
 };
 
 // max |A| over cnt complex entries into *out (bits of a double; *out must
@@ -112,21 +120,23 @@ void launch_pack_split(double2 *dst, const double *re, const double *im, size_t 
 
 template <class R>
 void launch_factor_level(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_t st);
-// Small fronts: the whole front of every node of the level assembled and
-// factorised in shared memory by one CTA (replaces launch_factor_level and
-// the level's contribution-block GEMM) when small_factor_level(L).
+// Fronts that fit shared memory whole, assembled and factorised by one CTA
+// each (replaces launch_factor_level and the level's contribution-block GEMM)
+// when front_factor_level(L).
 template <class R>
-bool small_factor_level(const LevelInfo &L);
+bool front_factor_level(const LevelInfo &L);
 template <class R>
-void launch_factor_small(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_t st);
-// Levels of fronts with at most NB pivots that do not fit the small kernel:
+void launch_factor_front(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_t st);
+std::vector<FrontClass> front_classes(const NodeDesc *desc, int count, size_t csize);
+int64_t front_words_of(int f, int s);   // shared-memory elements of one front there
+// Levels of fronts with at most NB pivots that do not fit it:
 // gather, operator entries, then one CTA per front factorises the pivot
 // panel in shared memory and applies the Schur update to the contribution
 // block (replaces the K3 / K4 steps and the level's contribution GEMM).
 template <class R>
 bool mid_factor_level(const LevelInfo &L);
 // the level's factorisation exchanges rows (FactorArgs::pivsrc) when
-// pivoting is on: every level but the small-front kernel's
+// pivoting is on: every level but the lowest (fronts of at most 100 KB)
 template <class R>
 bool level_pivots(const LevelInfo &L);
 template <class R>
