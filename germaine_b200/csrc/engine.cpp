@@ -190,8 +190,34 @@ extern "C" int gm_engine_create(int device, const gm_config *cfg, gm_engine **ou
                          [](const gm::NodeDesc &x, const gm::NodeDesc &y) { return x.nfront > y.nfront; });
         L.classes = gm::front_classes(fdesc.data() + L.first, L.count, e->csize());
     }
+    // small-front levels by pivot blocks, else in the dissection's order
+    // (neighbouring fronts share rows of x); groups of fewer than 256 fronts
+    // join the next larger
+    std::vector<gm::NodeDesc> sdesc = desc;
+    for (gm::LevelInfo &L : e->levels) {
+        L.groups.clear();
+        if (L.max_piv > 32) continue;
+        int p8[5] = {0, 1, 2, 3, 4}, cnt[5] = {0, 0, 0, 0, 0};   // p8[g]: the group that fronts of g blocks join
+        const int top = std::max(1, (L.max_piv + 7) / 8);
+        for (int t = L.first; t < L.first + L.count; ++t) ++cnt[std::max(1, (desc[t].npiv + 7) / 8)];
+        for (int g = 1; g < top; ++g)
+            if (cnt[g] < 256) {
+                cnt[g + 1] += cnt[g];
+                for (int q = 1; q <= g; ++q)
+                    if (p8[q] == g) p8[q] = g + 1;
+            }
+        int at = L.first;
+        for (int g = 1; g <= 4; ++g) {
+            const int first = at;
+            for (int t = L.first; t < L.first + L.count; ++t)
+                if (p8[std::max(1, (desc[t].npiv + 7) / 8)] == g) sdesc[at++] = desc[t];
+            if (at > first) L.groups.push_back(gm::PivGroup{first - L.first, at - first, g});
+        }
+    }
     int rc2;
-    if ((rc2 = upload(e->d_desc, desc, e->st)) || (rc2 = upload(e->d_fdesc, fdesc, e->st))) return rc2;
+    if ((rc2 = upload(e->d_desc, desc, e->st)) || (rc2 = upload(e->d_fdesc, fdesc, e->st)) ||
+        (rc2 = upload(e->d_sdesc, sdesc, e->st)))
+        return rc2;
     if ((rc2 = upload(e->d_npiv, s.npiv, e->st)) || (rc2 = upload(e->d_nfront, s.nfront, e->st)) ||
         (rc2 = upload(e->d_child0, s.child0, e->st)) || (rc2 = upload(e->d_child1, s.child1, e->st)) ||
         (rc2 = upload(e->d_vars, s.vars, e->st)) || (rc2 = upload(e->d_inv, s.inv, e->st)) ||
@@ -212,6 +238,7 @@ extern "C" int gm_engine_create(int device, const gm_config *cfg, gm_engine **ou
     d.front_total = s.front_total; d.rhs_total = s.rhs_total;
     d.desc = e->d_desc.as<gm::NodeDesc>();
     d.fdesc = e->d_fdesc.as<gm::NodeDesc>();
+    d.sdesc = e->d_sdesc.as<gm::NodeDesc>();
     d.y_off = e->d_y_off.as<int64_t>(); d.y_total = y_total;
 
     gm_stats &st = e->stats;
@@ -782,7 +809,9 @@ static const unsigned char *build_mask(gm_engine *e, int nrhs, const RhsPattern 
     e->work_w.assign(e->levels.size(), tcw_default);
     for (size_t h = 0; h < e->levels.size(); ++h) {
         e->work_off[h] = (int)work.size();
-        const int tcw = tuned && e->lvl_cfg[4 * h + 1] ? 8 * e->lvl_cfg[4 * h + 1] : tcw_default;
+        // (the small-front kernels take 32 columns whatever the tuned width)
+        const int tcw = e->levels[h].max_piv <= 32 ? 32
+                        : tuned && e->lvl_cfg[4 * h + 1] ? 8 * e->lvl_cfg[4 * h + 1] : tcw_default;
         e->work_w[h] = tcw;
         const int nslice = (nrhs + tcw - 1) / tcw;
         const LevelInfo &L = e->levels[h];

@@ -53,7 +53,7 @@ struct gm_engine {
 
     // device copy of the symbolic structure
     gm::DevBuf d_npiv, d_nfront, d_child0, d_child1, d_vars, d_inv, d_lvl_nodes;
-    gm::DevBuf d_front_off, d_var_off, d_inv_off, d_rhs_off, d_y_off, d_tri_off, d_desc, d_fdesc;
+    gm::DevBuf d_front_off, d_var_off, d_inv_off, d_rhs_off, d_y_off, d_tri_off, d_desc, d_fdesc, d_sdesc;
     int64_t tri_total = 0;   // entries of the triangle-inversion scratch per matrix
     gm::DevBuf d_ent_dst, d_ent_src;
     std::vector<gm::LevelInfo> levels;

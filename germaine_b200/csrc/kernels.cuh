@@ -55,6 +55,7 @@ struct DevSym {
     int n, nnodes;
     const NodeDesc *desc;   // [level position], parallel to lvl_nodes
     const NodeDesc *fdesc;  // the same with every level ordered by front size, largest first
+    const NodeDesc *sdesc;  // the same with every level ordered by pivot blocks (LevelInfo::groups)
     const int *npiv, *nfront, *child0, *child1, *vars, *inv, *lvl_nodes;
     const int64_t *front_off, *var_off, *inv_off, *rhs_off;
     int64_t front_total, rhs_total;
@@ -65,6 +66,9 @@ struct DevSym {
 };
 
 // ---------------- K2-K4 numeric factorisation ----------------
+// fronts first .. first + count - 1 of a level in DevSym::sdesc, with at most
+// 8 p8 pivots each
+struct PivGroup { int first, count, p8; };
 struct FrontClass {   // fronts first .. first + count - 1 of a level ordered by front size
     int first, count, max_rows;
     size_t smem;      // dynamic shared memory of the class's largest front
@@ -78,6 +82,7 @@ struct LevelInfo {
     int index;          // the level's height
     int64_t front_words;               // largest shared-memory need of the whole-front kernel (elements)
     std::vector<FrontClass> classes;   // its launches, over DevSym::fdesc
+    std::vector<PivGroup> groups;      // levels with at most 32 pivots: fronts by pivot blocks, over DevSym::sdesc
 };
 
 // Launches that put a level's fronts on grid.y are split into pieces of at

@@ -27,6 +27,7 @@
 // trans = 1 solves M^T x = b with the same factors: M^T = U^T L^T, the
 // forward pass runs with U^T and the backward pass with L^T; only the
 // factor indexing and which stored inverse is used change.
+#include <algorithm>
 #include <cstdlib>
 
 #include "solve_tile.cuh"
@@ -72,10 +73,11 @@ struct Ctx {
 };
 
 template <class R, int TC>
-__device__ __forceinline__ Ctx<R> make_ctx(const SolveArgs<R> &a, int lvl_first, int chunk, int pos = -1) {
+__device__ __forceinline__ Ctx<R> make_ctx(const SolveArgs<R> &a, int lvl_first, int chunk, int pos = -1,
+                                           const NodeDesc *desc = nullptr) {
     using C = cplx<R>;
     Ctx<R> c;
-    const NodeDesc d = a.s.desc[lvl_first + (pos < 0 ? (int)blockIdx.y : pos)];
+    const NodeDesc d = (desc ? desc : a.s.desc)[lvl_first + (pos < 0 ? (int)blockIdx.y : pos)];
     c.node = d.node;
     c.f = d.nfront;
     c.s = d.npiv;
@@ -354,6 +356,30 @@ __global__ void __launch_bounds__(NT) k_bwd_tri(SolveArgs<R> a, int lvl_first, i
 // 841 x 227, 10 matrices x 100 right-hand sides, complex64 forward levels 0-6:
 // 18.0 -> 14.4 ms over three passes against the unbounded 118 registers.)
 //
+// P8: the largest pivot count of the launch's fronts in blocks of 8 (1 .. 4);
+// the operand tiles and accumulators follow it.  These kernels wait for global
+// loads most of the time, so what counts is how many fronts an SM holds: six
+// with 80 registers, eight with 64, ten with 51.  Measured at 841 x 227 (10
+// matrices x 100 right-hand sides), backward levels 0-4, complex128:
+// 2.78, 0.83, 0.83, 0.57, 0.39 ms with one kernel of 32 pivot rows dealt to
+// the warps by rows; 2.64, 0.76, 0.75, 0.52, 0.35 dealt by columns;
+// 2.47, 0.57, 0.57, 0.43, 0.30 in these sizes, a level's fronts grouped by
+// theirs.
+template <class C, int P8>
+struct FwdSmall {
+    C L[8 * P8][SNB + SPAD];    // factor rows, [pivot][row]
+    C Y[8 * P8][32 + SPAD];     // pivot rows, [pivot][rhs]
+};
+template <class C, int P8>
+struct BwdSmall {
+    C L[SNB][8 * P8 + SPAD];    // factor tile, [column][pivot row]
+    C Y[SNB][32 + SPAD];        // right operand, [column][rhs]
+};
+template <class R, int P8>
+constexpr int small_ctas(bool fwd) {
+    return sizeof(R) == 8 ? (P8 == 4 ? 6 : P8 == 3 ? 7 : P8 == 2 || fwd ? 8 : 10) : P8 == 4 ? 9 : fwd ? 12 : 10;
+}
+
 // Forward pass of a whole front whose pivots fit one 32-pivot block (the
 // small fronts of the lower levels): the children's update vectors are added
 // into x at the pivots, y = Dinv x_piv is formed in shared memory and written
@@ -362,15 +388,15 @@ __global__ void __launch_bounds__(NT) k_bwd_tri(SolveArgs<R> a, int lvl_first, i
 // memory -- k_fwd_tri and k_fwd_ring in one CTA, y read once.
 // wofs >= 0: the CTA's (front position, slice) is work[wofs + blockIdx.x],
 // the live pairs of a pruned pass; wofs < 0: (blockIdx.y, blockIdx.x).
-template <class R, bool TRANS, int B>
-__global__ void __launch_bounds__(NT, 6) k_fwd_small(SolveArgs<R> a, int lvl_first, int wofs) {
+template <class R, bool TRANS, int P8>
+__global__ void __launch_bounds__(NT, small_ctas<R, P8>(true)) k_fwd_small(SolveArgs<R> a, int lvl_first, int wofs) {
     using C = cplx<R>;
-    constexpr int RT = 32;
+    constexpr int RT = 32, B = 4;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    SolveSmem<C, RT, B> &sm = *reinterpret_cast<SolveSmem<C, RT, B> *>(smem_raw);
+    FwdSmall<C, P8> &sm = *reinterpret_cast<FwdSmall<C, P8> *>(smem_raw);
     constexpr int TC = 8 * B;
     const int2 wk = wofs >= 0 ? a.work[wofs + blockIdx.x] : make_int2((int)blockIdx.y, (int)blockIdx.x);
-    const Ctx<R> c = make_ctx<R, TC>(a, lvl_first, wk.y, wk.x);
+    const Ctx<R> c = make_ctx<R, TC>(a, lvl_first, wk.y, wk.x, wofs >= 0 ? a.s.desc : a.s.sdesc);
     if (c.rn <= 0) return;
     const int r0 = wk.y * TC;
     if (!live(a, c.node, r0, c.rn)) return;   // y and the update vector are zero
@@ -392,15 +418,14 @@ __global__ void __launch_bounds__(NT, 6) k_fwd_small(SolveArgs<R> a, int lvl_fir
         if (threadIdx.x < s) prow[threadIdx.x] = a.pivsrc[solve_matrix(a) * (size_t)a.s.n + c.vars[threadIdx.x]];
         __syncthreads();
     }
-    TileAcc<C, RT, B> acc;
+    BlockTile<C> acc(c.rn, wk.x);
     if (s > 0) {
-        stage_dinv<C, true, TRANS, RT, B>(sm, c.F, c.f, 0, s);
-        stage_rows(sm, [&](int q) { return c.X + (size_t)c.vars[pv ? prow[q] : q] * ldr; }, s, c.rn);
+        stage_dinv_p<C, true, TRANS, RT>(sm.L, c.F, c.f, 0, s, 0, s, threadIdx.x, NT);
+        stage_rows_p<C, TC>(sm.Y, [&](int q) { return c.X + (size_t)c.vars[pv ? prow[q] : q] * ldr; }, s, c.rn, threadIdx.x, NT);
         staged_sync();
-        zero_acc(acc);
-        tile_mma<TRI_LOWER>(sm, s, acc, s, c.rn);   // y = Dinv x_piv
+        block_mma<TRI_LOWER>(sm.L, sm.Y, s, acc, s, c.rn);   // y = Dinv x_piv
         __syncthreads();
-        for_acc(acc, s, c.rn, threadIdx.x, [&](int row, int col, const C &v) { sm.Y[row][col] = v; });
+        acc.each(s, c.rn, [&](int row, int col, const C &v) { sm.Y[row][col] = v; });
         __syncthreads();
         for (int t = threadIdx.x; t < s * TC; t += NT) {
             const int q = t / TC, r = t % TC;
@@ -410,11 +435,11 @@ __global__ void __launch_bounds__(NT, 6) k_fwd_small(SolveArgs<R> a, int lvl_fir
     // w over the ring rows, 32-row tiles, y staying in sm.Y
     for (int i0 = s; i0 < c.f; i0 += RT) {
         const int rows = min(RT, c.f - i0);
-        stage_factor<C, TRANS, RT, B>(sm, c.F, c.f, i0, rows, 0, s);
+        stage_factor_p<C, TRANS, RT, 8 * P8>(sm.L, c.F, c.f, i0, rows, 0, s, threadIdx.x, NT);
         staged_sync();
-        zero_acc(acc);
-        tile_mma(sm, s, acc, rows, c.rn);
-        for_acc(acc, rows, c.rn, threadIdx.x, [&](int row, int r, const C &v) {
+        acc.zero();
+        block_mma<0>(sm.L, sm.Y, s, acc, rows, c.rn);
+        acc.each(rows, c.rn, [&](int row, int r, const C &v) {
             const int i = i0 + row;
             const int q0 = W0 ? inv[i] : -1, q1 = W1 ? inv[c.f + i] : -1;
             C g = czero<C>();
@@ -431,14 +456,14 @@ __global__ void __launch_bounds__(NT, 6) k_fwd_small(SolveArgs<R> a, int lvl_fir
 // the product accumulated in registers over 32-column ring blocks, t placed
 // in shared memory, then x_piv = Dinv t -- k_bwd_ring and k_bwd_tri in one
 // CTA, without writing t to x in between.
-template <class R, bool TRANS, int B>
-__global__ void __launch_bounds__(NT, 6) k_bwd_small(SolveArgs<R> a, int lvl_first) {
+template <class R, bool TRANS, int P8>
+__global__ void __launch_bounds__(NT, small_ctas<R, P8>(false)) k_bwd_small(SolveArgs<R> a, int lvl_first) {
     using C = cplx<R>;
-    constexpr int RT = 32;
+    constexpr int RT = 8 * P8, B = 4;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    SolveSmem<C, RT, B> &sm = *reinterpret_cast<SolveSmem<C, RT, B> *>(smem_raw);
+    BwdSmall<C, P8> &sm = *reinterpret_cast<BwdSmall<C, P8> *>(smem_raw);
     constexpr int TC = 8 * B;
-    const Ctx<R> c = make_ctx<R, TC>(a, lvl_first, blockIdx.x);
+    const Ctx<R> c = make_ctx<R, TC>(a, lvl_first, blockIdx.x, -1, a.s.sdesc);
     if (c.rn <= 0 || c.s == 0) return;
     const size_t ldr = a.ldr;
     const int s = c.s;   // <= SNB (launch condition)
@@ -448,14 +473,13 @@ __global__ void __launch_bounds__(NT, 6) k_bwd_small(SolveArgs<R> a, int lvl_fir
     __shared__ unsigned char prow[SNB];
     const bool pv = TRANS && a.pivsrc;
     if (pv && threadIdx.x < s) prow[threadIdx.x] = a.pivsrc[solve_matrix(a) * (size_t)a.s.n + c.vars[threadIdx.x]];
-    TileAcc<C, RT, B> acc;
-    zero_acc(acc);
+    BlockTile<C, (P8 < 2 ? 2 : P8)> acc(c.rn, blockIdx.y);
     for (int j0 = s; j0 < c.f; j0 += SNB) {
         const int jb = min(SNB, c.f - j0);
-        stage_factor<C, TRANS, RT, B>(sm, c.F, c.f, 0, s, j0, jb);
-        stage_rows(sm, [&](int q) { return c.X + (size_t)c.vars[j0 + q] * ldr; }, jb, c.rn);
+        stage_factor_p<C, TRANS, RT, SNB>(sm.L, c.F, c.f, 0, s, j0, jb, threadIdx.x, NT);
+        stage_rows_p<C, TC>(sm.Y, [&](int q) { return c.X + (size_t)c.vars[j0 + q] * ldr; }, jb, c.rn, threadIdx.x, NT);
         staged_sync();
-        tile_mma(sm, jb, acc, s, c.rn);
+        block_mma<0>(sm.L, sm.Y, jb, acc, s, c.rn);
         __syncthreads();
     }
     // t = y - acc in sm.Y (row q of the next product's right operand = pivot
@@ -469,16 +493,16 @@ __global__ void __launch_bounds__(NT, 6) k_bwd_small(SolveArgs<R> a, int lvl_fir
             else sm.Y[q][r] = czero<C>();
         }
     } else {
-        stage_rows(sm, [&](int q) { return c.X + (size_t)c.vars[q] * ldr; }, s, c.rn);
+        stage_rows_p<C, TC>(sm.Y, [&](int q) { return c.X + (size_t)c.vars[q] * ldr; }, s, c.rn, threadIdx.x, NT);
     }
-    stage_dinv<C, false, TRANS, RT, B>(sm, c.F, c.f, 0, s);
+    stage_dinv_p<C, false, TRANS, RT>(sm.L, c.F, c.f, 0, s, 0, s, threadIdx.x, NT);
     staged_sync();
-    for_acc(acc, s, c.rn, threadIdx.x, [&](int row, int col, const C &v) { sm.Y[row][col] = csub(sm.Y[row][col], v); });
+    acc.each(s, c.rn, [&](int row, int col, const C &v) { sm.Y[row][col] = csub(sm.Y[row][col], v); });
     __syncthreads();
-    zero_acc(acc);
-    tile_mma<TRI_UPPER>(sm, s, acc, s, c.rn);   // x_piv = Dinv t
-    for_acc(acc, s, c.rn, threadIdx.x,
-            [&](int row, int col, const C &v) { c.X[(size_t)c.vars[pv ? prow[row] : row] * ldr + col] = v; });
+    acc.zero();
+    block_mma<TRI_UPPER>(sm.L, sm.Y, s, acc, s, c.rn);   // x_piv = Dinv t
+    acc.each(s, c.rn,
+             [&](int row, int col, const C &v) { c.X[(size_t)c.vars[pv ? prow[row] : row] * ldr + col] = v; });
 }
 
 template <class R, int RT, int B>
@@ -492,6 +516,14 @@ static void set_smem(K kernel, size_t bytes) {
     cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+template <class R, int P8>
+static void set_small_attrs() {
+    set_smem(k_fwd_small<R, false, P8>, sizeof(FwdSmall<cplx<R>, P8>));
+    set_smem(k_fwd_small<R, true, P8>, sizeof(FwdSmall<cplx<R>, P8>));
+    set_smem(k_bwd_small<R, false, P8>, sizeof(BwdSmall<cplx<R>, P8>));
+    set_smem(k_bwd_small<R, true, P8>, sizeof(BwdSmall<cplx<R>, P8>));
+}
+
 template <class R, int RT, int B>
 static void set_attrs() {
     static bool done = false;
@@ -501,6 +533,12 @@ static void set_attrs() {
     set_smem(k_fwd_ring<R, true, RT, B>, sm);
     set_smem(k_bwd_ring<R, false, RT, B>, sm);
     set_smem(k_bwd_ring<R, true, RT, B>, sm);
+    if (RT == 32 && B == 4) {
+        set_small_attrs<R, 1>();
+        set_small_attrs<R, 2>();
+        set_small_attrs<R, 3>();
+        set_small_attrs<R, 4>();
+    }
     if (RT == 32) {
         set_smem(k_fwd_tri<R, false, B>, sm);
         set_smem(k_fwd_tri<R, true, B>, sm);
@@ -508,10 +546,6 @@ static void set_attrs() {
         set_smem(k_bwd_tri<R, true, B>, sm);
         set_smem(k_fwd_rhs<R, false, B>, 0);
         set_smem(k_fwd_rhs<R, true, B>, 0);
-        set_smem(k_fwd_small<R, false, B>, sms);
-        set_smem(k_fwd_small<R, true, B>, sms);
-        set_smem(k_bwd_small<R, false, B>, sms);
-        set_smem(k_bwd_small<R, true, B>, sms);
     }
     done = true;
 }
@@ -547,30 +581,64 @@ static int slice_b(int nrhs) {
 template <class R>
 static int solve_nfz(const SolveArgs<R> &a) { return a.fmap ? a.nfz : a.nf; }
 
+// the live (front, slice) pairs of a pruned forward pass
+template <class R, int P8>
+static void forward_small_work(const SolveArgs<R> &a, const LevelInfo &L, cudaStream_t st) {
+    const int wofs = a.work_off[L.index];
+    const int nlive = a.work_off[L.index + 1] - wofs;
+    if (nlive == 0) return;
+    const size_t smem = sizeof(FwdSmall<cplx<R>, P8>);
+    dim3 g(nlive, 1, solve_nfz(a));
+    if (a.trans) (k_fwd_small<R, true, P8><<<g, NT, smem, st>>>(a, L.first, wofs), note_launch());
+    else (k_fwd_small<R, false, P8><<<g, NT, smem, st>>>(a, L.first, wofs), note_launch());
+}
+
+// one group of a level's fronts
+template <class R, int P8>
+static void small_group(bool fwd, const SolveArgs<R> &a, const LevelInfo &L, const PivGroup &G, cudaStream_t st) {
+    for (int c0 = 0; c0 < G.count; c0 += kMaxGridY) {
+        const int first = L.first + G.first + c0;
+        dim3 g((a.nrhs + 31) / 32, std::min(kMaxGridY, G.count - c0), solve_nfz(a));
+        if (fwd) {
+            const size_t smem = sizeof(FwdSmall<cplx<R>, P8>);
+            if (a.trans) (k_fwd_small<R, true, P8><<<g, NT, smem, st>>>(a, first, -1), note_launch());
+            else (k_fwd_small<R, false, P8><<<g, NT, smem, st>>>(a, first, -1), note_launch());
+        } else {
+            const size_t smem = sizeof(BwdSmall<cplx<R>, P8>);
+            if (a.trans) (k_bwd_small<R, true, P8><<<g, NT, smem, st>>>(a, first), note_launch());
+            else (k_bwd_small<R, false, P8><<<g, NT, smem, st>>>(a, first), note_launch());
+        }
+    }
+}
+
+template <class R>
+static void small_level(bool fwd, const SolveArgs<R> &a, const LevelInfo &L, cudaStream_t st) {
+    set_attrs<R, 32, 4>();
+    if (fwd && a.work && a.work_w[L.index] == 32) {
+        if (L.max_piv <= 8) forward_small_work<R, 1>(a, L, st);
+        else if (L.max_piv <= 16) forward_small_work<R, 2>(a, L, st);
+        else if (L.max_piv <= 24) forward_small_work<R, 3>(a, L, st);
+        else forward_small_work<R, 4>(a, L, st);
+        return;
+    }
+    for (const PivGroup &G : L.groups) {
+        if (G.p8 == 1) small_group<R, 1>(fwd, a, L, G, st);
+        else if (G.p8 == 2) small_group<R, 2>(fwd, a, L, G, st);
+        else if (G.p8 == 3) small_group<R, 3>(fwd, a, L, G, st);
+        else small_group<R, 4>(fwd, a, L, G, st);
+    }
+}
+
 // Levels with at most 32 pivots per front take the fused small-front kernels
-// whatever the tile height; the others the four kernels above, RT being the
-// tile height of their ring parts.
+// in 32-column slices whatever the tile height and slice width; the others the
+// four kernels above, RT being the tile height of their ring parts.
 template <class R, int RT, int B>
 static void forward_level(const SolveArgs<R> &a, const LevelInfo &L, cudaStream_t st) {
     set_attrs<R, 32, B>();
     set_attrs<R, RT, B>();
-    const size_t smem = solve_smem<R, 32, B>();
     const int nchunk = (a.nrhs + 8 * B - 1) / (8 * B);
     if (L.max_piv <= SNB) {   // one pivot block per front: fused pivot + ring kernel
-        if (a.work && a.work_w[L.index] == 8 * B) {   // pruned pass: only the live (front, slice) pairs
-            const int wofs = a.work_off[L.index];
-            const int nlive = a.work_off[L.index + 1] - wofs;
-            if (nlive == 0) return;
-            dim3 g(nlive, 1, solve_nfz(a));
-            if (a.trans) (k_fwd_small<R, true, B><<<g, NT, smem, st>>>(a, L.first, wofs), note_launch());
-            else (k_fwd_small<R, false, B><<<g, NT, smem, st>>>(a, L.first, wofs), note_launch());
-            return;
-        }
-        for_level_pieces(L, [&](int first, int count) {
-            dim3 g(nchunk, count, solve_nfz(a));
-            if (a.trans) (k_fwd_small<R, true, B><<<g, NT, smem, st>>>(a, first, -1), note_launch());
-            else (k_fwd_small<R, false, B><<<g, NT, smem, st>>>(a, first, -1), note_launch());
-        });
+        small_level<R>(true, a, L, st);
         return;
     }
     const int nblk = (L.max_piv + SNB - 1) / SNB;
@@ -598,11 +666,7 @@ static void backward_level(const SolveArgs<R> &a, const LevelInfo &L, cudaStream
     set_attrs<R, RT, B>();
     const int nchunk = (a.nrhs + 8 * B - 1) / (8 * B);
     if (L.max_piv <= SNB) {   // one pivot block per front: fused ring + pivot kernel
-        for_level_pieces(L, [&](int first, int count) {
-            dim3 g(nchunk, count, solve_nfz(a));
-            if (a.trans) (k_bwd_small<R, true, B><<<g, NT, solve_smem<R, 32, B>(), st>>>(a, first), note_launch());
-            else (k_bwd_small<R, false, B><<<g, NT, solve_smem<R, 32, B>(), st>>>(a, first), note_launch());
-        });
+        small_level<R>(false, a, L, st);
         return;
     }
     const int nblk = (L.max_piv + SNB - 1) / SNB;

@@ -238,6 +238,114 @@ __device__ __forceinline__ void tile_mma(const SolveSmem<C, RT, B> &sm, int qb, 
     tile_mma_p<TRI, RT, B>(sm.L, sm.Y, qb, acc, rows, rn, threadIdx.x);
 }
 
+// 32 x 32 output tile of the small-front kernels in 8 x 8 blocks, dealt to
+// the four warps by columns (warp w: block column w, every row block) or, in
+// slices of at most 16 columns, by rows.  By rows alone a front of 6 pivots
+// kept one warp busy and one of 20 three -- and always the same ones, so that
+// one of the SM's four schedulers carried the level.
+// (NB8: blocks per warp kept, at least 2 for the slices dealt by rows)
+template <class C, int NB8 = 4>
+struct BlockTile {
+    static constexpr int N = NB8;
+    C v[N][2];   // this lane's two entries of the warp's blocks
+    bool bycol;
+    int w, lane;
+    // (by rows: the first row block goes to another warp in every front)
+    __device__ __forceinline__ BlockTile(int rn, int turn) {
+        lane = threadIdx.x & 31;
+        bycol = rn > 16;
+        w = (threadIdx.x >> 5) + (bycol ? 0 : turn) & 3;
+        zero();
+    }
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int i = 0; i < N; ++i) v[i][0] = v[i][1] = czero<C>();
+    }
+    __device__ __forceinline__ int row(int i) const { return 8 * (bycol ? i : w) + (lane >> 2); }
+    __device__ __forceinline__ int col(int i, int e) const {
+        return 8 * (bycol ? w : i) + (sizeof(C) == 16 ? 2 * (lane & 3) + e : (lane & 3) + 4 * e);
+    }
+    // f(row, col, value) over the lane's entries with row < rows, col < rn
+    template <class F>
+    __device__ __forceinline__ void each(int rows, int rn, F f) {
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                if (row(i) < rows && col(i, e) < rn) f(row(i), col(i, e), v[i][e]);
+    }
+};
+
+// one 8 x 8 block += its operands' fragments at pivots k0 .. k0 + 3 (complex128)
+__device__ __forceinline__ void block_mac(double2 *d, const double2 &a, const double2 &b) {
+    dmma_884(a.x, b.x, d[0].x, d[1].x);
+    dmma_884(-a.y, b.y, d[0].x, d[1].x);
+    dmma_884(a.x, b.y, d[0].y, d[1].y);
+    dmma_884(a.y, b.x, d[0].y, d[1].y);
+}
+
+// acc += L'[rows x qb] Y[qb x rn], operands and TRI as tile_mma_p
+template <int TRI, int LW, int N>
+__device__ __forceinline__ void block_mma(const double2 (*L)[LW], const double2 (*Y)[32 + SPAD], int qb,
+                                          BlockTile<double2, N> &acc, int rows, int rn) {
+    const int g = acc.lane >> 2, w = acc.w;
+    const int n = acc.bycol ? (rows + 7) / 8 : (rn + 7) / 8;   // blocks of this warp
+    if (8 * w >= (acc.bycol ? rn : rows)) return;              // warp-uniform
+    for (int k0 = 0; k0 < qb; k0 += 4) {
+        const int kk = k0 + (acc.lane & 3);
+        const bool kin = kk < qb;
+        if (acc.bycol) {
+            const double2 b = kin ? Y[kk][8 * w + g] : czero<double2>();
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                if (i >= n || (TRI == TRI_UPPER && 8 * i > k0 + 3)) break;
+                if (TRI == TRI_LOWER && 8 * i + 7 < k0) continue;
+                block_mac(acc.v[i], kin ? L[kk][8 * i + g] : czero<double2>(), b);
+            }
+        } else {
+            if ((TRI == TRI_UPPER && 8 * w > k0 + 3) || (TRI == TRI_LOWER && 8 * w + 7 < k0)) continue;
+            const double2 a = kin ? L[kk][8 * w + g] : czero<double2>();
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                if (i >= n) break;
+                block_mac(acc.v[i], a, kin ? Y[kk][8 * i + g] : czero<double2>());
+            }
+        }
+    }
+}
+template <int TRI, int LW, int N>
+__device__ __forceinline__ void block_mma(const float2 (*L)[LW], const float2 (*Y)[32 + SPAD], int qb,
+                                          BlockTile<float2, N> &acc, int rows, int rn) {
+    const int g = acc.lane >> 2, kq = acc.lane & 3, w = acc.w;
+    const int n = acc.bycol ? (rows + 7) / 8 : (rn + 7) / 8;
+    if (8 * w >= (acc.bycol ? rn : rows)) return;
+    if (acc.bycol) {
+#pragma unroll 2
+        for (int k = 0; k < qb; ++k) {
+            const float2 y0 = Y[k][8 * w + kq], y1 = Y[k][8 * w + kq + 4];
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                if (i >= n || (TRI == TRI_UPPER && 8 * i > k)) break;
+                if (TRI == TRI_LOWER && 8 * i + 7 < k) continue;
+                const float2 l = L[k][8 * i + g];
+                cfma(acc.v[i][0], l, y0);
+                cfma(acc.v[i][1], l, y1);
+            }
+        }
+    } else {
+        for (int k = 0; k < qb; ++k) {
+            if ((TRI == TRI_UPPER && 8 * w > k) || (TRI == TRI_LOWER && 8 * w + 7 < k)) continue;
+            const float2 l = L[k][8 * w + g];
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                if (i >= n) break;
+                cfma(acc.v[i][0], l, Y[k][8 * i + kq]);
+                cfma(acc.v[i][1], l, Y[k][8 * i + kq + 4]);
+            }
+        }
+    }
+}
+
 // Y[q][r] = row_ptr(q)[r] for q < qb, r < rn (entries outside: as above)
 template <class C, int TC, class RowPtr>
 __device__ __forceinline__ void stage_rows_p(C (*Y)[TC + SPAD], RowPtr row_ptr, int qb, int rn, int lt, int nt) {

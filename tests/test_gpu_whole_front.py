@@ -40,3 +40,24 @@ def test_whole_front_solve(nx, ny, leaf, pivot_tol):
                 for i, ds in enumerate(ops):
                     ref = ds.solve(b[i], trans=sys == GM_SYS_AT)
                     assert np.linalg.norm(x[i] - ref) / np.linalg.norm(ref) <= tol
+
+
+@pytest.mark.parametrize("nrhs", [1, 8, 9, 16, 17, 31, 33, 48, 100])
+def test_small_front_slices(nrhs):
+    """Substitution slices of the small fronts: dealt to the warps by columns
+    above 16 right-hand sides and by rows up to there, fronts of every pivot
+    group (leaves of 6 to 30 pivots on one grid)."""
+    nx, ny, dh, npml = 101, 67, 10.0, 3
+    vp = random_smooth(nx, ny, 1700.0, 3500.0, 5)
+    rho = random_smooth(nx, ny, 1000.0, 2200.0, 6)
+    g = O.Grid(nx=nx, ny=ny, dh=dh, npml=npml)
+    ds = OS.DirectSolver(OS.operator(OS.assembled_matrix(g, *O.Port(g).assemble(GM_PHYS_AC, 11.0, vp, rho))))
+    rng = np.random.default_rng(nrhs)
+    b = rng.standard_normal((g.n, nrhs)) + 1j * rng.standard_normal((g.n, nrhs))
+    for precision, tol in ((GM_PREC_FP64, 1e-10), (GM_PREC_C64_IR, 1e-8)):
+        with Engine(nx, ny, dh, npml, precision=precision) as e:
+            e.set_model(vp, rho)
+            e.factor([11.0])
+            for sys in (GM_SYS_A, GM_SYS_AT):
+                x, ref = e.solve(b, sys), ds.solve(b, trans=sys == GM_SYS_AT)
+                assert np.linalg.norm(x - ref) / np.linalg.norm(ref) <= tol
