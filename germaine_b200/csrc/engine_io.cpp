@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <unordered_set>
 #include <vector>
 
 #include "engine.hpp"
@@ -464,8 +465,15 @@ extern "C" int gm_grad_obj(gm_engine *e, int nshots, const float *src_x, const f
     std::vector<double2> stfu;
     if ((rc = residuals(e, nshots, ntr, pobs, stf_inv, misfit, l2, stfu))) return rc;
 
-    // adjoint sources and the adjoint solve with the same factors
-    if ((rc = upload(e->d_rec_k, g.kadj, e->st))) return rc;
+    // adjoint sources and the adjoint solve with the same factors; of the
+    // receivers sharing a grid point only the last one is kept
+    std::vector<int> klast(g.kadj);
+    {
+        std::unordered_set<int> later;
+        for (int t = ntr - 1; t >= 0; --t)
+            if (!later.insert(g.kadj[t]).second) klast[t] = -1;
+    }
+    if ((rc = upload(e->d_rec_k, klast, e->st))) return rc;
     const size_t cnt = (size_t)nf * nshots * ntr;
     // the reference's adjoint source is conj(res) / DH^2; the exact gradient's is conj(res)
     const double dh2 = exact ? 1.0 : (double)(e->cfg.dh * e->cfg.dh);

@@ -21,10 +21,17 @@ namespace gm {
 // patch's operator values (9 per grid point, shared by every right-hand
 // side; zero for neighbours outside the grid, so the stencil needs no
 // edge branches) are staged in shared memory once.
+//
+// Bound by the latency of the window's loads and by issue: 36 FP64
+// multiply-adds per point beside 9 shared and 3 global loads.  Line pointers
+// that step along the line, and edge cases by column and line instead of per
+// load, brought a point from 152 to about 110 instructions; two points' loads
+// in flight in 80 registers (three CTAs per SM) beat three in 120 (two).
+// 841 x 227, 10 matrices x 100 right-hand sides, norms only: 1.62 -> 1.29 ms.
 constexpr int PW = 32;      // grid columns per patch (steps per warp)
 constexpr int PL = 8;       // grid lines per patch (warps per CTA)
 constexpr int RLANES = 32;  // right-hand sides per CTA
-constexpr int RSTEP = 3;    // window steps whose loads are in flight together
+constexpr int RSTEP = 2;    // window steps whose loads are in flight together (at least 2)
 static_assert(PW == RLANES, "one patch point per thread when the patch is staged");
 
 // patches of the residual kernel on an nx x ny grid (partial-sum blocks)
@@ -50,7 +57,7 @@ __device__ __forceinline__ double2 op_coef(const double2 *A9, int n, int nx, boo
 // -- a warp instruction then serves SEG times the points where one lane per
 // right-hand side would leave most of the warp idle.
 template <class InC, class OutC, bool WRITE, bool PRODUCT, int SEG>
-__global__ void __launch_bounds__(RLANES *PL, 2) k_residual(ResidArgs a, const InC *__restrict__ xin, OutC *out,
+__global__ void __launch_bounds__(RLANES *PL, 3) k_residual(ResidArgs a, const InC *__restrict__ xin, OutC *out,
                                                           double *part, int r0) {
     constexpr int RL = RLANES / SEG, SW = PW / SEG;   // right-hand sides per warp, points per lane
     __shared__ double2 cf[9][PL][PW];   // operator values, zero for neighbours outside the grid
@@ -85,58 +92,78 @@ __global__ void __launch_bounds__(RLANES *PL, 2) k_residual(ResidArgs a, const I
     const int xs = seg * SW, xe = min(xs + SW, a.nx - x0);   // this lane's columns of the patch
     if (r < a.nrhs && y < a.ny && xs < xe) {
         const size_t per = (size_t)a.n * a.ldr;
-        const size_t base = (size_t)f * per + r;
         const size_t ldr = a.ldr;
-        const InC *X = xin + (size_t)(a.xmap ? a.xmap[fz] : f) * per + r;
-        OutC *O = out ? out + (size_t)(a.omap ? a.omap[fz] : f) * per + r : nullptr;
         const bool spikes = !PRODUCT && a.spike_k;
-        const int ks = spikes ? a.spike_k[r] : -1;
         const double2 amp = spikes ? a.spike_amp[f] : make_double2(0.0, 0.0);
-        const int n = a.n, nx = a.nx;
-        // x at flat index i, zero outside the array (such values are masked)
-        auto ld = [&](int i) { return (i >= 0 && i < n) ? cto_d(X[(size_t)i * ldr]) : make_double2(0.0, 0.0); };
+        const int nx = a.nx;
+        const int ne = xe - xs;            // points of this lane
         const int kb = y * nx + x0 + xs;   // flat index of the lane's first point
+        // the step (counted from kb) at which the spike enters, if it does here
+        const int hit = spikes ? a.spike_k[r] - kb : -1;
+        if (spikes && hit >= 0 && hit < ne) bb = amp.x * amp.x + amp.y * amp.y;
+        // x one column to the right of the current point on the line above,
+        // the same line and the line below; a line outside the grid is read
+        // as the same line (its operator values are zero), a column outside
+        // it as zero
+        const InC *xc = xin + (size_t)(a.xmap ? a.xmap[fz] : f) * per + r + (size_t)kb * ldr;
+        const ptrdiff_t line = (ptrdiff_t)nx * (ptrdiff_t)ldr;
+        const InC *p[3] = {y > 0 ? xc - line : xc, xc, y + 1 < a.ny ? xc + line : xc};
+        OutC *O = WRITE ? out + (size_t)(a.omap ? a.omap[fz] : f) * per + r + (size_t)kb * ldr : nullptr;
+        const double2 *bp = !PRODUCT && !spikes ? a.b + (size_t)f * per + r + (size_t)kb * ldr : nullptr;
+        const int last = nx - 1 - (x0 + xs);   // the step whose right-hand column lies outside the grid
         // window: wl[d] / wc[d] = x left of / at the current point on the
         // line above (d = 0), the same line (1) and the line below (2)
         double2 wl[3], wc[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            wl[d] = ld(kb - 1 + (d - 1) * nx);
-            wc[d] = ld(kb + (d - 1) * nx);
+            wl[d] = x0 + xs > 0 ? cto_d(*(p[d] - ldr)) : make_double2(0.0, 0.0);
+            wc[d] = cto_d(*p[d]);
+            p[d] += ldr;
         }
-        const int ne = xe - xs;   // points of this lane
-        for (int c0 = 0; c0 < ne; c0 += RSTEP) {
+        const double2 *cw = &cf[0][w][xs];
+        constexpr int CQ = PL * PW;   // operator values of one neighbour
+#pragma unroll 1
+        for (int c0 = 0; c0 < ne; c0 += RSTEP, cw += RSTEP) {
             double2 wr[RSTEP][3];   // the right-hand columns of the next RSTEP points
 #pragma unroll
-            for (int u = 0; u < RSTEP; ++u)
+            for (int u = 0; u < RSTEP; ++u) {
+                const bool in = c0 + u < ne && c0 + u < last;
 #pragma unroll
-                for (int d = 0; d < 3; ++d)
-                    wr[u][d] = c0 + u < ne ? ld(kb + c0 + u + 1 + (d - 1) * nx) : make_double2(0.0, 0.0);
+                for (int d = 0; d < 3; ++d) {
+                    wr[u][d] = in ? cto_d(*p[d]) : make_double2(0.0, 0.0);
+                    p[d] += ldr;
+                }
+            }
 #pragma unroll
             for (int u = 0; u < RSTEP; ++u) {
-                const int lx = xs + c0 + u;   // column in the patch
-                if (c0 + u >= ne) break;
-                const int k = kb + c0 + u;
-                double2 bv = make_double2(0.0, 0.0);
-                if (!PRODUCT) bv = spikes ? (k == ks ? amp : bv) : a.b[base + (size_t)k * ldr];
-                double2 acc = bv;
-                // no branches on the grid edges: a neighbour outside the grid
-                // has a zero operator value, and acc - 0 x is acc exactly
+                if (c0 + u < ne) {
+                    double2 bv = make_double2(0.0, 0.0);
+                    if (!PRODUCT) {
+                        if (spikes) {
+                            if (c0 + u == hit) bv = amp;
+                        } else {
+                            bv = bp[(size_t)(c0 + u) * ldr];
+                            bb += bv.x * bv.x + bv.y * bv.y;
+                        }
+                    }
+                    double2 acc = bv;
+                    // no branches on the grid edges: a neighbour outside the grid
+                    // has a zero operator value, and acc - 0 x is acc exactly
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    cfms(acc, cf[3 * d][w][lx], wl[d]);
-                    cfms(acc, cf[3 * d + 1][w][lx], wc[d]);
-                    cfms(acc, cf[3 * d + 2][w][lx], wr[u][d]);
+                    for (int d = 0; d < 3; ++d) {
+                        cfms(acc, cw[3 * d * CQ + u], u == 0 ? wl[d] : u == 1 ? wc[d] : wr[u - 2][d]);
+                        cfms(acc, cw[(3 * d + 1) * CQ + u], u == 0 ? wc[d] : wr[u - 1][d]);
+                        cfms(acc, cw[(3 * d + 2) * CQ + u], wr[u][d]);
+                    }
+                    if (PRODUCT) acc = make_double2(-acc.x, -acc.y);
+                    if (WRITE) O[(size_t)(c0 + u) * ldr] = cconv<OutC>(acc);
+                    rr += acc.x * acc.x + acc.y * acc.y;
                 }
-                if (PRODUCT) acc = make_double2(-acc.x, -acc.y);
-                if (WRITE) O[(size_t)k * ldr] = cconv<OutC>(acc);
-                rr += acc.x * acc.x + acc.y * acc.y;
-                bb += bv.x * bv.x + bv.y * bv.y;
+            }
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    wl[d] = wc[d];
-                    wc[d] = wr[u][d];
-                }
+            for (int d = 0; d < 3; ++d) {
+                wl[d] = wr[RSTEP - 2][d];
+                wc[d] = wr[RSTEP - 1][d];
             }
         }
     }
