@@ -546,59 +546,96 @@ __global__ void __launch_bounds__(256) k_panel_mm(FactorArgs<R> a, int lvl_first
     });
 }
 
-// Trailing update C -= Lp * Up on TL x TL tiles, 256 threads.  Only the part
-// of the trailing matrix that still belongs to pivot rows or pivot columns is
-// updated here; the contribution block (rows and columns >= npiv) receives
-// all pivot steps at once in one K = npiv GEMM at the end of the level
-// (launch_gemm_sub_cc).  The first CTA takes the next diagonal block alone,
-// updates and factors it (it starts first, so this overlaps the tiles); the
-// others take tile blockIdx.x - 1 without that block.
+// acc -= A B over k < K for one TL x TL tile (A: column-major rows 0 .. mrows
+// of K columns, B: columns 0 .. ncols of K rows), 256 threads.  K runs in
+// chunks of GKC staged through shared memory by asynchronous copies, two
+// buffers: the next chunk's loads are in flight while the current one is
+// multiplied.  Entries outside mrows and ncols are not staged (they only feed
+// accumulators that are never stored).  sm: GEMM_SMEM<TL> complex values.
+constexpr int GKC = 16;
+template <int TL>
+constexpr int GEMM_SMEM = 4 * GKC * (TL + 2);
+
+template <class C, bool MMA, int TL>
+__device__ __forceinline__ void gemm_chunks(const C *A, int lda, const C *B, int ldb, int K, int mrows, int ncols,
+                                            TileCC<C, MMA, TL> &acc, C *sm) {
+    constexpr int SS = TL + 2;   // padded stride of the staged operands
+    C *As = sm;                  // [2][GKC][SS]: As[c * SS + r]
+    C *Bs = As + 2 * GKC * SS;   // [2][GKC][SS]: Bs[c * SS + col]
+    auto stage = [&](int buf, int k0) {
+        const int kb = min(GKC, K - k0);
+        C *Ab = As + buf * GKC * SS, *Bb = Bs + buf * GKC * SS;
+        for (int t = threadIdx.x; t < GKC * TL; t += 256) {
+            const int r = t % TL, c = t / TL;
+            if (c < kb && r < mrows) cp_async_elem(Ab + c * SS + r, A + (size_t)r + (size_t)(k0 + c) * lda);
+            const int col = t / GKC, cc = t % GKC;   // B: contiguous along k
+            if (cc < kb && col < ncols) cp_async_elem(Bb + cc * SS + col, B + (size_t)(k0 + cc) + (size_t)col * ldb);
+        }
+        async_commit();
+    };
+    const int nk = (K + GKC - 1) / GKC;
+    if (nk > 0) stage(0, 0);
+    for (int kc = 0; kc < nk; ++kc) {
+        async_wait_group<0>();   // chunk kc has landed
+        __syncthreads();         // and every warp is past chunk kc - 1
+        if (kc + 1 < nk) stage((kc + 1) & 1, (kc + 1) * GKC);
+        mma_tile<true>(As + (kc & 1) * GKC * SS, SS, 1, Bs + (kc & 1) * GKC * SS, SS, 1, min(GKC, K - kc * GKC), mrows,
+                       ncols, acc, threadIdx.x);
+    }
+}
+
+// Trailing update C -= L U of the pivots k0 .. k0 + kw - 1 on TL x TL tiles,
+// 256 threads, over the trailing rows and columns from k0 + kw on of which one
+// at least is a pivot before `lim`.  The contribution block (rows and columns
+// >= npiv) receives all pivot steps at once in one K = npiv GEMM at the end of
+// the level (launch_gemm_sub_cc), and the pivots from `lim` on their outer
+// block's at once: with every 32-pivot step applied to all of them, a front's
+// pivot rows and columns went through global memory once per step (64 KB read
+// and written per 4.3 us of products in a 64 x 64 tile).  So fronts of many
+// pivots take them in outer blocks of kOuter: the inner steps update the outer
+// block's own rows and columns, one kw = kOuter step the rest.
+// The first CTA takes the next diagonal block alone, updates and factors it
+// (it starts first, so this overlaps the tiles); the others take tile
+// blockIdx.x - 1 without that block.
 //
 // Tile size: a 64 x 64 x 32 complex128 product keeps one SM's FP64 pipe busy
 // for 4.3 us, a 32 x 32 one for 1.1 us, so where the level's 64-row tiles do
 // not fill the chip twice (kTileFill CTAs) the smaller ones shorten the step:
 // one 241 x 141 matrix, contribution GEMMs of the top levels 22-39 -> 11-15 us,
 // updates without a diagonal block behind them 19 -> 11 us.
+// (complex64 keeps one block: its products are short against the steps there.
+// 2060 x 1060, one matrix, levels 11-15: 18.9 -> 17.8 ms in blocks of 128, 17.9
+// in 64, 18.2 in 256.)
+template <class R>
+constexpr int kOuter = sizeof(R) == 8 ? 128 : 1 << 20;
 static_assert(DIAG_THREADS == 256, "k_update's first CTA factors the next diagonal block");
 template <class R, int TL>
-__global__ void __launch_bounds__(256) k_update(FactorArgs<R> a, int lvl_first, int k0, int ntmax, int piv) {
+__global__ void __launch_bounds__(256) k_update(FactorArgs<R> a, int lvl_first, int k0, int kw, int lim, int ntmax,
+                                                int piv) {
     using C = cplx<R>;
-    constexpr int SS = TL + 2;   // padded row stride of the staged operands
     const NodeDesc d = a.s.desc[lvl_first + blockIdx.y];
-    const int s = d.npiv;
-    if (k0 >= s) return;
-    const int f = d.nfront;
-    const int kb = min(NB, s - k0);
-    const int i0 = k0 + kb, m = f - i0;
+    if (k0 >= d.npiv) return;
+    const int f = d.nfront, s = min(d.npiv, lim);
+    const int i0 = min(d.npiv, k0 + kw), m = f - i0;
     const int nt = (m + TL - 1) / TL;
     C *F = reinterpret_cast<C *>(a.front) + (size_t)blockIdx.z * a.s.front_total + d.front_off;
     const bool next = blockIdx.x == 0;   // the next diagonal block
     const int ti = next ? 0 : (blockIdx.x - 1) / ntmax, tj = next ? 0 : (blockIdx.x - 1) % ntmax;
     if (ti >= nt || tj >= nt) return;
-    if (i0 + ti * TL >= s && i0 + tj * TL >= s) return;   // tile inside the contribution block
+    if (i0 + ti * TL >= s && i0 + tj * TL >= s) return;   // no pivot before lim
     const int nd = min(NB, s - i0);                        // size of the next diagonal block
     const bool first = !next && ti == 0 && tj == 0;        // the tile that holds it
     if (first && TL <= NB && nd == NB) return;
     if (next && nd <= 0) return;
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    C *Ls = reinterpret_cast<C *>(smem_raw);   // [NB][SS]: Ls[c * SS + r]
-    C *Us = Ls + NB * SS;                      // [NB][SS]: Us[c * SS + col]
+    C *sm = reinterpret_cast<C *>(smem_raw);
     const int r0 = i0 + ti * TL, c0 = i0 + tj * TL;
-    // a tile whose columns all lie in the contribution block needs only its
-    // pivot rows (and the other way round): the product is cut to them
+    // a tile whose columns all lie from lim on needs only its rows before it
+    // (and the other way round): the product is cut to them
     const int mrows = next ? nd : c0 >= s ? min(TL, s - r0) : min(TL, f - r0);
     const int ncols = next ? nd : r0 >= s ? min(TL, s - c0) : min(TL, f - c0);
-    // asynchronous copies, all in flight at once; entries outside those rows
-    // and columns or beyond kb are not staged (the product reads k < kb only
-    // and treats rows / columns outside them as zero)
-    for (int t = threadIdx.x; t < NB * TL; t += blockDim.x) {
-        const int r = t % TL, c = t / TL;
-        if (c < kb && r < mrows) cp_async_elem(Ls + c * SS + r, F + (r0 + r) + (size_t)(k0 + c) * f);
-        const int col = t / NB, cc = t % NB;   // U: contiguous along the pivot index
-        if (cc < kb && col < ncols) cp_async_elem(Us + cc * SS + col, F + (k0 + cc) + (size_t)(c0 + col) * f);
-    }
-    // the tile's current values go into the accumulators while the staged
+    // the tile's current values go into the accumulators while the first
     // operands land (read after the products, their latency was exposed)
     TileCC<C, sizeof(R) == 8, TL> acc;
     auto mine = [&](int rr, int cc) {
@@ -607,79 +644,40 @@ __global__ void __launch_bounds__(256) k_update(FactorArgs<R> a, int lvl_first, 
     for_tile(acc, threadIdx.x, [&](int rr, int cc, C &v) {
         v = mine(rr, cc) ? F[(r0 + rr) + (size_t)(c0 + cc) * f] : czero<C>();
     });
-    staged_sync();
-    mma_tile<true>(Ls, SS, 1, Us, SS, 1, kb, mrows, ncols, acc, threadIdx.x);
+    gemm_chunks(F + r0 + (size_t)k0 * f, f, F + k0 + (size_t)c0 * f, f, i0 - k0, mrows, ncols, acc, sm);
     for_tile(acc, threadIdx.x, [&](int rr, int cc, C &v) {
         if (mine(rr, cc)) F[(r0 + rr) + (size_t)(c0 + cc) * f] = v;
     });
     if (next) {
-        __syncthreads();   // the block's global writes are visible; Ls / Us are free
-        diag_block<R>(a, F, d, blockIdx.z, i0, nd, Ls, piv != 0);
+        __syncthreads();   // the block's global writes are visible; the staged operands are free
+        diag_block<R>(a, F, d, blockIdx.z, i0, nd, sm, piv != 0);
     }
 }
 
 // Batched C -= A * B (TL x TL output tiles, 256 threads): the
-// contribution-block update of every front of a level in one launch.  K runs
-// in chunks of GKC staged through shared memory by asynchronous copies, two
-// buffers: the next chunk's loads are in flight while the current one is
-// multiplied.  Tile entries outside A's rows or B's columns are not staged
-// (they only feed accumulators that are never stored); the chunk loop reads
-// only the k < kb part.
-constexpr int GKC = 16;
-
+// contribution-block update of every front of a level in one launch.
 template <class R, int TL>
-__global__ void __launch_bounds__(256) k_gemm_sub_cc(const GemmProb<R> *__restrict__ probs,
+__global__ void __launch_bounds__(256, 2) k_gemm_sub_cc(const GemmProb<R> *__restrict__ probs,
                                                      const int4 *__restrict__ tiles) {
     using C = cplx<R>;
-    constexpr int SS = TL + 2;
     const int4 tl = tiles[blockIdx.x];
     const GemmProb<R> p = probs[tl.x];
     const int r0 = tl.y * TL, c0 = tl.z * TL;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    C *As = reinterpret_cast<C *>(smem_raw);   // [2][GKC][SS]: As[c * SS + r]
-    C *Bs = As + 2 * GKC * SS;                 // [2][GKC][SS]: Bs[c * SS + col]
-    auto stage = [&](int buf, int k0) {
-        const int kb = min(GKC, p.k - k0);
-        C *Ab = As + buf * GKC * SS, *Bb = Bs + buf * GKC * SS;
-        for (int t = threadIdx.x; t < GKC * TL; t += blockDim.x) {
-            const int r = t % TL, c = t / TL;
-            if (c < kb && r0 + r < p.m) cp_async_elem(Ab + c * SS + r, p.A + (size_t)(r0 + r) + (size_t)(k0 + c) * p.lda);
-            const int col = t / GKC, cc = t % GKC;   // B: contiguous along k
-            if (cc < kb && c0 + col < p.n)
-                cp_async_elem(Bb + cc * SS + col, p.B + (size_t)(k0 + cc) + (size_t)(c0 + col) * p.ldb);
-        }
-        async_commit();
-    };
-    TileCC<C, sizeof(R) == 8, TL> acc;
-    for_tile(acc, threadIdx.x, [](int, int, C &v) { v = czero<C>(); });
     const int mrows = min(TL, p.m - r0), ncols = min(TL, p.n - c0);
-    const int nk = (p.k + GKC - 1) / GKC;
-    if (nk > 0) stage(0, 0);
-    for (int kc = 0; kc < nk; ++kc) {
-        if (kc + 1 < nk) {
-            stage((kc + 1) & 1, (kc + 1) * GKC);
-            async_wait_group<1>();   // chunk kc has landed
-        } else {
-            async_wait_group<0>();
-        }
-        __syncthreads();
-        const int kb = min(GKC, p.k - kc * GKC);
-        mma_tile<false>(As + (kc & 1) * GKC * SS, SS, 1, Bs + (kc & 1) * GKC * SS, SS, 1, kb, mrows, ncols, acc,
-                        threadIdx.x);
-        __syncthreads();   // this buffer is staged again for chunk kc + 2
-    }
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    TileCC<C, sizeof(R) == 8, TL> acc;
     for_tile(acc, threadIdx.x, [&](int rr, int cc, C &v) {
-        const int row = r0 + rr, col = c0 + cc;
-        if (row < p.m && col < p.n) {
-            C &d = p.C[(size_t)row + (size_t)col * p.ldc];
-            d = csub(d, v);
-        }
+        v = rr < mrows && cc < ncols ? p.C[(size_t)(r0 + rr) + (size_t)(c0 + cc) * p.ldc] : czero<C>();
+    });
+    gemm_chunks(p.A + r0, p.lda, p.B + (size_t)c0 * p.ldb, p.ldb, p.k, mrows, ncols, acc, reinterpret_cast<C *>(smem_raw));
+    for_tile(acc, threadIdx.x, [&](int rr, int cc, C &v) {
+        if (rr < mrows && cc < ncols) p.C[(size_t)(r0 + rr) + (size_t)(c0 + cc) * p.ldc] = v;
     });
 }
 
 template <class R, int TL>
 static void launch_gemm_tl(const GemmProb<R> *d_probs, const int4 *d_tiles, int ntiles, cudaStream_t st) {
-    const size_t smem = 4 * GKC * (TL + 2) * sizeof(cplx<R>);
+    const size_t smem = GEMM_SMEM<TL> * sizeof(cplx<R>);
     static bool attr = false;
     if (!attr) {
         cudaFuncSetAttribute(k_gemm_sub_cc<R, TL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -698,17 +696,27 @@ void launch_gemm_sub_cc(const GemmProb<R> *d_probs, const int4 *d_tiles, int nti
 template void launch_gemm_sub_cc<double>(const GemmProb<double> *, const int4 *, int, int, cudaStream_t);
 template void launch_gemm_sub_cc<float>(const GemmProb<float> *, const int4 *, int, int, cudaStream_t);
 
-// trailing update of pivot block k0 over TL x TL tiles
+// one trailing update of a level's fronts over TL x TL tiles
 template <class R, int TL>
-static void launch_update(const FactorArgs<R> &a, int first, int count, int mmax, int k0, int piv, cudaStream_t st) {
-    const size_t smem = std::max<size_t>(2 * NB * (TL + 2), DIAG_SCRATCH) * sizeof(cplx<R>);
+static void launch_update_tl(const FactorArgs<R> &a, int first, int count, int mmax, int k0, int kw, int lim, int piv,
+                             cudaStream_t st) {
+    const size_t smem = std::max<size_t>(GEMM_SMEM<TL>, DIAG_SCRATCH) * sizeof(cplx<R>);
     static bool attr = false;
     if (!attr) {
         cudaFuncSetAttribute(k_update<R, TL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         attr = true;
     }
     const int nt = (mmax + TL - 1) / TL;
-    (k_update<R, TL><<<dim3(nt * nt + 1, count, a.nf), 256, smem, st>>>(a, first, k0, nt, piv), note_launch());
+    (k_update<R, TL><<<dim3(nt * nt + 1, count, a.nf), 256, smem, st>>>(a, first, k0, kw, lim, nt, piv), note_launch());
+}
+template <class R>
+static void launch_update(const FactorArgs<R> &a, const LevelInfo &L, int mmax, int k0, int kw, int lim, int piv,
+                          cudaStream_t st) {
+    const int64_t nt = (mmax + TILE - 1) / TILE;
+    for_level_pieces(L, [&](int first, int count) {
+        if (nt * nt * L.count * a.nf < kTileFill) launch_update_tl<R, 32>(a, first, count, mmax, k0, kw, lim, piv, st);
+        else launch_update_tl<R, 64>(a, first, count, mmax, k0, kw, lim, piv, st);
+    });
 }
 
 template <class R>
@@ -740,11 +748,10 @@ void launch_factor_level(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_
         // the trailing tiles only update pivot rows and columns still to
         // come (and factor the next diagonal block): after the level's last
         // pivot block there is nothing left for them
-        if (ntmax > 0 && L.max_piv > k0 + NB)
-            for_level_pieces(L, [&](int first, int count) {
-                if ((int64_t)ntmax * ntmax * L.count * a.nf < kTileFill) launch_update<R, 32>(a, first, count, mmax, k0, piv, st);
-                else launch_update<R, 64>(a, first, count, mmax, k0, piv, st);
-            });
+        const int lim = (k0 / kOuter<R> + 1) * kOuter<R>;   // end of the outer block
+        if (ntmax > 0 && std::min(L.max_piv, lim) > k0 + NB) launch_update<R>(a, L, mmax, k0, NB, lim, piv, st);
+        if (ntmax > 0 && k0 + NB == lim && L.max_piv > lim)
+            launch_update<R>(a, L, L.max_front - lim, lim - kOuter<R>, kOuter<R>, L.max_piv, piv, st);
     }
 }
 
