@@ -407,13 +407,13 @@ static int build_cb_plan(gm_engine *e) {
             for (int t = L.first; t < L.first + L.count; ++t) {
                 const int v = s.lvl_nodes[t];
                 const int fr = s.nfront[v], sp = s.npiv[v], m = fr - sp;
-                if (sp == 0 || m == 0) continue;
+                if (m == 0 || (backend && sp == 0)) continue;
                 C *F = base + (size_t)f * s.front_total + s.front_off[v];
                 GemmProb<R> p{F + sp, F + (size_t)sp * fr, F + sp + (size_t)sp * fr, fr, fr, fr, m, m, sp};
-                const int id = (int)(probs.size() - pl.prob_off);
-                probs.push_back(p);
+                const int id = backend ? (int)(probs.size() - pl.prob_off) : t - L.first;
+                if (backend) probs.push_back(p);
                 for (int a = 0; a < (m + tr - 1) / tr; ++a)
-                    for (int b = 0; b < (m + tc - 1) / tc; ++b) tiles.push_back(make_int4(id, a, b, 0));
+                    for (int b = 0; b < (m + tc - 1) / tc; ++b) tiles.push_back(make_int4(id, a, b, f));
             }
         pl.ntiles = (int)(tiles.size() - pl.tile_off);
         if (backend == 1) e->stats.tc_tiles += pl.ntiles;
@@ -467,13 +467,13 @@ static int factor_batch(gm_engine *e, double pivscale) {
             } else if (use_mid_factor<R>(e->levels[h])) {
                 launch_factor_mid<R>(a, e->levels[h], e->st);
             } else {
-                launch_factor_level<R>(a, e->levels[h], e->st);
                 const auto &pl = e->cb_plan[h];
+                launch_factor_level<R>(a, e->levels[h], pl.backend == 1, e->st);
                 if (pl.backend == 1)
                     launch_cgemm_sub(1, reinterpret_cast<const CgemmProb *>(probs + pl.prob_off), tiles + pl.tile_off,
                                      pl.ntiles, e->d_tcerr.as<int>(), e->st);
                 else
-                    launch_gemm_sub_cc<R>(probs + pl.prob_off, tiles + pl.tile_off, pl.ntiles, pl.tile, e->st);
+                    launch_contribution<R>(a, e->levels[h], tiles + pl.tile_off, pl.ntiles, pl.tile, e->st);
             }
             if (e->levels[h].max_piv > 32 && !inverted) {   // beside the levels above (the last level's: nothing is)
                 cudaEventRecord(e->ev_fork, e->st);

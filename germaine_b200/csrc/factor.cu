@@ -4,8 +4,9 @@
 //
 // Fronts live in HBM as dense column-major nfront x nfront complex blocks
 // (one block per node per frequency).  A level is processed by
-//   K2 gather   -- each front pulls its children's contribution blocks
-//                  (extend-add by inverse maps: deterministic, no atomics),
+//   K2 gather   -- each front's pivot rows and columns pull their children's
+//                  contribution blocks (extend-add by inverse maps:
+//                  deterministic, no atomics),
 //   K3 diag     -- adds the operator entries owned by the front (first block),
 //                  then per NB-wide pivot block: LU of the diagonal block with
 //                  threshold partial pivoting inside the block (static
@@ -162,11 +163,14 @@ __device__ __forceinline__ void mma_tile(const double2 *As, int ak, int ar, cons
     }
 }
 
+// (pivots: only the pivot rows and columns, the contribution-block kernel
+// gathers the rest itself)
 template <class R>
-__global__ void k_front_gather(FactorArgs<R> a, int lvl_first) {
+__global__ void k_front_gather(FactorArgs<R> a, int lvl_first, int pivots) {
     using C = cplx<R>;
     const NodeDesc d = a.s.desc[lvl_first + blockIdx.y];
     const int f = d.nfront;
+    const int rows = pivots && blockIdx.x * GATHER_COLS >= (unsigned)d.npiv ? d.npiv : f;   // of this CTA's columns
     const int j = blockIdx.x * GATHER_COLS + (threadIdx.x >> 5);   // one warp per front column
     if (j >= f) return;   // warp-uniform (no barrier below)
     C *base = reinterpret_cast<C *>(a.front) + (size_t)blockIdx.z * a.s.front_total;
@@ -176,7 +180,7 @@ __global__ void k_front_gather(FactorArgs<R> a, int lvl_first) {
     const int b1 = d.child1 >= 0 ? inv[f + j] : -1;
     const C *cb0 = b0 >= 0 ? base + d.cb0 + (size_t)b0 * d.ld0 : nullptr;
     const C *cb1 = b1 >= 0 ? base + d.cb1 + (size_t)b1 * d.ld1 : nullptr;
-    for (int i = threadIdx.x & 31; i < f; i += 32) {
+    for (int i = threadIdx.x & 31; i < rows; i += 32) {
         C v = czero<C>();
         if (cb0) { const int r = inv[i]; if (r >= 0) v = cadd(v, cb0[r]); }
         if (cb1) { const int r = inv[f + i]; if (r >= 0) v = cadd(v, cb1[r]); }
@@ -588,7 +592,7 @@ __device__ __forceinline__ void gemm_chunks(const C *A, int lda, const C *B, int
 // 256 threads, over the trailing rows and columns from k0 + kw on of which one
 // at least is a pivot before `lim`.  The contribution block (rows and columns
 // >= npiv) receives all pivot steps at once in one K = npiv GEMM at the end of
-// the level (launch_gemm_sub_cc), and the pivots from `lim` on their outer
+// the level (launch_contribution), and the pivots from `lim` on their outer
 // block's at once: with every 32-pivot step applied to all of them, a front's
 // pivot rows and columns went through global memory once per step (64 KB read
 // and written per 4.3 us of products in a 64 x 64 tile).  So fronts of many
@@ -654,47 +658,70 @@ __global__ void __launch_bounds__(256) k_update(FactorArgs<R> a, int lvl_first, 
     }
 }
 
-// Batched C -= A * B (TL x TL output tiles, 256 threads): the
-// contribution-block update of every front of a level in one launch.
+// Contribution blocks of a level, C = (children's contribution blocks) - L21
+// U12 with all of the front's pivots (TL x TL tiles, 256 threads): tiles[t] =
+// (level position, tile row, tile column, matrix).  The extend-add of the
+// block happens here, into the accumulators: gathered by a kernel of its own
+// the block went through global memory twice more (841 x 227, 10 matrices,
+// levels 5-8: 4.19 -> 3.73 ms; 2060 x 1060, one matrix, factorisation 37.4 ->
+// 35.8 ms).
 template <class R, int TL>
-__global__ void __launch_bounds__(256, 2) k_gemm_sub_cc(const GemmProb<R> *__restrict__ probs,
-                                                     const int4 *__restrict__ tiles) {
+__global__ void __launch_bounds__(256, 2) k_contribution(FactorArgs<R> a, int lvl_first, const int4 *__restrict__ tiles) {
     using C = cplx<R>;
     const int4 tl = tiles[blockIdx.x];
-    const GemmProb<R> p = probs[tl.x];
-    const int r0 = tl.y * TL, c0 = tl.z * TL;
-    const int mrows = min(TL, p.m - r0), ncols = min(TL, p.n - c0);
+    const NodeDesc d = a.s.desc[lvl_first + tl.x];
+    const int f = d.nfront, s = d.npiv;
+    const int r0 = s + tl.y * TL, c0 = s + tl.z * TL;   // first row / column of the tile
+    const int mrows = min(TL, f - r0), ncols = min(TL, f - c0);
+    C *base = reinterpret_cast<C *>(a.front) + (size_t)tl.w * a.s.front_total;
+    C *F = base + d.front_off;
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int map[2][2][TL];   // children's positions of the tile's rows / columns
+    for (int t = threadIdx.x; t < 4 * TL; t += 256) {
+        const int ch = t / (2 * TL), rc = t / TL % 2, i = t % TL;
+        int v = -1;
+        if ((ch ? d.child1 : d.child0) >= 0 && i < (rc ? ncols : mrows)) v = a.s.inv[d.inv_off + ch * f + (rc ? c0 : r0) + i];
+        map[ch][rc][i] = v;
+    }
+    __syncthreads();
+    const C *cb0 = base + d.cb0, *cb1 = base + d.cb1;
     TileCC<C, sizeof(R) == 8, TL> acc;
     for_tile(acc, threadIdx.x, [&](int rr, int cc, C &v) {
-        v = rr < mrows && cc < ncols ? p.C[(size_t)(r0 + rr) + (size_t)(c0 + cc) * p.ldc] : czero<C>();
+        v = czero<C>();
+        const int i0 = map[0][0][rr], j0 = map[0][1][cc], i1 = map[1][0][rr], j1 = map[1][1][cc];
+        if (i0 >= 0 && j0 >= 0) v = cb0[i0 + (size_t)j0 * d.ld0];
+        if (i1 >= 0 && j1 >= 0) v = cadd(v, cb1[i1 + (size_t)j1 * d.ld1]);
     });
-    gemm_chunks(p.A + r0, p.lda, p.B + (size_t)c0 * p.ldb, p.ldb, p.k, mrows, ncols, acc, reinterpret_cast<C *>(smem_raw));
+    gemm_chunks(F + r0, f, F + (size_t)c0 * f, f, s, mrows, ncols, acc, reinterpret_cast<C *>(smem_raw));
     for_tile(acc, threadIdx.x, [&](int rr, int cc, C &v) {
-        if (rr < mrows && cc < ncols) p.C[(size_t)(r0 + rr) + (size_t)(c0 + cc) * p.ldc] = v;
+        if (rr < mrows && cc < ncols) F[(r0 + rr) + (size_t)(c0 + cc) * f] = v;
     });
 }
 
 template <class R, int TL>
-static void launch_gemm_tl(const GemmProb<R> *d_probs, const int4 *d_tiles, int ntiles, cudaStream_t st) {
+static void launch_contribution_tl(const FactorArgs<R> &a, const LevelInfo &L, const int4 *d_tiles, int ntiles,
+                                   cudaStream_t st) {
     const size_t smem = GEMM_SMEM<TL> * sizeof(cplx<R>);
     static bool attr = false;
     if (!attr) {
-        cudaFuncSetAttribute(k_gemm_sub_cc<R, TL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_contribution<R, TL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         attr = true;
     }
-    (k_gemm_sub_cc<R, TL><<<ntiles, 256, smem, st>>>(d_probs, d_tiles), note_launch());
+    (k_contribution<R, TL><<<ntiles, 256, smem, st>>>(a, L.first, d_tiles), note_launch());
 }
 
 template <class R>
-void launch_gemm_sub_cc(const GemmProb<R> *d_probs, const int4 *d_tiles, int ntiles, int tile, cudaStream_t st) {
+void launch_contribution(const FactorArgs<R> &a, const LevelInfo &L, const int4 *d_tiles, int ntiles, int tile,
+                         cudaStream_t st) {
     if (ntiles <= 0) return;
-    if (tile == 32) launch_gemm_tl<R, 32>(d_probs, d_tiles, ntiles, st);
-    else launch_gemm_tl<R, 64>(d_probs, d_tiles, ntiles, st);
+    if (tile == 32) launch_contribution_tl<R, 32>(a, L, d_tiles, ntiles, st);
+    else launch_contribution_tl<R, 64>(a, L, d_tiles, ntiles, st);
 }
 
-template void launch_gemm_sub_cc<double>(const GemmProb<double> *, const int4 *, int, int, cudaStream_t);
-template void launch_gemm_sub_cc<float>(const GemmProb<float> *, const int4 *, int, int, cudaStream_t);
+template void launch_contribution<double>(const FactorArgs<double> &, const LevelInfo &, const int4 *, int, int,
+                                          cudaStream_t);
+template void launch_contribution<float>(const FactorArgs<float> &, const LevelInfo &, const int4 *, int, int,
+                                         cudaStream_t);
 
 // one trailing update of a level's fronts over TL x TL tiles
 template <class R, int TL>
@@ -720,12 +747,12 @@ static void launch_update(const FactorArgs<R> &a, const LevelInfo &L, int mmax, 
 }
 
 template <class R>
-void launch_factor_level(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_t st) {
+void launch_factor_level(const FactorArgs<R> &a, const LevelInfo &L, bool whole_gather, cudaStream_t st) {
     using C = cplx<R>;
     if (L.count == 0) return;
     for_level_pieces(L, [&](int first, int count) {
         (k_front_gather<R><<<dim3((L.max_front + GATHER_COLS - 1) / GATHER_COLS, count, a.nf), 32 * GATHER_COLS, 0,
-                             st>>>(a, first),
+                             st>>>(a, first, !whole_gather),
          note_launch());
     });
     const size_t smem = 2 * NB * TSTR * sizeof(C);
@@ -755,8 +782,8 @@ void launch_factor_level(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_
     }
 }
 
-template void launch_factor_level<double>(const FactorArgs<double> &, const LevelInfo &, cudaStream_t);
-template void launch_factor_level<float>(const FactorArgs<float> &, const LevelInfo &, cudaStream_t);
+template void launch_factor_level<double>(const FactorArgs<double> &, const LevelInfo &, bool, cudaStream_t);
+template void launch_factor_level<float>(const FactorArgs<float> &, const LevelInfo &, bool, cudaStream_t);
 
 // ---------------------------------------------------------------------
 // Fronts that fit shared memory whole (the lower levels of the tree): one CTA
@@ -1511,7 +1538,7 @@ template <class R>
 void launch_factor_mid(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_t st) {
     for_level_pieces(L, [&](int first, int count) {
         (k_front_gather<R><<<dim3((L.max_front + GATHER_COLS - 1) / GATHER_COLS, count, a.nf), 32 * GATHER_COLS, 0,
-                             st>>>(a, first),
+                             st>>>(a, first, 0),
          note_launch());
     });
     if (L.max_piv <= 16)

@@ -124,7 +124,7 @@ void launch_amax(const double2 *A, size_t cnt, unsigned long long *out, cudaStre
 void launch_pack_split(double2 *dst, const double *re, const double *im, size_t cnt, cudaStream_t st);
 
 template <class R>
-void launch_factor_level(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_t st);
+void launch_factor_level(const FactorArgs<R> &a, const LevelInfo &L, bool whole_gather, cudaStream_t st);
 // Fronts that fit shared memory whole, assembled and factorised by one CTA
 // each (replaces launch_factor_level and the level's contribution-block GEMM)
 // when front_factor_level(L).
@@ -163,9 +163,11 @@ struct GemmProb {
     cplx_any<R> *C;
     int lda, ldb, ldc, m, n, k;
 };
-// batched GEMM over tile x tile output tiles (64 or 32): tiles[t] = (problem, tile row, tile col)
+// a level's contribution blocks over tile x tile output tiles (64 or 32), their
+// extend-add included: tiles[t] = (level position, tile row, tile column, matrix)
 template <class R>
-void launch_gemm_sub_cc(const GemmProb<R> *d_probs, const int4 *d_tiles, int ntiles, int tile, cudaStream_t st);
+void launch_contribution(const FactorArgs<R> &a, const LevelInfo &L, const int4 *d_tiles, int ntiles, int tile,
+                         cudaStream_t st);
 constexpr int kGemmTileCC = 64;
 // fewer 64 x 64 tiles than this in a launch: 32 x 32 ones instead (two per SM)
 constexpr int kGemmTileFill = 2 * 148;
