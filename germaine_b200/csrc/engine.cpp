@@ -45,13 +45,6 @@ using gm::fail;
 
 namespace {
 
-template <class T>
-int upload(gm::DevBuf &buf, const std::vector<T> &v, cudaStream_t st) {
-    GM_ALLOC(buf, v.size() * sizeof(T));
-    if (!v.empty()) GM_CUDA(cudaMemcpyAsync(buf.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st));
-    return GM_OK;
-}
-
 int check_config(const gm_config *c) {
     if (!c) return fail(GM_ERROR_INVALID, "null config");
     if (c->nx < 3 || c->ny < 3) return fail(GM_ERROR_INVALID, "grid must be at least 3 x 3 (got %d x %d)", c->nx, c->ny);
@@ -111,6 +104,7 @@ extern "C" int gm_engine_create(int device, const gm_config *cfg, gm_engine **ou
     GM_CUDA(cudaEventCreate(&e->ev_s0));
     GM_CUDA(cudaEventCreate(&e->ev_s1));
     GM_CUDA(cudaEventCreate(&e->ev_sm));
+    GM_CUDA(cudaEventCreate(&e->ev_r));
     GM_CUDA(cudaStreamCreateWithFlags(&e->st2, cudaStreamNonBlocking));
     GM_CUDA(cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming));
     GM_CUDA(cudaEventCreateWithFlags(&e->ev_join, cudaEventDisableTiming));
@@ -214,32 +208,36 @@ extern "C" int gm_engine_create(int device, const gm_config *cfg, gm_engine **ou
             if (at > first) L.groups.push_back(gm::PivGroup{first - L.first, at - first, g});
         }
     }
-    int rc2;
-    if ((rc2 = upload(e->d_desc, desc, e->st)) || (rc2 = upload(e->d_fdesc, fdesc, e->st)) ||
-        (rc2 = upload(e->d_sdesc, sdesc, e->st)))
-        return rc2;
-    if ((rc2 = upload(e->d_npiv, s.npiv, e->st)) || (rc2 = upload(e->d_nfront, s.nfront, e->st)) ||
-        (rc2 = upload(e->d_child0, s.child0, e->st)) || (rc2 = upload(e->d_child1, s.child1, e->st)) ||
-        (rc2 = upload(e->d_vars, s.vars, e->st)) || (rc2 = upload(e->d_inv, s.inv, e->st)) ||
-        (rc2 = upload(e->d_lvl_nodes, s.lvl_nodes, e->st)) || (rc2 = upload(e->d_front_off, s.front_off, e->st)) ||
-        (rc2 = upload(e->d_var_off, s.var_off, e->st)) || (rc2 = upload(e->d_inv_off, s.inv_off, e->st)) ||
-        (rc2 = upload(e->d_rhs_off, s.rhs_off, e->st)) || (rc2 = upload(e->d_ent_dst, ent_dst, e->st)) ||
-        (rc2 = upload(e->d_y_off, y_off, e->st)) || (rc2 = upload(e->d_tri_off, tri_off, e->st)) ||
-        (rc2 = upload(e->d_ent_src, ent_src, e->st)))
-        return rc2;
-    GM_CUDA(cudaStreamSynchronize(e->st));
+    // one allocation for all of them, each on a 256-byte boundary (18 small
+    // allocations and their release cost more than the copies)
     gm::DevSym &d = e->dsym;
     d.n = s.n; d.nnodes = s.nnodes;
-    d.npiv = e->d_npiv.as<int>(); d.nfront = e->d_nfront.as<int>();
-    d.child0 = e->d_child0.as<int>(); d.child1 = e->d_child1.as<int>();
-    d.vars = e->d_vars.as<int>(); d.inv = e->d_inv.as<int>(); d.lvl_nodes = e->d_lvl_nodes.as<int>();
-    d.front_off = e->d_front_off.as<int64_t>(); d.var_off = e->d_var_off.as<int64_t>();
-    d.inv_off = e->d_inv_off.as<int64_t>(); d.rhs_off = e->d_rhs_off.as<int64_t>();
-    d.front_total = s.front_total; d.rhs_total = s.rhs_total;
-    d.desc = e->d_desc.as<gm::NodeDesc>();
-    d.fdesc = e->d_fdesc.as<gm::NodeDesc>();
-    d.sdesc = e->d_sdesc.as<gm::NodeDesc>();
-    d.y_off = e->d_y_off.as<int64_t>(); d.y_total = y_total;
+    d.front_total = s.front_total; d.rhs_total = s.rhs_total; d.y_total = y_total;
+    size_t sym_bytes = 0;
+    std::vector<std::pair<const void *, size_t>> parts;   // host array, bytes
+    std::vector<std::pair<const void **, size_t>> where;  // device pointer, offset
+    const auto part = [&](const auto &v, auto **dst) {
+        const size_t nb = v.size() * sizeof(v[0]);
+        parts.emplace_back(v.data(), nb);
+        where.emplace_back((const void **)dst, sym_bytes);
+        sym_bytes += (nb + 255) / 256 * 256;
+    };
+    part(desc, &d.desc); part(fdesc, &d.fdesc); part(sdesc, &d.sdesc);
+    part(s.npiv, &d.npiv); part(s.nfront, &d.nfront); part(s.child0, &d.child0); part(s.child1, &d.child1);
+    part(s.vars, &d.vars); part(s.inv, &d.inv); part(s.lvl_nodes, &d.lvl_nodes);
+    part(s.front_off, &d.front_off); part(s.var_off, &d.var_off); part(s.inv_off, &d.inv_off);
+    part(s.rhs_off, &d.rhs_off); part(y_off, &d.y_off); part(tri_off, &e->tri_off);
+    part(ent_dst, &e->ent_dst); part(ent_src, &e->ent_src);
+    GM_ALLOC(e->d_sym, sym_bytes);
+    for (size_t i = 0; i < parts.size(); ++i) {
+        char *p = e->d_sym.as<char>() + where[i].second;
+        *where[i].first = p;
+        if (parts[i].second)
+            GM_CUDA(cudaMemcpyAsync(p, parts[i].first, parts[i].second, cudaMemcpyHostToDevice, e->st));
+    }
+    GM_CUDA(cudaStreamSynchronize(e->st));
+    e->node_at.resize(s.nnodes);
+    for (int t = 0; t < s.nnodes; ++t) e->node_at[s.lvl_nodes[t]] = t;
 
     gm_stats &st = e->stats;
     st.n = s.n;
@@ -420,7 +418,6 @@ static int build_cb_plan(gm_engine *e) {
     }
     GM_ALLOC(e->d_cb_probs, probs.size() * sizeof(GemmProb<R>) + 16);
     GM_ALLOC(e->d_cb_tiles, tiles.size() * sizeof(int4) + 16);
-    GM_ALLOC(e->d_tcerr, sizeof(int));
     if (!probs.empty())
         GM_CUDA(cudaMemcpyAsync(e->d_cb_probs.p, probs.data(), probs.size() * sizeof(GemmProb<R>), cudaMemcpyHostToDevice, e->st));
     if (!tiles.empty())
@@ -437,20 +434,20 @@ static int factor_batch(gm_engine *e, double pivscale) {
     a.s = e->dsym;
     a.front = e->d_front.p;
     a.A = e->d_A.as<double2>();
-    a.ent_dst = e->d_ent_dst.as<int64_t>();
-    a.ent_src = e->d_ent_src.as<int>();
+    a.ent_dst = e->ent_dst;
+    a.ent_src = e->ent_src;
     a.nf = e->nf;
-    a.amax = e->d_amax.as<unsigned long long>();
+    gm_engine::FactorReport *report = e->d_report.as<gm_engine::FactorReport>();
+    a.amax = &report->amax;
     a.pivscale = pivscale;
-    a.npert = e->d_npert.as<unsigned long long>();
-    a.nswap = a.npert + 1;
+    a.npert = &report->npert;
+    a.nswap = &report->nswap;
     a.pivtau2 = e->cfg.pivot_tol > 0 ? e->cfg.pivot_tol * e->cfg.pivot_tol : 0.0;
     a.pivsrc = e->cfg.pivot_tol > 0 ? e->d_pivsrc.as<unsigned char>() : nullptr;
     if (e->cb_plan_base != e->d_front.p || e->cb_plan_nf != e->nf) {
         const int rc = build_cb_plan<R>(e);
         if (rc) return rc;
     }
-    GM_CUDA(cudaMemsetAsync(e->d_tcerr.p, 0, sizeof(int), e->st));
     const GemmProb<R> *probs = e->d_cb_probs.as<GemmProb<R>>();
     const int4 *tiles = e->d_cb_tiles.as<int4>();
     // GM_TRACE_LEVELS=1: device time of every level on stderr
@@ -471,14 +468,14 @@ static int factor_batch(gm_engine *e, double pivscale) {
                 launch_factor_level<R>(a, e->levels[h], pl.backend == 1, e->st);
                 if (pl.backend == 1)
                     launch_cgemm_sub(1, reinterpret_cast<const CgemmProb *>(probs + pl.prob_off), tiles + pl.tile_off,
-                                     pl.ntiles, e->d_tcerr.as<int>(), e->st);
+                                     pl.ntiles, &report->tcerr, e->st);
                 else
                     launch_contribution<R>(a, e->levels[h], tiles + pl.tile_off, pl.ntiles, pl.tile, e->st);
             }
             if (e->levels[h].max_piv > 32 && !inverted) {   // beside the levels above (the last level's: nothing is)
                 cudaEventRecord(e->ev_fork, e->st);
                 cudaStreamWaitEvent(e->st2, e->ev_fork, 0);
-                launch_tri_inverse<R>(a, e->levels[h], e->d_tri.p, e->tri_total, e->d_tri_off.as<int64_t>(), e->st2);
+                launch_tri_inverse<R>(a, e->levels[h], e->d_tri.p, e->tri_total, e->tri_off, e->st2);
                 forked = true;
             }
             if (evs) cudaEventRecord(evs[1 + h], e->st);
@@ -494,9 +491,9 @@ static int factor_batch(gm_engine *e, double pivscale) {
         // with new buffers launches directly (which also sets every kernel's
         // attributes outside any capture), the second captures the graph.
         gm_engine::FactorGraphKey key;
-        key.front = e->d_front.p; key.A = e->d_A.p; key.amax = e->d_amax.p; key.npert = e->d_npert.p;
+        key.front = e->d_front.p; key.A = e->d_A.p; key.report = report;
         key.pivsrc = e->d_pivsrc.p; key.tri = e->d_tri.p;
-        key.tcerr = e->d_tcerr.p; key.probs = probs; key.tiles = tiles; key.nf = e->nf; key.fp64 = sizeof(R) == 8;
+        key.probs = probs; key.tiles = tiles; key.nf = e->nf; key.fp64 = sizeof(R) == 8;
         if (!(e->fgraph && key == e->fgraph_key) && key == e->fgraph_seen) {
             if (e->fgraph) cudaGraphExecDestroy(e->fgraph);
             e->fgraph = nullptr;
@@ -582,8 +579,7 @@ static int factor_assembled(gm_engine *e) {
     const bool fp64 = e->cfg.precision == GM_PREC_FP64;
     const size_t fbytes = (size_t)e->nf * e->sym.front_total * e->csize();
     GM_ALLOC(e->d_front, fbytes);
-    GM_ALLOC(e->d_npert, 2 * sizeof(unsigned long long));   // perturbed pivots, row exchanges
-    GM_ALLOC(e->d_amax, sizeof(unsigned long long));
+    GM_ALLOC(e->d_report, sizeof(gm_engine::FactorReport));
     GM_ALLOC(e->d_tri, (size_t)e->nf * e->tri_total * e->csize());
     if (e->cfg.pivot_tol > 0) {
         GM_ALLOC(e->d_pivsrc, (size_t)e->nf * e->n);
@@ -591,31 +587,27 @@ static int factor_assembled(gm_engine *e) {
         if (rc) return rc;
     }
     GM_CUDA(cudaEventRecord(e->ev0, e->st));
-    GM_CUDA(cudaMemsetAsync(e->d_npert.p, 0, 2 * sizeof(unsigned long long), e->st));
-    GM_CUDA(cudaMemsetAsync(e->d_amax.p, 0, sizeof(unsigned long long), e->st));
-    launch_amax(e->d_A.as<double2>(), (size_t)e->nf * 9 * e->n, e->d_amax.as<unsigned long long>(), e->st);
+    gm_engine::FactorReport *report = e->d_report.as<gm_engine::FactorReport>();
+    GM_CUDA(cudaMemsetAsync(report, 0, sizeof *report, e->st));
+    launch_amax(e->d_A.as<double2>(), (size_t)e->nf * 9 * e->n, &report->amax, e->st);
     const int rc = fp64 ? factor_batch<double>(e, 1e-13) : factor_batch<float>(e, 1e-6);
     if (rc) return rc;
     GM_CUDA(cudaEventRecord(e->ev1, e->st));
-    GM_CUDA(cudaEventSynchronize(e->ev1));
+    gm_engine::FactorReport h{};
+    GM_CUDA(cudaMemcpyAsync(&h, report, sizeof h, cudaMemcpyDeviceToHost, e->st));
+    GM_CUDA(cudaStreamSynchronize(e->st));   // the call's only wait
     float ms = 0;
     cudaEventElapsedTime(&ms, e->ev0, e->ev1);
     e->stats.ms_factor = ms;
-    unsigned long long np = 0, amax_bits = 0, nsw = 0;
-    GM_CUDA(cudaMemcpy(&np, e->d_npert.p, sizeof np, cudaMemcpyDeviceToHost));
-    GM_CUDA(cudaMemcpy(&nsw, e->d_npert.as<unsigned long long>() + 1, sizeof nsw, cudaMemcpyDeviceToHost));
-    e->stats.pivot_swaps = (int64_t)nsw;
-    GM_CUDA(cudaMemcpy(&amax_bits, e->d_amax.p, sizeof amax_bits, cudaMemcpyDeviceToHost));
+    e->stats.pivot_swaps = (int64_t)h.nswap;
     double amax = 0;
-    std::memcpy(&amax, &amax_bits, sizeof amax);
+    std::memcpy(&amax, &h.amax, sizeof amax);
     if (!std::isfinite(amax))   // NaN bits order above every finite value in the max reduction
         return fail(GM_ERROR_NONFINITE, "factor: the operator holds non-finite values (NaN or Inf material?)");
-    int tcerr = 0;
-    GM_CUDA(cudaMemcpy(&tcerr, e->d_tcerr.p, sizeof tcerr, cudaMemcpyDeviceToHost));
-    if (tcerr) return fail(GM_ERROR_CUDA, "factor: a tensor-core wait timed out in the contribution-block update");
-    e->stats.perturbed_pivots = (int64_t)np;
+    if (h.tcerr) return fail(GM_ERROR_CUDA, "factor: a tensor-core wait timed out in the contribution-block update");
+    e->stats.perturbed_pivots = (int64_t)h.npert;
     e->factored = true;
-    return np ? GM_WARNING_PERTURBED : GM_OK;
+    return h.npert ? GM_WARNING_PERTURBED : GM_OK;
 }
 
 }  // namespace gm
@@ -636,15 +628,16 @@ extern "C" int gm_factor_models(gm_engine *e, int nmat, const float *h_freqs, co
     if (h_models) e->models.assign(h_models, h_models + nmat);
     else e->models.assign(nmat, 0);
 
-    GM_CUDA(cudaEventRecord(e->ev0, e->st));
+    GM_CUDA(cudaEventRecord(e->ev_s0, e->st));
     int rc = gm::assemble_batch(e);
     if (rc) return rc;
-    GM_CUDA(cudaEventRecord(e->ev1, e->st));
-    GM_CUDA(cudaEventSynchronize(e->ev1));
+    GM_CUDA(cudaEventRecord(e->ev_s1, e->st));
+    rc = gm::factor_assembled(e);
+    cudaEventSynchronize(e->ev_s1);   // past already, unless the factorisation failed to start
     float ms = 0;
-    cudaEventElapsedTime(&ms, e->ev0, e->ev1);
+    cudaEventElapsedTime(&ms, e->ev_s0, e->ev_s1);
     e->stats.ms_assemble = ms;
-    return gm::factor_assembled(e);
+    return rc;
 }
 
 extern "C" int gm_factor(gm_engine *e, int nfreq, const float *h_freqs) {
@@ -702,6 +695,21 @@ extern "C" int gm_get_triplets(gm_engine *e, int ifreq, double *Ar, double *Ai, 
 
 namespace gm {
 
+// Adds the last substitution's device times to the stats.  substitute() does
+// not wait for the device; its times are taken after the next wait that the
+// solve has anyway.
+static void collect_subst_times(gm_engine *e) {
+    if (!e->subst_timed) return;
+    e->subst_timed = false;
+    cudaEventSynchronize(e->ev_s1);
+    float ms = 0;
+    cudaEventElapsedTime(&ms, e->ev_s0, e->ev_s1);
+    e->stats.ms_subst += ms;
+    cudaEventElapsedTime(&ms, e->ev_sm, e->ev_s1);
+    e->stats.ms_subst_bwd += ms;
+    e->stats.n_subst += 1;
+}
+
 // One substitution over the right-hand sides in xT; fmap (device, nfz
 // entries) restricts it to those matrices of the batch (NULL: all); y is the
 // pivot workspace.
@@ -709,6 +717,7 @@ template <class R>
 static void substitute(gm_engine *e, void *xT, void *y, int nrhs, int trans, const unsigned char *mask = nullptr,
                        const int *fmap = nullptr, int nfz = 0, const int *xmap = nullptr,
                        const SpikeRhs *spikes = nullptr) {
+    collect_subst_times(e);   // the events are used again
     cudaEventRecord(e->ev_s0, e->st);
     SolveArgs<R> a{};
     a.s = e->dsym;
@@ -725,7 +734,6 @@ static void substitute(gm_engine *e, void *xT, void *y, int nrhs, int trans, con
     if (mask && e->have_work) {   // the pruned pass launches only the live pairs
         a.work = e->d_work.as<int2>();
         a.work_off = e->work_off.data();
-        a.work_w = e->work_w.data();
     }
     a.nrhs = nrhs;
     a.ldr = nrhs;
@@ -772,13 +780,7 @@ static void substitute(gm_engine *e, void *xT, void *y, int nrhs, int trans, con
         for (auto &x : ev) cudaEventDestroy(x);
     }
     cudaEventRecord(e->ev_s1, e->st);
-    cudaEventSynchronize(e->ev_s1);
-    float ms = 0;
-    cudaEventElapsedTime(&ms, e->ev_s0, e->ev_s1);
-    e->stats.ms_subst += ms;
-    cudaEventElapsedTime(&ms, e->ev_sm, e->ev_s1);
-    e->stats.ms_subst_bwd += ms;
-    e->stats.n_subst += 1;
+    e->subst_timed = true;
 }
 
 // Forward-pass pruning mask from a right-hand-side pattern: node v is live
@@ -790,9 +792,13 @@ static const unsigned char *build_mask(gm_engine *e, int nrhs, const RhsPattern 
     const Symbolic &sy = e->sym;
     const int nch = (nrhs + 31) / 32, nn = sy.nnodes;
     std::vector<unsigned char> m((size_t)nn * nch, 0);
+    std::vector<unsigned char> live((size_t)nn + 8, 0);   // by level position
     auto mark = [&](int row, int g) {
         if (row < 0 || row >= sy.n) return;
-        for (int v = sy.owner[row]; v >= 0 && !m[(size_t)v * nch + g]; v = sy.parent[v]) m[(size_t)v * nch + g] = 1;
+        for (int v = sy.owner[row]; v >= 0 && !m[(size_t)v * nch + g]; v = sy.parent[v]) {
+            m[(size_t)v * nch + g] = 1;
+            live[e->node_at[v]] = 1;
+        }
     };
     if (pat->per_col)
         for (int r = 0; r < std::min(nrhs, pat->ncol); ++r) mark(pat->per_col[r], r / 32);
@@ -800,28 +806,27 @@ static const unsigned char *build_mask(gm_engine *e, int nrhs, const RhsPattern 
         for (int g = 0; g < nch; ++g) mark(pat->common[i], g);
     if (e->d_mask.ensure(m.size()) != cudaSuccess) return nullptr;   // fall back to the dense pass
     if (cudaMemcpyAsync(e->d_mask.p, m.data(), m.size(), cudaMemcpyHostToDevice, e->st) != cudaSuccess) return nullptr;
-    // the live (front position, slice) pairs of every level, for slices of
-    // the width the level's forward pass will use (tuned or default)
-    const int tcw_default = solve_slice_width(nrhs, e->cfg.precision == GM_PREC_FP64);
-    const bool tuned = !e->lvl_cfg.empty() && e->tuned_nrhs == nrhs;
+    // the live (front position, 32-column slice) pairs of the small-front
+    // levels, whose kernels are launched over them; the other levels read
+    // the mask.  Eight positions are looked at together: few are live.
     std::vector<int2> work;
     e->work_off.assign(e->levels.size() + 1, 0);
-    e->work_w.assign(e->levels.size(), tcw_default);
     for (size_t h = 0; h < e->levels.size(); ++h) {
         e->work_off[h] = (int)work.size();
-        // (the small-front kernels take 32 columns whatever the tuned width)
-        const int tcw = e->levels[h].max_piv <= 32 ? 32
-                        : tuned && e->lvl_cfg[4 * h + 1] ? 8 * e->lvl_cfg[4 * h + 1] : tcw_default;
-        e->work_w[h] = tcw;
-        const int nslice = (nrhs + tcw - 1) / tcw;
         const LevelInfo &L = e->levels[h];
-        for (int t = 0; t < L.count; ++t) {
-            const int v = sy.lvl_nodes[L.first + t];
-            for (int c = 0; c < nslice; ++c) {
-                const int r0 = c * tcw, r1 = std::min(nrhs, r0 + tcw) - 1;
-                bool lv = false;
-                for (int g = r0 >> 5; g <= (r1 >> 5) && !lv; ++g) lv = m[(size_t)v * nch + g] != 0;
-                if (lv) work.push_back(make_int2(t, c));
+        if (L.max_piv > 32) continue;
+        for (int t = 0; t < L.count;) {
+            unsigned long long eight;
+            std::memcpy(&eight, &live[L.first + t], 8);
+            if (!eight) {
+                t += 8;
+                continue;
+            }
+            for (const int stop = std::min(L.count, t + 8); t < stop; ++t) {
+                if (!live[L.first + t]) continue;
+                const unsigned char *mv = &m[(size_t)sy.lvl_nodes[L.first + t] * nch];
+                for (int c = 0; c < nch; ++c)
+                    if (mv[c]) work.push_back(make_int2(t, c));
             }
         }
     }
@@ -829,7 +834,6 @@ static const unsigned char *build_mask(gm_engine *e, int nrhs, const RhsPattern 
     e->have_work = e->d_work.ensure((work.size() + 1) * sizeof(int2)) == cudaSuccess &&
                    cudaMemcpyAsync(e->d_work.p, work.data(), work.size() * sizeof(int2), cudaMemcpyHostToDevice,
                                    e->st) == cudaSuccess;
-    cudaStreamSynchronize(e->st);   // m and work are released on return
     return e->d_mask.as<unsigned char>();
 }
 
@@ -1138,6 +1142,7 @@ int engine_solve_device(gm_engine *e, int sys, int nrhs, double2 *d_x, const dou
     e->stats.ms_subst = 0;
     e->stats.ms_subst_bwd = 0;
     e->stats.n_subst = 0;
+    e->subst_timed = false;
     GM_CUDA(cudaEventRecord(t0, e->st));
     // initial solve in working precision: in FP64 in place in x (b copied
     // into it), in complex64 in the work buffer and then added into x = 0
@@ -1158,11 +1163,8 @@ int engine_solve_device(gm_engine *e, int sys, int nrhs, double2 *d_x, const dou
         launch_add_up<float>(d_x, e->d_t.p, cnt, e->st);
     }
     GM_CUDA(cudaGetLastError());
-    GM_CUDA(cudaEventRecord(t1, e->st));
-    GM_CUDA(cudaEventSynchronize(t1));
+    GM_CUDA(cudaEventRecord(t1, e->st));   // read after the first residual's wait
     float ms = 0;
-    cudaEventElapsedTime(&ms, t0, t1);
-    e->stats.ms_solve = ms;
 
     // Refinement, per matrix: r = b - M' x (FP64), x += M'^{-1} r (working
     // precision), until the matrix's worst right-hand side meets the target.
@@ -1187,7 +1189,6 @@ int engine_solve_device(gm_engine *e, int sys, int nrhs, double2 *d_x, const dou
     e->refine_info.assign(e->nf, gm_refine_info{0.0, 0.0, 0, GM_REFINE_NONE});
     double worst = 0;
     int it = 0;
-    GM_CUDA(cudaEventRecord(t0, e->st));
     for (;; ++it) {
         const int na = (int)act.size();
         GM_CUDA(cudaMemcpyAsync(d_act, act.data(), na * sizeof(int), cudaMemcpyHostToDevice, e->st));
@@ -1204,8 +1205,14 @@ int engine_solve_device(gm_engine *e, int sys, int nrhs, double2 *d_x, const dou
         const int cntn = na * nrhs * 2;
         launch_reduce_norms(e->d_part.as<double>(), nblk, cntn, e->d_norm.as<double>(), e->st);
         GM_CUDA(cudaGetLastError());
+        GM_CUDA(cudaEventRecord(e->ev_r, e->st));
         GM_CUDA(cudaMemcpyAsync(norms.data(), e->d_norm.p, cntn * sizeof(double), cudaMemcpyDeviceToHost, e->st));
         GM_CUDA(cudaStreamSynchronize(e->st));
+        collect_subst_times(e);
+        if (it == 0) {
+            cudaEventElapsedTime(&ms, t0, t1);
+            e->stats.ms_solve = ms;
+        }
         bool finite = true;
         std::vector<int> next;
         for (int z = 0; z < na; ++z) {
@@ -1269,6 +1276,9 @@ int engine_solve_device(gm_engine *e, int sys, int nrhs, double2 *d_x, const dou
         if (irset.empty()) {
             worst = 0;
             for (const gm_refine_info &ri : e->refine_info) worst = std::max(worst, ri.final_residual);
+            GM_CUDA(cudaEventRecord(e->ev_r, e->st));
+            GM_CUDA(cudaEventSynchronize(e->ev_r));
+            collect_subst_times(e);
             ++it;
             break;
         }
@@ -1295,9 +1305,7 @@ int engine_solve_device(gm_engine *e, int sys, int nrhs, double2 *d_x, const dou
             e->refine_info[f].method = GM_REFINE_IR;
         }
     }
-    GM_CUDA(cudaEventRecord(t1, e->st));
-    GM_CUDA(cudaEventSynchronize(t1));
-    cudaEventElapsedTime(&ms, t0, t1);
+    cudaEventElapsedTime(&ms, t1, e->ev_r);
     e->stats.ms_refine = ms;
     e->stats.ir_iterations = it;
     e->stats.ir_residual = worst;

@@ -7,6 +7,8 @@
 #include <vector>
 
 #include "../../include/germaine_gpu.h"
+#include <cstdlib>
+
 #include "common.hpp"
 #include "kernels.cuh"
 #include "symbolic.hpp"
@@ -41,6 +43,36 @@ struct DevBuf {
     template <class T> T *as() const { return reinterpret_cast<T *>(p); }
 };
 
+// Owning host allocation, page-locked where that is granted: a copy from the
+// device into pageable memory runs at a fifth of the link's rate.
+struct HostBuf {
+    void *p = nullptr;
+    size_t bytes = 0;
+    bool locked = false;
+    HostBuf() = default;
+    HostBuf(const HostBuf &) = delete;
+    HostBuf &operator=(const HostBuf &) = delete;
+    ~HostBuf() { release(); }
+    void release() {
+        if (p && locked) cudaFreeHost(p);
+        else std::free(p);
+        p = nullptr;
+        bytes = 0;
+    }
+    bool ensure(size_t nb) {  // grow-only
+        if (nb <= bytes && p) return true;
+        release();
+        locked = cudaMallocHost(&p, nb) == cudaSuccess;
+        if (!locked) {
+            (void)cudaGetLastError();
+            p = std::malloc(nb);
+        }
+        if (p) bytes = nb;
+        return p != nullptr;
+    }
+    template <class T> T *as() const { return reinterpret_cast<T *>(p); }
+};
+
 }  // namespace gm
 
 struct gm_engine {
@@ -51,11 +83,13 @@ struct gm_engine {
     int n = 0;
     gm::Symbolic sym;
 
-    // device copy of the symbolic structure
-    gm::DevBuf d_npiv, d_nfront, d_child0, d_child1, d_vars, d_inv, d_lvl_nodes;
-    gm::DevBuf d_front_off, d_var_off, d_inv_off, d_rhs_off, d_y_off, d_tri_off, d_desc, d_fdesc, d_sdesc;
+    // device copy of the symbolic structure, one allocation (dsym and the
+    // pointers here point into it)
+    gm::DevBuf d_sym;
+    const int64_t *tri_off = nullptr, *ent_dst = nullptr;
+    const int *ent_src = nullptr;
     int64_t tri_total = 0;   // entries of the triangle-inversion scratch per matrix
-    gm::DevBuf d_ent_dst, d_ent_src;
+    std::vector<int> node_at;   // position of each node in sym.lvl_nodes
     std::vector<gm::LevelInfo> levels;
     gm::DevSym dsym{};
 
@@ -68,7 +102,13 @@ struct gm_engine {
     int nf = 0;
     std::vector<float> freqs;
     std::vector<int> models;    // material model of each matrix of the batch
-    gm::DevBuf d_A, d_mass, d_pml, d_fq, d_front, d_npert, d_amax, d_tri;
+    gm::DevBuf d_A, d_mass, d_pml, d_fq, d_front, d_tri;
+    // what a factorisation reports, cleared and read back as one block
+    struct FactorReport {
+        unsigned long long npert, nswap, amax;   // perturbed pivots, row exchanges, max |A| (bits)
+        int tcerr, pad;                          // a tensor-core wait ran out
+    };
+    gm::DevBuf d_report;
     // threshold pivoting record [nf][n] (FactorArgs::pivsrc): every slot up
     // to pivsrc_ready_nf of the buffer at pivsrc_ready holds the identity
     // outside the pivoted levels
@@ -82,19 +122,18 @@ struct gm_engine {
     // storage moves or the batch size changes)
     struct CbPlan { int backend; int64_t prob_off, tile_off; int ntiles, tile; };
     std::vector<CbPlan> cb_plan;
-    gm::DevBuf d_cb_probs, d_cb_tiles, d_tcerr;
+    gm::DevBuf d_cb_probs, d_cb_tiles;
     const void *cb_plan_base = nullptr;
     int cb_plan_nf = 0;
     // the factorisation's launch sequence as a CUDA graph, replayed while
     // the buffers and the batch it was captured for stay the same
     struct FactorGraphKey {
-        const void *front = nullptr, *A = nullptr, *amax = nullptr, *npert = nullptr, *tcerr = nullptr;
+        const void *front = nullptr, *A = nullptr, *report = nullptr;
         const void *probs = nullptr, *tiles = nullptr, *pivsrc = nullptr, *tri = nullptr;
         int nf = 0, fp64 = 0;
         bool operator==(const FactorGraphKey &o) const {
-            return front == o.front && A == o.A && amax == o.amax && npert == o.npert && tcerr == o.tcerr &&
-                   probs == o.probs && tiles == o.tiles && pivsrc == o.pivsrc && tri == o.tri && nf == o.nf &&
-                   fp64 == o.fp64;
+            return front == o.front && A == o.A && report == o.report && probs == o.probs && tiles == o.tiles &&
+                   pivsrc == o.pivsrc && tri == o.tri && nf == o.nf && fp64 == o.fp64;
         }
     };
     FactorGraphKey fgraph_key, fgraph_seen;
@@ -117,6 +156,7 @@ struct gm_engine {
 
     // epilogue state
     gm::DevBuf d_src_k, d_rec_k, d_seis, d_field, d_res, d_grad, d_frame, d_frame_pass, d_misc;
+    gm::DevBuf d_amp, d_scal, d_sq;   // source amplitudes; gradient / Hessian scalars; Hessian sums
     gm::DevBuf d_xf, d_xa;   // forward / adjoint solutions kept for the gradient
     int xf_ns = 0, xa_ns = 0; // right-hand sides held in d_xf / d_xa (0: none valid)
     gm::DevBuf d_mask;       // forward-pass pruning mask of the current solve
@@ -126,9 +166,11 @@ struct gm_engine {
     std::vector<int> lvl_cfg;
     int tuned_nrhs = 0;
     std::vector<int> work_off;
-    std::vector<int> work_w; // per level: slice width the pairs were built for
     bool have_work = false;
-    std::vector<double> last_grad0, last_grad1;
+    // FP64 gradient of the last gm_grad_obj, diagonal Hessian of the last
+    // gm_hessian: one or two arrays of n doubles (0: none yet)
+    gm::HostBuf last_grad, last_hess;
+    int last_grad_arrays = 0, last_hess_arrays = 0;
     // per-shot gradient taper of ass_grad (SWS_TAPER_CIRCULAR_PER_SHOT 0, 1, 2),
     // its radius (SRTRADIUS, metres) and square half-width (FILTSIZE)
     int invmat = 1;               // INVMAT of calc_res_AC: 1 FWI residuals, 2 RTM (observed data)
@@ -140,10 +182,10 @@ struct gm_engine {
     float srt_radius = 0.0f;
     int filtsize = 0;
     gm::DevBuf d_taper;   // the taper's tables for the gradient kernel
-    std::vector<double> last_hess0, last_hess1;
 
     gm_stats stats{};
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_s0 = nullptr, ev_s1 = nullptr, ev_sm = nullptr;
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_s0 = nullptr, ev_s1 = nullptr, ev_sm = nullptr, ev_r = nullptr;
+    bool subst_timed = false;   // ev_s0, ev_sm, ev_s1 hold a substitution not yet in the stats
 
     gm_engine() = default;
     gm_engine(const gm_engine &) = delete;
@@ -154,6 +196,7 @@ struct gm_engine {
         if (ev_s0) cudaEventDestroy(ev_s0);
         if (ev_s1) cudaEventDestroy(ev_s1);
         if (ev_sm) cudaEventDestroy(ev_sm);
+        if (ev_r) cudaEventDestroy(ev_r);
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_join) cudaEventDestroy(ev_join);
         if (fgraph) cudaGraphExecDestroy(fgraph);

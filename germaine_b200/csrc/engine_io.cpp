@@ -79,7 +79,7 @@ int upload(gm::DevBuf &buf, const std::vector<T> &v, cudaStream_t st) {
 // spike right-hand sides of every shot and frequency into e->d_b, forward solve into xout;
 // the spike amplitude is that of src_physics's source routine (RHS_source_AC / _TE)
 int forward_solve(gm_engine *e, int ns, const Geometry &g, double2 *xout, int src_physics = 0) {
-    const int nf = e->nf, n = e->n;
+    const int nf = e->nf;
     if (!src_physics) src_physics = e->cfg.physics;
     std::vector<double2> amp(nf);
     if (!e->wavelet.empty() && e->wavelet.size() != 2 * (size_t)nf)
@@ -93,18 +93,14 @@ int forward_solve(gm_engine *e, int ns, const Geometry &g, double2 *xout, int sr
     }
     int rc;
     if ((rc = upload(e->d_src_k, g.ksrc, e->st))) return rc;
-    gm::DevBuf amp_buf;
-    if ((rc = upload(amp_buf, amp, e->st))) return rc;
-    (void)n;
+    if ((rc = upload(e->d_amp, amp, e->st))) return rc;
     gm::RhsPattern pat;   // one spike per shot: prune the forward pass
     pat.per_col = g.ksrc.data();
     pat.ncol = ns;
     gm::SpikeRhs sp;      // and never form the dense right-hand sides
     sp.k = e->d_src_k.as<int>();
-    sp.amp = amp_buf.as<double2>();
-    rc = gm::engine_solve_device(e, GM_SYS_A, ns, xout, nullptr, &pat, &sp);
-    GM_CUDA(cudaStreamSynchronize(e->st));  // amp_buf is released on return
-    return rc;
+    sp.amp = e->d_amp.as<double2>();
+    return gm::engine_solve_device(e, GM_SYS_A, ns, xout, nullptr, &pat, &sp);
 }
 
 // cp_grad_frame's taper (coefficient and number of passes per grid point) on the device
@@ -507,20 +503,20 @@ extern "C" int gm_grad_obj(gm_engine *e, int nshots, const float *src_x, const f
         om2[f] = make_double2(a[0], a[1]);
         om[f] = make_double2(b[0], b[1]);
     }
-    gm::DevBuf scal;
     std::vector<double2> sc;
     sc.insert(sc.end(), stfu.begin(), stfu.end());
     sc.insert(sc.end(), om2.begin(), om2.end());
     sc.insert(sc.end(), om.begin(), om.end());
-    if ((rc = upload(scal, sc, e->st))) return rc;
-    GM_ALLOC(e->d_grad, 2 * (size_t)n * sizeof(double));
+    if ((rc = upload(e->d_scal, sc, e->st))) return rc;
+    GM_ALLOC(e->d_grad, 2 * (size_t)n * (sizeof(double) + sizeof(float)));
     gm::GradArgs ga{};
     ga.n = n; ga.nf = nf; ga.ns = nshots; ga.te = te;
     ga.xf = e->d_xf.as<double2>(); ga.xa = e->d_xa.as<double2>();
-    ga.stfu = scal.as<double2>(); ga.om2 = ga.stfu + stfu.size(); ga.om = ga.om2 + nf;
+    ga.stfu = e->d_scal.as<double2>(); ga.om2 = ga.stfu + stfu.size(); ga.om = ga.om2 + nf;
     ga.m0 = e->d_m0.as<float>() + (size_t)e->models[0] * n; ga.m1 = e->d_m1.as<float>() + (size_t)e->models[0] * n;
     ga.frame = e->d_frame.as<float>(); ga.passes = e->d_frame_pass.as<unsigned char>();
     ga.g0 = e->d_grad.as<double>(); ga.g1 = ga.g0 + n;
+    ga.f0 = reinterpret_cast<float *>(ga.g1 + n); ga.f1 = ga.f0 + n;
     if ((rc = shot_taper_tables(e, nshots, src_x, src_y, ntr, rec_x, rec_y, ga))) return rc;
     if (exact) {
         if (e->shot_taper) return fail(GM_ERROR_INVALID, "gm_grad_obj: the exact gradient takes no per-shot taper");
@@ -531,20 +527,15 @@ extern "C" int gm_grad_obj(gm_engine *e, int nshots, const float *src_x, const f
         gm::launch_gradient(ga, e->st);
     }
     GM_CUDA(cudaGetLastError());
-    e->last_grad0.resize(n);
-    e->last_grad1.assign(te ? n : 0, 0.0);
-    GM_CUDA(cudaMemcpyAsync(e->last_grad0.data(), ga.g0, n * sizeof(double), cudaMemcpyDeviceToHost, e->st));
-    if (te) GM_CUDA(cudaMemcpyAsync(e->last_grad1.data(), ga.g1, n * sizeof(double), cudaMemcpyDeviceToHost, e->st));
+    e->last_grad_arrays = 0;
+    if (!e->last_grad.ensure(2 * (size_t)n * sizeof(double)))
+        return fail(GM_ERROR_OUT_OF_MEMORY, "gm_grad_obj: host allocation failed");
+    e->last_grad_arrays = te ? 2 : 1;
+    GM_CUDA(cudaMemcpyAsync(e->last_grad.p, ga.g0, e->last_grad_arrays * (size_t)n * sizeof(double),
+                            cudaMemcpyDeviceToHost, e->st));
+    if (grad0) GM_CUDA(cudaMemcpyAsync(grad0, ga.f0, n * sizeof(float), cudaMemcpyDefault, e->st));
+    if (grad1 && te) GM_CUDA(cudaMemcpyAsync(grad1, ga.f1, n * sizeof(float), cudaMemcpyDefault, e->st));
     GM_CUDA(cudaStreamSynchronize(e->st));
-    std::vector<float> tmp(n);
-    if (grad0) {
-        for (int k = 0; k < n; ++k) tmp[k] = (float)e->last_grad0[k];
-        GM_CUDA(cudaMemcpy(grad0, tmp.data(), n * sizeof(float), cudaMemcpyDefault));
-    }
-    if (grad1 && te) {
-        for (int k = 0; k < n; ++k) tmp[k] = (float)e->last_grad1[k];
-        GM_CUDA(cudaMemcpy(grad1, tmp.data(), n * sizeof(float), cudaMemcpyDefault));
-    }
     if (l2_out) *l2_out = (float)(0.5 * l2);
     return worst;
 }
@@ -573,9 +564,10 @@ extern "C" int gm_get_misfit_fp64(gm_engine *e, int nmat, double *l2, double *l2
 
 extern "C" int gm_get_gradient_fp64(gm_engine *e, double *g0, double *g1) {
     if (!e) return fail(GM_ERROR_INVALID, "null engine");
-    if (e->last_grad0.empty()) return fail(GM_ERROR_STATE, "no gradient computed yet");
-    if (g0) std::memcpy(g0, e->last_grad0.data(), e->last_grad0.size() * sizeof(double));
-    if (g1 && !e->last_grad1.empty()) std::memcpy(g1, e->last_grad1.data(), e->last_grad1.size() * sizeof(double));
+    if (!e->last_grad_arrays) return fail(GM_ERROR_STATE, "no gradient computed yet");
+    const size_t n = (size_t)e->n;
+    if (g0) std::memcpy(g0, e->last_grad.as<double>(), n * sizeof(double));
+    if (g1 && e->last_grad_arrays == 2) std::memcpy(g1, e->last_grad.as<double>() + n, n * sizeof(double));
     return GM_OK;
 }
 
@@ -618,9 +610,8 @@ extern "C" int gm_hessian(gm_engine *e, int mode, int nshots, const float *src_x
     int worst = forward_solve(e, nshots, g, e->d_xf.as<double2>(), src_phys);
     if (worst < 0) return worst;
     e->xf_ns = nshots;
-    gm::DevBuf sq;
-    GM_ALLOC(sq, 2 * (size_t)nf * n * sizeof(double));
-    double *sqf = sq.as<double>(), *sqg = sqf + (size_t)nf * n;
+    GM_ALLOC(e->d_sq, 2 * (size_t)nf * n * sizeof(double));
+    double *sqf = e->d_sq.as<double>(), *sqg = sqf + (size_t)nf * n;
     gm::launch_hess_sq(e->d_xf.as<double2>(), n, nf, nshots, sqf, 0, e->st);
     GM_CUDA(cudaGetLastError());
 
@@ -629,8 +620,7 @@ extern "C" int gm_hessian(gm_engine *e, int mode, int nshots, const float *src_x
         const int blk = std::min(ntr, std::max(nshots, 32));
         const double a = gmh_hess_green_amp(e->cfg.physics, e->cfg.dh);
         std::vector<double2> amp(nf, make_double2(a, 0.0));
-        gm::DevBuf amp_buf;
-        if ((rc = upload(amp_buf, amp, e->st))) return rc;
+        if ((rc = upload(e->d_amp, amp, e->st))) return rc;
         if ((rc = upload(e->d_rec_k, g.kadj, e->st))) return rc;
         GM_ALLOC(e->d_xa, (size_t)nf * n * blk * sizeof(double2));
         for (int r0 = 0; r0 < ntr; r0 += blk) {
@@ -641,14 +631,13 @@ extern "C" int gm_hessian(gm_engine *e, int mode, int nshots, const float *src_x
             pat.ncol = nr;
             gm::SpikeRhs sp;
             sp.k = e->d_rec_k.as<int>() + r0;
-            sp.amp = amp_buf.as<double2>();
+            sp.amp = e->d_amp.as<double2>();
             const int src = gm::engine_solve_device(e, GM_SYS_A, nr, e->d_xa.as<double2>(), nullptr, &pat, &sp);
             if (src < 0) return src;
             if (src > worst) worst = src;
             gm::launch_hess_sq(e->d_xa.as<double2>(), n, nf, nr, sqg, r0 > 0, e->st);
             GM_CUDA(cudaGetLastError());
         }
-        GM_CUDA(cudaStreamSynchronize(e->st));   // amp_buf is released on return
     }
 
     if ((rc = ensure_frame(e))) return rc;
@@ -661,24 +650,25 @@ extern "C" int gm_hessian(gm_engine *e, int mode, int nshots, const float *src_x
         w[f] = te ? a1 : 4.0 * a2;                                          // AC: |2 Omega^2|^2
         w[nf + f] = te ? a2 : 0.0;
     }
-    gm::DevBuf wbuf;
-    if ((rc = upload(wbuf, w, e->st))) return rc;
+    if ((rc = upload(e->d_scal, w, e->st))) return rc;
     GM_ALLOC(e->d_grad, 2 * (size_t)n * sizeof(double));
     GM_ALLOC(e->d_misc, 2 * (size_t)n * sizeof(float));
     gm::HessArgs ha{};
     ha.n = n; ha.nf = nf; ha.te = te;
     ha.sqf = sqf; ha.sqg = mode == GM_HESS_GREEN ? sqg : nullptr;
-    ha.w0 = wbuf.as<double>(); ha.w1 = ha.w0 + nf;
+    ha.w0 = e->d_scal.as<double>(); ha.w1 = ha.w0 + nf;
     ha.m0 = e->d_m0.as<float>() + (size_t)e->models[0] * n; ha.m1 = e->d_m1.as<float>() + (size_t)e->models[0] * n;
     ha.frame = e->d_frame.as<float>(); ha.passes = e->d_frame_pass.as<unsigned char>();
     ha.h0 = e->d_grad.as<double>(); ha.h1 = ha.h0 + n;
     ha.f0 = e->d_misc.as<float>(); ha.f1 = ha.f0 + n;
     gm::launch_hess_final(ha, e->st);
     GM_CUDA(cudaGetLastError());
-    e->last_hess0.resize(n);
-    e->last_hess1.assign(te ? n : 0, 0.0);
-    GM_CUDA(cudaMemcpyAsync(e->last_hess0.data(), ha.h0, n * sizeof(double), cudaMemcpyDeviceToHost, e->st));
-    if (te) GM_CUDA(cudaMemcpyAsync(e->last_hess1.data(), ha.h1, n * sizeof(double), cudaMemcpyDeviceToHost, e->st));
+    e->last_hess_arrays = 0;
+    if (!e->last_hess.ensure(2 * (size_t)n * sizeof(double)))
+        return fail(GM_ERROR_OUT_OF_MEMORY, "gm_hessian: host allocation failed");
+    e->last_hess_arrays = te ? 2 : 1;
+    GM_CUDA(cudaMemcpyAsync(e->last_hess.p, ha.h0, e->last_hess_arrays * (size_t)n * sizeof(double),
+                            cudaMemcpyDeviceToHost, e->st));
     if (hess0) GM_CUDA(cudaMemcpyAsync(hess0, ha.f0, n * sizeof(float), cudaMemcpyDefault, e->st));
     if (hess1 && te) GM_CUDA(cudaMemcpyAsync(hess1, ha.f1, n * sizeof(float), cudaMemcpyDefault, e->st));
     GM_CUDA(cudaStreamSynchronize(e->st));
@@ -687,8 +677,9 @@ extern "C" int gm_hessian(gm_engine *e, int mode, int nshots, const float *src_x
 
 extern "C" int gm_get_hessian_fp64(gm_engine *e, double *h0, double *h1) {
     if (!e) return fail(GM_ERROR_INVALID, "null engine");
-    if (e->last_hess0.empty()) return fail(GM_ERROR_STATE, "no Hessian computed yet");
-    if (h0) std::memcpy(h0, e->last_hess0.data(), e->last_hess0.size() * sizeof(double));
-    if (h1 && !e->last_hess1.empty()) std::memcpy(h1, e->last_hess1.data(), e->last_hess1.size() * sizeof(double));
+    if (!e->last_hess_arrays) return fail(GM_ERROR_STATE, "no Hessian computed yet");
+    const size_t n = (size_t)e->n;
+    if (h0) std::memcpy(h0, e->last_hess.as<double>(), n * sizeof(double));
+    if (h1 && e->last_hess_arrays == 2) std::memcpy(h1, e->last_hess.as<double>() + n, n * sizeof(double));
     return GM_OK;
 }

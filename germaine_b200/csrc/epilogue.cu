@@ -252,7 +252,10 @@ __global__ void k_gradient(GradArgs a) {
     const int p = a.passes[k];
     for (int q = 0; q < p; ++q) { g0 *= c; g1 *= c; }
     a.g0[k] = g0;
-    if (a.te) a.g1[k] = g1;
+    a.f0[k] = (float)g0;
+    if (!a.te) return;
+    a.g1[k] = g1;
+    a.f1[k] = (float)g1;
 }
 
 void launch_gradient(const GradArgs &a, cudaStream_t st) {
@@ -298,6 +301,7 @@ __global__ void k_gradient_exact(GradArgs a, double wa, double wb, double wc) {
     const int p = a.passes[k];
     for (int q = 0; q < p; ++q) g *= c;
     a.g0[k] = g;
+    a.f0[k] = (float)g;
 }
 
 void launch_gradient_exact(const GradArgs &a, const float w[3], cudaStream_t st) {

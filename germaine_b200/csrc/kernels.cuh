@@ -195,10 +195,10 @@ struct SolveArgs {
     const int *xmap;
     // live (front position in its level, slice) pairs of a pruned forward
     // pass (device), level h at work[work_off[h] .. work_off[h + 1]) (host
-    // offsets), for slices of work_w[h] right-hand sides (host); NULL: no list
+    // offsets), for slices of 32 right-hand sides; empty above the small-front
+    // levels; NULL: no list
     const int2 *work;
     const int *work_off;
-    const int *work_w;
     // host: per level {forward rt, forward B, backward rt, backward B} chosen
     // by the autotuner (gm_autotune; 0 entries keep the default rule), or NULL
     const int *lvl_cfg;

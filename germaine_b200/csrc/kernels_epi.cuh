@@ -15,6 +15,7 @@ struct GradArgs {
     const float *frame;         // PML taper coefficient per grid point
     const unsigned char *passes;
     double *g0, *g1;            // [n] outputs (FP64)
+    float *f0, *f1;             // the same rounded to float
     // per-shot taper (0 none; 1 radial around the shot's source and every
     // receiver; 2 the term replaced by 1e-5 on the marked squares)
     int nx, shot_taper;

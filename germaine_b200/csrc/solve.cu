@@ -614,7 +614,7 @@ static void small_group(bool fwd, const SolveArgs<R> &a, const LevelInfo &L, con
 template <class R>
 static void small_level(bool fwd, const SolveArgs<R> &a, const LevelInfo &L, cudaStream_t st) {
     set_attrs<R, 32, 4>();
-    if (fwd && a.work && a.work_w[L.index] == 32) {
+    if (fwd && a.work) {
         if (L.max_piv <= 8) forward_small_work<R, 1>(a, L, st);
         else if (L.max_piv <= 16) forward_small_work<R, 2>(a, L, st);
         else if (L.max_piv <= 24) forward_small_work<R, 3>(a, L, st);
