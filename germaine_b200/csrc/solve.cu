@@ -51,6 +51,25 @@ __device__ __forceinline__ bool col_live(const SolveArgs<R> &a, int v, int col) 
     return !a.mask || a.mask[(size_t)v * a.mask_nch + (col >> 5)];
 }
 
+// The columns r of a slice in which child v's update vector was formed.  The
+// small-front levels form 32-column slices, pruned one by one; a wider slice
+// of a level above can cover a live and a pruned one, whose columns hold
+// what an earlier solve left there.
+template <int TC>
+struct LiveCols {
+    static_assert(TC <= 40, "a slice meets at most two 32-column groups");
+    int lo = 0, n = TC;
+    template <class R>
+    __device__ __forceinline__ LiveCols(const SolveArgs<R> &a, int v, int r0, int rn) {
+        if (TC % 32 == 0 || v < 0 || !a.mask || (r0 & 31) + rn <= 32) return;
+        const unsigned char *m = a.mask + (size_t)v * a.mask_nch + (r0 >> 5);
+        const int cut = 32 - (r0 & 31);
+        lo = m[0] ? 0 : cut;
+        n = (m[1] ? rn : cut) - lo;
+    }
+    __device__ __forceinline__ bool has(int r) const { return TC % 32 == 0 || (unsigned)(r - lo) < (unsigned)n; }
+};
+
 // matrix handled by this CTA: blockIdx.z indexes the launch's matrix list
 template <class R>
 __device__ __forceinline__ size_t solve_matrix(const SolveArgs<R> &a) {
@@ -200,6 +219,7 @@ __global__ void __launch_bounds__(NT) k_fwd_rhs(SolveArgs<R> a, int lvl_first, i
     const int c0 = a.s.child0[c.node], c1 = a.s.child1[c.node];
     const C *W0 = c0 >= 0 && live(a, c0, r0, c.rn) ? Wall + (size_t)a.s.rhs_off[c0] * a.ldr : nullptr;
     const C *W1 = c1 >= 0 && live(a, c1, r0, c.rn) ? Wall + (size_t)a.s.rhs_off[c1] * a.ldr : nullptr;
+    const LiveCols<TC> l0(a, c0, r0, c.rn), l1(a, c1, r0, c.rn);
     const size_t ldr = a.ldr;
     const bool implicit = a.spike_k != nullptr;
     const bool pv = !TRANS && a.pivsrc;
@@ -222,8 +242,8 @@ __global__ void __launch_bounds__(NT) k_fwd_rhs(SolveArgs<R> a, int lvl_first, i
                 v[e] = c.X[(size_t)row * ldr + r];
             }
             C g = czero<C>();
-            if (q0 >= 0) g = cadd(g, W0[(size_t)q0 * ldr + r]);
-            if (q1 >= 0) g = cadd(g, W1[(size_t)q1 * ldr + r]);
+            if (q0 >= 0 && l0.has(r)) g = cadd(g, W0[(size_t)q0 * ldr + r]);
+            if (q1 >= 0 && l1.has(r)) g = cadd(g, W1[(size_t)q1 * ldr + r]);
             v[e] = cadd(v[e], g);
         }
     }
@@ -282,13 +302,14 @@ __global__ void __launch_bounds__(NT) k_fwd_ring(SolveArgs<R> a, int lvl_first, 
     const int c0 = a.s.child0[c.node], c1 = a.s.child1[c.node];
     const C *W0 = c0 >= 0 && live(a, c0, chunk * TC, c.rn) ? Wall + (size_t)a.s.rhs_off[c0] * a.ldr : nullptr;
     const C *W1 = c1 >= 0 && live(a, c1, chunk * TC, c.rn) ? Wall + (size_t)a.s.rhs_off[c1] * a.ldr : nullptr;
+    const LiveCols<TC> l0(a, c0, chunk * TC, c.rn), l1(a, c1, chunk * TC, c.rn);
     TileAcc<C, RT, B> acc;
     zero_acc(acc);
     for_acc(acc, rows, c.rn, threadIdx.x, [&](int row, int r, C &v) {
         const int i = i0 + row;
         const int q0 = W0 ? inv[i] : -1, q1 = W1 ? inv[c.f + i] : -1;
-        if (q0 >= 0) v = csub(v, W0[(size_t)q0 * ldr + r]);
-        if (q1 >= 0) v = csub(v, W1[(size_t)q1 * ldr + r]);
+        if (q0 >= 0 && l0.has(r)) v = csub(v, W0[(size_t)q0 * ldr + r]);
+        if (q1 >= 0 && l1.has(r)) v = csub(v, W1[(size_t)q1 * ldr + r]);
     });
     pipe_product<R, TRANS, true, false, RT, B>(st, c.F, c.f, i0, rows, 0, c.s,
                                                [&](int k) { return Y + (size_t)k * ldr; }, c.rn, acc);
