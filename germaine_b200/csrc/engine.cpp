@@ -712,11 +712,12 @@ static void collect_subst_times(gm_engine *e) {
 
 // One substitution over the right-hand sides in xT; fmap (device, nfz
 // entries) restricts it to those matrices of the batch (NULL: all); y is the
-// pivot workspace.
+// pivot workspace.  Right-hand sides given by spikes or b are read from there
+// (x need not hold anything).
 template <class R>
 static void substitute(gm_engine *e, void *xT, void *y, int nrhs, int trans, const unsigned char *mask = nullptr,
                        const int *fmap = nullptr, int nfz = 0, const int *xmap = nullptr,
-                       const SpikeRhs *spikes = nullptr) {
+                       const SpikeRhs *spikes = nullptr, const double2 *b = nullptr) {
     collect_subst_times(e);   // the events are used again
     cudaEventRecord(e->ev_s0, e->st);
     SolveArgs<R> a{};
@@ -742,9 +743,11 @@ static void substitute(gm_engine *e, void *xT, void *y, int nrhs, int trans, con
     a.trans = trans;
     a.mask = mask;
     a.mask_nch = (nrhs + 31) / 32;
-    if (spikes && mask) {   // implicit right-hand sides: x not cleared beforehand
+    if (spikes) {
         a.spike_k = spikes->k;
         a.spike_amp = spikes->amp;
+    } else {
+        a.b = b;
     }
     // GM_TRACE_LEVELS=1: device time of every level of both passes on stderr
     static const bool trace = std::getenv("GM_TRACE_LEVELS") != nullptr;
@@ -1144,23 +1147,17 @@ int engine_solve_device(gm_engine *e, int sys, int nrhs, double2 *d_x, const dou
     e->stats.n_subst = 0;
     e->subst_timed = false;
     GM_CUDA(cudaEventRecord(t0, e->st));
-    // initial solve in working precision: in FP64 in place in x (b copied
-    // into it), in complex64 in the work buffer and then added into x = 0
+    // initial solve in working precision: in FP64 in x, in complex64 in the
+    // work buffer and then converted into x; the right-hand sides are read
+    // where they are (pruned fronts: y = 0)
     const unsigned char *mask = build_mask(e, nrhs, pattern);
     const bool implicit = !d_b;
-    // FP64 with implicit spikes and a pruning mask: x is not cleared, the
-    // passes take b from the spike list (pruned fronts: y = 0)
-    const bool lazy_b = implicit && fp64 && mask;
-    if (implicit && !lazy_b) launch_spikes(d_x, e->n, e->nf, nrhs, spikes->k, spikes->amp, e->st);   // x = b
     if (fp64) {
-        if (!implicit) GM_CUDA(cudaMemcpyAsync(d_x, d_b, cnt * sizeof(double2), cudaMemcpyDeviceToDevice, e->st));
-        substitute<double>(e, d_x, e->d_t.p, nrhs, sys, mask, nullptr, 0, nullptr, lazy_b ? spikes : nullptr);
+        substitute<double>(e, d_x, e->d_t.p, nrhs, sys, mask, nullptr, 0, nullptr, implicit ? spikes : nullptr, d_b);
     } else {
         if (const int rc = ensure_y(e, nrhs)) return rc;
-        launch_convert_down<float>(implicit ? d_x : d_b, e->d_t.p, cnt, e->st);
-        GM_CUDA(cudaMemsetAsync(d_x, 0, cnt * sizeof(double2), e->st));
-        substitute<float>(e, e->d_t.p, e->d_y.p, nrhs, sys, mask);
-        launch_add_up<float>(d_x, e->d_t.p, cnt, e->st);
+        substitute<float>(e, e->d_t.p, e->d_y.p, nrhs, sys, mask, nullptr, 0, nullptr, implicit ? spikes : nullptr, d_b);
+        launch_convert_up(d_x, e->d_t.as<float2>(), cnt, e->st);
     }
     GM_CUDA(cudaGetLastError());
     GM_CUDA(cudaEventRecord(t1, e->st));   // read after the first residual's wait

@@ -14,18 +14,6 @@
 
 namespace gm {
 
-__global__ void k_spikes(double2 *b, int n, int nf, int ns, const int *ksrc, const double2 *amp) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nf * ns) return;
-    const int f = t / ns, s = t % ns;
-    b[((size_t)f * n + ksrc[s]) * ns + s] = amp[f];
-}
-
-void launch_spikes(double2 *b, int n, int nf, int ns, const int *ksrc, const double2 *amp, cudaStream_t st) {
-    cudaMemsetAsync(b, 0, (size_t)nf * n * ns * sizeof(double2), st);
-    (k_spikes<<<(nf * ns + 255) / 256, 256, 0, st>>>(b, n, nf, ns, ksrc, amp), note_launch());
-}
-
 __device__ __forceinline__ double2 shifted(const double2 *x, int n, int ns, int k, int s) {
     // vec2mat: field value of grid point k is x[k + 1]; x[n] is defined as 0
     return (k + 1 < n) ? x[(size_t)(k + 1) * ns + s] : make_double2(0.0, 0.0);

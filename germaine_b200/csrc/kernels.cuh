@@ -202,13 +202,15 @@ struct SolveArgs {
     // host: per level {forward rt, forward B, backward rt, backward B} chosen
     // by the autotuner (gm_autotune; 0 entries keep the default rule), or NULL
     const int *lvl_cfg;
-    // implicit spike right-hand sides (with a pruning mask only; NULL: x
-    // holds b on entry): column r is spike_amp[matrix] on row spike_k[r] and
-    // zero elsewhere.  x is not cleared beforehand: the forward pass writes
-    // b + the children's updates at the pivot rows of every live front, and
-    // the backward pass takes y = 0 at the pivot rows of pruned fronts.
+    // right-hand sides that x does not hold on entry: implicit spikes (column
+    // r is spike_amp[matrix] on row spike_k[r] and zero elsewhere) or b
+    // ([nf][n][ldr], FP64); both NULL: x holds them.  x is not cleared
+    // beforehand: the forward pass writes b + the children's updates at the
+    // pivot rows of every live front, and the backward pass takes y = 0 at
+    // the pivot rows of pruned fronts.
     const int *spike_k;
     const double2 *spike_amp;
+    const double2 *b;
     // row exchanges of the factorisation's threshold pivoting (FactorArgs::
     // pivsrc; NULL: none): within each 32-pivot block of the pivoted fronts,
     // the forward pass of M x = b gathers the block's right-hand-side rows
@@ -267,6 +269,8 @@ int launch_matvec(const ResidArgs &a, const void *x, double2 *out, double *part,
 // y(T) <- x(double) and x(double) += d(T) over [nf][n][ldr]
 template <class R>
 void launch_convert_down(const double2 *src, void *dst, size_t count, cudaStream_t st);
+// x = d, converted up
+void launch_convert_up(double2 *x, const float2 *d, size_t count, cudaStream_t st);
 template <class R>
 void launch_add_up(double2 *x, const void *d, size_t count, cudaStream_t st);
 // x[f] += d[f] for the matrices f = fmap[0 .. nfz) (device list), per_f entries each

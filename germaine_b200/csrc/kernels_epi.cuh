@@ -37,7 +37,6 @@ struct HessArgs {
     float *f0, *f1;             // [n] float outputs: the sum rounded to float, then tapered in float
 };
 
-void launch_spikes(double2 *b, int n, int nf, int ns, const int *ksrc, const double2 *amp, cudaStream_t st);
 void launch_gather_seis(const double2 *x, int n, int nf, int ns, int ntr, const int *krec, float2 *seis, double2 *cal,
                         cudaStream_t st);
 void launch_field(const double2 *x, int n, int nf, int ns, float2 *field, cudaStream_t st);

@@ -292,6 +292,16 @@ void launch_add_up(double2 *x, const void *d, size_t count, cudaStream_t st) {
     (k_add_up<R><<<(unsigned)((count + 255) / 256), 256, 0, st>>>(x, reinterpret_cast<const cplx<R> *>(d), count), note_launch());
 }
 
+__global__ void k_convert_up(double2 *__restrict__ x, const float2 *__restrict__ d, size_t count) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < count) x[i] = cto_d(d[i]);
+}
+
+void launch_convert_up(double2 *x, const float2 *d, size_t count, cudaStream_t st) {
+    if (!count) return;
+    (k_convert_up<<<(unsigned)((count + 255) / 256), 256, 0, st>>>(x, d, count), note_launch());
+}
+
 // x[f] += d[f] over the matrices f = fmap[0 .. nfz) (per_f entries each)
 template <class R>
 __global__ void k_add_up_f(double2 *__restrict__ x, const cplx<R> *__restrict__ d, size_t per_f, const int *fmap) {

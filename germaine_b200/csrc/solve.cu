@@ -110,28 +110,52 @@ __device__ __forceinline__ Ctx<R> make_ctx(const SolveArgs<R> &a, int lvl_first,
     return c;
 }
 
+// Right-hand sides that x does not hold (implicit spikes, or the caller's FP64
+// b): the entry of a row and column of this slice.  Copied into x first, b
+// went through memory twice more, and in complex64 the spikes were written,
+// converted and the solution added to a cleared x (841 x 227, 100 right-hand
+// sides: 10 matrices in complex64 63.0 -> 60.7 ms a call, the gradient of 3
+// matrices, dense adjoint sources in FP64, 13.4 -> 13.0 ms).
+template <class R>
+struct OuterRhs {
+    using C = cplx<R>;
+    const int *spike_k;
+    const double2 *b;
+    C amp;
+    __device__ __forceinline__ OuterRhs(const SolveArgs<R> &a, int r0) {
+        const size_t f = solve_matrix(a);
+        spike_k = a.spike_k ? a.spike_k + r0 : nullptr;
+        b = a.b ? a.b + f * (size_t)a.s.n * a.ldr + r0 : nullptr;
+        amp = spike_k ? cconv<C>(a.spike_amp[f]) : czero<C>();
+    }
+    __device__ __forceinline__ bool given() const { return spike_k || b; }
+    __device__ __forceinline__ C at(int row, int r, size_t ldr) const {
+        if (b) return cconv<C>(b[(size_t)row * ldr + r]);
+        return spike_k[r] == row ? amp : czero<C>();
+    }
+};
+
 // The pivot rows of this front's slice of x receive the children's update
-// vectors (W0, W1: NULL for a child that is absent or pruned); with implicit
-// spike right-hand sides they become b + the updates, x not being read
+// vectors (W0, W1: NULL for a child that is absent or pruned); where x does
+// not hold the right-hand sides they become b + the updates, x not being read
 // (it is not cleared before the solve).
 template <class R>
 __device__ __forceinline__ void pivot_rhs(const SolveArgs<R> &a, const Ctx<R> &c, const int *inv, const cplx<R> *W0,
                                           const cplx<R> *W1, int r0, size_t ldr) {
     using C = cplx<R>;
-    const bool implicit = a.spike_k != nullptr;
-    if (!(W0 || W1 || implicit)) return;   // CTA-uniform
+    const OuterRhs<R> outer(a, r0);
+    if (!(W0 || W1 || outer.given())) return;   // CTA-uniform
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const C amp = implicit ? cconv<C>(a.spike_amp[solve_matrix(a)]) : czero<C>();
     for (int i = warp; i < c.s; i += NT / 32) {
         const int q0 = W0 ? inv[i] : -1, q1 = W1 ? inv[c.f + i] : -1;
-        if (!implicit && q0 < 0 && q1 < 0) continue;
+        if (!outer.given() && q0 < 0 && q1 < 0) continue;
         const int row = c.vars[i];
         for (int r = lane; r < c.rn; r += 32) {
             C v = czero<C>();
             if (q0 >= 0) v = cadd(v, W0[(size_t)q0 * ldr + r]);
             if (q1 >= 0) v = cadd(v, W1[(size_t)q1 * ldr + r]);
             C &x = c.X[(size_t)row * ldr + r];
-            x = implicit ? (a.spike_k[r0 + r] == row ? cadd(amp, v) : v) : cadd(x, v);
+            x = cadd(outer.given() ? outer.at(row, r, ldr) : x, v);
         }
     }
     __syncthreads();
@@ -221,11 +245,10 @@ __global__ void __launch_bounds__(NT) k_fwd_rhs(SolveArgs<R> a, int lvl_first, i
     const C *W1 = c1 >= 0 && live(a, c1, r0, c.rn) ? Wall + (size_t)a.s.rhs_off[c1] * a.ldr : nullptr;
     const LiveCols<TC> l0(a, c0, r0, c.rn), l1(a, c1, r0, c.rn);
     const size_t ldr = a.ldr;
-    const bool implicit = a.spike_k != nullptr;
+    const OuterRhs<R> outer(a, r0);
     const bool pv = !TRANS && a.pivsrc;
-    if (!(W0 || W1 || implicit || pv)) return;   // CTA-uniform: x holds the block's right-hand sides already
+    if (!(W0 || W1 || outer.given() || pv)) return;   // CTA-uniform: x holds the block's right-hand sides already
     const unsigned char *psrc = pv ? a.pivsrc + solve_matrix(a) * (size_t)a.s.n : nullptr;
-    const C amp = implicit ? cconv<C>(a.spike_amp[solve_matrix(a)]) : czero<C>();
     const int kb = min(SNB, c.s - k0);
     C v[NE];   // all of the block's rows are read before any is written
 #pragma unroll
@@ -236,11 +259,7 @@ __global__ void __launch_bounds__(NT) k_fwd_rhs(SolveArgs<R> a, int lvl_first, i
             const int p = k0 + (pv ? psrc[c.vars[k0 + q]] : q);
             const int row = c.vars[p];
             const int q0 = W0 ? inv[p] : -1, q1 = W1 ? inv[c.f + p] : -1;
-            if (implicit) {
-                if (a.spike_k[r0 + r] == row) v[e] = amp;
-            } else {
-                v[e] = c.X[(size_t)row * ldr + r];
-            }
+            v[e] = outer.given() ? outer.at(row, r, ldr) : c.X[(size_t)row * ldr + r];
             C g = czero<C>();
             if (q0 >= 0 && l0.has(r)) g = cadd(g, W0[(size_t)q0 * ldr + r]);
             if (q1 >= 0 && l1.has(r)) g = cadd(g, W1[(size_t)q1 * ldr + r]);
@@ -505,8 +524,8 @@ __global__ void __launch_bounds__(NT, small_ctas<R, P8>(false)) k_bwd_small(Solv
     }
     // t = y - acc in sm.Y (row q of the next product's right operand = pivot
     // q); y = 0 where the pruned forward pass skipped the front (its rows of
-    // x are not cleared when the right-hand sides are implicit spikes)
-    if (a.spike_k) {   // y = 0 in the right-hand sides the pruned forward pass skipped
+    // x are not cleared when x does not hold the right-hand sides)
+    if ((a.spike_k || a.b) && a.mask) {   // y = 0 in the right-hand sides the pruned forward pass skipped
         for (int t = threadIdx.x; t < s * TC; t += NT) {
             const int q = t / TC, r = t % TC;
             if (r >= c.rn) continue;
