@@ -115,8 +115,9 @@ extern "C" int gm_engine_create(int device, const gm_config *cfg, gm_engine **ou
     std::vector<int64_t> ent_dst;
     std::vector<int> ent_src;
     std::vector<int64_t> ent_lvl_off(s.nnodes + 1, 0);
-    ent_dst.reserve(s.ent_pos.size());
-    ent_src.reserve(s.ent_pos.size());
+    ent_dst.resize(s.ent_pos.size());
+    ent_src.resize(s.ent_pos.size());
+    int64_t ne = 0;
     e->levels.resize(s.nlevels);
     for (int h = 0; h < s.nlevels; ++h) {
         gm::LevelInfo &L = e->levels[h];
@@ -134,24 +135,24 @@ extern "C" int gm_engine_create(int device, const gm_config *cfg, gm_engine **ou
             L.mid_words = std::max(L.mid_words, (int64_t)(fv + 1) * sv + (int64_t)(sv | 1) * (fv - sv));
             L.front_words = std::max(L.front_words, gm::front_words_of(fv, sv));
         }
-        L.ent_first = (int64_t)ent_dst.size();
+        L.ent_first = ne;
         for (int t = L.first; t < L.first + L.count; ++t) {
             const int v = s.lvl_nodes[t];
-            ent_lvl_off[t] = (int64_t)ent_dst.size();
-            for (int64_t q = s.ent_off[v]; q < s.ent_off[v + 1]; ++q) {
-                ent_dst.push_back(s.front_off[v] + s.ent_pos[q]);
+            ent_lvl_off[t] = ne;
+            for (int64_t q = s.ent_off[v]; q < s.ent_off[v + 1]; ++q, ++ne) {
+                ent_dst[ne] = s.front_off[v] + s.ent_pos[q];
                 int id = s.ent_id[q];
                 if (e->cfg.op_mode == GM_OP_EXACT) {   // M = A: entry (r, c) reads A[r][c]
                     const int dir = id / s.n, c = id % s.n;
                     const int r = c + gm::stencil_di(dir) + gm::stencil_dj(dir) * s.nx;
                     id = (8 - dir) * s.n + r;
                 }
-                ent_src.push_back(id);
+                ent_src[ne] = id;
             }
         }
-        L.ent_count = (int64_t)ent_dst.size() - L.ent_first;
+        L.ent_count = ne - L.ent_first;
     }
-    ent_lvl_off[s.nnodes] = (int64_t)ent_dst.size();
+    ent_lvl_off[s.nnodes] = ne;
     // levels with more than 32 pivots: rows of the pivot workspace, and each
     // front's part of the triangle-inversion scratch (one level at a time)
     std::vector<int64_t> y_off(s.nnodes, -1), tri_off(s.nnodes, 0);
@@ -1394,13 +1395,9 @@ extern "C" int gm_autotune(gm_engine *e, int nrhs, int reps) {
         time_pass(sf, sb);
         const float margin = c[0] ? 0.97f : 1.0f;
         for (int h = 0; h < nl; ++h) {
-            // forward levels of fronts with at most 32 pivots keep 32-row
-            // tiles: only that kernel runs the pruned first pass of
-            // spike right-hand sides from a work list
-            const bool fwd_ok = !(c[0] == 64 && e->levels[h].max_piv <= 32);
-            if (fwd_ok && sf[h] < margin * best_f[h]) {
-                best_f[h] = sf[h]; pick[4 * h + 0] = c[0]; pick[4 * h + 1] = c[1];
-            }
+            // (fronts of at most 32 pivots: one kernel, sized by the pivots)
+            if (c[0] && e->levels[h].max_piv <= 32) continue;
+            if (sf[h] < margin * best_f[h]) { best_f[h] = sf[h]; pick[4 * h + 0] = c[0]; pick[4 * h + 1] = c[1]; }
             if (sb[h] < margin * best_b[h]) { best_b[h] = sb[h]; pick[4 * h + 2] = c[0]; pick[4 * h + 3] = c[1]; }
         }
     }
@@ -1429,8 +1426,9 @@ extern "C" int gm_autotune(gm_engine *e, int nrhs, int reps) {
     for (int h = 0; h < nl; ++h)
         for (int d = 0; d < 2; ++d)
             if (pick[4 * h + 2 * d] == 0) {
-                pick[4 * h + 2 * d] = gm::solve_level_rt(e->levels[h]);
-                pick[4 * h + 2 * d + 1] = b_def;
+                const bool small = e->levels[h].max_piv <= 32;
+                pick[4 * h + 2 * d] = small ? 32 : gm::solve_level_rt();
+                pick[4 * h + 2 * d + 1] = small ? 4 : b_def;
             }
     GM_CUDA(cudaGetLastError());
     e->lvl_cfg = pick;

@@ -222,7 +222,7 @@ struct SolveArgs {
 // right-hand sides per substitution slice for nrhs right-hand sides
 int solve_slice_width(int nrhs, bool fp64);
 // the built-in tile height of a level's substitution kernels (32 or 64)
-int solve_level_rt(const LevelInfo &L);
+int solve_level_rt();
 
 template <class R>
 void launch_solve_forward_level(const SolveArgs<R> &a, const LevelInfo &L, cudaStream_t st);

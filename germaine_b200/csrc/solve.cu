@@ -546,9 +546,6 @@ __global__ void __launch_bounds__(NT, small_ctas<R, P8>(false)) k_bwd_small(Solv
 }
 
 template <class R, int RT, int B>
-static size_t solve_smem() { return sizeof(SolveSmem<cplx<R>, RT, B>); }
-
-template <class R, int RT, int B>
 static size_t pipe_smem() { return PST * sizeof(PipeStage<cplx<R>, RT, B>); }
 
 template <class K>
@@ -568,7 +565,7 @@ template <class R, int RT, int B>
 static void set_attrs() {
     static bool done = false;
     if (done) return;
-    const size_t sm = pipe_smem<R, RT, B>(), sms = solve_smem<R, RT, B>();
+    const size_t sm = pipe_smem<R, RT, B>();
     set_smem(k_fwd_ring<R, false, RT, B>, sm);
     set_smem(k_fwd_ring<R, true, RT, B>, sm);
     set_smem(k_bwd_ring<R, false, RT, B>, sm);
@@ -595,22 +592,23 @@ static int env_int(const char *name) {
     return v ? std::atoi(v) : 0;
 }
 
-// Tile height of a level: 32-row tiles wherever the level has many fronts
-// (measured on 841 x 227: 14 % less substitution time than 64-row tiles,
-// the gain coming from the 4096 .. 16-front levels), 64-row tiles on the
-// top levels of at most four fronts, where the tiles of one front are the
-// parallelism.  GM_SOLVE_RT=32 / 64 forces one height on every level.
-static int level_rt(const LevelInfo &L) {
+// Tile height of the levels with more than 32 pivots: 32 rows.  64-row tiles
+// read each right operand half as often, but leave too few CTAs on the top
+// levels and hold fewer per SM.  Backward pass, 32 / 64 rows: 2060 x 1060, one
+// matrix, 100 right-hand sides 8.44 / 8.90 ms; 841 x 227, 10 matrices 6.25 /
+// 6.28 ms, in complex64 (four passes) 19.0 / 18.8 ms.  (64 rows on levels of at
+// most four fronts only: 8.55, 6.25 and 19.1 ms.)  GM_SOLVE_RT=64 forces 64;
+// gm_autotune times both.
+static int level_rt() {
     static const int forced = env_int("GM_SOLVE_RT");
-    if (forced == 32 || forced == 64) return forced;
-    return L.count > 4 ? 32 : 64;
+    return forced == 64 ? 64 : 32;
 }
 
-// Right-hand-side slice width (8 B).  Measured on 841 x 227 with 100
-// right-hand sides: 32 / 40 / 56 columns give 36.6 / 36.6 / 38.0 ms per
-// complex128 substitution and 19.9 / 19.1 / 19.8 ms per complex64 one, so
-// the lower levels are not bound by re-reading the factors per slice.
-// GM_SOLVE_B=4 / 5 forces 32 / 40.
+// Right-hand-side slice width (8 B) of the same levels.  With 100 right-hand
+// sides 32 / 40 columns: 841 x 227, 10 matrices, both passes 7.14 / 7.34 ms
+// (one substitution), in complex64 38.6 / 38.7 ms (four); the wider slices
+// read the factors less often and are kept in complex64.  GM_SOLVE_B=4 / 5
+// forces 32 / 40.
 template <class R>
 static int slice_b(int nrhs) {
     static const int forced = env_int("GM_SOLVE_B");
@@ -724,18 +722,7 @@ static void backward_level(const SolveArgs<R> &a, const LevelInfo &L, cudaStream
 }
 
 template <class R, int B>
-static void level_pass(bool fwd, const SolveArgs<R> &a, const LevelInfo &L, cudaStream_t st) {
-    if (level_rt(L) == 32) {
-        if (fwd) forward_level<R, 32, B>(a, L, st);
-        else backward_level<R, 32, B>(a, L, st);
-    } else {
-        if (fwd) forward_level<R, 64, B>(a, L, st);
-        else backward_level<R, 64, B>(a, L, st);
-    }
-}
-
-template <class R, int B>
-static void level_pass_rt(bool fwd, int rt, const SolveArgs<R> &a, const LevelInfo &L, cudaStream_t st) {
+static void level_pass(bool fwd, int rt, const SolveArgs<R> &a, const LevelInfo &L, cudaStream_t st) {
     if (rt == 32) {
         if (fwd) forward_level<R, 32, B>(a, L, st);
         else backward_level<R, 32, B>(a, L, st);
@@ -753,15 +740,10 @@ static void dispatch(bool fwd, const SolveArgs<R> &a_in, const LevelInfo &L, cud
     if (L.count == 0 || solve_nfz(a_in) <= 0) return;
     SolveArgs<R> a = a_in;
     if (!level_pivots<R>(L)) a.pivsrc = nullptr;   // no row exchanges on this level
-    if (a.lvl_cfg) {
-        const int *c = a.lvl_cfg + 4 * L.index + (fwd ? 0 : 2);
-        const int rt = c[0] ? c[0] : level_rt(L), b = c[1] ? c[1] : slice_b<R>(a.nrhs);
-        if (b == 5) level_pass_rt<R, 5>(fwd, rt, a, L, st);
-        else level_pass_rt<R, 4>(fwd, rt, a, L, st);
-        return;
-    }
-    if (slice_b<R>(a.nrhs) == 5) level_pass<R, 5>(fwd, a, L, st);
-    else level_pass<R, 4>(fwd, a, L, st);
+    const int *c = a.lvl_cfg ? a.lvl_cfg + 4 * L.index + (fwd ? 0 : 2) : nullptr;
+    const int rt = c && c[0] ? c[0] : level_rt(), b = c && c[1] ? c[1] : slice_b<R>(a.nrhs);
+    if (b == 5) level_pass<R, 5>(fwd, rt, a, L, st);
+    else level_pass<R, 4>(fwd, rt, a, L, st);
 }
 
 template <class R>
@@ -790,7 +772,7 @@ void preload_solve_kernels() {
 }
 
 int solve_slice_width(int nrhs, bool fp64) { return 8 * (fp64 ? slice_b<double>(nrhs) : slice_b<float>(nrhs)); }
-int solve_level_rt(const LevelInfo &L) { return level_rt(L); }
+int solve_level_rt() { return level_rt(); }
 
 template void launch_solve_forward_level<double>(const SolveArgs<double> &, const LevelInfo &, cudaStream_t);
 template void launch_solve_forward_level<float>(const SolveArgs<float> &, const LevelInfo &, cudaStream_t);

@@ -91,10 +91,6 @@ __device__ __forceinline__ void stage_dinv_p(C (*L)[RT + SPAD], const C *F, int 
         }
     }
 }
-template <class C, bool FWD, bool TRANS, int RT, int B>
-__device__ __forceinline__ void stage_dinv(SolveSmem<C, RT, B> &sm, const C *F, int f, int k0, int kb) {
-    stage_dinv_p<C, FWD, TRANS, RT>(sm.L, F, f, k0, kb, 0, kb, threadIdx.x, NT);
-}
 
 // Per-thread accumulators of an RT x 8B complex output tile (128 threads,
 // lt = 0 .. 127), in the layout of the tile product that fills them.
@@ -353,10 +349,6 @@ __device__ __forceinline__ void stage_rows_p(C (*Y)[TC + SPAD], RowPtr row_ptr, 
         const int q = t / TC, r = t % TC;
         if (r < rn) cp_async_elem(&Y[q][r], row_ptr(q) + r);
     }
-}
-template <class C, int RT, int B, class RowPtr>
-__device__ __forceinline__ void stage_rows(SolveSmem<C, RT, B> &sm, RowPtr row_ptr, int qb, int rn) {
-    stage_rows_p<C, 8 * B>(sm.Y, row_ptr, qb, rn, threadIdx.x, NT);
 }
 
 }  // namespace gm
