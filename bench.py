@@ -49,7 +49,7 @@ DH, NPML, ROW = 25.0, 20, 2
 RESIDUAL_TARGET = 1e-10
 METRIC = "shot-solves/s (factor+solve) mixed vs FP64 on B200 at resid<=1e-10; %roofline"
 # DRAM bytes of one complex128 backward substitution pass on 4 frequencies
-# (the k_bwd_small / k_bwd_ring / k_bwd_piv launches of the FP64 engine's
+# (the k_bwd_small / k_bwd_ring / k_bwd_tri launches of the FP64 engine's
 # timed step, ncu dram__bytes_read.sum + dram__bytes_write.sum, summed)
 BWD_TRAFFIC_FP64_4FREQ = 3.585e9
 PEAK_KIND = "measured FP64 rate, the higher of CUDA-core DFMA (gm_peak_fp64) and FP64 MMA (gm_peak_fp64_mma)"
@@ -428,7 +428,7 @@ def run_gpu(args):
     value = units / (head["ms"] * 1e-3)
     st = head["stats"]
     # roofline of the backward substitution pass (K5 k_bwd_small on the
-    # fronts with at most 32 pivots, k_bwd_ring + k_bwd_piv above them;
+    # fronts with at most 32 pivots, k_bwd_ring + k_bwd_tri above them;
     # the dense part of every solve: the forward pass is pruned to the
     # fronts on the paths from the sources to the root): the stored U
     # entries read once + the right-hand sides read (y, ancestors' x) and the
@@ -498,7 +498,7 @@ def run_gpu(args):
                   for n in ("fp64", "mixed")},
         "mixed_over_fp64": fp64["ms"] / mixed["ms"],
         "per_frequency": per_freq,
-        "roofline": {"kernel": "K5 backward substitution (k_bwd_small, k_bwd_ring + k_bwd_piv, %s)" % ("complex128" if csize == 16 else "complex64"),
+        "roofline": {"kernel": "K5 backward substitution (k_bwd_small, k_bwd_ring + k_bwd_tri, %s)" % ("complex128" if csize == 16 else "complex64"),
                      "bound": "hbm", "achieved": achieved, "peak": peak_hbm, "unit": "GB/s",
                      "frac": achieved / peak_hbm, "peak_kind": peak_kind, "traffic": traffic,
                      "algorithmic_bytes": subst_bytes, "ms_per_launch_group": subst_ms},
