@@ -10,6 +10,7 @@
 // All wavefield reads honour the reference's vec2mat one-slot shift: the
 // value used at grid point k is x[k+1], and x[N] is defined as 0.
 #include "kernels_epi.cuh"
+#include "adjoint_index.hpp"
 #include "cplx.cuh"
 
 namespace gm {
@@ -146,12 +147,12 @@ void launch_residual_shot(const double2 *cal, const float2 *obs, int nfs, int nt
 // as before, took 846 us for 3 x 100 shots x 801 receivers; so 7 us).
 __global__ void k_adjoint_src(double2 *b, int n, int nf, int ns, int ntr, const int *kadj, const double2 *res,
                               double dh2) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;   // receiver * ns + shot
-    if (t >= ntr * ns) return;
-    const int q = t / ns, s = t - q * ns, f = blockIdx.y, k = kadj[q];
+    const AdjointItem it = adjoint_item((size_t)blockIdx.x * blockDim.x + threadIdx.x, ns, ntr);
+    if (!it.in) return;
+    const int f = blockIdx.y, k = kadj[it.receiver];
     if (k < 0) return;
-    const double2 r = res[((size_t)f * ns + s) * ntr + q];
-    b[((size_t)f * n + k) * ns + s] = make_double2(r.x / dh2, -r.y / dh2);
+    const double2 r = res[((size_t)f * ns + it.shot) * ntr + it.receiver];
+    b[((size_t)f * n + k) * ns + it.shot] = make_double2(r.x / dh2, -r.y / dh2);
 }
 
 void launch_adjoint_src(double2 *b, int n, int nf, int ns, int ntr, const int *kadj, const double2 *res, double dh2,
