@@ -204,7 +204,9 @@ __device__ __forceinline__ void add_entries(const FactorArgs<R> &a, const NodeDe
 
 // Static pivoting: a pivot of magnitude below pivtol (or NaN) is replaced by
 // itself scaled to magnitude pivtol (pivtol when it is zero) and counted.
-// The test compares squares, so the common case takes no square root.
+// The test compares squares, so the common case takes no square root; where
+// pivtol^2 underflows to zero every square would pass, and magnitudes are
+// compared (a caller that tests the square first has to come here then).
 template <class R>
 __device__ __forceinline__ cplx<R> static_pivot(cplx<R> piv, R pivtol, int &npert) {
     const R m2 = cabs2(piv), tol2 = pivtol * pivtol;
@@ -303,7 +305,7 @@ __device__ void factor_diag_block(const FactorArgs<R> &a, cplx<R> *F, int f, int
     C *Bb = Ab + NB * ASTR;                   // [PW8][BSTR]
     C *rd = Bb + PW8 * BSTR;                  // [NB] reciprocal pivots
     __shared__ int rowat[NB];                 // block row (equation order) at pivot position q
-    const R pivtol = (R)(a.pivscale * __longlong_as_double((long long)*a.amax));
+    const R pivtol = (R)(a.pivscale * __longlong_as_double((long long)*a.amax)), tol2 = pivtol * pivtol;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid < NB) {
         rowat[tid] = tid;
@@ -363,7 +365,7 @@ __device__ void factor_diag_block(const FactorArgs<R> &a, cplx<R> *F, int f, int
                         }
                     }
                     C piv = pr[0];
-                    if (!(cabs2(piv) >= pivtol * pivtol) || !(pivtol > R(0))) {   // rare, off the chain: rp is formed already
+                    if (!(cabs2(piv) >= tol2) || !(tol2 > R(0))) {   // rare, off the chain: rp is formed already
                         piv = static_pivot<R>(piv, pivtol, np);
                         rp = crcp(piv);
                     }
@@ -983,7 +985,7 @@ __global__ void __launch_bounds__(NTH, NTH == 128 ? (sizeof(R) == 8 ? 5 : 8) : N
         __syncthreads();
     }
 
-    const R pivtol = (R)(a.pivscale * __longlong_as_double((long long)*a.amax));
+    const R pivtol = (R)(a.pivscale * __longlong_as_double((long long)*a.amax)), tol2 = pivtol * pivtol;
     int np = 0, nsw = 0;   // the panels' warp: the same in every lane
     // 1. the panel at p0 (one warp): lane l holds pivot row p0 + l in registers,
     // x[i] its entry in column p + i
@@ -1029,7 +1031,7 @@ __global__ void __launch_bounds__(NTH, NTH == 128 ? (sizeof(R) == 8 ? 5 : 8) : N
                     }
                 }
             }
-            if (!(cabs2(piv) >= pivtol * pivtol) || !(pivtol > R(0))) {   // rare, off the chain: rp is formed already
+            if (!(cabs2(piv) >= tol2) || !(tol2 > R(0))) {   // rare, off the chain: rp is formed already
                 piv = static_pivot<R>(piv, pivtol, np);
                 rp = crcp(piv);
             }
