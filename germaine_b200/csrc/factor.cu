@@ -344,6 +344,7 @@ __device__ void factor_diag_block(const FactorArgs<R> &a, cplx<R> *F, int f, int
                         if (cabs2(pr[0]) < (R)a.pivtau2 * from_lead(top, R(0))) {   // warp-uniform
                             const int arg = __ffs(__ballot_sync(ALL, key == top)) - 1;
                             if (arg > p) {   // rows p and arg trade places
+                                __syncwarp();   // the multipliers that other lanes stored (shuffles order no memory)
                                 const int from = lane == p ? arg : lane == arg ? p : lane;
 #pragma unroll
                                 for (int i = 0; i < W; ++i) {
@@ -1008,6 +1009,7 @@ __global__ void __launch_bounds__(NTH, NTH == 128 ? (sizeof(R) == 8 ? 5 : 8) : N
                 if (cabs2(piv) < (R)a.pivtau2 * from_lead(top, R(0))) {   // warp-uniform
                     const int arg = __ffs(__ballot_sync(ALL, key == top)) - 1;
                     if (arg > j) {   // rows p and p0 + arg trade places: the panel's columns here, the others in step 2
+                        __syncwarp();   // the multipliers that other lanes stored (shuffles order no memory)
                         const int from = lane == j ? arg : lane == arg ? j : lane;
 #pragma unroll
                         for (int i = 0; i < PW8; ++i)
