@@ -795,7 +795,9 @@ static const unsigned char *build_mask(gm_engine *e, int nrhs, const RhsPattern 
     if (!pat || (!pat->per_col && !pat->common) || std::getenv("GM_NO_PRUNE")) return nullptr;
     const Symbolic &sy = e->sym;
     const int nch = (nrhs + 31) / 32, nn = sy.nnodes;
-    std::vector<unsigned char> m((size_t)nn * nch, 0);
+    if (e->mask_upload) cudaStreamSynchronize(e->st);   // a solve that failed before its wait
+    std::vector<unsigned char> &m = e->h_mask;
+    m.assign((size_t)nn * nch, 0);
     std::vector<unsigned char> live((size_t)nn + 8, 0);   // by level position
     auto mark = [&](int row, int g) {
         if (row < 0 || row >= sy.n) return;
@@ -809,11 +811,13 @@ static const unsigned char *build_mask(gm_engine *e, int nrhs, const RhsPattern 
     for (int i = 0; i < pat->ncommon; ++i)
         for (int g = 0; g < nch; ++g) mark(pat->common[i], g);
     if (e->d_mask.ensure(m.size()) != cudaSuccess) return nullptr;   // fall back to the dense pass
+    e->mask_upload = true;
     if (cudaMemcpyAsync(e->d_mask.p, m.data(), m.size(), cudaMemcpyHostToDevice, e->st) != cudaSuccess) return nullptr;
     // the live (front position, 32-column slice) pairs of the small-front
     // levels, whose kernels are launched over them; the other levels read
     // the mask.  Eight positions are looked at together: few are live.
-    std::vector<int2> work;
+    std::vector<int2> &work = e->h_work;
+    work.clear();
     e->work_off.assign(e->levels.size() + 1, 0);
     for (size_t h = 0; h < e->levels.size(); ++h) {
         e->work_off[h] = (int)work.size();
@@ -1206,6 +1210,7 @@ int engine_solve_device(gm_engine *e, int sys, int nrhs, double2 *d_x, const dou
         GM_CUDA(cudaEventRecord(e->ev_r, e->st));
         GM_CUDA(cudaMemcpyAsync(norms.data(), e->d_norm.p, cntn * sizeof(double), cudaMemcpyDeviceToHost, e->st));
         GM_CUDA(cudaStreamSynchronize(e->st));
+        e->mask_upload = false;
         collect_subst_times(e);
         if (it == 0) {
             cudaEventElapsedTime(&ms, t0, t1);

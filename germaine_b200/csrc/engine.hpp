@@ -167,6 +167,11 @@ struct gm_engine {
     int tuned_nrhs = 0;
     std::vector<int> work_off;
     bool have_work = false;
+    // host copies of d_mask and d_work, kept while their uploads may be in
+    // flight (mask_upload: until the solve's first wait)
+    std::vector<unsigned char> h_mask;
+    std::vector<int2> h_work;
+    bool mask_upload = false;
     // FP64 gradient of the last gm_grad_obj, diagonal Hessian of the last
     // gm_hessian: one or two arrays of n doubles (0: none yet)
     gm::HostBuf last_grad, last_hess;

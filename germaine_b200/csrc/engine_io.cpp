@@ -100,7 +100,9 @@ int forward_solve(gm_engine *e, int ns, const Geometry &g, double2 *xout, int sr
     gm::SpikeRhs sp;      // and never form the dense right-hand sides
     sp.k = e->d_src_k.as<int>();
     sp.amp = e->d_amp.as<double2>();
-    return gm::engine_solve_device(e, GM_SYS_A, ns, xout, nullptr, &pat, &sp);
+    rc = gm::engine_solve_device(e, GM_SYS_A, ns, xout, nullptr, &pat, &sp);
+    if (rc < 0) cudaStreamSynchronize(e->st);   // the uploads above read the caller's arrays and this one's
+    return rc;
 }
 
 // cp_grad_frame's taper (coefficient and number of passes per grid point) on the device
@@ -633,7 +635,10 @@ extern "C" int gm_hessian(gm_engine *e, int mode, int nshots, const float *src_x
             sp.k = e->d_rec_k.as<int>() + r0;
             sp.amp = e->d_amp.as<double2>();
             const int src = gm::engine_solve_device(e, GM_SYS_A, nr, e->d_xa.as<double2>(), nullptr, &pat, &sp);
-            if (src < 0) return src;
+            if (src < 0) {
+                cudaStreamSynchronize(e->st);   // the upload above reads amp
+                return src;
+            }
             if (src > worst) worst = src;
             gm::launch_hess_sq(e->d_xa.as<double2>(), n, nf, nr, sqg, r0 > 0, e->st);
             GM_CUDA(cudaGetLastError());
