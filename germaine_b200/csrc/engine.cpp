@@ -444,6 +444,7 @@ static int factor_batch(gm_engine *e, double pivscale) {
     a.npert = &report->npert;
     a.nswap = &report->nswap;
     a.pivtau2 = e->cfg.pivot_tol > 0 ? e->cfg.pivot_tol * e->cfg.pivot_tol : 0.0;
+    a.pivreach = a.pivtau2 > 0 ? std::min(1e30, (1.0 - 1.0 / (1 << 20)) / a.pivtau2) : 0.0;
     a.pivsrc = e->cfg.pivot_tol > 0 ? e->d_pivsrc.as<unsigned char>() : nullptr;
     if (e->cb_plan_base != e->d_front.p || e->cb_plan_nf != e->nf) {
         const int rc = build_cb_plan<R>(e);

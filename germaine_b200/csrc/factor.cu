@@ -248,8 +248,8 @@ __device__ __forceinline__ cplx<R> static_pivot(cplx<R> piv, R pivtol, int &nper
 //      row per lane;
 //   3. all warps form the 16 products a_r b_c on 8 x 8 blocks.
 // Row exchanges: position p goes to the row of largest |D(r, p)| among those
-// left (by the leading 32 bits of |D|^2) when the row there has |D(p, p)|^2 <
-// pivtau2 |D(r, p)|^2; whole rows of the array trade places (a few per front).
+// left when the row there has |D(p, p)|^2 < pivtau2 |D(r, p)|^2; whole rows of
+// the array trade places (a few per front).
 // The block's permutation goes to pivsrc[vars[k0 + q]] (q: pivot position,
 // value: block row in equation order); columns right of the block are
 // exchanged when the U panel is staged, columns left of it (earlier blocks'
@@ -293,6 +293,29 @@ __device__ __forceinline__ void block8_sub(const float2 *Ab, int sa, const float
         cfms(acc[0], v, Bb[j * sb + 2 * kq]);
         cfms(acc[1], v, Bb[j * sb + 2 * kq + 1]);
     }
+}
+
+// The lane whose row takes the pivot's place by the threshold rule: the largest
+// m2 = |entry|^2 of the column (the lowest lane among equals) when piv2 =
+// |pivot|^2 is below pivtau2 times that, else -1; the same in every lane.
+// key: lead_bits(m2), -1 where the lane has no candidate.  The chain of the
+// pivots carries one warp reduction over the keys.  In complex128 it sees half
+// of the bits: rows can only be exchanged if the leading bits of piv2 pivreach
+// (below piv2 / pivtau2 by more than it is rounded; formed while the reduction
+// is out) do not lead its result, and behind that the remaining bits decide.
+__device__ __forceinline__ int exchange_lane(const FactorArgs<double> &a, double m2, int key, double piv2) {
+    constexpr unsigned ALL = 0xffffffffu;
+    const int top = __reduce_max_sync(ALL, key);
+    if (lead_bits(piv2 * a.pivreach) > top) return -1;
+    const unsigned lo = key == top ? (unsigned)__double2loint(m2) : 0u;
+    const unsigned l = __reduce_max_sync(ALL, lo);
+    const int arg = __ffs(__ballot_sync(ALL, key == top && lo == l)) - 1;
+    return piv2 < a.pivtau2 * __hiloint2double(top, (int)l) ? arg : -1;
+}
+__device__ __forceinline__ int exchange_lane(const FactorArgs<float> &a, float, int key, float piv2) {
+    const int top = __reduce_max_sync(0xffffffffu, key);
+    if (!(piv2 < (float)a.pivtau2 * from_lead(top, 0.f))) return -1;
+    return __ffs(__ballot_sync(0xffffffffu, key == top)) - 1;
 }
 
 template <class R, bool PIV>
@@ -340,29 +363,26 @@ __device__ void factor_diag_block(const FactorArgs<R> &a, cplx<R> *F, int f, int
                     if (PIV) {
                         const R m2 = cabs2(x[0]);
                         const int key = lane >= p && lane < kb ? lead_bits(m2) : -1;
-                        const int top = __reduce_max_sync(ALL, key);
-                        if (cabs2(pr[0]) < (R)a.pivtau2 * from_lead(top, R(0))) {   // warp-uniform
-                            const int arg = __ffs(__ballot_sync(ALL, key == top)) - 1;
-                            if (arg > p) {   // rows p and arg trade places
-                                __syncwarp();   // the multipliers that other lanes stored (shuffles order no memory)
-                                const int from = lane == p ? arg : lane == arg ? p : lane;
+                        const int arg = exchange_lane(a, m2, key, cabs2(pr[0]));
+                        if (arg > p) {   // rows p and arg trade places
+                            __syncwarp();   // the multipliers that other lanes stored (shuffles order no memory)
+                            const int from = lane == p ? arg : lane == arg ? p : lane;
 #pragma unroll
-                                for (int i = 0; i < W; ++i) {
-                                    pr[i] = mk(__shfl_sync(ALL, x[i].x, arg), __shfl_sync(ALL, x[i].y, arg));
-                                    x[i] = mk(__shfl_sync(ALL, x[i].x, from), __shfl_sync(ALL, x[i].y, from));
-                                }
-                                const C u = T[p * DSTR + lane], v = T[arg * DSTR + lane];
-                                T[p * DSTR + lane] = v;
-                                T[arg * DSTR + lane] = u;
-                                if (lane == 0) {
-                                    const int t = rowat[p];
-                                    rowat[p] = rowat[arg];
-                                    rowat[arg] = t;
-                                }
-                                __syncwarp();
-                                rp = crcp(pr[0]);
-                                ++nsw;
+                            for (int i = 0; i < W; ++i) {
+                                pr[i] = mk(__shfl_sync(ALL, x[i].x, arg), __shfl_sync(ALL, x[i].y, arg));
+                                x[i] = mk(__shfl_sync(ALL, x[i].x, from), __shfl_sync(ALL, x[i].y, from));
                             }
+                            const C u = T[p * DSTR + lane], v = T[arg * DSTR + lane];
+                            T[p * DSTR + lane] = v;
+                            T[arg * DSTR + lane] = u;
+                            if (lane == 0) {
+                                const int t = rowat[p];
+                                rowat[p] = rowat[arg];
+                                rowat[arg] = t;
+                            }
+                            __syncwarp();
+                            rp = crcp(pr[0]);
+                            ++nsw;
                         }
                     }
                     C piv = pr[0];
@@ -1004,33 +1024,31 @@ __global__ void __launch_bounds__(NTH, NTH == 128 ? (sizeof(R) == 8 ? 5 : 8) : N
             C piv = mk(__shfl_sync(ALL, x[0].x, j), __shfl_sync(ALL, x[0].y, j));
             C rp = crcp(piv);
             if (PIV) {
-                const int key = lane >= j && p0 + lane < s ? lead_bits(cabs2(x[0])) : -1;
-                const int top = __reduce_max_sync(ALL, key);
-                if (cabs2(piv) < (R)a.pivtau2 * from_lead(top, R(0))) {   // warp-uniform
-                    const int arg = __ffs(__ballot_sync(ALL, key == top)) - 1;
-                    if (arg > j) {   // rows p and p0 + arg trade places: the panel's columns here, the others in step 2
-                        __syncwarp();   // the multipliers that other lanes stored (shuffles order no memory)
-                        const int from = lane == j ? arg : lane == arg ? j : lane;
+                const R m2 = cabs2(x[0]);
+                const int key = lane >= j && p0 + lane < s ? lead_bits(m2) : -1;
+                const int arg = exchange_lane(a, m2, key, cabs2(piv));
+                if (arg > j) {   // rows p and p0 + arg trade places: the panel's columns here, the others in step 2
+                    __syncwarp();   // the multipliers that other lanes stored (shuffles order no memory)
+                    const int from = lane == j ? arg : lane == arg ? j : lane;
 #pragma unroll
-                        for (int i = 0; i < PW8; ++i)
-                            x[i] = mk(__shfl_sync(ALL, x[i].x, from), __shfl_sync(ALL, x[i].y, from));
-                        piv = mk(__shfl_sync(ALL, x[0].x, j), __shfl_sync(ALL, x[0].y, j));
-                        if (lane < j) {   // the multipliers stored so far
-                            C *c = S + (p0 + lane) * ld;
-                            const C t = c[p];
-                            c[p] = c[p0 + arg];
-                            c[p0 + arg] = t;
-                        }
-                        if (lane == 0) {
-                            const int t = rowat[p];
-                            rowat[p] = rowat[p0 + arg];
-                            rowat[p0 + arg] = t;
-                            swaps[1 + nx] = p | (p0 + arg) << 16;
-                        }
-                        __syncwarp();
-                        ++nx;
-                        rp = crcp(piv);
+                    for (int i = 0; i < PW8; ++i)
+                        x[i] = mk(__shfl_sync(ALL, x[i].x, from), __shfl_sync(ALL, x[i].y, from));
+                    piv = mk(__shfl_sync(ALL, x[0].x, j), __shfl_sync(ALL, x[0].y, j));
+                    if (lane < j) {   // the multipliers stored so far
+                        C *c = S + (p0 + lane) * ld;
+                        const C t = c[p];
+                        c[p] = c[p0 + arg];
+                        c[p0 + arg] = t;
                     }
+                    if (lane == 0) {
+                        const int t = rowat[p];
+                        rowat[p] = rowat[p0 + arg];
+                        rowat[p0 + arg] = t;
+                        swaps[1 + nx] = p | (p0 + arg) << 16;
+                    }
+                    __syncwarp();
+                    ++nx;
+                    rp = crcp(piv);
                 }
             }
             if (!(cabs2(piv) >= tol2) || !(tol2 > R(0))) {   // rare, off the chain: rp is formed already

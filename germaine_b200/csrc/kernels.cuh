@@ -112,7 +112,7 @@ struct FactorArgs {
     // levels (fronts with more than NB pivots): pivtau2 = tolerance^2 (0 =
     // off); pivsrc[matrix * n + vars[k]] = the row of pivot k's block (0 ..
     // 31, equation order) that pivot position k took; nswap counts exchanges
-    double pivtau2;
+    double pivtau2, pivreach;   // pivreach: (1 - 2^-20) / pivtau2, at most 1e30 (exchanges ruled out by leading bits)
     unsigned char *pivsrc;
     unsigned long long *nswap;
 };
