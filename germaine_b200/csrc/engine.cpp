@@ -335,29 +335,28 @@ static int assemble_batch(gm_engine *e) {
     return GM_OK;
 }
 
-// Builds the per-level list of contribution-block products
-// C[s:f, s:f] -= L21 * U12 (K = npiv) over every front and frequency, and
-// their output tiles: tcgen05 tiles (128 x 64) for the complex64 path on
-// levels whose blocks are large enough to fill them, CUDA-core tiles
-// (64 x 64) otherwise.
-// Levels of fronts with at most 16 pivots that are too large for the
-// whole-front kernel go to the fused mid-level kernel; GM_NO_FACTOR_MID=1 keeps them on
-// the blocked diagonal / panel / contribution-GEMM sequence.  With 17-32
-// pivots the fused kernel holds 32-entry pivot rows in registers and fits
-// one CTA per SM; measured at 841 x 227 (10 frequencies) the blocked
-// sequence is faster there (levels 5-6, 26-28 pivots: 1.64 -> 1.26 and
-// 1.22 -> 1.10 ms) and slower with 14 pivots (level 4: 1.05 vs 1.39 ms).
-// GM_MID_MAX_PIV=<n> moves the limit (32: every level the kernel takes).
+// GM_MID_MAX_PIV=<n> (n <= 32) gives the levels of at most n pivots per front
+// that are too large for the whole-front kernel to the fused mid-level kernel
+// instead of the blocked diagonal / panel / contribution sequence.  By default
+// none: it holds 32-entry pivot rows in registers and fits one CTA per SM, and
+// with 26-28 pivots the blocked sequence is faster (841 x 227, 10 frequencies,
+// levels 5-6: 1.64 -> 1.26 and 1.22 -> 1.10 ms when it was chosen); every level
+// of at most 16 pivots fits the whole-front kernel (grids of 6 x 40 to 900 x
+// 220, leaves of 8 to 100 points, both precisions).
 template <class R>
 static bool use_mid_factor(const LevelInfo &L) {
-    static const bool off = std::getenv("GM_NO_FACTOR_MID") != nullptr;
     static const int max_piv = [] {
         const char *v = std::getenv("GM_MID_MAX_PIV");
-        return v ? std::atoi(v) : 16;
+        return v ? std::atoi(v) : 0;
     }();
-    return !off && L.max_piv <= max_piv && mid_factor_level<R>(L);
+    return L.max_piv > 0 && L.max_piv <= max_piv && mid_factor_level<R>(L);
 }
 
+// Builds the per-level list of contribution-block updates
+// C[s:f, s:f] -= L21 * U12 (K = npiv) over every front and frequency, as
+// output tiles: tcgen05 tiles (128 x 64) for the complex64 path on levels
+// whose blocks are large enough to fill them, else 64 x 64 tiles, or 32 x 32
+// ones where those do not fill the chip.
 template <class R>
 static int build_cb_plan(gm_engine *e) {
     using C = cplx_any<R>;

@@ -27,13 +27,14 @@
 // multipliers of earlier blocks in equation order, and the block's
 // permutation is in FactorArgs::pivsrc.
 //
-// Two fused kernels leave the same layout on the levels where they pay:
+// Two fused kernels leave the same layout:
 //   k_factor_front  fronts that fit shared memory whole (the lower levels):
 //                   extend-add, entries, LU and Schur complement in one CTA;
-//   k_factor_mid    fronts with at most NB pivots and at most 256 rows above
-//                   those: after K2, one CTA factorises the pivot columns
-//                   and applies the Schur update to the contribution block
-//                   once, in place of K3 / K4 and the contribution GEMM.
+//   k_factor_mid    on request (GM_MID_MAX_PIV): fronts with at most NB pivots
+//                   and at most 256 rows above those: after K2, one CTA
+//                   factorises the pivot columns and applies the Schur update
+//                   to the contribution block once, in place of K3 / K4 and the
+//                   contribution GEMM.
 // The remaining (upper) levels take the blocked K2-K4 sequence.
 #include <algorithm>
 #include <cstdlib>
@@ -1329,7 +1330,8 @@ namespace gm {
 
 // ---------------------------------------------------------------------
 // Mid-level fronts: at most NB pivots and at most MID_FT rows, but too
-// large for the whole-front kernel.  After the extend-add
+// large for the whole-front kernel.  Taken on request only (GM_MID_MAX_PIV,
+// engine.cpp).  After the extend-add
 // gather and the operator entries (K2), one CTA per front and frequency
 //   1. factorises the pivot columns (f x s) right-looking with each thread
 //      holding one front row in registers: per pivot, warp 0 picks the
@@ -1383,9 +1385,10 @@ __device__ __forceinline__ void mid_select_pivot(R c2, int &pos, int kp, int s, 
     }
 }
 
-template <class R, int NPR>
+template <class R>
 __global__ void __launch_bounds__(MID_FT) k_factor_mid(FactorArgs<R> a, int lvl_first) {
     using C = cplx<R>;
+    constexpr int NPR = NB;   // entries of a pivot row in registers
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ C Dinv[NB][NB + 1];
     __shared__ C urow[2][NPR];   // pivot row k at columns k .. s-1, alternating buffers
@@ -1523,7 +1526,7 @@ __global__ void __launch_bounds__(MID_FT) k_factor_mid(FactorArgs<R> a, int lvl_
     // values loaded into the accumulators first
     for (int i0 = 0; i0 < m; i0 += 64)
         for (int j0 = 0; j0 < m; j0 += 64) {
-            TileCC<C, (sizeof(R) == 8 && NPR > 16), 64> acc;   // short K (<= 16 pivots): CUDA-core FMAs
+            TileCC<C, sizeof(R) == 8, 64> acc;
             for_tile(acc, tid, [&](int rr, int cc, C &v) {
                 const int i = i0 + rr, j = j0 + cc;
                 v = (i < m && j < m) ? F[s + i + (size_t)(s + j) * f] : czero<C>();
@@ -1545,14 +1548,14 @@ bool mid_factor_level(const LevelInfo &L) {
            (size_t)L.mid_words * sizeof(cplx<R>) <= MID_FACTOR_SMEM;
 }
 
-template <class R, int NPR>
+template <class R>
 static void launch_mid(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_t st) {
     static bool attr_set = false;
     if (!attr_set) {
-        cudaFuncSetAttribute(k_factor_mid<R, NPR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MID_FACTOR_SMEM);
+        cudaFuncSetAttribute(k_factor_mid<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MID_FACTOR_SMEM);
         attr_set = true;
     }
-    (k_factor_mid<R, NPR><<<dim3(L.count, a.nf), MID_FT, (size_t)L.mid_words * sizeof(cplx<R>), st>>>(a, L.first),
+    (k_factor_mid<R><<<dim3(L.count, a.nf), MID_FT, (size_t)L.mid_words * sizeof(cplx<R>), st>>>(a, L.first),
      note_launch());
 }
 
@@ -1563,10 +1566,7 @@ void launch_factor_mid(const FactorArgs<R> &a, const LevelInfo &L, cudaStream_t 
                              st>>>(a, first, 0),
          note_launch());
     });
-    if (L.max_piv <= 16)
-        launch_mid<R, 16>(a, L, st);
-    else
-        launch_mid<R, NB>(a, L, st);
+    launch_mid<R>(a, L, st);
 }
 
 template bool mid_factor_level<double>(const LevelInfo &);
