@@ -135,7 +135,6 @@ extern "C" int gm_engine_create(int device, const gm_config *cfg, gm_engine **ou
             L.mid_words = std::max(L.mid_words, (int64_t)(fv + 1) * sv + (int64_t)(sv | 1) * (fv - sv));
             L.front_words = std::max(L.front_words, gm::front_words_of(fv, sv));
         }
-        L.ent_first = ne;
         for (int t = L.first; t < L.first + L.count; ++t) {
             const int v = s.lvl_nodes[t];
             ent_lvl_off[t] = ne;
@@ -150,7 +149,6 @@ extern "C" int gm_engine_create(int device, const gm_config *cfg, gm_engine **ou
                 ent_src[ne] = id;
             }
         }
-        L.ent_count = ne - L.ent_first;
     }
     ent_lvl_off[s.nnodes] = ne;
     // levels with more than 32 pivots: rows of the pivot workspace, and each
@@ -739,8 +737,6 @@ static void substitute(gm_engine *e, void *xT, void *y, int nrhs, int trans, con
     }
     a.nrhs = nrhs;
     a.ldr = nrhs;
-    const int nchunk = (nrhs + 31) / 32;
-    a.rch = (nrhs + nchunk - 1) / nchunk;
     a.trans = trans;
     a.mask = mask;
     a.mask_nch = (nrhs + 31) / 32;
@@ -1335,8 +1331,6 @@ static void time_levels(gm_engine *e, void *xT, int nrhs, std::vector<float> &fw
     a.nf = e->nf;
     a.nrhs = nrhs;
     a.ldr = nrhs;
-    const int nchunk = (nrhs + 31) / 32;
-    a.rch = (nrhs + nchunk - 1) / nchunk;
     a.lvl_cfg = e->lvl_cfg.data();
     std::vector<cudaEvent_t> ev(2 * nl + 1);
     for (auto &x : ev) cudaEventCreate(&x);

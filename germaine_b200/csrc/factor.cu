@@ -42,6 +42,7 @@
 #include "kernels.cuh"
 #include "cplx.cuh"
 #include "async_copy.cuh"
+#include "mma_f64.cuh"
 
 namespace gm {
 
@@ -116,20 +117,6 @@ __device__ __forceinline__ void mma_tile(const C *As, int ak, int ar, const C *B
                 else cfma(acc.v[i][j], lv[i], uv[j]);
             }
     }
-}
-
-__device__ __forceinline__ void dmma_884(double a, double b, double &d0, double &d1) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
-}
-
-// one complex 8 x 8 x 4 block
-__device__ __forceinline__ void cmma_884(const double2 &a, const double2 &b, double2 &d0, double2 &d1) {
-    dmma_884(a.x, b.x, d0.x, d1.x);    // Re += Ar Br
-    dmma_884(-a.y, b.y, d0.x, d1.x);   //     - Ai Bi
-    dmma_884(a.x, b.y, d0.y, d1.y);    // Im += Ar Bi
-    dmma_884(a.y, b.x, d0.y, d1.y);    //     + Ai Br
 }
 
 template <bool NEG, int TL>

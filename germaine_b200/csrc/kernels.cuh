@@ -77,7 +77,6 @@ struct LevelInfo {
     int first;      // offset into lvl_nodes
     int count;      // nodes in the level
     int max_front, max_piv, max_ring;
-    int64_t ent_first, ent_count;  // level's entry range in ent_dst/ent_src
     int64_t mid_words;  // largest (f + 1) s + (s | 1)(f - s) of the level's fronts: k_factor_mid's tile
     int index;          // the level's height
     int64_t front_words;               // largest shared-memory need of the whole-front kernel (elements)
@@ -181,7 +180,6 @@ struct SolveArgs {
     void *w;                  // cplx<R> [nf][rhs_total][ldr] update vectors (ring rows)
     void *y;                  // cplx<R> [nf][y_total][ldr] pivot rows of the levels with more than 32 pivots
     int nf, nrhs, ldr;
-    int rch;                  // right-hand sides per CTA (<= 32)
     int trans;                // 0: M x = b, 1: M^T x = b
     // forward-pass pruning (NULL: every front carries data): mask[v * mask_nch + g]
     // is 0 when right-hand sides 32 g .. 32 g + 31 are zero on every pivot row of

@@ -84,8 +84,6 @@ void substitute_into(gm_engine *e, void *xT, void *w, void *y, int nrhs, int tra
     a.nf = e->nf;
     a.nrhs = nrhs;
     a.ldr = nrhs;
-    const int nchunk = (nrhs + 31) / 32;
-    a.rch = (nrhs + nchunk - 1) / nchunk;
     a.trans = trans;
     for (int h = 0; h < (int)e->levels.size(); ++h) gm::launch_solve_forward_level<R>(a, e->levels[h], e->st);
     for (int h = (int)e->levels.size() - 1; h >= 0; --h) gm::launch_solve_backward_level<R>(a, e->levels[h], e->st);

@@ -213,7 +213,7 @@ __device__ __forceinline__ void pipe_product(PipeStage<cplx<R>, RT, B> *st, cons
         __syncthreads();               // and every warp is past chunk j - 1
         stage(j + PST - 1);
         const PipeStage<C, RT, B> &sm = st[j % PST];
-        tile_mma_p<0, RT, B>(sm.L, sm.Y, min(PKC, k1 - k0 - j * PKC), acc, rows, rn, threadIdx.x);
+        tile_mma_p<RT, B>(sm.L, sm.Y, min(PKC, k1 - k0 - j * PKC), acc, rows, rn, threadIdx.x);
     }
 }
 

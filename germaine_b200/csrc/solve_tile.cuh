@@ -6,6 +6,7 @@
 #include "kernels.cuh"
 #include "cplx.cuh"
 #include "async_copy.cuh"
+#include "mma_f64.cuh"
 
 namespace gm {
 
@@ -30,23 +31,18 @@ struct SolveSmem {
     C Y[SNB][8 * B + SPAD];    // right operand, [pivot q][rhs]
 };
 
-// factor element M'(i, c) of the forward (L') or backward (U') factor:
-// F[i + c f] for M x = b, F[c + i f] for M^T x = b
-template <class C, bool TRANS>
-__device__ __forceinline__ C elem(const C *F, int f, int i, int c) {
-    return TRANS ? F[c + (size_t)i * f] : F[i + (size_t)c * f];
-}
-
+// Below, M'(i, c) is the element of the forward (L') or backward (U') factor:
+// F[i + c f] for M x = b, F[c + i f] for M^T x = b.
+//
 // The staging helpers below issue asynchronous copies (every load of the
 // tile in flight at once, no register round trip); the tile is complete
 // after staged_sync().
 //
-// sm.L[q][row] = M'(i0 + row, c0 + q) for row < rows, q < qb.  Entries
-// outside are left as they are: tile_mma reads only q < qb, and rows >= rows
+// L[q][row] = M'(i0 + row, c0 + q) for row < rows, q < qb.  Entries
+// outside are left as they are: the products read only q < qb, and rows >= rows
 // (or right-hand sides >= rn) only feed accumulators that are never stored,
 // so partial tiles stage only what they use.
-// (the _p forms take the tile by pointer and the participating threads as
-// lt = 0 .. nt - 1; the SolveSmem forms are the CTA-wide ones)
+// (lt = 0 .. nt - 1: the participating threads)
 template <class C, bool TRANS, int RT, int KQ = SNB>
 __device__ __forceinline__ void stage_factor_p(C (*L)[RT + SPAD], const C *F, int f, int i0, int rows, int c0, int qb,
                                                int lt, int nt) {
@@ -61,10 +57,6 @@ __device__ __forceinline__ void stage_factor_p(C (*L)[RT + SPAD], const C *F, in
             if (q < qb) cp_async_elem(&L[q][row], F + (c0 + q) + (size_t)(i0 + row) * f);
         }
     }
-}
-template <class C, bool TRANS, int RT, int B>
-__device__ __forceinline__ void stage_factor(SolveSmem<C, RT, B> &sm, const C *F, int f, int i0, int rows, int c0, int qb) {
-    stage_factor_p<C, TRANS, RT>(sm.L, F, f, i0, rows, c0, qb, threadIdx.x, NT);
 }
 
 // L[q][p] = entry (p, q0 + q) of the inverse diagonal-block operator of
@@ -146,17 +138,13 @@ __device__ __forceinline__ void for_acc(TileAcc<C, RT, B> &acc, int rows, int rn
 // Y[q][col] the right operand.  Rows >= `rows` and columns >= rn of the
 // tile only feed accumulators that are never stored; row and column groups
 // that lie entirely outside are skipped warp-uniformly, so small fronts and
-// short slices do not pay for the full tile.  TRI: 0 a full operator;
-// TRI_LOWER / TRI_UPPER a triangular one (the diagonal-block inverses),
-// whose column q has no entries above / below row q: row groups that column
-// q does not reach are skipped for that q.
-constexpr int TRI_LOWER = 1, TRI_UPPER = 2;
-
+// short slices do not pay for the full tile.
+//
 // complex64: each thread accumulates its 16-row-strided rows x 8-column-
 // strided columns with CUDA-core FMAs, one pivot q at a time
-template <int TRI, int RT, int B>
+template <int RT, int B>
 __device__ __forceinline__ void tile_mma_p(const float2 (*L)[RT + SPAD], const float2 (*Y)[8 * B + SPAD], int qb,
-                                           TileAcc<float2, RT, B> &acc, int rows, int rn, int lt, int q0 = 0) {
+                                           TileAcc<float2, RT, B> &acc, int rows, int rn, int lt) {
     constexpr int A = RT / 16;
     const int tr = lt / 8, tc = lt % 8;
     const int wrow = (lt >> 5) * 4;   // a warp owns rows 4w .. 4w + 3 of each 16-row group
@@ -165,17 +153,14 @@ __device__ __forceinline__ void tile_mma_p(const float2 (*L)[RT + SPAD], const f
     if (na == 0) return;   // warp-uniform: this warp owns no row of the tile
 #pragma unroll 2
     for (int q = 0; q < qb; ++q) {
-        const int alo = TRI == TRI_LOWER ? (q0 + q) / 16 : 0;       // rows >= q only
-        const int ahi = TRI == TRI_UPPER ? (q0 + q) / 16 : A - 1;   // rows <= q only
         float2 l[A], y[B];
 #pragma unroll
-        for (int a = 0; a < A; ++a) l[a] = a < na && a >= alo && a <= ahi ? L[q][tr + 16 * a] : czero<float2>();
+        for (int a = 0; a < A; ++a) l[a] = a < na ? L[q][tr + 16 * a] : czero<float2>();
 #pragma unroll
         for (int b = 0; b < B; ++b) y[b] = b < nb ? Y[q][tc + 8 * b] : czero<float2>();
 #pragma unroll
         for (int a = 0; a < A; ++a) {
             if (a >= na) break;
-            if (a < alo || a > ahi) continue;
 #pragma unroll
             for (int b = 0; b < B; ++b)
                 if (b < nb) cfma(acc.v[a][b], l[a], y[b]);
@@ -183,22 +168,13 @@ __device__ __forceinline__ void tile_mma_p(const float2 (*L)[RT + SPAD], const f
     }
 }
 
-// d = a b + d on one 8 x 8 x 4 FP64 block (warp-wide; a: this lane's entry
-// of the 8 x 4 row-major left block, b: of the 4 x 8 column-major right
-// block, d: this lane's two entries of the 8 x 8 result)
-__device__ __forceinline__ void dmma_884(double a, double b, double &d0, double &d1) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
-}
-
 // complex128: per 4 pivots and per 8 x 8 block, four FP64 matrix
 // instructions (Re += Ar Br - Ai Bi, Im += Ar Bi + Ai Br); a lane loads one
 // complex entry of each left and right fragment.  Pivots q >= qb enter as
 // zeros.
-template <int TRI, int RT, int B>
+template <int RT, int B>
 __device__ __forceinline__ void tile_mma_p(const double2 (*L)[RT + SPAD], const double2 (*Y)[8 * B + SPAD], int qb,
-                                           TileAcc<double2, RT, B> &acc, int rows, int rn, int lt, int q0 = 0) {
+                                           TileAcc<double2, RT, B> &acc, int rows, int rn, int lt) {
     constexpr int NRB = RT / 32;
     const int w = lt >> 5, lane = lt & 31;
     const int nb = min(B, (rn + 7) / 8);
@@ -212,26 +188,14 @@ __device__ __forceinline__ void tile_mma_p(const double2 (*L)[RT + SPAD], const 
         for (int i = 0; i < NRB; ++i) {
             const int rb = w + 4 * i;   // row block: rows 8 rb .. 8 rb + 7
             if (8 * rb >= rows) break;   // warp-uniform
-            if (TRI == TRI_UPPER && 8 * rb > q0 + k0 + 3) continue;   // rows <= q only
-            if (TRI == TRI_LOWER && 8 * rb + 7 < q0 + k0) continue;   // rows >= q only
             const double2 af = kin ? L[kk][8 * rb + (lane >> 2)] : czero<double2>();
 #pragma unroll
             for (int b = 0; b < B; ++b) {
                 if (b >= nb) break;
-                double2 &d0 = acc.v[i][2 * b], &d1 = acc.v[i][2 * b + 1];
-                dmma_884(af.x, bf[b].x, d0.x, d1.x);
-                dmma_884(-af.y, bf[b].y, d0.x, d1.x);
-                dmma_884(af.x, bf[b].y, d0.y, d1.y);
-                dmma_884(af.y, bf[b].x, d0.y, d1.y);
+                cmma_884(af, bf[b], acc.v[i][2 * b], acc.v[i][2 * b + 1]);
             }
         }
     }
-}
-
-template <int TRI = 0, class C, int RT, int B>
-__device__ __forceinline__ void tile_mma(const SolveSmem<C, RT, B> &sm, int qb, TileAcc<C, RT, B> &acc, int rows,
-                                         int rn) {
-    tile_mma_p<TRI, RT, B>(sm.L, sm.Y, qb, acc, rows, rn, threadIdx.x);
 }
 
 // 32 x 32 output tile of the small-front kernels in 8 x 8 blocks, dealt to
@@ -272,15 +236,11 @@ struct BlockTile {
     }
 };
 
-// one 8 x 8 block += its operands' fragments at pivots k0 .. k0 + 3 (complex128)
-__device__ __forceinline__ void block_mac(double2 *d, const double2 &a, const double2 &b) {
-    dmma_884(a.x, b.x, d[0].x, d[1].x);
-    dmma_884(-a.y, b.y, d[0].x, d[1].x);
-    dmma_884(a.x, b.y, d[0].y, d[1].y);
-    dmma_884(a.y, b.x, d[0].y, d[1].y);
-}
-
-// acc += L'[rows x qb] Y[qb x rn], operands and TRI as tile_mma_p
+// acc += L'[rows x qb] Y[qb x rn], operands as tile_mma_p.  TRI: 0 a full
+// operator; TRI_LOWER / TRI_UPPER a triangular one (the diagonal-block
+// inverses), whose column q has no entries above / below row q: row blocks that
+// column q does not reach are skipped for that q.
+constexpr int TRI_LOWER = 1, TRI_UPPER = 2;
 template <int TRI, int LW, int N>
 __device__ __forceinline__ void block_mma(const double2 (*L)[LW], const double2 (*Y)[32 + SPAD], int qb,
                                           BlockTile<double2, N> &acc, int rows, int rn) {
@@ -296,7 +256,7 @@ __device__ __forceinline__ void block_mma(const double2 (*L)[LW], const double2 
             for (int i = 0; i < N; ++i) {
                 if (i >= n || (TRI == TRI_UPPER && 8 * i > k0 + 3)) break;
                 if (TRI == TRI_LOWER && 8 * i + 7 < k0) continue;
-                block_mac(acc.v[i], kin ? L[kk][8 * i + g] : czero<double2>(), b);
+                cmma_884(kin ? L[kk][8 * i + g] : czero<double2>(), b, acc.v[i][0], acc.v[i][1]);
             }
         } else {
             if ((TRI == TRI_UPPER && 8 * w > k0 + 3) || (TRI == TRI_LOWER && 8 * w + 7 < k0)) continue;
@@ -304,7 +264,7 @@ __device__ __forceinline__ void block_mma(const double2 (*L)[LW], const double2 
 #pragma unroll
             for (int i = 0; i < N; ++i) {
                 if (i >= n) break;
-                block_mac(acc.v[i], a, kin ? Y[kk][8 * i + g] : czero<double2>());
+                cmma_884(a, kin ? Y[kk][8 * i + g] : czero<double2>(), acc.v[i][0], acc.v[i][1]);
             }
         }
     }

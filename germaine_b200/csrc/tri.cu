@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(NT) k_tri_inverse(FactorArgs<R> a, int lvl_fir
             async_wait_group<0>();
         }
         __syncthreads();
-        tile_mma_p<0, SNB, TRB>(st[buf].L, st[buf].Y, min(SNB, q_hi - q0), acc, rows, cols, threadIdx.x);
+        tile_mma_p<SNB, TRB>(st[buf].L, st[buf].Y, min(SNB, q_hi - q0), acc, rows, cols, threadIdx.x);
         __syncthreads();
     }
     C *out = PHASE == 0 ? T : const_cast<C *>(F);
