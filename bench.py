@@ -49,9 +49,9 @@ DH, NPML, ROW = 25.0, 20, 2
 RESIDUAL_TARGET = 1e-10
 METRIC = "shot-solves/s (factor+solve) mixed vs FP64 on B200 at resid<=1e-10; %roofline"
 # DRAM bytes of one complex128 backward substitution pass on 4 frequencies
-# (the k_bwd_small / k_bwd_ring / k_bwd_tri launches of the FP64 engine's
-# timed step, ncu dram__bytes_read.sum + dram__bytes_write.sum, summed)
-BWD_TRAFFIC_FP64_4FREQ = 3.585e9
+# (the 22 k_bwd_small / k_bwd_ring / k_bwd_tri launches of one forward call,
+# ncu dram__bytes_read.sum + dram__bytes_write.sum, summed; profiles/)
+BWD_TRAFFIC_FP64_4FREQ = 3.859e9
 PEAK_KIND = "measured FP64 rate, the higher of CUDA-core DFMA (gm_peak_fp64) and FP64 MMA (gm_peak_fp64_mma)"
 
 # the benchmark workload; --nx0/--ny0/--nfreq/--nshots shrink it for

@@ -1,12 +1,13 @@
 // gm_engine: the C-ABI of the per-frequency engine (include/germaine_gpu.h).
 //
 // Memory plan (HBM, per engine):
-//   symbolic structure        ~ 40 B per grid point (uploaded once)
+//   symbolic structure        ~ 180 B per grid point (uploaded once)
 //   A      [nf][9][n] c128    assembled stencils of the frequency batch
 //   fronts [nf][sum f^2]      c128 (GM_PREC_FP64) or c64 (GM_PREC_C64_IR)
-//   x, b, r[nf][n][nrhs] c128 solution, right-hand side, residual
-//   t      [nf][n][nrhs]      working precision copy for the substitution
-//   w      [nf][sum f][nrhs]  front-vector workspace of the substitution
+//   x, b   [nf][n][nrhs] c128 solution, dense right-hand sides
+//   t      [nf][n][nrhs]      residual / correction in working precision
+//   y      [nf][pivots of the levels above 32][nrhs]  pivot workspace
+//   w      [nf][sum of ring rows][nrhs]  update vectors of the substitution
 // At 841 x 227 (n = 190,907) with 10 frequencies x 100 shots this is about
 // 8 GB of fronts in FP64 plus 12 GB of vectors -- resident in one B200.
 #include "engine.hpp"
@@ -339,8 +340,8 @@ static int assemble_batch(gm_engine *e) {
 // none: it holds 32-entry pivot rows in registers and fits one CTA per SM, and
 // with 26-28 pivots the blocked sequence is faster (841 x 227, 10 frequencies,
 // levels 5-6: 1.64 -> 1.26 and 1.22 -> 1.10 ms when it was chosen); every level
-// of at most 16 pivots fits the whole-front kernel (grids of 6 x 40 to 900 x
-// 220, leaves of 8 to 100 points, both precisions).
+// of at most 16 pivots fits the whole-front kernel (checked over grids of up to
+// 1600 points by 220, leaves of 8 to 100 points, both precisions).
 template <class R>
 static bool use_mid_factor(const LevelInfo &L) {
     static const int max_piv = [] {

@@ -76,8 +76,9 @@ int upload(gm::DevBuf &buf, const std::vector<T> &v, cudaStream_t st) {
     return GM_OK;
 }
 
-// spike right-hand sides of every shot and frequency into e->d_b, forward solve into xout;
-// the spike amplitude is that of src_physics's source routine (RHS_source_AC / _TE)
+// forward solve of every shot and frequency into xout; the right-hand sides are spikes
+// (RHS_source_AC, src/AC/RHS_source_AC.c:32-53, and RHS_source_TE) that the substitution
+// takes from their rows and amplitudes, the amplitude that of src_physics's source routine
 int forward_solve(gm_engine *e, int ns, const Geometry &g, double2 *xout, int src_physics = 0) {
     const int nf = e->nf;
     if (!src_physics) src_physics = e->cfg.physics;

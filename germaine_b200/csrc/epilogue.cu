@@ -1,7 +1,6 @@
 // K7: per-shot work around the block solves, fused over all shots and
 // frequencies (replaces the per-shot host loops of forward_shot_AC and
 // grad_obj_AC):
-//   spike sources        RHS_source_AC / RHS_source_TE (src/AC/RHS_source_AC.c:32-53)
 //   receiver gather      vec2mat + calc_seis_AC (src/vec2mat.c:19-26, src/AC/calc_seis_AC.c:18-22)
 //   wavefield export     vec2mat layout, [nf][nshots][N] complex64 (tiled transpose)
 //   residual + misfit    calc_res_AC (src/AC/calc_res_AC.c:10-95)

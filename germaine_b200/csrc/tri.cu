@@ -15,10 +15,12 @@
 // level is eliminated, so these launches run on their own stream beside the
 // levels above: the work is s^3 / 3 complex multiply-adds per triangle pair,
 // small against the fronts' Schur updates, and the upper levels leave most of
-// the chip idle.  Accuracy (multifrontal replay in double precision, worst
-// relative residual of shots over the 2-11 Hz, 5-25 Hz SH and 100-400 MHz
-// georadar operators): within a factor of two of the block substitution
-// either way, 1.5e-11 against 1.3e-11 at worst.
+// the chip idle.  Accuracy, against inverses of the 32 x 32 blocks only: direct
+// residuals within a factor of two either way over the 2-11 Hz, 5-25 Hz SH and
+// 100-400 MHz georadar operators (multifrontal replay in double precision); on
+// the device 841 x 227, 9 / 10 / 11 Hz 1.3e-12 -> 1.5e-12, 1.2e-11 -> 1.7e-11
+// (the worst), 4.3e-13 -> 3.6e-13.  The fields are no further from a 64-bit
+// solution.
 #include "solve_tile.cuh"
 
 namespace gm {
