@@ -203,12 +203,14 @@ int residuals(gm_engine *e, int ns, int ntr, const float *pobs, int stf_inv, int
 namespace {
 
 // Device bytes per shot of one block solve over the batch: the FP64
-// solutions, the working-precision copy, the front update vectors, the
-// complex64 path's pivot workspace and the residual partial sums.
+// solutions, the working-precision copy, the front update vectors, the pivot
+// workspace (of the refinement sweeps and the complex64 path) and the residual
+// partial sums.
+size_t pivot_bytes_per_shot(const gm_engine *e) { return (size_t)e->nf * e->dsym.y_total * e->csize(); }
 size_t bytes_per_shot(const gm_engine *e) {
     const size_t n = (size_t)e->n, nf = (size_t)e->nf;
-    const size_t y = e->cfg.precision == GM_PREC_FP64 ? 0 : (size_t)e->dsym.y_total;
-    return nf * (n * sizeof(double2) + n * e->csize() + ((size_t)e->sym.rhs_total + y) * e->csize() +
+    return pivot_bytes_per_shot(e) +
+           nf * (n * sizeof(double2) + n * e->csize() + (size_t)e->sym.rhs_total * e->csize() +
                  (size_t)gm::residual_blocks(e->cfg.nx, e->cfg.ny) * 2 * sizeof(double) + 2 * sizeof(double));
 }
 
@@ -217,10 +219,12 @@ size_t bytes_per_shot(const gm_engine *e) {
 // workspaces already hold, less a reserve of 5 % of the device and 1 GB),
 // or the caller's cap (gm_set_shot_block).
 int shot_block(const gm_engine *e, int nshots) {
-    const size_t held = e->d_xf.bytes + e->d_t.bytes + e->d_w.bytes + e->d_part.bytes + e->d_norm.bytes +
-                        (e->cfg.precision == GM_PREC_FP64 ? 0 : e->d_y.bytes);
+    const size_t held = e->d_xf.bytes + e->d_t.bytes + e->d_w.bytes + e->d_part.bytes + e->d_norm.bytes + e->d_y.bytes;
     const size_t per = std::max<size_t>(1, bytes_per_shot(e));
-    if (e->shot_block <= 0 && per * (size_t)nshots <= held) return nshots;   // workspaces in place already
+    // workspaces in place already (in FP64 the pivot workspace comes with the first sweep, if any)
+    const bool fp64 = e->cfg.precision == GM_PREC_FP64;
+    const size_t need = per - (fp64 ? pivot_bytes_per_shot(e) : 0), have = held - (fp64 ? e->d_y.bytes : 0);
+    if (e->shot_block <= 0 && need * (size_t)nshots <= have) return nshots;
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return nshots;
     const size_t reserve = tot / 20 + ((size_t)1 << 30);
